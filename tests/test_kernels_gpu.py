@@ -441,6 +441,25 @@ def test_gemm_f32_is_true_32_bit(m, n, k_):
         assert torch.equal(one[0], out[m - 1])
 
 
+@pytest.mark.parametrize("m,n,k_,pad", [(1, 9, 64, 0), (2, 17, 65, 0), (4, 24, 2048 + 72, 8), (5, 24584, 136, 0),
+                                        (8, 33, 4160, 0), (9, 70, 1032, 3), (16, 24577, 72, 8), (17, 63, 200, 0),
+                                        (65, 130, 61, 0), (129, 65, 128, 5)])
+def test_gemm_f32_forms_sum_in_one_order(m, n, k_, pad):
+    """Few rows, few rows of many columns and tiles, with rows that are and are not whole 32-byte pieces: every row
+    equals the one-row product bit for bit, and 64 bits to the bound of a chain of 64 products and K / 64 sums (each
+    rounding 2^-24 of a partial sum, which random terms keep within a few standard deviations of the result)."""
+    k = K()
+    xs, ws = rnd(m, k_ + pad, seed=1).to(DEV), rnd(n, k_ + pad, seed=2).to(DEV)
+    x, w = xs[:, :k_], ws[:, :k_]
+    out = torch.full((m, n), float("nan"), device=DEV)
+    k.gemm_f32(out, x, w)
+    assert rel(out, x.double() @ w.double().t()) <= 2e-6
+    for r in {0, m // 2, m - 1}:
+        one = torch.empty(1, n, device=DEV)
+        k.gemm_f32(one, x[r:r + 1], w)
+        assert torch.equal(one[0], out[r])
+
+
 @pytest.mark.parametrize("m,n,k_", [(17, 256, 128), (64, 2560, 4096), (33, 1000, 1000), (1, 128, 64),
                                     (48, 331 * 2, 80), (64, 6144, 2560), (24, 1280, 2560),
                                     (24, 20012, 2560)])
