@@ -867,6 +867,53 @@ def attention_prefill_bf16(out, q, n_tokens, positions, token_slot, cu_seqlens, 
                        float(softcap or 0.0), _stream())
 
 
+_attn_prefill_f32 = Function("attention_prefill_f32", "ek_attention_prefill_f32",
+                             [_P, _P, c_int, _P, _P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, c_int, c_int,
+                              c_float, c_int, c_float, _P, c_int, _P, c_int, c_int, c_float, _P])
+PREFILL_F32_ROWS = 64           # tokens a block of attention_prefill_f32 takes
+PREFILL_F32_ROUND = 1024        # (see attention_prefill_f32_wins)
+
+
+def attention_prefill_f32_supported(out, q, k_pages, v_pages, head_dim):
+    return (q.dtype == torch.float32 and head_dim % 4 == 0 and 4 <= head_dim <= 128 and q.stride(0) % 4 == 0
+            and all(t.data_ptr() % 16 == 0 for t in (out, q, k_pages, v_pages)))
+
+
+def attention_prefill_f32_wins(n_tokens, n_seqs, n_q_heads, visible, device):
+    """Whether blocks of 64 tokens beat the general kernel's block a token and head.  A page of 64 keys takes a
+    block about 0.1 us a dimension of the head, two blocks an SM side by side; the general kernel works off
+    600,000 (token, head, key, dimension) products a microsecond once it fills the GPU.  Both grow with the keys
+    and the head size alike, which leaves the rows: 1,024 (token, head) rows for every round of blocks (heads of
+    128, keys before the prompt: 32 tokens x 16 heads 118 us here against 215, 64 x 32 1,565 against 780).  Below
+    two pages of keys what a block fetches first decides (64 tokens x 16 heads alone: 15 us against 22)."""
+    blocks = (n_tokens // PREFILL_F32_ROWS + n_seqs) * n_q_heads
+    rounds = -(-blocks // (2 * sm_count(device)))
+    return visible >= 2 * PAGE and n_tokens * n_q_heads >= PREFILL_F32_ROUND * rounds
+
+
+def attention_prefill_f32(out, q, n_tokens, positions, token_slot, cu_seqlens, n_seqs, k_pages, v_pages,
+                          block_table, n_q_heads, n_kv_heads, head_dim, scale, window=None, sink=None, sinks=None,
+                          keep_first=0, gate=None, chunk=None, softcap=None):
+    """Several new tokens per sequence in true 32-bit: sequence b owns rows cu_seqlens[b] .. cu_seqlens[b+1] of
+    ``q``, which stand at consecutive positions; their keys and values are already in the pages.  Options as in
+    :func:`attention_generic`."""
+    _need_cuda(out, q, positions, token_slot, cu_seqlens, k_pages, v_pages, block_table, gate)
+    _need(out.dtype == q.dtype == k_pages.dtype, "attention: one dtype for q, cache and out")
+    _need(attention_prefill_f32_supported(out, q, k_pages, v_pages, head_dim),
+          "attention_prefill_f32: 32-bit, head sizes up to 128 in multiples of 4, rows on 16-byte boundaries")
+    _need(out.is_contiguous() and out.shape[-1] == n_q_heads * head_dim, "attention: out [T, NQ*D]")
+    _need(q.stride(-1) == 1, "attention: q rows must be dense")
+    _need(gate is None or (gate.dtype == q.dtype and gate.stride(-1) == 1 and gate.shape[-1] >= n_q_heads),
+          "attention: the gate holds one value per token and query head, in q's dtype")
+    _need(cu_seqlens.dtype == torch.int32 and cu_seqlens.numel() >= n_seqs + 1, "attention: cu_seqlens")
+    _attention_cost(q, n_tokens, positions, n_q_heads, n_kv_heads, head_dim, window, True, chunk)
+    _attn_prefill_f32(_ptr(out), _ptr(q), q.stride(0), _ptr(positions), _ptr(token_slot), _ptr(cu_seqlens), n_seqs,
+                      n_tokens, _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.stride(0), n_q_heads,
+                      n_kv_heads, head_dim, float(scale), int(window or 0), _sink(sink), _sinks(sinks, n_q_heads),
+                      int(keep_first or 0), _ptr(gate), gate.stride(0) if gate is not None else 0, int(chunk or 0),
+                      float(softcap or 0.0), _stream())
+
+
 _attn_prefill_tc = Function("attention_prefill_tc", "ek_attention_prefill_tc",
                             [_P, _P, c_int, _P, c_int, c_int, _P, _P, c_int, _P, c_int, c_int,
                              c_int, c_int, c_float, c_int, _P, c_float, _P, c_int, c_float, _P])

@@ -301,6 +301,12 @@ class Attention(Mixer):
                                           entry.block_table, nh, nkv, big, self.scale, self.window, splits, 0, acc, ml,
                                           keep_first=self.keep_first, gate=gate, **mask)
             return self._project(out, ctx, None, leave_bias)
+        if not ctx.is_decode and kernels.attention_prefill_f32_supported(out, rows, entry.k_pages, entry.v_pages, big) \
+                and kernels.attention_prefill_f32_wins(t, ctx.n_seqs, nh, visible, self.device):
+            kernels.attention_prefill_f32(out, rows, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
+                                          entry.k_pages, entry.v_pages, entry.block_table, nh, nkv, big, self.scale,
+                                          self.window, keep_first=self.keep_first, gate=gate, **mask)
+            return self._project(out, ctx, None, leave_bias)
         splits, per_split, acc, ml = 1, 0, None, None
         blocks = t * nh
         if blocks < 2 * kernels.sm_count(self.device) and visible > 512:
@@ -499,6 +505,14 @@ class Attention(Mixer):
                 out, qkv, t, ctx.positions, ctx.token_slot, entry.k_pages, entry.v_pages,
                 entry.block_table, self.num_heads, self.num_kv_heads, self.head_dim, self.scale,
                 self.window, splits, sink=self.sink, **mask)
+            return
+        if not ctx.is_decode and kernels.attention_prefill_f32_supported(
+                out, qkv, entry.k_pages, entry.v_pages, self.head_dim) and kernels.attention_prefill_f32_wins(
+                t, ctx.n_seqs, self.num_heads, visible, self.device):
+            kernels.attention_prefill_f32(
+                out, qkv, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs, entry.k_pages, entry.v_pages,
+                entry.block_table, self.num_heads, self.num_kv_heads, self.head_dim, self.scale, self.window,
+                sink=self.sink, **mask)
             return
         if fast_decode:
             # blocks = tokens x KV heads (x 16-row blocks of the group); three fit an SM.  Split

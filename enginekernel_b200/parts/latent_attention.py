@@ -188,6 +188,11 @@ class LatentAttention(Mixer):
             kernels.attention_prefill_bf16(out, q, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
                                            pages, pages, table, nh, 1, row, self.scale, self.window, **common)
             return
+        if not ctx.is_decode and kernels.attention_prefill_f32_supported(out, q, pages, pages, row) \
+                and kernels.attention_prefill_f32_wins(t, ctx.n_seqs, nh, visible, self.device):
+            kernels.attention_prefill_f32(out, q, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
+                                          pages, pages, table, nh, 1, row, self.scale, self.window, **common)
+            return
         fast = ctx.is_decode and kernels.attention_decode_supported(self.dtype, row)
         if fast:
             blocks = t * -(-nh // 16)

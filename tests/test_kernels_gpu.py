@@ -939,3 +939,44 @@ def test_a_wait_that_runs_out_reaches_the_caller_and_is_cleared():
         k.check_tc_status(DEV)
     with pytest.raises(KernelError):
         k.wait_that_runs_out(DEV, code=1, limit=10**9)       # refused: only short waits
+
+
+@pytest.mark.parametrize("nq,nkv,d", [(4, 2, 4), (3, 1, 60), (4, 4, 64), (6, 2, 68), (8, 1, 128)])
+@pytest.mark.parametrize("options", [{}, {"window": 70, "keep_first": 5, "gate": True}, {"window": 1}, {"chunk": 100},
+                                     {"softcap": 3.0, "sinks": True}, {"sink": 0.5, "window": 64, "keep_first": 130}])
+def test_attention_prefill_f32(nq, nkv, d, options):
+    """Blocks of 64 tokens beside the general kernel, which takes a token and head a block: prompts of 1 to 200
+    tokens (tiles with 1, 63, 64, 65 rows), some behind 65 and 300 earlier tokens, every option.  Both sum up to
+    500 terms in 32-bit, each its own way: 2e-6 of the largest value, as the general kernel's own tests allow.  A
+    value that is not a number reaches only the tokens that see its key."""
+    k = K()
+    new, past = [1, 64, 200, 63, 65], [0, 0, 300, 65, 0]
+    t = sum(new)
+    pages = Pages(len(new), 500, nkv, d, torch.float32, seed=3)
+    for s in range(len(new)):
+        n = new[s] + past[s]
+        pages.fill(s, rnd(n, nkv, d, seed=10 + s), rnd(n, nkv, d, seed=20 + s))
+    q = rnd(t, nq * d + 4 + 4 * nq, seed=30)
+    pos = torch.tensor([p0 + i for n, p0 in zip(new, past) for i in range(n)], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([s for s, n in enumerate(new) for _ in range(n)], dtype=torch.int32, device=DEV)
+    cu = torch.tensor([0, 1, 65, 265, 328, 393], dtype=torch.int32, device=DEV)
+    kw = dict(options)
+    if kw.pop("gate", False):
+        kw["gate"] = q[:, nq * d + 4:]
+    if kw.pop("sinks", False):
+        kw["sinks"] = rnd(nq, seed=5)
+    window = kw.pop("window", None)
+    place = lambda: (pages.k, pages.v, pages.table, nq, nkv, d, d ** -0.5, window)
+    want, got = torch.empty(t, nq * d, device=DEV), torch.full((t, nq * d), 7.0, device=DEV)
+    k.attention_generic(want, q, t, pos, slots, *place(), **kw)
+    k.attention_prefill_f32(got, q, t, pos, slots, cu, len(new), *place(), **kw)
+    assert rel(got, want) <= 2e-6
+    alone = torch.empty(200, nq * d, device=DEV)               # a sequence's rows do not depend on the others
+    k.attention_prefill_f32(alone, q[65:], 200, pos[65:], slots[65:], torch.tensor([0, 200], dtype=torch.int32, device=DEV),
+                            1, *place(), **dict(kw, **({"gate": kw["gate"][65:]} if "gate" in kw else {})))
+    assert torch.equal(alone, got[65:265])
+    page = int(pages.table[2, 330 // 64])
+    pages.v[page, :, 330 % 64] = float("nan")
+    k.attention_generic(want, q, t, pos, slots, *place(), **kw)
+    k.attention_prefill_f32(got, q, t, pos, slots, cu, len(new), *place(), **kw)
+    assert torch.equal(got.isnan(), want.isnan()) and want.isnan().any() and not want[:65 + 30].isnan().any()
