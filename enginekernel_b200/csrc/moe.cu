@@ -16,7 +16,7 @@
 //             stretch, made on the device: the host never sees who chose what.
 //   expert product  out[row] = f(x[row] . W_e^T) over the tiles of the plan: FFMA with 32-bit
 //             sums in ascending k (the 32-bit path, and 16-bit rows that cannot be read 16 bytes
-//             at a time), or mma.sync on bfloat16 tiles with 32-bit accumulators; either way a
+//             at a time; the others run on pairs of SMs, moe_pair.cu); either way a
 //             pair's result does not depend on its neighbours.  The up form gathers its rows by
 //             token and applies the activation, the down form scales by the pair's weight and
 //             scatters 32-bit rows by pair.  `gated` up form: the expert's weight rows alternate
@@ -26,7 +26,7 @@
 //             which is the product of the weighted input; `limit` belongs to the clamped activation.
 //   combine   out[t] = sum over the token's choices, in the order they were chosen (a choice that names an
 //             expert without weights adds weight * x[t]) (+ add[t], the result of an expert that every token shares).
-#include "common.cuh"
+#include "moe_common.cuh"
 
 namespace ek {
 
@@ -134,11 +134,17 @@ moe_route_kernel(int* __restrict__ sel_expert, float* __restrict__ sel_weight,
 constexpr int kTileRows = 64;
 
 // One block.  sel_expert [P] -> sorted_pair [P] (pairs grouped by expert), tiles [max_tiles][3] =
-// (expert, first sorted row, rows), n_tiles[0].
+// (expert, first sorted row, rows), n_tiles[0].  Tiles hold up to `tile_rows` rows; with `even` > 0 an expert's
+// tiles are as few as that allows and equal, up to the next multiple of `even` rows.
 __global__ void __launch_bounds__(1024)
 moe_plan_kernel(int* __restrict__ sorted_pair, int* __restrict__ tiles, int* __restrict__ n_tiles,
-                const int* __restrict__ sel_expert, int P, int E) {
+                const int* __restrict__ sel_expert, int P, int E, int tile_rows, int even) {
   extern __shared__ int plan_s[];               // counts [E], first row [E], first tile [E + 1]
+  auto rows_of = [&](int n) {                   // rows of the tiles of an expert with n pairs
+    if (even <= 0 || n <= 0) return tile_rows;
+    const int tiles_n = (n + tile_rows - 1) / tile_rows, each = (n + tiles_n - 1) / tiles_n;
+    return (each + even - 1) / even * even;
+  };
   pdl_launch_dependents();
   pdl_wait();
   int* counts = plan_s;
@@ -151,24 +157,36 @@ moe_plan_kernel(int* __restrict__ sorted_pair, int* __restrict__ tiles, int* __r
     if (e >= 0 && e < E) atomicAdd(&counts[e], 1);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {                       // first rows and first tiles: a scan, a lane an expert
+    const int lane = threadIdx.x;
     int row = 0, tile = 0;
-    for (int e = 0; e < E; ++e) {
-      first[e] = row;
-      tile0[e] = tile;
-      row += counts[e];
-      tile += (counts[e] + kTileRows - 1) / kTileRows;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane, n = e < E ? counts[e] : 0, each = rows_of(n), t = (n + each - 1) / each;
+      int rows_to = n, tiles_to = t;            // up to and with this lane's
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int r = __shfl_up_sync(0xffffffffu, rows_to, o), q = __shfl_up_sync(0xffffffffu, tiles_to, o);
+        if (lane >= o) { rows_to += r; tiles_to += q; }
+      }
+      if (e < E) {
+        first[e] = row + rows_to - n;
+        tile0[e] = tile + tiles_to - t;
+      }
+      row += __shfl_sync(0xffffffffu, rows_to, 31);
+      tile += __shfl_sync(0xffffffffu, tiles_to, 31);
     }
-    tile0[E] = tile;
-    n_tiles[0] = tile;
+    if (lane == 0) {
+      tile0[E] = tile;
+      n_tiles[0] = tile;
+    }
   }
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    const int n = counts[e];
-    for (int i = 0, tile = tile0[e]; i < n; i += kTileRows, ++tile) {
+    const int n = counts[e], each = rows_of(n);
+    for (int i = 0, tile = tile0[e]; i < n; i += each, ++tile) {
       tiles[3 * tile] = e;
       tiles[3 * tile + 1] = first[e] + i;
-      tiles[3 * tile + 2] = min(kTileRows, n - i);
+      tiles[3 * tile + 2] = min(each, n - i);
     }
     counts[e] = first[e];                       // from here on: the next free row of the expert
   }
@@ -177,24 +195,6 @@ moe_plan_kernel(int* __restrict__ sorted_pair, int* __restrict__ tiles, int* __r
     const int e = sel_expert[p];
     if (e >= 0 && e < E) sorted_pair[atomicAdd(&counts[e], 1)] = p;
   }
-}
-
-constexpr int ACT_RELU2 = 1, ACT_SILU = 2, ACT_GELU_TANH = 3, ACT_CLAMPED = 4;      // 0: none
-
-__device__ __forceinline__ float activate(float z, int act) {
-  if (act == ACT_RELU2) { const float r = fmaxf(z, 0.f); return r * r; }
-  if (act == ACT_SILU) return z / (1.f + expf(-z));
-  if (act == ACT_GELU_TANH) return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-  return z;
-}
-
-// act(gate) * up; the clamped form is g sigmoid(1.702 g) (u + 1) with g = min(gate, limit), u = clamp(up, -limit, limit).
-__device__ __forceinline__ float gated_value(float gate, float up, int act, float limit) {
-  if (act == ACT_CLAMPED) {
-    const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
-    return g / (1.f + expf(-1.702f * g)) * (u + 1.f);
-  }
-  return activate(gate, act) * up;
 }
 
 // grid (max tiles, column tiles).  UP: a[row] = x[pair / top], out T [sorted row][N] = act(.).
@@ -277,152 +277,19 @@ moe_expert_product_kernel(void* __restrict__ out_, const T* __restrict__ a, cons
   }
 }
 
-// ---------------------------------------------------------------------------------------------
-// The same product on the tensor cores (bfloat16 operands, 32-bit accumulators): a block takes a
-// 64-row tile of the plan and 128 columns, eight warps of 32 x 32 each, K in steps of 64 through a
-// ring of three shared-memory stages filled by cp.async (rows padded by 16 bytes: ldmatrix without
-// bank conflicts).  K % 8 == 0.
-__device__ __forceinline__ void ldsm_x4(uint32_t r[4], const bf16* p) {
-  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
-}
-__device__ __forceinline__ void mma_bf16_16816(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// 16 bytes global -> shared without passing through registers; `bytes` = 0 writes zeros instead.
-__device__ __forceinline__ void cp_async_16(void* dst, const void* src, int bytes) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-constexpr int kTcCols = 128, kTcK = 64, kTcLd = kTcK + 8, kTcStages = 3;
-constexpr size_t kTcSmem = (size_t)kTcStages * (kTileRows + kTcCols) * kTcLd * sizeof(bf16);
-
-template <bool UP>
+// out[sorted row] = x[token of the pair], 16 bytes a thread: the rows of the up product side by side.  A warp a row.
 __global__ void __launch_bounds__(256)
-moe_expert_product_tc_kernel(void* __restrict__ out_, const bf16* __restrict__ a, const bf16* __restrict__ w,
-                             const int* __restrict__ tiles, const int* __restrict__ n_tiles,
-                             const int* __restrict__ sorted_pair, const float* __restrict__ pair_weight,
-                             int top, int N, int K, int act, int gated, float limit) {
-  constexpr int BM = kTileRows, BN = kTcCols, BK = kTcK, LD = kTcLd, STAGES = kTcStages;
-  extern __shared__ __align__(16) unsigned char tc_smem[];
-  typedef bf16 (*Tile)[LD];
-  bf16* const a_base = reinterpret_cast<bf16*>(tc_smem);                  // [STAGES][BM][LD]
-  bf16* const w_base = a_base + STAGES * BM * LD;                          // [STAGES][BN][LD]
-  __shared__ int src_row[BM];
-  __shared__ int pair_s[BM];
+moe_gather_kernel(uint4* __restrict__ out, const uint4* __restrict__ x, const int* __restrict__ sorted_pair,
+                  const int* __restrict__ tiles, const int* __restrict__ n_tiles, int P, int top, int pieces) {
   pdl_launch_dependents();
   pdl_wait();
-  if ((int)blockIdx.x >= n_tiles[0]) return;
-  const int e = tiles[3 * blockIdx.x], row0 = tiles[3 * blockIdx.x + 1], rows = tiles[3 * blockIdx.x + 2];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid < BM) {
-    const int p = tid < rows ? sorted_pair[row0 + tid] : -1;
-    pair_s[tid] = p;
-    src_row[tid] = p < 0 ? -1 : (UP ? p / top : row0 + tid);
-  }
-  __syncthreads();
-  const int n0 = blockIdx.y * BN;
-  const bf16* we = w + (size_t)e * N * K;
-  const int wm = warp >> 2, wn = warp & 3;      // the warp's 32 x 32 piece: rows wm * 32, columns wn * 32
-  float acc[2][4][4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.f;
-
-  // a K step is (64 + 128) rows of 8 pieces of 16 bytes: six pieces a thread
-  auto load = [&](int stage, int kt) {
-    const int k0 = kt * BK;
-#pragma unroll
-    for (int it = 0; it < (BM + BN) * (BK / 8) / 256; ++it) {
-      const int idx = tid + it * 256, row = idx / (BK / 8), piece = idx % (BK / 8);
-      const int gk = k0 + piece * 8;
-      if (row < BM) {
-        const int src = src_row[row];
-        const bool ok = src >= 0 && gk < K;
-        cp_async_16(a_base + ((size_t)stage * BM + row) * LD + piece * 8, ok ? a + (size_t)src * K + gk : a, ok ? 16 : 0);
-      } else {
-        const int gn = n0 + row - BM;
-        const bool ok = gn < N && gk < K;
-        cp_async_16(w_base + ((size_t)stage * BN + row - BM) * LD + piece * 8, ok ? we + (size_t)gn * K + gk : w, ok ? 16 : 0);
-      }
-    }
-  };
-  const int KT = (K + BK - 1) / BK;
-#pragma unroll
-  for (int st = 0; st < STAGES - 1; ++st) {
-    if (st < KT) load(st, st);
-    cp_async_commit();
-  }
-  for (int kt = 0; kt < KT; ++kt) {
-    cp_async_wait_group<STAGES - 2>();           // this step's tiles have landed
-    __syncthreads();                             // ... for everyone, and the stage refilled below is free
-    if (kt + STAGES - 1 < KT) load((kt + STAGES - 1) % STAGES, kt + STAGES - 1);
-    cp_async_commit();
-    const int st = kt % STAGES;
-    Tile As = reinterpret_cast<Tile>(a_base + (size_t)st * BM * LD);
-    Tile Ws = reinterpret_cast<Tile>(w_base + (size_t)st * BN * LD);
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 16) {
-      uint32_t af[2][4], bfr[2][4];
-#pragma unroll
-      for (int i = 0; i < 2; ++i)                // rows (lane % 16), k half (lane / 16)
-        ldsm_x4(af[i], &As[wm * 32 + i * 16 + (lane & 15)][kk + (lane >> 4) * 8]);
-#pragma unroll
-      for (int j = 0; j < 2; ++j)                // two n8 tiles a load: n = (lane / 16) * 8 + lane % 8, k half (lane / 8) % 2
-        ldsm_x4(bfr[j], &Ws[wn * 32 + j * 16 + (lane >> 4) * 8 + (lane & 7)][kk + ((lane >> 3) & 1) * 8]);
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          mma_bf16_16816(acc[i][j], af[i], bfr[j >> 1][(j & 1) * 2], bfr[j >> 1][(j & 1) * 2 + 1]);
-    }
-  }
-  cp_async_wait_group<0>();
-  const int g = lane >> 2, tq = lane & 3;
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int r = wm * 32 + i * 16 + g + half * 8;
-      if (r >= rows) continue;
-      const int p = pair_s[r];
-      const float pw = pair_weight != nullptr ? pair_weight[p] : 1.f;
-      if (UP && gated) {                          // a lane's two neighbouring columns are (gate, up)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int gn = n0 + wn * 32 + j * 8 + tq * 2;
-          if (gn + 1 < N)
-            ((bf16*)out_)[(size_t)(row0 + r) * (N / 2) + gn / 2] =
-                __float2bfloat16_rn(gated_value(acc[i][j][half * 2] * pw, acc[i][j][half * 2 + 1] * pw, act, limit));
-        }
-        continue;
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int gn = n0 + wn * 32 + j * 8 + tq * 2 + c;
-          if (gn >= N) continue;
-          const float v = acc[i][j][half * 2 + c];
-          if (UP) ((bf16*)out_)[(size_t)(row0 + r) * N + gn] = __float2bfloat16_rn(activate(v * pw, act));
-          else ((float*)out_)[(size_t)p * N + gn] = v * pw;
-        }
-    }
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int last = n_tiles[0] - 1;               // (pairs whose expert has no weights have no row)
+  if (last < 0 || row >= min(P, tiles[3 * last + 1] + tiles[3 * last + 2])) return;
+  const uint4* from = x + (size_t)(sorted_pair[row] / top) * pieces;
+  uint4* to = out + (size_t)row * pieces;
+#pragma unroll 8
+  for (int i = lane; i < pieces; i += 32) to[i] = from[i];
 }
 
 // out[t, :] = sum_k pair_out[t * top + k, :], k ascending (+ add[t, :]).  A choice k whose expert number is E or more
@@ -493,46 +360,21 @@ EK_EXPORT int ek_moe_route(int* sel_expert, float* sel_weight, const float* logi
 }
 
 EK_EXPORT int ek_moe_plan(int* sorted_pair, int* tiles, int* n_tiles, const int* sel_expert, int P, int E,
-                          cudaStream_t stream) {
+                          int tile_rows, int even, cudaStream_t stream) {
   if (P <= 0) return 0;
-  if (E <= 0 || E > 8192) return EK_ERR_ARG;
+  if (E <= 0 || E > 8192 || tile_rows <= 0 || even < 0 || (even > 0 && tile_rows % even)) return EK_ERR_ARG;
   ek::moe_plan_kernel<<<1, 1024, (size_t)(3 * E + 1) * sizeof(int), stream>>>(sorted_pair, tiles, n_tiles,
-                                                                             sel_expert, P, E);
+                                                                             sel_expert, P, E, tile_rows, even);
   EK_RETURN_LAUNCH_STATUS();
 }
 
-// The tensor-core forms: bfloat16, K a multiple of 8, operands on 16-byte boundaries.
-EK_EXPORT int ek_moe_expert_up_tc(void* out, const void* x, const void* w, const int* tiles, const int* n_tiles,
-                                  const int* sorted_pair, int max_tiles, int top, int N, int K, int act,
-                                  int gated, float limit, const float* row_weight, cudaStream_t stream) {
-  using namespace ek;
-  if (max_tiles <= 0) return 0;
-  if ((gated && N % 2) || (act == ACT_CLAMPED && !(gated && limit > 0.f))) return EK_ERR_ARG;
-  if (N <= 0 || K <= 0 || K % 8 || top <= 0 || (N + 127) / 128 > 65535 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15))
-    return EK_ERR_ARG;
-  dim3 grid(max_tiles, (N + 127) / 128);
-  cudaError_t e = cudaFuncSetAttribute(moe_expert_product_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kTcSmem);
-  if (e != cudaSuccess) return (int)e;
-  moe_expert_product_tc_kernel<true><<<grid, 256, kTcSmem, stream>>>(out, (const bf16*)x, (const bf16*)w, tiles, n_tiles,
-                                                              sorted_pair, row_weight, top, N, K, act, gated, limit);
-  EK_RETURN_LAUNCH_STATUS();
-}
-
-EK_EXPORT int ek_moe_expert_down_tc(float* out, const void* a, const void* w, const int* tiles, const int* n_tiles,
-                                    const int* sorted_pair, const float* pair_weight, int max_tiles, int N, int K,
-                                    cudaStream_t stream) {
-  using namespace ek;
-  if (max_tiles <= 0) return 0;
-  if (N <= 0 || K <= 0 || K % 8 || (N + 127) / 128 > 65535 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15))
-    return EK_ERR_ARG;
-  dim3 grid(max_tiles, (N + 127) / 128);
-  cudaError_t e = cudaFuncSetAttribute(moe_expert_product_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kTcSmem);
-  if (e != cudaSuccess) return (int)e;
-  moe_expert_product_tc_kernel<false><<<grid, 256, kTcSmem, stream>>>(out, (const bf16*)a, (const bf16*)w, tiles, n_tiles,
-                                                               sorted_pair, pair_weight, 1, N, K, 0, 0, 0.f);
-  EK_RETURN_LAUNCH_STATUS();
+// out [P, width] = x [T, width] by the plan's order; bfloat16 rows of whole 16-byte pieces.
+EK_EXPORT int ek_moe_gather(void* out, const void* x, const int* sorted_pair, const int* tiles, const int* n_tiles,
+                            int P, int top, int width, cudaStream_t stream) {
+  if (P <= 0) return 0;
+  if (top <= 0 || width <= 0 || width % 8 || ((uintptr_t)x & 15) || ((uintptr_t)out & 15)) return EK_ERR_ARG;
+  return (int)ek::launch_pdl(ek::moe_gather_kernel, dim3((P + 7) / 8), dim3(256), 0, stream, (uint4*)out,
+                             (const uint4*)x, sorted_pair, tiles, n_tiles, P, top, width / 8);
 }
 
 #define EK_INSTANTIATE(SUFFIX, T)                                                                     \

@@ -1972,27 +1972,46 @@ def xlstm_out(y, o, m_run, proj, col_g, w, eps, q_scale, positions, n_tokens, he
 
 # ------------------------------------------------------------------ routed experts
 _moe_route = Function("moe", "ek_moe_route", [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, _P, _P])
-_moe_plan = Function("moe", "ek_moe_plan", [_P, _P, _P, _P, c_int, c_int, _P])
+_moe_plan = Function("moe", "ek_moe_plan", [_P, _P, _P, _P, c_int, c_int, c_int, c_int, _P])
 _moe_up = _per_dtype("moe", "ek_moe_expert_up",
                      [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_float, _P, _P])
 _moe_down = _per_dtype("moe", "ek_moe_expert_down", [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, _P])
 _moe_combine = _per_dtype("moe", "ek_moe_combine", [_P, _P, c_int, c_int, c_int, _P, _P, _P, _P, c_int, _P])
-_moe_up_tc = Function("moe", "ek_moe_expert_up_tc",
-                      [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_float, _P, _P])
-_moe_down_tc = Function("moe", "ek_moe_expert_down_tc", [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, _P])
+_moe_up_pair = Function("moe_pair", "ek_moe_pair_up",
+                        [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, _P, _P,
+                         _P])
+_moe_gather = Function("moe", "ek_moe_gather", [_P, _P, _P, _P, _P, c_int, c_int, c_int, _P])
+_moe_down_pair = Function("moe_pair", "ek_moe_pair_down",
+                          [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P])
 
 
-def _moe_on_tensor_cores(a, w) -> bool:
-    """bfloat16 rows that can be read 16 bytes at a time go to the mma.sync form of the expert products."""
-    return (a.dtype == torch.bfloat16 and w.shape[-1] % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+def _moe_on_pairs(a, w) -> bool:
+    """What TMA can address: bfloat16 rows of whole 16-byte pieces."""
+    return (a.dtype == torch.bfloat16 and w.shape[-1] % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+            and w.shape[0] * w.shape[1] < 1 << 31)
+
+
 MOE_TILE_ROWS = 64          # must equal kTileRows in csrc/moe.cu
+MOE_PAIR_TILE_ROWS, MOE_PAIR_EVEN = 256, 32     # must equal kMoeTile and kMoeEven in csrc/moe_pair.cu
+# From here on the up product reads a copy of x with a row per pair instead of gathering rows: the copy costs a pass
+# over the rows, gathered rows reach shared memory half as fast (8,192 pairs of 2,048 values: 128 us against 61 + 9;
+# 256 pairs 59 against 64; 512 to 1,024 pairs alike)
+MOE_GATHER_PAIRS = 1024
 EXPERT_ACTIVATIONS = {"none": 0, "relu2": 1, "silu": 2, "gelu_tanh": 3, "clamped": 4}
 ROUTE_WEIGHTS = {"scores_of_chosen": 0, "softmax_of_chosen": 1, "sigmoid": 2, "softmax": 3}
 
 
-def moe_max_tiles(n_pairs: int, n_experts: int) -> int:
+def moe_max_tiles(n_pairs: int, n_experts: int, wide: bool = False) -> int:
     """Most row tiles a plan of ``n_pairs`` (token, choice) pairs can have."""
-    return -(-n_pairs // MOE_TILE_ROWS) + min(n_experts, n_pairs)
+    return -(-n_pairs // (MOE_PAIR_TILE_ROWS if wide else MOE_TILE_ROWS)) + min(n_experts, n_pairs)
+
+
+def moe_on_pairs(x, w_up, w_down) -> bool:
+    """Whether the experts' products run on pairs of SMs, over a wide plan: every bfloat16 layer whose rows TMA can
+    address.  From one token on they were ahead of the 64 x 128 tiles on mma.sync that stood here before (32
+    experts of 1,024 gated, width 2,048, 4 chosen; up + down in us): 1 token 41 -> 32, 8 tokens 94 -> 68, 256
+    tokens 124 -> 98, 2,048 tokens 467 -> 162, 4,096 tokens 873 -> 259."""
+    return _moe_on_pairs(x, w_up) and _moe_on_pairs(x, w_down)
 
 
 def moe_route(sel_expert, sel_weight, logits, n_tokens, n_groups, keep, top, scale, weights="scores_of_chosen",
@@ -2013,17 +2032,22 @@ def moe_route(sel_expert, sel_weight, logits, n_tokens, n_groups, keep, top, sca
                top, float(scale), ROUTE_WEIGHTS[weights], _ptr(correction), _stream())
 
 
-def moe_plan(sorted_pair, tiles, n_tiles, sel_expert, n_pairs, n_experts):
+def moe_plan(sorted_pair, tiles, n_tiles, sel_expert, n_pairs, n_experts, wide=False):
+    """Sort the pairs by expert and cut every expert's stretch into row tiles: of 64, or (``wide``) into equal
+    ones of up to 256."""
     _need_cuda(sorted_pair, tiles, n_tiles, sel_expert)
-    _moe_plan(_ptr(sorted_pair), _ptr(tiles), _ptr(n_tiles), _ptr(sel_expert), n_pairs, n_experts, _stream())
+    _moe_plan(_ptr(sorted_pair), _ptr(tiles), _ptr(n_tiles), _ptr(sel_expert), n_pairs, n_experts,
+              *((MOE_PAIR_TILE_ROWS, MOE_PAIR_EVEN) if wide else (MOE_TILE_ROWS, 0)), _stream())
 
 
 def moe_expert_up(out, x, w, tiles, n_tiles, sorted_pair, n_pairs, top, activation, gated=False, limit=0.0,
-                  input_weight=None):
+                  input_weight=None, wide=False, scratch=None):
     """out[sorted row] = act(x[token of the pair] . w[expert]^T); ``w`` [E, N, K].  ``gated``: the
     rows of an expert's ``w`` alternate gate, up, gate, up ...; out [pairs, N / 2] holds
     act(gate) * up, taken from the 32-bit sums (``"clamped"`` as in :func:`act_mul`, with ``limit``).
-    ``input_weight`` [pairs] (32-bit): a pair's input is multiplied by its weight (in the 32-bit sums)."""
+    ``input_weight`` [pairs] (32-bit): a pair's input is multiplied by its weight (in the 32-bit sums).
+    ``wide``: the plan is a wide one (:func:`moe_plan`), the product runs on pairs of SMs; ``scratch``: memory
+    for a copy of x with a row per pair, which many pairs (MOE_GATHER_PAIRS) make first."""
     _need_cuda(out, x, w, tiles, n_tiles, sorted_pair, input_weight)
     _need(activation != "clamped" or (gated and limit > 0), "moe_expert_up: the clamped gate needs gate rows and a limit")
     _need(input_weight is None or (input_weight.dtype == torch.float32 and input_weight.is_contiguous()
@@ -2033,15 +2057,28 @@ def moe_expert_up(out, x, w, tiles, n_tiles, sorted_pair, n_pairs, top, activati
     e, n, k = w.shape
     if lib.recording():
         lib.annotate(bytes=x.element_size() * (min(e, n_pairs) * n * k + n_pairs * (n + k)), flops=2 * n_pairs * n * k)
-    fn = _moe_up_tc if _moe_on_tensor_cores(x, w) else _moe_up[x.dtype]
-    fn(_ptr(out), _ptr(x), _ptr(w), _ptr(tiles), _ptr(n_tiles), _ptr(sorted_pair),
-       moe_max_tiles(n_pairs, e), top, n, k, EXPERT_ACTIVATIONS[activation], 1 if gated else 0, float(limit),
-       _ptr(input_weight), _stream())
+    if wide:
+        _need(_moe_on_pairs(x, w) and x.shape[0] * top >= n_pairs, "moe_expert_up: a wide plan takes bfloat16 rows "
+              "that can be read 16 bytes at a time")
+        rows, gathered = -(-n_pairs // top), 0
+        if scratch is not None and n_pairs >= MOE_GATHER_PAIRS:
+            _need_cuda(scratch)
+            _need(scratch.is_contiguous() and scratch.data_ptr() % 16 == 0
+                  and scratch.numel() * scratch.element_size() >= n_pairs * k * x.element_size(), "moe_expert_up: scratch")
+            _moe_gather(_ptr(scratch), _ptr(x), _ptr(sorted_pair), _ptr(tiles), _ptr(n_tiles), n_pairs, top, k, _stream())
+            x, rows, gathered = scratch, n_pairs, 1
+        _moe_up_pair(_ptr(out), _ptr(x), _ptr(w), _ptr(tiles), _ptr(n_tiles), _ptr(sorted_pair), rows, gathered, e,
+                     moe_max_tiles(n_pairs, e, True), top, n, k, EXPERT_ACTIVATIONS[activation], 1 if gated else 0,
+                     float(limit), _ptr(input_weight), _ptr(tc_status(w.device)), _stream())
+        return
+    _moe_up[x.dtype](_ptr(out), _ptr(x), _ptr(w), _ptr(tiles), _ptr(n_tiles), _ptr(sorted_pair),
+                     moe_max_tiles(n_pairs, e), top, n, k, EXPERT_ACTIVATIONS[activation], 1 if gated else 0,
+                     float(limit), _ptr(input_weight), _stream())
 
 
-def moe_expert_down(pair_out, a, w, tiles, n_tiles, sorted_pair, pair_weight, n_pairs):
+def moe_expert_down(pair_out, a, w, tiles, n_tiles, sorted_pair, pair_weight, n_pairs, wide=False):
     """pair_out[pair] = weight[pair] * (a[sorted row] . w[expert]^T) in 32-bit; ``w`` [E, N, K];
-    ``pair_weight`` None: ones."""
+    ``pair_weight`` None: ones.  ``wide`` as in :func:`moe_expert_up`."""
     _need_cuda(pair_out, a, w, tiles, n_tiles, sorted_pair, pair_weight)
     _need(a.dtype == w.dtype and pair_out.dtype == torch.float32 and a.is_contiguous() and w.is_contiguous(),
           "moe_expert_down: 32-bit output")
@@ -2049,9 +2086,14 @@ def moe_expert_down(pair_out, a, w, tiles, n_tiles, sorted_pair, pair_weight, n_
     if lib.recording():
         lib.annotate(bytes=a.element_size() * (min(e, n_pairs) * n * k + n_pairs * k) + 4 * n_pairs * n,
                      flops=2 * n_pairs * n * k)
-    fn = _moe_down_tc if _moe_on_tensor_cores(a, w) else _moe_down[a.dtype]
-    fn(_ptr(pair_out), _ptr(a), _ptr(w), _ptr(tiles), _ptr(n_tiles), _ptr(sorted_pair),
-       _ptr(pair_weight), moe_max_tiles(n_pairs, e), n, k, _stream())
+    if wide:
+        _need(_moe_on_pairs(a, w) and a.shape[0] >= n_pairs, "moe_expert_down: a wide plan takes bfloat16 rows "
+              "that can be read 16 bytes at a time")
+        _moe_down_pair(_ptr(pair_out), _ptr(a), _ptr(w), _ptr(tiles), _ptr(n_tiles), _ptr(sorted_pair), _ptr(pair_weight),
+                       n_pairs, e, moe_max_tiles(n_pairs, e, True), n, k, _ptr(tc_status(a.device)), _stream())
+        return
+    _moe_down[a.dtype](_ptr(pair_out), _ptr(a), _ptr(w), _ptr(tiles), _ptr(n_tiles), _ptr(sorted_pair),
+                       _ptr(pair_weight), moe_max_tiles(n_pairs, e), n, k, _stream())
 
 
 def moe_combine(out, pair_out, n_tokens, top, add=None, identity=None):

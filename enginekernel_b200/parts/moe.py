@@ -129,15 +129,17 @@ class RoutedExperts(FeedForward):
         kernels.moe_route(chosen, weight, logits[:, :self.routed], t, self.groups, self.keep, top, self.scale,
                           weights=self.weights, correction=self.correction)
         sorted_pair = ws.get("moe_sorted", (pairs,), torch.int32)
-        tiles = ws.get("moe_tiles", (kernels.moe_max_tiles(pairs, self.experts), 3), torch.int32)
+        wide = kernels.moe_on_pairs(x, self.w_up, self.w_down)
+        tiles = ws.get("moe_tiles", (kernels.moe_max_tiles(pairs, self.experts, wide), 3), torch.int32)
         n_tiles = ws.get("moe_n_tiles", (1,), torch.int32)
-        kernels.moe_plan(sorted_pair, tiles, n_tiles, chosen, pairs, self.experts)
+        kernels.moe_plan(sorted_pair, tiles, n_tiles, chosen, pairs, self.experts, wide=wide)
         act = ws.get("moe_act", (pairs, self.inter), self.dtype)
+        pair_out = ws.get("moe_pair_out", (pairs, self.hidden), torch.float32)      # (free until the down product)
         kernels.moe_expert_up(act, x, self.w_up, tiles, n_tiles, sorted_pair, pairs, top, self.activation,
-                              gated=self.gated, limit=self.limit, input_weight=weight if self.weigh_input else None)
-        pair_out = ws.get("moe_pair_out", (pairs, self.hidden), torch.float32)
+                              gated=self.gated, limit=self.limit, input_weight=weight if self.weigh_input else None, wide=wide,
+                              scratch=pair_out)
         kernels.moe_expert_down(pair_out, act, self.w_down, tiles, n_tiles, sorted_pair,
-                                None if self.weigh_input else weight, pairs)
+                                None if self.weigh_input else weight, pairs, wide=wide)
         add = None
         if self.shared is not None:
             self.shared.product_image = self.product_image
