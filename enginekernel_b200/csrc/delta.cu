@@ -39,8 +39,12 @@ struct DeltaShape {
 };
 
 // out[t, c] = f(bias[c] + sum_r w2t[r][c] * proj[t, offset + r]) for c < channels: f = sigmoid (mode 1), or
-// the decay exp(-exp(a_log[c / dim]) * softplus(.)) (mode 0).  grid (token tiles of 16, channel tiles of 128).
+// the decay exp(-exp(a_log[c / dim]) * softplus(.)) (mode 0).  grid (token tiles of 16, channel tiles of 128 x PER).
+// A thread takes PER channels: every 16-byte read of a token's inputs feeds 4 PER FMAs, and a warp's read takes
+// shared memory four cycles.  Four where rows are whole 16-byte pieces and the tokens give blocks enough (2,048 tokens,
+// rank 64, 2,048 channels: 45 us with one, 33 with four), else one.
 constexpr int kRankTokens = 16;
+template <int PER>
 __global__ void __launch_bounds__(128)
 delta_low_rank_kernel(float* __restrict__ out, const float* __restrict__ proj, int proj_stride, int offset,
                       int rank, const float* __restrict__ w2t, const float* __restrict__ bias,
@@ -51,37 +55,53 @@ delta_low_rank_kernel(float* __restrict__ out, const float* __restrict__ proj, i
   const int t0 = blockIdx.x * kRankTokens, tid = threadIdx.x;
   const int nt = min(kRankTokens, n_tokens - t0);
   const int ld = (rank + 3) & ~3;
-  for (int idx = tid; idx < kRankTokens * rank; idx += blockDim.x) {
-    const int tt = idx / rank, r = idx % rank;
-    x_s[tt * ld + r] = tt < nt ? proj[(size_t)(t0 + tt) * proj_stride + offset + r] : 0.f;
+  for (int idx = tid; idx < kRankTokens * ld; idx += blockDim.x) {
+    const int tt = idx / ld, r = idx % ld;
+    x_s[idx] = tt < nt && r < rank ? proj[(size_t)(t0 + tt) * proj_stride + offset + r] : 0.f;
   }
   __syncthreads();
-  const int c = blockIdx.y * 128 + tid;
+  const int c = (blockIdx.y * 128 + tid) * PER;
   if (c >= channels) return;
-  float acc[kRankTokens];
-  const float b = bias ? bias[c] : 0.f;
+  auto fetch = [&](float (&w)[PER], const float* from) {
+    if (PER == 4) *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(from);
+    else w[0] = *from;
+  };
+  float acc[kRankTokens][PER], b[PER];
+  if (bias) fetch(b, bias + c);
 #pragma unroll
-  for (int tt = 0; tt < kRankTokens; ++tt) acc[tt] = b;
-  int r = 0;
-  for (; r + 4 <= rank; r += 4) {               // four weights, then one 16-byte read of a token's four inputs
-    const float w0 = w2t[(size_t)r * channels + c], w1 = w2t[(size_t)(r + 1) * channels + c];
-    const float w2 = w2t[(size_t)(r + 2) * channels + c], w3 = w2t[(size_t)(r + 3) * channels + c];
+  for (int tt = 0; tt < kRankTokens; ++tt)
+#pragma unroll
+    for (int p = 0; p < PER; ++p) acc[tt][p] = bias ? b[p] : 0.f;
+  for (int r = 0; r < rank; r += 4) {           // four rows of weights, then one 16-byte read of a token's four inputs
+    float w[4][PER];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (r + j < rank) fetch(w[j], w2t + (size_t)(r + j) * channels + c);
+      else
+#pragma unroll
+        for (int p = 0; p < PER; ++p) w[j][p] = 0.f;
+    }
 #pragma unroll
     for (int tt = 0; tt < kRankTokens; ++tt) {
       const float4 x = *reinterpret_cast<const float4*>(x_s + tt * ld + r);
-      acc[tt] = fmaf(w3, x.w, fmaf(w2, x.z, fmaf(w1, x.y, fmaf(w0, x.x, acc[tt]))));
+#pragma unroll
+      for (int p = 0; p < PER; ++p)
+        acc[tt][p] = fmaf(w[3][p], x.w, fmaf(w[2][p], x.z, fmaf(w[1][p], x.y, fmaf(w[0][p], x.x, acc[tt][p]))));
     }
   }
-  for (; r < rank; ++r) {
-    const float wv = w2t[(size_t)r * channels + c];
+  float rate[PER];
 #pragma unroll
-    for (int tt = 0; tt < kRankTokens; ++tt) acc[tt] = fmaf(wv, x_s[tt * ld + r], acc[tt]);
+  for (int p = 0; p < PER; ++p) rate[p] = mode == 0 ? expf(a_log[(c + p) / dim]) : 0.f;
+#pragma unroll
+  for (int tt = 0; tt < kRankTokens; ++tt) {    // (a fixed trip count keeps acc in registers)
+    if (tt >= nt) continue;
+    float y[PER];
+#pragma unroll
+    for (int p = 0; p < PER; ++p) y[p] = mode == 0 ? expf(-rate[p] * softplus_f(acc[tt][p])) : sigmoid_f(acc[tt][p]);
+    float* to = out + (size_t)(t0 + tt) * channels + c;
+    if (PER == 4) *reinterpret_cast<float4*>(to) = *reinterpret_cast<const float4*>(y);
+    else *to = y[0];
   }
-  const float rate = mode == 0 ? expf(a_log[c / dim]) : 0.f;
-#pragma unroll
-  for (int tt = 0; tt < kRankTokens; ++tt)      // (a fixed trip count keeps acc in registers)
-    if (tt < nt)
-      out[(size_t)(t0 + tt) * channels + c] = mode == 0 ? expf(-rate * softplus_f(acc[tt])) : sigmoid_f(acc[tt]);
 }
 
 // grid (tokens, key heads): a block convolves one q head, one k head and the v channels of the value
@@ -141,6 +161,92 @@ delta_prepare_kernel(float* __restrict__ qn, float* __restrict__ kn, float* __re
     const float f = rsqrtf(ss + 1e-6f) * (which == 0 ? rsqrtf((float)sh.dim) : 1.f);
     float* dst = (which == 0 ? qn : kn) + (size_t)t * cq + (size_t)g * sh.dim;
     for (int i = tid; i < sh.dim; i += blockDim.x) dst[i] = x[i] * f;
+  }
+}
+
+// The same for many tokens: a block takes one head's channels - a q head, a k head or a value head - of 8 (kPrepTokens)
+// neighbouring tokens, a thread a channel, so that an input is fetched once for all its taps (11 loads for 8 tokens of 4
+// taps) and the taps stay in registers.  Bound by memory (2,048 tokens of 6,144 channels, 50 MB in and out: 100 us with a
+// block a token, 45 so).  grid (token tiles, 2 kv_heads + heads); blockDim = the head's channels rounded up to a warp.
+constexpr int kPrepTokens = 8;
+template <int K>
+__global__ void __launch_bounds__(256)
+delta_prepare_tile_kernel(float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vc,
+                          float* __restrict__ beta, const float* __restrict__ proj, int proj_stride,
+                          const float* __restrict__ conv_w, const float* __restrict__ state, size_t slot_stride,
+                          size_t tail_offset, const int* __restrict__ positions, const int* __restrict__ token_slot,
+                          int n_tokens, DeltaShape sh) {
+  __shared__ int n_prev_s[kPrepTokens], slot_s[kPrepTokens];
+  __shared__ float sums[kPrepTokens][8];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t0 = blockIdx.x * kPrepTokens, nt = min(kPrepTokens, n_tokens - t0), tid = threadIdx.x;
+  const int unit = blockIdx.y, cq = sh.cq();
+  const bool is_v = unit >= 2 * sh.kv_heads;
+  const int size = is_v ? sh.vdim : sh.dim;
+  const int c0 = is_v ? 2 * cq + (unit - 2 * sh.kv_heads) * sh.vdim : unit * sh.dim;      // (q heads, then k heads)
+  if (tid < nt) {
+    const int t = t0 + tid, pos = positions[t], slot = token_slot[t];
+    int n = 0;                                  // predecessors of this token inside the step
+    while (n < K - 1 && t - n - 1 >= 0 && token_slot[t - n - 1] == slot && positions[t - n - 1] == pos - n - 1) ++n;
+    n_prev_s[tid] = pos < 0 ? -1 : n;
+    slot_s[tid] = slot;
+    if (is_v && pos >= 0) {
+      const int h = unit - 2 * sh.kv_heads;
+      beta[(size_t)t * sh.heads + h] = sigmoid_f(proj[(size_t)t * proj_stride + sh.off_beta() + h]);
+    }
+  }
+  __syncthreads();
+  const bool live = tid < size;
+  const int c = c0 + (live ? tid : 0);
+  float w[K], x[kPrepTokens + K - 1], y[kPrepTokens];
+#pragma unroll
+  for (int j = 0; j < K; ++j) w[j] = conv_w[(size_t)c * K + j];
+#pragma unroll
+  for (int i = 0; i < kPrepTokens + K - 1; ++i) {          // rows t0 - (K - 1) ..
+    const int t = t0 + i - (K - 1);
+    x[i] = t >= 0 && t < n_tokens ? proj[(size_t)t * proj_stride + c] : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < kPrepTokens; ++i) {
+    y[i] = 0.f;
+    const int n_prev = i < nt ? n_prev_s[i] : -1;
+    if (n_prev < 0) continue;
+    float acc = w[K - 1] * x[i + K - 1];
+    if (n_prev == K - 1) {
+#pragma unroll
+      for (int j = 1; j < K; ++j) acc = fmaf(w[K - 1 - j], x[i + K - 1 - j], acc);
+    } else {                                    // the sequence's first tokens of the step
+      const float* tail = state + (size_t)slot_s[i] * slot_stride + tail_offset + (size_t)c * (K - 1);
+#pragma unroll
+      for (int j = 1; j < K; ++j)
+        acc = fmaf(w[K - 1 - j], j <= n_prev ? x[i + K - 1 - j] : tail[n_prev - j + K - 1], acc);
+    }
+    y[i] = live ? acc * sigmoid_f(acc) : 0.f;
+  }
+  if (is_v) {
+    const int at = c - 2 * cq;
+#pragma unroll
+    for (int i = 0; i < kPrepTokens; ++i)
+      if (live && i < nt && n_prev_s[i] >= 0) vc[(size_t)(t0 + i) * sh.cv() + at] = y[i];
+    return;
+  }
+  // unit vectors: q (also times dim^-1/2), then k
+  const int warp = tid >> 5, lane = tid & 31;
+#pragma unroll
+  for (int i = 0; i < kPrepTokens; ++i) {
+    const float ss = warp_sum(y[i] * y[i]);
+    if (lane == 0) sums[i][warp] = ss;
+  }
+  __syncthreads();
+  const bool is_q = unit < sh.kv_heads;
+  const float scale = is_q ? rsqrtf((float)sh.dim) : 1.f;
+  float* dst = (is_q ? qn : kn) + (is_q ? c : c - cq);
+#pragma unroll
+  for (int i = 0; i < kPrepTokens; ++i) {
+    float ss = 0.f;
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) ss += sums[i][q];
+    if (live && i < nt && n_prev_s[i] >= 0) dst[(size_t)(t0 + i) * cq] = y[i] * (rsqrtf(ss + 1e-6f) * scale);
   }
 }
 
@@ -442,14 +548,18 @@ EK_EXPORT int ek_delta_low_rank(float* out, const float* proj, int proj_stride, 
   if (rank <= 0 || rank > 2048 || channels <= 0 || dim <= 0 || offset < 0 || proj_stride < offset + rank ||
       (mode == 0 && !a_log) || (channels + 127) / 128 > 65535)
     return EK_ERR_ARG;
-  dim3 grid((n_tokens + kRankTokens - 1) / kRankTokens, (channels + 127) / 128);
+  const int token_tiles = (n_tokens + kRankTokens - 1) / kRankTokens;
+  const bool four = channels % 4 == 0 && (long long)token_tiles * ((channels + 511) / 512) >= sm_count() &&
+                    (((uintptr_t)out | (uintptr_t)w2t | (uintptr_t)bias) & 15) == 0;
   const size_t smem = (size_t)kRankTokens * ((rank + 3) & ~3) * sizeof(float);
+  auto kernel = four ? delta_low_rank_kernel<4> : delta_low_rank_kernel<1>;
   if (smem > 40 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(delta_low_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  delta_low_rank_kernel<<<grid, 128, smem, stream>>>(out, proj, proj_stride, offset, rank, w2t, bias, a_log, dim,
-                                                     channels, n_tokens, mode);
+  const int wide = four ? 512 : 128;
+  kernel<<<dim3(token_tiles, (channels + wide - 1) / wide), 128, smem, stream>>>(
+      out, proj, proj_stride, offset, rank, w2t, bias, a_log, dim, channels, n_tokens, mode);
   EK_RETURN_LAUNCH_STATUS();
 }
 
@@ -462,6 +572,17 @@ EK_EXPORT int ek_delta_prepare(float* qn, float* kn, float* vc, float* beta,
   if (n_tokens <= 0) return 0;
   DeltaShape sh{heads, kv_heads, dim, vdim, taps, rank_a, rank_g};
   if (!shape_ok(sh) || proj_stride < sh.row()) return EK_ERR_ARG;
+  // (tiles from where they give every SM two blocks on; taps beyond 4 and heads beyond 256 channels take the others)
+  const int units = 2 * kv_heads + heads, widest = dim > vdim ? dim : vdim;
+  if (taps >= 2 && taps <= 4 && widest <= 256 && units <= 65535 &&
+      (long long)(n_tokens / kPrepTokens) * units >= 2 * sm_count()) {
+    const dim3 grid((n_tokens + kPrepTokens - 1) / kPrepTokens, units);
+    auto kernel = taps == 2 ? delta_prepare_tile_kernel<2> : taps == 3 ? delta_prepare_tile_kernel<3> : delta_prepare_tile_kernel<4>;
+    kernel<<<grid, (widest + 31) / 32 * 32, 0, stream>>>(qn, kn, vc, beta, proj, proj_stride, conv_w, state,
+                                                         (size_t)slot_stride, (size_t)tail_offset, positions, token_slot,
+                                                         n_tokens, sh);
+    EK_RETURN_LAUNCH_STATUS();
+  }
   if (n_tokens >= 512) {
     const size_t smem = (size_t)(2 * sh.cq()) * sizeof(float);
     if (smem > 200 * 1024) return EK_ERR_ARG;

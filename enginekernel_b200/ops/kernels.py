@@ -1655,11 +1655,26 @@ def delta_conv_tail(state, tail_offset, proj, cu_seqlens, positions, token_slot,
                      _ptr(positions), _ptr(token_slot), n_seqs, channels, taps, _stream())
 
 
+_delta_chunks = Function("delta_chunk", "ek_delta_chunks",
+                         [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, c_longlong, _P, _P, _P, c_int, c_int, c_int, c_int, c_int,
+                          c_int, c_int, _P])
+DELTA_CHUNK = 32                # must equal kChunk in csrc/delta_chunk.cu
+# Tokens a sequence brings on average from which the walk by chunks wins (16 to 20 heads of 128 x 128, us token by token
+# and by chunks: 64 tokens 28 / 35, 128 tokens 59 / 50, 16 x 128 323 / 298, 2,048 699 / 307, 8 x 2,048 2,722 / 2,005)
+DELTA_CHUNK_TOKENS = 96
+
+
+def delta_by_chunks(n_tokens, n_seqs, dim, vdim) -> bool:
+    """Whether the recurrence over ``n_tokens`` tokens runs by chunks (csrc/delta_chunk.cu) or token by token."""
+    return (n_tokens >= DELTA_CHUNK_TOKENS * n_seqs and dim in (64, 128) and vdim % 4 == 0 and vdim <= 2 * dim)
+
+
 def delta_scan(out, qn, kn, vc, beta, decay, state, cu_seqlens, positions, token_slot, n_seqs, heads,
-               kv_heads, dim, vdim, n_tokens=0, decay_per_head=False):
+               kv_heads, dim, vdim, n_tokens=0, decay_per_head=False, workspace=None):
     """The recurrence over every sequence's tokens; S [heads, vdim, rows] at the start of a slot's state
     is read and written back.  ``decay`` is [T, heads * dim] (one per key channel) or, with
-    ``decay_per_head``, [T, heads]."""
+    ``decay_per_head``, [T, heads].  ``workspace`` (with ``n_tokens``): scratch for long stretches of tokens, which then
+    run by chunks (:func:`delta_by_chunks`) and leave other values in ``vc`` and ``decay``."""
     _need_cuda(out, qn, kn, vc, beta, decay, state, cu_seqlens, positions, token_slot)
     _need(decay.is_contiguous() and decay.shape[-1] == (heads if decay_per_head else heads * dim),
           "delta_scan: decays [T, heads * dim], or [T, heads] with decay_per_head")
@@ -1667,6 +1682,19 @@ def delta_scan(out, qn, kn, vc, beta, decay, state, cu_seqlens, positions, token
         lib.annotate(bytes=4 * (n_tokens * (2 * kv_heads * dim + heads * dim + 2 * heads * vdim + heads)
                                 + 2 * n_seqs * heads * vdim * delta_state_rows(dim)),
                      flops=6 * n_tokens * heads * dim * vdim)
+    if workspace is not None and delta_by_chunks(n_tokens, n_seqs, dim, vdim):
+        _need_f32("delta_scan", out, qn, kn, vc, beta, decay)
+        _need(all(t.is_contiguous() for t in (out, qn, kn, vc, beta)) and state.stride(0) % 4 == 0, "delta_scan: contiguous")
+        chunks = n_tokens // DELTA_CHUNK + n_seqs
+        w = workspace.get("delta_chunk_w", (n_tokens, heads * dim), torch.float32)
+        qp = workspace.get("delta_chunk_q", (n_tokens, heads * dim), torch.float32)
+        kh = workspace.get("delta_chunk_k", (n_tokens, heads * dim), torch.float32) if decay_per_head else decay
+        gam = workspace.get("delta_chunk_decay", (chunks, heads, dim), torch.float32)
+        _delta_chunks(_ptr(out), _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(decay), _ptr(w), _ptr(qp), _ptr(kh), _ptr(gam),
+                      _ptr(state), state.stride(0), _ptr(cu_seqlens), _ptr(positions), _ptr(token_slot), n_seqs, chunks,
+                      heads, kv_heads, dim, vdim, 1 if decay_per_head else 0, _stream())
+        count_extra_launches()
+        return
     _delta_scan(_ptr(out), _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(decay), _ptr(state), state.stride(0),
                 _ptr(cu_seqlens), _ptr(positions), _ptr(token_slot), n_seqs, heads, kv_heads, dim, vdim,
                 1 if decay_per_head else 0, _stream())

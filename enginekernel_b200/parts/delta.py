@@ -116,7 +116,7 @@ class ChannelDelta(Mixer):
                                     ctx.n_seqs, self.channels, self.taps)
         o = ws.get("delta_o", (t, nh * e), f32)
         kernels.delta_scan(o, qn, kn, vc, beta, decay, state, ctx.cu_seqlens, ctx.positions, ctx.token_slot,
-                           ctx.n_seqs, nh, g, d, e, n_tokens=t)
+                           ctx.n_seqs, nh, g, d, e, n_tokens=t, workspace=ws)
         y = ws.get("attn_out", (t, nh * e), self.dtype)
         kernels.delta_out_norm(y, o, gate, self.norm_w, self.eps, ctx.positions, t, self.shape())
         return linear(y, self.w_o, ctx, "attn_proj", n_rows=t)
@@ -213,7 +213,7 @@ class HeadDelta(Mixer):
                                     ctx.n_seqs, self.channels, self.taps)
         o = ws.get("delta_o", (t, nh * e), f32)
         kernels.delta_scan(o, qn, kn, vc, beta, decay, state, ctx.cu_seqlens, ctx.positions, ctx.token_slot,
-                           ctx.n_seqs, nh, g, d, e, n_tokens=t, decay_per_head=True)
+                           ctx.n_seqs, nh, g, d, e, n_tokens=t, decay_per_head=True, workspace=ws)
         y = ws.get("attn_out", (t, nh * e), self.dtype)
         kernels.delta_out_norm(y, o, proj[:, col_a + nh:], self.norm_w, self.eps, ctx.positions, t, self.shape(),
                                gate_activation="silu")
