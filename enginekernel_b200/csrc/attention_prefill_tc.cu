@@ -35,14 +35,13 @@ namespace ek {
 constexpr int kFaRows = 128;
 constexpr int kFaKeys = EK_PAGE;             // 64
 constexpr int kFaThreads = 224;              // 4 softmax warps, a producer warp, two MMA warps
-constexpr int kFaKStages = 3;                // K pages in flight: two pages of lookahead for the scores
-constexpr int kFaVStages = 2;
+// K pages in flight: two pages of lookahead for the scores; where the values are the keys' pages (`shared`) a
+// page also waits there for its P.V
+__host__ __device__ constexpr int fa_k_stages(bool shared) { return shared ? 4 : 3; }
+__host__ __device__ constexpr int fa_v_stages(bool shared) { return shared ? 0 : 2; }
 // mbarriers: K full / empty per K stage, V full / empty per V stage, then per S buffer (2):
 // scores complete, P written, P.V done; and Q landed
-constexpr int kBarKFull = 0, kBarKEmpty = kBarKFull + kFaKStages, kBarVFull = kBarKEmpty + kFaKStages,
-              kBarVEmpty = kBarVFull + kFaVStages, kBarSFull = kBarVEmpty + kFaVStages,
-              kBarPFull = kBarSFull + 2, kBarPvDone = kBarPFull + 2, kBarQFull = kBarPvDone + 2,
-              kFaBars = kBarQFull + 1;
+__host__ __device__ constexpr int fa_bars(bool shared) { return 2 * (fa_k_stages(shared) + fa_v_stages(shared)) + 7; }
 
 // Two 32-bit values at once (sm_100's packed single-precision pipe): the softmax warps are short
 // of issue slots, and the scale-and-shift before each exponential and the running sums are half
@@ -74,18 +73,35 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
 // row sees the keys of its own chunk of positions only.
 constexpr float kBoundedCap = 40.f * 1.4426950408889634f;
 
-template <int D, bool CAP>
-__global__ void __launch_bounds__(kFaThreads, 2)
+// KEEP: with a window, the first `keep_first` positions of a sequence stay visible (their pages come before the
+// window's), and a head's result is multiplied by the sigmoid of `gate` [token, head], if there is one.
+// SHARED (D = 256): one row a token serves as key and as value (attention through a latent) - a page is fetched
+// once, K-major for the scores and MN-major for P.V as it lies, and only the first `v_cols` values are wanted of
+// the result.  Q (64 KB), four pages (128 KB) and 384 columns of tensor memory leave room for one block an SM; the
+// group may be any number of heads up to 128 (rows past the last whole token stay unused).
+// Measured against the mma.sync kernel that took these prompts before: three of 2,500, 965 and 755 tokens under a
+// window of 1,024 with 4 kept, 16 heads of 128 on 8, gated: 215 -> 42 us; one of 2,048 tokens, 16 heads on rows of 256
+// (192 wanted): 216 -> 40 us (850 TFLOP/s of its 34 GFLOP).
+template <int D, bool CAP, bool KEEP, bool SHARED>
+__global__ void __launch_bounds__(kFaThreads, SHARED ? 1 : 2)
 attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUtensorMap map_q,
                             const int4* __restrict__ tiles,
                             const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const int* block_table,
                             int table_stride, int n_kv_heads, int n_q_heads, float scale_log2,
                             int window, int tok_per_tile, int* status, float sink_log2,
-                            const float* __restrict__ sinks, int chunk, SoftCap cap) {
+                            const float* __restrict__ sinks, int chunk, SoftCap cap, int keep_first,
+                            const bf16* __restrict__ gate, int gate_stride, int v_cols) {
+  constexpr int kFaKStages = fa_k_stages(SHARED), kFaVStages = fa_v_stages(SHARED);
+  constexpr int kBarKFull = 0, kBarKEmpty = kBarKFull + kFaKStages, kBarVFull = kBarKEmpty + kFaKStages,
+                kBarVEmpty = kBarVFull + kFaVStages, kBarSFull = kBarVEmpty + kFaVStages,
+                kBarPFull = kBarSFull + 2, kBarPvDone = kBarPFull + 2, kBarQFull = kBarPvDone + 2,
+                kFaBars = fa_bars(SHARED);
+  static_assert(kBarQFull + 1 == kFaBars, "all barriers");
+  const int cols = SHARED ? v_cols : D;            // of O
   constexpr int DB = D / 64;                       // 64-wide blocks of the head dimension
   constexpr uint32_t kSub = kFaKeys * 128;         // one [64 x 64] bfloat16 sub-tile: 8 KB
-  constexpr uint32_t kTmemCols = 256;
+  constexpr uint32_t kTmemCols = SHARED ? 512 : 256;
   constexpr uint32_t kColS = 0, kColO = 128;        // S buffers at 0 and 64, O at 128
   // No static shared memory in this kernel, so the dynamic part starts at the block's first
   // shared byte, which is 1024-byte aligned as the 128-byte swizzle needs; the kernel checks it.
@@ -100,7 +116,9 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
   const int kv_head = blockIdx.x;             // heads fastest: blocks start longest key range first
   const int group = n_q_heads / n_kv_heads;
 
-  pdl_launch_dependents();
+  // (SHARED: not before the tensor memory is ours - a block of the next kernel that took part of it meanwhile would
+  // wait for this one)
+  if (!SHARED) pdl_launch_dependents();
   // The tile's tokens, position and slot come from a table made once per step (sequence bounds,
   // positions and slots were uploaded before the step's first kernel, and the table is made
   // before its first attention kernel): one 16-byte load instead of a search through the
@@ -124,6 +142,7 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (SHARED) pdl_launch_dependents();
   const int n_rows = n_tok * group;
   const bool misplaced = (smem_u32(smem) & 1023u) != 0;   // never seen; the swizzled tiles would be wrong
   const int pos0 = misplaced ? -1 : tile.z;
@@ -146,7 +165,10 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
   const int hi_tile = pos0 + n_tok - 1;
   const int lo_tile = first_key(pos0, window, chunk);
   const int kt_lo = lo_tile / kFaKeys, kt_hi = hi_tile / kFaKeys;
-  const int n_iter = kt_hi - kt_lo + 1;
+  // pages of kept first keys that the window's pages do not cover: 0 .. n_first - 1
+  const int n_first = KEEP && keep_first > 0 ? min((keep_first + kFaKeys - 1) / kFaKeys, kt_lo) : 0;
+  const int n_iter = n_first + kt_hi - kt_lo + 1;
+  auto page_of = [&](int it) { return KEEP && it < n_first ? it : kt_lo + it - n_first; };
   pdl_wait();                                      // Q and the newest keys and values: the kernel ahead
 
   bool ok = true;
@@ -154,26 +176,30 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
     // ------------------------------------------------------------------- TMA producer
     // Rows of Q past this tile's tokens are the next sequence's or zeros (past the last token);
     // they make rows of S and O that nobody stores.
-    mbar_expect_tx(bar(kBarQFull), DB * 2 * kSub);
+    mbar_expect_tx(bar(kBarQFull), SHARED ? DB * 128u * group * tok_per_tile : DB * 2 * kSub);
 #pragma unroll
     for (int j = 0; j < DB; ++j)
       tma_load_3d(smem_u32(q_s + j * 2 * kSub), &map_q, 64 * j, kv_head * group, t_first, bar(kBarQFull));
     for (int it = 0; it < n_iter; ++it) {
-      const int ks = it % kFaKStages, vs = it % kFaVStages;
-      const uint32_t k_phase = (it / kFaKStages) & 1, v_phase = (it / kFaVStages) & 1;
-      const int row = (table[kt_lo + it] * n_kv_heads + kv_head) * kFaKeys;
+      const int ks = it % kFaKStages;
+      const uint32_t k_phase = (it / kFaKStages) & 1;
+      const int row = (table[page_of(it)] * n_kv_heads + kv_head) * kFaKeys;
       ok = mbar_wait(bar(kBarKEmpty + ks), k_phase ^ 1, status, 11);
       if (!ok) break;
       mbar_expect_tx(bar(kBarKFull + ks), DB * kSub);
 #pragma unroll
       for (int j = 0; j < DB; ++j)
         tma_load_2d(smem_u32(k_s + (ks * DB + j) * kSub), &map_k, 64 * j, row, bar(kBarKFull + ks));
-      ok = mbar_wait(bar(kBarVEmpty + vs), v_phase ^ 1, status, 12);
-      if (!ok) break;
-      mbar_expect_tx(bar(kBarVFull + vs), DB * kSub);
+      if (!SHARED) {
+        constexpr int stages = SHARED ? 1 : kFaVStages;
+        const int vs = it % stages;
+        ok = mbar_wait(bar(kBarVEmpty + vs), ((it / stages) & 1) ^ 1, status, 12);
+        if (!ok) break;
+        mbar_expect_tx(bar(kBarVFull + vs), DB * kSub);
 #pragma unroll
-      for (int j = 0; j < DB; ++j)
-        tma_load_2d(smem_u32(v_s + (vs * DB + j) * kSub), &map_v, 64 * j, row, bar(kBarVFull + vs));
+        for (int j = 0; j < DB; ++j)
+          tma_load_2d(smem_u32(v_s + (vs * DB + j) * kSub), &map_v, 64 * j, row, bar(kBarVFull + vs));
+      }
     }
   } else if (tid == 160) {
     // ------------------------------------------------------------------- issuer of S = Q.K^T
@@ -200,26 +226,28 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
           tc_mma(tmem_base + kColS + 64 * s, dq + (uint64_t)(2 * k), dk + (uint64_t)(2 * k), idesc_s,
                  (j | k) ? 1u : 0u);
       }
-      tc_commit(bar(kBarKEmpty + ks));             // the K stage is free when these are done
+      if (!SHARED) tc_commit(bar(kBarKEmpty + ks));   // the K stage is free when these are done
       tc_commit(bar(kBarSFull + s));               // S is complete
     }
   } else if (tid == 192) {
     // ------------------------------------------------------------------- issuer of O += P.V
-    constexpr uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
-                                  ((uint32_t)(D >> 3) << 17) | ((uint32_t)(kFaRows >> 4) << 24);
+    const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
+                              ((uint32_t)(cols >> 3) << 17) | ((uint32_t)(kFaRows >> 4) << 24);
     for (int u = 0; u < n_iter; ++u) {
       const int s = u & 1;
-      const int vs = u % kFaVStages;
+      constexpr int stages = SHARED ? kFaKStages : kFaVStages;
+      const int vs = u % stages;
       ok = mbar_wait(bar(kBarPFull + s), (u >> 1) & 1, status, 23);   // P written (O rescaled)
-      if (ok) ok = mbar_wait(bar(kBarVFull + vs), (u / kFaVStages) & 1, status, 24);   // V landed
+      // V landed (SHARED: its scores have been computed from it)
+      if (!SHARED && ok) ok = mbar_wait(bar(kBarVFull + vs), (u / stages) & 1, status, 24);
       if (!ok) break;
       tc_fence_after();
-      const uint64_t dv = smem_desc_mn_sw128(smem_u32(v_s + vs * DB * kSub), kSub, 1024);
+      const uint64_t dv = smem_desc_mn_sw128(smem_u32((SHARED ? k_s : v_s) + vs * DB * kSub), kSub, 1024);
 #pragma unroll
       for (int k = 0; k < 4; ++k)                  // 16 keys a step: 8 columns of P,
         tc_mma_ts(tmem_base + kColO, tmem_base + kColS + 64 * s + 8 * k, dv + (uint64_t)(128 * k),
                   idesc_pv, (u | k) ? 1u : 0u);    // 16 rows (2048 bytes) down V
-      tc_commit(bar(kBarVEmpty + vs));             // the V stage is free
+      tc_commit(bar((SHARED ? kBarKEmpty : kBarVEmpty) + vs));   // the stage is free
       tc_commit(bar(kBarPvDone + s));              // O holds pages 0..u
     }
   }
@@ -236,7 +264,7 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
     for (int it = 0; it < n_iter && ok; ++it) {
       const int s = it & 1;
       const uint32_t phase = (it >> 1) & 1;
-      const int key0 = (kt_lo + it) * kFaKeys;
+      const int key0 = page_of(it) * kFaKeys;
       ok = mbar_wait(bar(kBarSFull + s), phase, status, 31);
       if (!ok) break;
       tc_fence_after();
@@ -244,16 +272,15 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
       // two blocks of 7 warps an SM set: first the maximum (keys 32..63 are only looked at,
       // keys 0..31 stay in registers), then the exponentials of keys 0..31, their P, and the
       // same for keys 32..63, read from TMEM once more.
-      const bool full = key0 + kFaKeys - 1 <= pos_r && key0 >= first_r;
+      const bool full = key0 + kFaKeys - 1 <= pos_r && (key0 >= first_r || (KEEP && key0 + kFaKeys <= keep_first));
+      auto sees = [&](int key) { return key <= pos_r && (key >= first_r || (KEEP && key < keep_first)); };
       auto load_half = [&](int h, float* v) {      // scores of keys key0 + 32 h .., masked
         tmem_ld32_nowait(lane_addr + kColS + 64 * s + 32 * h, v);
         tmem_ld_wait();
         if (!full) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            const int key = key0 + 32 * h + i;
-            const bool seen = key <= pos_r && key >= first_r;
-            v[i] = seen ? v[i] : -INFINITY;
+            v[i] = sees(key0 + 32 * h + i) ? v[i] : -INFINITY;
           }
         }
       };
@@ -282,6 +309,7 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
         tc_fence_after();
 #pragma unroll
         for (int c = 0; c < D; c += 32) {
+          if (SHARED && c >= cols) break;
           float v[32];
           tmem_ld32_nowait(lane_addr + kColO + c, v);
           tmem_ld_wait();
@@ -320,8 +348,8 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
           float2 p = make_float2(ex2_approx(a.x), ex2_approx(a.y));
           if (CAP && !full) {
             const int key = key0 + 32 * h + i;
-            p.x = key <= pos_r && key >= first_r ? p.x : 0.f;
-            p.y = key + 1 <= pos_r && key + 1 >= first_r ? p.y : 0.f;
+            p.x = sees(key) ? p.x : 0.f;
+            p.y = sees(key + 1) ? p.y : 0.f;
           }
           psum[(i >> 1) & 1] = add2(psum[(i >> 1) & 1], p);
           __nv_bfloat162 hh = __floats2bfloat162_rn(p.x, p.y);
@@ -347,20 +375,25 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
     if (tid < kFaRows) {                           // whole warps: tcgen05.ld is warp-wide
       // a sink: one more term exp(sink) in the denominator, with no value (-inf: none)
       // (`sinks`: one score per query head instead of the same for all)
-      const float sk = sinks ? sinks[kv_head * group + r % group] * 1.4426950408889634f : sink_log2;
+      const float sk = sinks ? sinks[kv_head * group + min(r, n_rows - 1) % group] * 1.4426950408889634f : sink_log2;
       if (sk > -INFINITY && l_run > 0.f) l_run += exp2f(sk - m_ref);
-      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+      float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       const bool wide_out = ((uintptr_t)out & 31) == 0;     // rows of D values are then 32-byte aligned
       const int row = min(r, n_rows - 1);
       bf16* o = out + ((size_t)(t_first + row / group) * n_q_heads + kv_head * group + row % group) * D;
+      if (KEEP && gate != nullptr)
+        inv *= 1.f / (1.f + expf(-__bfloat162float(
+            gate[(size_t)(t_first + row / group) * gate_stride + kv_head * group + row % group])));
 #pragma unroll
       for (int c = 0; c < D; c += 32) {
+        if (SHARED && c >= cols) break;
         float v[32];
         tmem_ld32_nowait(lane_addr + kColO + c, v);
         tmem_ld_wait();
         if (r < n_rows) {
 #pragma unroll
           for (int j = 0; j < 32; j += 16) {     // 32 bytes a store: whole sectors of L2, a row a lane
+            if (SHARED && c + j >= cols) break;
             uint32_t w[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -473,12 +506,13 @@ attention_prefill_tiles_kernel(int4* tiles, int max_tiles, const int* cu_seqlens
   for (int i = total + tid; i < max_tiles; i += kFaTileThreads) tiles[i] = make_int4(0, 0, -1, 0);
 }
 
-template <int D, bool CAP>
+template <int D, bool CAP, bool KEEP, bool SHARED>
 static int launch_fa(bf16* out, const bf16* q, int q_row_stride, const int4* tiles, int n_tiles, int n_tokens,
                      const void* k_pages, const void* v_pages, long long page_rows,
                      const int* block_table, int table_stride, int n_q_heads, int n_kv_heads,
                      float scale, int window, int* status, float sink, const float* sinks, int chunk,
-                     float softcap, cudaStream_t stream) {
+                     float softcap, int keep_first, const bf16* gate, int gate_stride, int v_cols,
+                     cudaStream_t stream) {
   const int group = n_q_heads / n_kv_heads;
   const int tok_per_tile = kFaRows / group;
   CUtensorMap mq, mk, mv;
@@ -487,8 +521,9 @@ static int launch_fa(bf16* out, const bf16* q, int q_row_stride, const int4* til
   if ((rc = tensor_map(k_pages, page_rows, D, D, kFaKeys, &mk))) return rc;
   if ((rc = tensor_map(v_pages, page_rows, D, D, kFaKeys, &mv))) return rc;
   constexpr int DB = D / 64;
-  constexpr size_t smem = (size_t)(2 * DB + (kFaKStages + kFaVStages) * DB) * kFaKeys * 128 + kFaBars * 8 + 16;
-  auto kernel = attention_prefill_tc_kernel<D, CAP>;
+  constexpr size_t smem = (size_t)(2 * DB + (fa_k_stages(SHARED) + fa_v_stages(SHARED)) * DB) * kFaKeys * 128 +
+                          fa_bars(SHARED) * 8 + 16;
+  auto kernel = attention_prefill_tc_kernel<D, CAP, KEEP, SHARED>;
   static bool configured[kMaxDevices] = {};
   int device = 0;
   cudaError_t e = cudaGetDevice(&device);
@@ -505,7 +540,7 @@ static int launch_fa(bf16* out, const bf16* q, int q_row_stride, const int4* til
   return (int)launch_pdl(kernel, grid, dim3(kFaThreads), smem, stream, out, mq, tiles, mk, mv, block_table,
                          table_stride, n_kv_heads, n_q_heads, scale * 1.4426950408889634f,
                          window, tok_per_tile, status, sink * 1.4426950408889634f, sinks, chunk,
-                         soft_cap(scale, softcap));
+                         soft_cap(scale, softcap), keep_first, gate, gate_stride, v_cols);
 }
 
 }  // namespace ek
@@ -530,31 +565,47 @@ EK_EXPORT int ek_attention_prefill_tiles(int* tiles, int max_tiles, const int* c
 // `tiles` / n_tiles: the table ek_attention_prefill_tiles made for this step and group size.
 // `sink`: score of a key without a value that every query also sees (one more term in the softmax
 // denominator); -INFINITY for none.  `chunk` > 0 instead of a window: keys of a token's own chunk only.
-// `softcap` > 0: scores become softcap tanh(score / softcap).
+// `softcap` > 0: scores become softcap tanh(score / softcap).  `keep_first` > 0 (with a window): the sequence's first
+// positions stay visible; `gate` (may be null): one value per token and query head, whose sigmoid multiplies the
+// head's result.  head_dim 256 with one KV head: attention over rows that are keys and values alike (v_pages is
+// k_pages), any group up to 128, and only the first `v_cols` values (rounded up to 16) of every head are written.
 EK_EXPORT int ek_attention_prefill_tc(void* out, const void* q, int q_row_stride, const int* tiles,
                                       int n_tiles, int n_tokens,
                                       const void* k_pages, const void* v_pages, int n_pages,
                                       const int* block_table, int table_stride, int n_q_heads,
                                       int n_kv_heads, int head_dim, float scale, int window,
                                       int* status, float sink, const float* sinks, int chunk,
-                                      float softcap, cudaStream_t stream) {
+                                      float softcap, int keep_first, const void* gate, int gate_stride, int v_cols,
+                                      cudaStream_t stream) {
   using namespace ek;
   if (n_tokens <= 0 || n_tiles <= 0) return 0;
-  if (chunk < 0 || (chunk > 0 && window > 0)) return EK_ERR_ARG;
-  if ((head_dim != 64 && head_dim != 128) || n_kv_heads <= 0 || n_q_heads % n_kv_heads ||
-      kFaRows % (n_q_heads / n_kv_heads) || q_row_stride % 8 || ((uintptr_t)q & 15) || !status ||
-      !(scale > 0.f) || n_pages <= 0 || !tiles || ((uintptr_t)tiles & 15))
+  if (chunk < 0 || (chunk > 0 && (window > 0 || keep_first > 0)) || keep_first < 0) return EK_ERR_ARG;
+  const bool shared = head_dim == 256;
+  if ((head_dim != 64 && head_dim != 128 && !shared) || n_kv_heads <= 0 || n_q_heads % n_kv_heads ||
+      n_q_heads / n_kv_heads > kFaRows || (!shared && kFaRows % (n_q_heads / n_kv_heads)) || q_row_stride % 8 ||
+      ((uintptr_t)q & 15) || !status || !(scale > 0.f) || n_pages <= 0 || !tiles || ((uintptr_t)tiles & 15) ||
+      (shared && (n_kv_heads != 1 || v_pages != k_pages || v_cols <= 0 || v_cols > head_dim || softcap > 0.f)))
     return EK_ERR_ARG;
   const long long page_rows = (long long)n_pages * n_kv_heads * EK_PAGE;
-#define EK_FA(D_, CAP_)                                                                                  \
-  return launch_fa<D_, CAP_>((bf16*)out, (const bf16*)q, q_row_stride, (const int4*)tiles, n_tiles,       \
+  if (window <= 0) keep_first = 0;
+  const bool keep = keep_first > 0 || gate != nullptr;
+  v_cols = (v_cols + 15) / 16 * 16;
+#define EK_FA(D_, CAP_, KEEP_, SHARED_)                                                                  \
+  return launch_fa<D_, CAP_, KEEP_, SHARED_>((bf16*)out, (const bf16*)q, q_row_stride, (const int4*)tiles, n_tiles, \
                              n_tokens, k_pages, v_pages, page_rows, block_table, table_stride, n_q_heads, \
-                             n_kv_heads, scale, window, status, sink, sinks, chunk, softcap, stream)
-  if (head_dim == 64) {
-    if (softcap > 0.f) EK_FA(64, true);
-    EK_FA(64, false);
+                             n_kv_heads, scale, window, status, sink, sinks, chunk, softcap, keep_first, \
+                             (const bf16*)gate, gate_stride, v_cols, stream)
+  if (shared) {
+    if (keep) EK_FA(256, false, true, true);
+    EK_FA(256, false, false, true);
   }
-  if (softcap > 0.f) EK_FA(128, true);
-  EK_FA(128, false);
+  if (head_dim == 64) {
+    if (softcap > 0.f) { if (keep) EK_FA(64, true, true, false); EK_FA(64, true, false, false); }
+    if (keep) EK_FA(64, false, true, false);
+    EK_FA(64, false, false, false);
+  }
+  if (softcap > 0.f) { if (keep) EK_FA(128, true, true, false); EK_FA(128, true, false, false); }
+  if (keep) EK_FA(128, false, true, false);
+  EK_FA(128, false, false, false);
 #undef EK_FA
 }

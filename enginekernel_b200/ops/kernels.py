@@ -916,7 +916,7 @@ def attention_prefill_f32(out, q, n_tokens, positions, token_slot, cu_seqlens, n
 
 _attn_prefill_tc = Function("attention_prefill_tc", "ek_attention_prefill_tc",
                             [_P, _P, c_int, _P, c_int, c_int, _P, _P, c_int, _P, c_int, c_int,
-                             c_int, c_int, c_float, c_int, _P, c_float, _P, c_int, c_float, _P])
+                             c_int, c_int, c_float, c_int, _P, c_float, _P, c_int, c_float, c_int, _P, c_int, c_int, _P])
 _attn_prefill_tiles = Function("attention_prefill_tc", "ek_attention_prefill_tiles",
                                [_P, c_int, _P, _P, _P, c_int, c_int, c_int, _P])
 _attn_prefill_cross = Function("attention_prefill_bf16", "ek_attention_prefill_cross_bf16",
@@ -946,6 +946,11 @@ PREFILL_TC_MAX_SEQS = 1024
 def attention_prefill_tc_supported(dtype, head_dim, n_q_heads, n_kv_heads):
     group = n_q_heads // n_kv_heads
     return dtype == torch.bfloat16 and head_dim in (64, 128) and 128 % group == 0
+
+
+def attention_prefill_shared_supported(dtype, row, n_q_heads):
+    """Rows that are keys and values alike (attention through a latent): 256 values, up to 128 heads on one."""
+    return dtype == torch.bfloat16 and row == 256 and n_q_heads <= PREFILL_TC_ROWS
 
 
 _l2_bytes = {}
@@ -986,15 +991,23 @@ def attention_prefill_tiles(tiles, n_tokens, positions, token_slot, cu_seqlens, 
 
 def attention_prefill_tc(out, q, n_tokens, positions, token_slot, cu_seqlens, n_seqs, k_pages,
                          v_pages, block_table, n_q_heads, n_kv_heads, head_dim, scale, window=None,
-                         tiles=None, n_tiles=0, sink=None, chunk=None, softcap=None, sinks=None):
+                         tiles=None, n_tiles=0, sink=None, chunk=None, softcap=None, sinks=None, keep_first=0, gate=None,
+                         v_cols=None):
     """:func:`attention_prefill_bf16` on tcgen05 tensor cores (head sizes 64 and 128, groups
-    that divide 128): TMA-fed pages, scores and P.V in TMEM.  ``tiles`` / ``n_tiles``: the table
+    that divide 128): TMA-fed pages, scores and P.V in TMEM.  With ``v_cols``, rows of 256 values that are keys and
+    values alike (``v_pages`` is ``k_pages``, one KV head, up to 128 query heads): only the first ``v_cols`` values of a
+    head's result are written.  ``tiles`` / ``n_tiles``: the table
     :func:`attention_prefill_tiles` made for this step (made once, before the step's first
     kernel, and used by every layer); without it the table is made here and the stream is
     waited for, which suits a single call, not a model's step."""
     _need_cuda(out, q, positions, token_slot, cu_seqlens, k_pages, v_pages, block_table, tiles)
-    _need(attention_prefill_tc_supported(q.dtype, head_dim, n_q_heads, n_kv_heads),
-          "attention_prefill_tc: bfloat16, head size 64 or 128, a group size that divides 128")
+    if v_cols is not None:
+        _need(attention_prefill_shared_supported(q.dtype, head_dim, n_q_heads) and n_kv_heads == 1
+              and v_pages.data_ptr() == k_pages.data_ptr() and 0 < v_cols <= head_dim and not softcap,
+              "attention_prefill_tc: shared rows are 256 bfloat16 values of one KV head, without a soft cap")
+    else:
+        _need(attention_prefill_tc_supported(q.dtype, head_dim, n_q_heads, n_kv_heads),
+              "attention_prefill_tc: bfloat16, head size 64 or 128, a group size that divides 128")
     _need(out.dtype == q.dtype == k_pages.dtype, "attention: one dtype for q, cache and out")
     _need(out.is_contiguous() and out.shape[-1] == n_q_heads * head_dim, "attention: out [T, NQ*D]")
     _need(q.stride(-1) == 1 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0,
@@ -1014,7 +1027,8 @@ def attention_prefill_tc(out, q, n_tokens, positions, token_slot, cu_seqlens, n_
                      _ptr(v_pages), k_pages.shape[0], _ptr(block_table), block_table.stride(0), n_q_heads,
                      n_kv_heads, head_dim, float(scale), int(window or 0),
                      _ptr(tc_status(q.device)), _sink(sink), _sinks(sinks, n_q_heads), int(chunk or 0),
-                     float(softcap or 0.0), _stream())
+                     float(softcap or 0.0), int(keep_first or 0), *_gate_args(gate, q, n_q_heads), int(v_cols or 0),
+                     _stream())
 
 
 # ------------------------------------------------------------------ matrix products

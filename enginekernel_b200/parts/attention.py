@@ -49,8 +49,8 @@ Optional parameters, all off by default, for designs that differ there:
                        all its key heads (``q_norm`` [NH*D], ``k_norm`` [NKV*D]) instead of one per head.
 ``sinks``              True: a learned sink score per query head (tensor ``sink`` [NH]) instead of one constant.
 ``value_dim``, ``unit_norm_after_rotation``, ``keep_first`` and ``head_gate`` send the layer down one path: a single
-product for everything that reads the input, a prepare kernel that knows padded heads, and the ``mma.sync`` or the
-general attention kernel.  The others ride on the ordinary path.
+product for everything that reads the input, a prepare kernel that knows padded heads, and the attention kernel that
+takes the padded head size (tcgen05 for prompts of 64 and 128, ``mma.sync``, or the general one).  The others ride on the ordinary path.
 """
 
 from __future__ import annotations
@@ -66,6 +66,24 @@ from .spec import CacheSpec, TensorSpec
 
 FUSE_ROPE_ROWS = 64       # the q/k/v product does norm, rotation and cache write itself up to here
 WIDE_CLUSTER_PAGES = 64     # clusters of more than 8 key splits only from this many pages of context
+
+
+def make_prefill_tiles(ctx, key, num_heads, num_kv_heads, head_dim):
+    """The table of tiles of the tcgen05 prompt attention, once per step and shape of the heads (``ctx.shared[key]``)."""
+    if key in ctx.shared:
+        return
+    per_tile = kernels.PREFILL_TC_ROWS // (num_heads // num_kv_heads)
+    rows = -(-ctx.n_tokens // per_tile) + ctx.n_seqs
+    tiles = ctx.workspace.get(f"prefill_tc_tiles_{key[1]}_{key[2]}", (rows, 4), torch.int32)
+    n = kernels.attention_prefill_tiles(tiles, ctx.n_tokens, ctx.positions, ctx.token_slot, ctx.cu_seqlens,
+                                        ctx.n_seqs, num_heads, num_kv_heads, head_dim)
+    ctx.shared[key] = (tiles, n)
+
+
+def prefill_tiles(ctx, key):
+    """The table made for this step as arguments of the kernel (a part driven alone has none)."""
+    made = ctx.shared.get(key)
+    return {} if made is None else dict(tiles=made[0], n_tiles=made[1])
 
 
 @register_part("mixer", "attention")
@@ -187,23 +205,17 @@ class Attention(Mixer):
             self.position.prepare(max_positions)
 
     def _tiles_key(self):
-        return ("prefill_tc_tiles", self.num_heads // self.num_kv_heads, self.num_kv_heads * self.head_dim)
+        return ("prefill_tc_tiles", self.num_heads // self.num_kv_heads, self.num_kv_heads * self.padded_dim)
+
+    def _on_prefill_tc(self, ctx):
+        """Whether a prompt of this step runs on the tcgen05 kernel."""
+        return (not ctx.is_decode and ctx.n_seqs <= kernels.PREFILL_TC_MAX_SEQS and self.scale > 0
+                and kernels.attention_prefill_tc_supported(self.dtype, self.padded_dim, self.num_heads, self.num_kv_heads))
 
     def begin_step(self, ctx):
         """The table of tiles of the tcgen05 prompt attention, once per step and shape of the heads."""
-        if self.general or ctx.is_decode or ctx.n_seqs > kernels.PREFILL_TC_MAX_SEQS or not self.scale > 0 or \
-                not kernels.attention_prefill_tc_supported(self.dtype, self.head_dim, self.num_heads,
-                                                           self.num_kv_heads):
-            return
-        key = self._tiles_key()
-        if key in ctx.shared:
-            return
-        per_tile = kernels.PREFILL_TC_ROWS // (self.num_heads // self.num_kv_heads)
-        rows = -(-ctx.n_tokens // per_tile) + ctx.n_seqs
-        tiles = ctx.workspace.get(f"prefill_tc_tiles_{key[1]}_{key[2]}", (rows, 4), torch.int32)
-        n = kernels.attention_prefill_tiles(tiles, ctx.n_tokens, ctx.positions, ctx.token_slot, ctx.cu_seqlens,
-                                            ctx.n_seqs, self.num_heads, self.num_kv_heads, self.head_dim)
-        ctx.shared[key] = (tiles, n)
+        if self._on_prefill_tc(ctx):
+            make_prefill_tiles(ctx, self._tiles_key(), self.num_heads, self.num_kv_heads, self.padded_dim)
 
     def _by_head(self, t, n, reorder):
         """[n * size, ...] -> [n * padded_dim, ...]: a head's values in the kernels' order (``reorder``: they turn
@@ -283,6 +295,12 @@ class Attention(Mixer):
         visible = self._visible(ctx)
         gate = rows[:, gate_col:] if self.head_gate else None
         mask = {"chunk": self.chunk, "softcap": self.softcap, "sinks": self.sinks}
+        if self._on_prefill_tc(ctx):
+            kernels.attention_prefill_tc(out, rows, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
+                                         entry.k_pages, entry.v_pages, entry.block_table, nh, nkv, big, self.scale,
+                                         self.window, keep_first=self.keep_first, gate=gate, **mask,
+                                         **prefill_tiles(ctx, self._tiles_key()))
+            return self._project(out, ctx, None, leave_bias)
         if not ctx.is_decode and kernels.attention_prefill_supported(self.dtype, big, nh, nkv):
             kernels.attention_prefill_bf16(out, rows, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
                                            entry.k_pages, entry.v_pages, entry.block_table, nh, nkv, big, self.scale,
@@ -475,16 +493,9 @@ class Attention(Mixer):
         fast_decode = ctx.is_decode and kernels.attention_decode_supported(self.dtype, self.head_dim)
         if not ctx.is_decode and kernels.attention_prefill_supported(
                 self.dtype, self.head_dim, self.num_heads, self.num_kv_heads):
-            prefill = kernels.attention_prefill_bf16
-            if ctx.n_seqs <= kernels.PREFILL_TC_MAX_SEQS and self.scale > 0 and \
-                    kernels.attention_prefill_tc_supported(self.dtype, self.head_dim, self.num_heads,
-                                                           self.num_kv_heads):
-                prefill = kernels.attention_prefill_tc      # tcgen05: head sizes 64 and 128
-            extra = {}
-            if prefill is kernels.attention_prefill_tc:
-                made = ctx.shared.get(self._tiles_key())
-                if made is not None:                 # (made in begin_step; a part driven alone has none)
-                    extra = dict(tiles=made[0], n_tiles=made[1])
+            prefill, extra = kernels.attention_prefill_bf16, {}
+            if self._on_prefill_tc(ctx):
+                prefill, extra = kernels.attention_prefill_tc, prefill_tiles(ctx, self._tiles_key())   # tcgen05
             prefill(
                 out, qkv, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
                 entry.k_pages, entry.v_pages, entry.block_table, self.num_heads, self.num_kv_heads,

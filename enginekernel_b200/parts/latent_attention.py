@@ -16,8 +16,8 @@ with zeros to the row length D that the attention kernels take, and attention ru
 form: the query of head h becomes [W_uk,h^T q_h,flat ; rot(q_h,rot)] (D values), all H heads read
 the same cached rows as keys AND as values, and W_uv,h is applied to the first c values of each
 head's result.  That is grouped-query attention with one key head, so the framework's attention
-kernels run it (with a sink score per head): the mma.sync kernels for rows of up to 256 values, the
-general kernel beyond (up to 1,024).
+kernels run it (with a sink score per head): for rows of 256 values the tcgen05 prompt kernel, which fetches a row
+once for both uses, the mma.sync kernels for the others up to 256, the general kernel beyond (up to 1,024).
 
 Parameters: ``hidden_size``, ``num_heads``, ``head_dim`` (d), ``rot_dim`` (r), ``v_dim`` (e),
 ``q_rank`` (a), ``kv_rank`` (c), ``scale``, ``eps``, ``position`` (a rotary PartSpec over ``rot_dim``
@@ -43,6 +43,7 @@ import torch
 from ..ops import kernels
 from ..ops.linear import linear
 from ..registry import lookup_part, register_part
+from .attention import make_prefill_tiles, prefill_tiles
 from .base import Mixer
 from .rope import neighbours_to_halves
 from .spec import CacheSpec, TensorSpec
@@ -109,6 +110,17 @@ class LatentAttention(Mixer):
     def prepare(self, max_positions):
         if self.position is not None:
             self.position.prepare(max_positions)
+
+    def _on_prefill_tc(self, ctx):
+        return (not ctx.is_decode and ctx.n_seqs <= kernels.PREFILL_TC_MAX_SEQS and self.scale > 0
+                and kernels.attention_prefill_shared_supported(self.dtype, self.row, self.num_heads))
+
+    def _tiles_key(self):
+        return ("prefill_tc_tiles", self.num_heads, self.row)
+
+    def begin_step(self, ctx):
+        if self._on_prefill_tc(ctx):
+            make_prefill_tiles(ctx, self._tiles_key(), self.num_heads, 1, self.row)
 
     def load(self, tensors):
         w = self.spec.weights
@@ -184,6 +196,11 @@ class LatentAttention(Mixer):
         pages, table = entry.k_pages, entry.block_table
         common = dict(sinks=self.sinks, gate=gate)
         visible = min(ctx.max_context, self.window) if self.window else ctx.max_context
+        if self._on_prefill_tc(ctx):
+            kernels.attention_prefill_tc(out, q, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
+                                         pages, pages, table, nh, 1, row, self.scale, self.window, v_cols=self.kv_rank,
+                                         **common, **prefill_tiles(ctx, self._tiles_key()))
+            return
         if not ctx.is_decode and kernels.attention_prefill_supported(self.dtype, row, nh, 1):
             kernels.attention_prefill_bf16(out, q, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
                                            pages, pages, table, nh, 1, row, self.scale, self.window, **common)

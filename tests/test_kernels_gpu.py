@@ -980,3 +980,84 @@ def test_attention_prefill_f32(nq, nkv, d, options):
     k.attention_generic(want, q, t, pos, slots, *place(), **kw)
     k.attention_prefill_f32(got, q, t, pos, slots, cu, len(new), *place(), **kw)
     assert torch.equal(got.isnan(), want.isnan()) and want.isnan().any() and not want[:65 + 30].isnan().any()
+
+
+def _prompt_rows(lens, first):
+    pos = [p for n, p0 in zip(lens, first) for p in range(p0, p0 + n)]
+    slot = [s for s, n in enumerate(lens) for _ in range(n)]
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    as_dev = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    return as_dev(pos), as_dev(slot), as_dev(cu)
+
+
+@pytest.mark.parametrize("nq,nkv,d", [(4, 2, 64), (16, 8, 128), (8, 8, 128), (32, 1, 64)])
+@pytest.mark.parametrize("window,keep,softcap", [(9, 3, None), (64, 64, None), (70, 5, 4.0), (130, 200, None), (1, 1, None),
+                                                 (None, 0, None)])
+def test_attention_prefill_tc_keeps_first_tokens_and_gates(nq, nkv, d, window, keep, softcap):
+    """The tcgen05 prompt kernel beside the mma.sync one: a window with kept first tokens (their pages apart from the
+    window's, touching it, covered by it, more of them than the window), a gate per head, per-head sinks; prompts and
+    portions behind earlier keys.  Both round P and the result to bfloat16 (2^-9 each) around 32-bit sums: 2^-7 of the
+    largest value.  One key that fits every query decides the result exactly where the rule sees it."""
+    k = K()
+    new, past = [1, 70, 300, 128], [0, 200, 0, 130]
+    t, dtype = sum(new), torch.bfloat16
+    pages = Pages(len(new), 300, nkv, d, dtype, seed=3)
+    for s in range(len(new)):
+        n = new[s] + past[s]
+        pages.fill(s, rnd(n, nkv, d, dtype=dtype, seed=10 + s), rnd(n, nkv, d, dtype=dtype, seed=20 + s))
+    q = rnd(t, nq * d + 8 * nq, dtype=dtype, seed=30)
+    pos, slots, cu = _prompt_rows(new, past)
+    args = (q, t, pos, slots, cu, len(new))
+    place = (pages.k, pages.v, pages.table, nq, nkv, d, d ** -0.5, window)
+    kw = dict(keep_first=keep, gate=q[:, nq * d:], softcap=softcap, sinks=rnd(nq, seed=5))
+    want, got = (torch.full((t, nq * d), 7.0, dtype=dtype, device=DEV) for _ in range(2))
+    k.attention_prefill_bf16(want, *args, *place, **kw)
+    k.attention_prefill_tc(got, *args, *place, **kw)
+    k.check_tc_status(DEV)
+    assert rel(got, want) <= 2 ** -7
+    if window is None or softcap:
+        return
+    last, row = 299, 1 + 70 + 299
+    q2 = torch.zeros_like(q)
+    q2[:, :nq * d].view(t, nq, d)[:, :, 0] = 30.0
+    for j in sorted({0, keep - 1, keep, last - window, last - window + 1, 63, 64, last} & set(range(300))):
+        saved = pages.k[:, :, :, 0].clone()
+        pages.k[:, :, :, 0] = 0
+        pages.k[int(pages.table[2, j // 64]), :, j % 64, 0] = 30.0
+        k.attention_prefill_tc(got, q2, *args[1:], *place, keep_first=keep)
+        value = pages.v[int(pages.table[2, j // 64]), :, j % 64].repeat_interleave(nq // nkv, 0)
+        seen = last - j < window or j < keep
+        assert (rel(got[row].view(nq, d), value) <= 2e-2) == seen, (j, seen)
+        pages.k[:, :, :, 0] = saved
+
+
+@pytest.mark.parametrize("heads", [1, 16, 20, 128])
+@pytest.mark.parametrize("v_cols,window", [(192, None), (256, 100), (16, None), (200, 1)])
+def test_attention_prefill_tc_over_rows_that_are_keys_and_values(heads, v_cols, window):
+    """Rows of 256 values read once for both uses, beside the mma.sync kernel that reads them twice: groups that do and
+    do not divide 128, prompts and portions; the same bound as above.  Only the wanted values are written."""
+    k = K()
+    new, past = [1, 70, 200, 129], [0, 200, 0, 63]
+    t, dtype = sum(new), torch.bfloat16
+    pages = Pages(len(new), 300, 1, 256, dtype, seed=3)
+    for s in range(len(new)):
+        n = new[s] + past[s]
+        rows = rnd(n, 1, 256, dtype=dtype, seed=10 + s)
+        pages.fill(s, rows, rows)
+    q = rnd(t, heads * 256, dtype=dtype, seed=30)
+    pos, slots, cu = _prompt_rows(new, past)
+    args = (q, t, pos, slots, cu, len(new))
+    place = (pages.k, pages.k, pages.table, heads, 1, 256, 256 ** -0.5, window)
+    gate = rnd(t, heads, dtype=dtype, seed=6)
+    want, got = (torch.full((t, heads * 256), 7.0, dtype=dtype, device=DEV) for _ in range(2))
+    for kw in (dict(sinks=rnd(heads, seed=5)), dict(gate=gate)):
+        k.attention_prefill_bf16(want, *args, *place, **kw)
+        got.fill_(7.0)
+        k.attention_prefill_tc(got, *args, *place, v_cols=v_cols, **kw)
+        k.check_tc_status(DEV)
+        written = -(-v_cols // 16) * 16
+        g, w = got.view(t, heads, 256), want.view(t, heads, 256)
+        assert rel(g[..., :v_cols], w[..., :v_cols]) <= 2 ** -7
+        assert (g[..., written:] == 7.0).all()
