@@ -86,6 +86,80 @@ conv_silu_kernel(float* __restrict__ out, int out_stride, const float* __restric
   }
 }
 
+// The same for many tokens: a thread takes four neighbouring channels (V = 4; one where rows are not whole 16-byte
+// pieces) of 8 (kConvTile) neighbouring tokens, so that an input is fetched once for all its taps - 11 loads for 8 tokens
+// of 4 taps, all of them before the first use - and the taps stay in registers.  Bound by memory (3,824 tokens of 6,144
+// channels, 188 MB in and out: 150 us with a token's taps fetched one by one, 67 so).
+constexpr int kConvTile = 8;
+template <int K, int V>
+__global__ void __launch_bounds__(128)
+conv_silu_tile_kernel(float* __restrict__ out, int out_stride, const float* __restrict__ proj, int proj_stride, int col0,
+                      const float* __restrict__ conv_w, const float* __restrict__ conv_b,
+                      const float* __restrict__ state, size_t slot_stride, size_t tail_offset,
+                      const int* __restrict__ positions, const int* __restrict__ token_slot, int n_tokens, int channels,
+                      const float* __restrict__ in_bias, int act) {
+  __shared__ int n_prev_s[kConvTile], slot_s[kConvTile], pos_s[kConvTile];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t0 = blockIdx.x * kConvTile, nt = min(kConvTile, n_tokens - t0);
+  if ((int)threadIdx.x < nt) {
+    const int t = t0 + threadIdx.x, pos = positions[t];
+    n_prev_s[threadIdx.x] = pos >= 0 ? step_predecessors(positions, token_slot, t, K - 1) : -1;
+    slot_s[threadIdx.x] = pos >= 0 ? token_slot[t] : 0;
+    pos_s[threadIdx.x] = pos;
+  }
+  __syncthreads();
+  const int c = (blockIdx.y * 128 + threadIdx.x) * V;
+  if (c >= channels) return;
+  auto fetch = [](float (&to)[V], const float* from) {
+    if (V == 4) *reinterpret_cast<float4*>(to) = *reinterpret_cast<const float4*>(from);
+    else to[0] = *from;
+  };
+  float x[kConvTile + K - 1][V], w[V][K], bias[V], xb[V];
+#pragma unroll
+  for (int i = 0; i < kConvTile + K - 1; ++i) {            // rows t0 - (K - 1) ..
+    const int t = t0 + i - (K - 1);
+    if (t >= 0 && t < n_tokens) fetch(x[i], proj + (size_t)t * proj_stride + col0 + c);
+    else
+#pragma unroll
+      for (int v = 0; v < V; ++v) x[i][v] = 0.f;
+  }
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    bias[v] = conv_b ? conv_b[c + v] : 0.f;
+    xb[v] = in_bias ? in_bias[c + v] : 0.f;                // of the projection itself: only real tokens carry it
+#pragma unroll
+    for (int j = 0; j < K; ++j) w[v][j] = conv_w[(size_t)(c + v) * K + j];
+  }
+#pragma unroll
+  for (int i = 0; i < kConvTile; ++i) {
+    if (i >= nt) break;
+    const int n_prev = n_prev_s[i];
+    if (n_prev < 0) continue;
+    float y[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      float acc = bias[v] + w[v][K - 1] * (x[i + K - 1][v] + xb[v]);
+      if (n_prev == K - 1) {
+#pragma unroll
+        for (int j = 1; j < K; ++j) acc = fmaf(w[v][K - 1 - j], x[i + K - 1 - j][v] + xb[v], acc);
+      } else {                                             // the sequence's first tokens of the step
+        const float* tail = state + (size_t)slot_s[i] * slot_stride + tail_offset + (size_t)(c + v) * (K - 1);
+#pragma unroll
+        for (int j = 1; j < K; ++j) {
+          float z = j <= n_prev ? x[i + K - 1 - j][v] : tail[n_prev - j + K - 1];
+          if (pos_s[i] - j >= 0) z += xb[v];
+          acc = fmaf(w[v][K - 1 - j], z, acc);
+        }
+      }
+      y[v] = act ? acc * sigmoid_f(acc) : acc;
+    }
+    float* to = out + (size_t)(t0 + i) * out_stride + c;
+    if (V == 4) *reinterpret_cast<float4*>(to) = *reinterpret_cast<const float4*>(y);
+    else *to = y[0];
+  }
+}
+
 // grid (sequences, channel tiles).  After the step the tail holds the sequence's last taps-1 inputs.
 __global__ void conv_tail_kernel(float* __restrict__ state, size_t slot_stride, size_t tail_offset,
                                  const float* __restrict__ proj, int proj_stride, int col0,
@@ -710,13 +784,49 @@ __global__ void __launch_bounds__(1024)
 ssm_out_kernel(T* __restrict__ y, const float* __restrict__ o, const float* __restrict__ x, int x_stride,
                const float* __restrict__ proj, int proj_stride, int col_z, const float* __restrict__ d_skip,
                const float* __restrict__ w, float eps, const int* __restrict__ positions, int inner, int vdim,
-               int parts) {
+               int parts, int vec) {
   __shared__ float scratch[33];
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x, part = blockIdx.y;
   if (positions[t] < 0) return;
   const int size = inner / parts, c0 = part * size;
+  if (vec) {                                     // four neighbours a thread, everything fetched before the sum
+    constexpr int kKeep4 = kOutKeep / 4;
+    float4 u[kKeep4], x4[kKeep4], z4[kKeep4];
+    float ss = 0.f;
+#pragma unroll
+    for (int m = 0; m < kKeep4; ++m) {
+      const int i = (threadIdx.x + m * blockDim.x) * 4, c = c0 + i;
+      u[m] = x4[m] = z4[m] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < size) {
+        u[m] = *reinterpret_cast<const float4*>(o + (size_t)t * inner + c);
+        x4[m] = *reinterpret_cast<const float4*>(x + (size_t)t * x_stride + c);
+        z4[m] = *reinterpret_cast<const float4*>(proj + (size_t)t * proj_stride + col_z + c);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < kKeep4; ++m) {
+      const int i = (threadIdx.x + m * blockDim.x) * 4, c = c0 + i;
+      if (i >= size) continue;
+      const float d = d_skip[c / vdim];          // (vdim is a multiple of 4)
+      u[m].x = (u[m].x + d * x4[m].x) * (z4[m].x * sigmoid_f(z4[m].x));
+      u[m].y = (u[m].y + d * x4[m].y) * (z4[m].y * sigmoid_f(z4[m].y));
+      u[m].z = (u[m].z + d * x4[m].z) * (z4[m].z * sigmoid_f(z4[m].z));
+      u[m].w = (u[m].w + d * x4[m].w) * (z4[m].w * sigmoid_f(z4[m].w));
+      ss += u[m].x * u[m].x + u[m].y * u[m].y + u[m].z * u[m].z + u[m].w * u[m].w;
+    }
+    const float rstd = rsqrtf(block_sum(ss, scratch) / (float)size + eps);
+#pragma unroll
+    for (int m = 0; m < kKeep4; ++m) {
+      const int i = (threadIdx.x + m * blockDim.x) * 4, c = c0 + i;
+      if (i >= size) continue;
+      const float4 w4 = *reinterpret_cast<const float4*>(w + c);
+      Vec4<T>::store(y + (size_t)t * inner + c, make_float4(u[m].x * rstd * w4.x, u[m].y * rstd * w4.y,
+                                                            u[m].z * rstd * w4.z, u[m].w * rstd * w4.w));
+    }
+    return;
+  }
   auto value = [&](int c) {
     const float z = proj[(size_t)t * proj_stride + col_z + c];
     return (o[(size_t)t * inner + c] + d_skip[c / vdim] * x[(size_t)t * x_stride + c]) * (z * sigmoid_f(z));
@@ -792,18 +902,45 @@ xlstm_out_kernel(T* __restrict__ y, const float* __restrict__ o, const float* __
 
 }  // namespace ek
 
+namespace ek {
+
+static int launch_conv(float* out, int out_stride, const float* proj, int proj_stride, int col0, const float* conv_w,
+                       const float* conv_b, const float* in_bias, int act, const float* state, long long slot_stride,
+                       long long tail_offset, const int* positions, const int* token_slot, int n_tokens, int channels,
+                       int taps, cudaStream_t stream) {
+  // tiles of tokens from where they give every SM four blocks on; more taps than 4 take the other kernel
+  const bool four = channels % 4 == 0 && out_stride % 4 == 0 && proj_stride % 4 == 0 && col0 % 4 == 0 &&
+                    (((uintptr_t)out | (uintptr_t)proj) & 15) == 0;
+  const int wide = four ? 512 : 128, columns = (channels + wide - 1) / wide;
+  if (taps >= 2 && taps <= 4 && columns <= 65535 && (long long)(n_tokens / kConvTile) * columns >= 4 * sm_count()) {
+    const dim3 grid((n_tokens + kConvTile - 1) / kConvTile, columns);
+#define EK_CONV(K_)                                                                                                  \
+  return (int)launch_pdl(four ? conv_silu_tile_kernel<K_, 4> : conv_silu_tile_kernel<K_, 1>, grid, dim3(128), 0, stream, \
+                         out, out_stride, proj, proj_stride, col0, conv_w, conv_b, state, (size_t)slot_stride,       \
+                         (size_t)tail_offset, positions, token_slot, n_tokens, channels, in_bias, act)
+    if (taps == 2) EK_CONV(2);
+    if (taps == 3) EK_CONV(3);
+    EK_CONV(4);
+#undef EK_CONV
+  }
+  const int tiles = (channels + 255) / 256;
+  const int per_block = n_tokens >= 2048 ? kConvTokens : n_tokens >= 256 ? 4 : 1;
+  return (int)launch_pdl(conv_silu_kernel, dim3((n_tokens + per_block - 1) / per_block, tiles < 65535 ? tiles : 65535),
+                         dim3(256), 0, stream, out, out_stride, proj, proj_stride, col0, conv_w, conv_b, state,
+                         (size_t)slot_stride, (size_t)tail_offset, positions, token_slot, n_tokens, channels,
+                         taps, per_block, in_bias, act);
+}
+
+}  // namespace ek
+
 EK_EXPORT int ek_conv_silu(float* out, int out_stride, const float* proj, int proj_stride, int col0,
                            const float* conv_w, const float* conv_b, const float* state, long long slot_stride,
                            long long tail_offset, const int* positions, const int* token_slot, int n_tokens,
                            int channels, int taps, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (channels <= 0 || taps < 1) return EK_ERR_ARG;
-  const int tiles = (channels + 255) / 256;
-  const int per_block = n_tokens >= 2048 ? ek::kConvTokens : n_tokens >= 256 ? 4 : 1;
-  return (int)ek::launch_pdl(ek::conv_silu_kernel, dim3((n_tokens + per_block - 1) / per_block, tiles < 65535 ? tiles : 65535),
-                             dim3(256), 0, stream, out, out_stride, proj, proj_stride, col0, conv_w, conv_b, state,
-                             (size_t)slot_stride, (size_t)tail_offset, positions, token_slot, n_tokens, channels,
-                             taps, per_block, (const float*)nullptr, 1);
+  return ek::launch_conv(out, out_stride, proj, proj_stride, col0, conv_w, conv_b, nullptr, 1, state, slot_stride, tail_offset,
+                         positions, token_slot, n_tokens, channels, taps, stream);
 }
 
 // The same convolution with two options: `in_bias` [channels] is added to every input that belongs to a
@@ -814,12 +951,8 @@ EK_EXPORT int ek_conv_act(float* out, int out_stride, const float* proj, int pro
                           const int* token_slot, int n_tokens, int channels, int taps, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (channels <= 0 || taps < 1) return EK_ERR_ARG;
-  const int tiles = (channels + 255) / 256;
-  const int per_block = n_tokens >= 2048 ? ek::kConvTokens : n_tokens >= 256 ? 4 : 1;
-  return (int)ek::launch_pdl(ek::conv_silu_kernel, dim3((n_tokens + per_block - 1) / per_block, tiles < 65535 ? tiles : 65535),
-                             dim3(256), 0, stream, out, out_stride, proj, proj_stride, col0, conv_w, conv_b, state,
-                             (size_t)slot_stride, (size_t)tail_offset, positions, token_slot, n_tokens, channels,
-                             taps, per_block, in_bias, act);
+  return ek::launch_conv(out, out_stride, proj, proj_stride, col0, conv_w, conv_b, in_bias, act, state, slot_stride, tail_offset,
+                         positions, token_slot, n_tokens, channels, taps, stream);
 }
 
 // Both gates of the gated linear recurrence and what enters it: a[t, c] and x[t, c] (see lru_gates_kernel).
@@ -1135,9 +1268,13 @@ EK_EXPORT int ek_rotate_heads(float* x, int stride, int col0, int heads, int dim
       return EK_ERR_ARG;                                                                                       \
     const int size = inner / parts; /* a thread takes up to four channels of a part */                         \
     const int threads = size >= 4096 ? 1024 : size <= 256 ? 64 : (size / 4 + 31) / 32 * 32;                    \
+    /* (3,824 tokens of 4,096 channels in 8 parts: 82 us one by one, 51 four neighbours a thread) */    \
+    const int vec = size % 4 == 0 && vdim % 4 == 0 && x_stride % 4 == 0 && proj_stride % 4 == 0 &&             \
+                    col_z % 4 == 0 && size <= threads * ek::kOutKeep && ((uintptr_t)y & (4 * sizeof(T) - 1)) == 0 && \
+                    (((uintptr_t)o | (uintptr_t)x | (uintptr_t)proj | (uintptr_t)w) & 15) == 0;                \
     return (int)ek::launch_pdl(ek::ssm_out_kernel<T>, dim3(n_tokens, parts), dim3(threads), 0, stream, (T*)y,  \
                                o, x, x_stride, proj, proj_stride, col_z, d_skip, w, eps, positions, inner,     \
-                               vdim, parts);                                                                   \
+                               vdim, parts, vec);                                                              \
   }                                                                                                            \
   EK_EXPORT int ek_norm_gate_out_##SUFFIX(void* y, const float* o, const float* proj, int proj_stride, int col_g, \
                                           const float* w, float eps, const int* positions, int n_tokens,       \

@@ -148,3 +148,53 @@ def test_low_rank_halves_of_many_tokens(channels, rank, tokens):
     k.delta_low_rank(out, proj, tokens, 5, w, bias=bias, a_log=a_log, dim=-(-channels // 4))
     rate = torch.exp(a_log.double())[torch.arange(channels, device=DEV) // -(-channels // 4)]
     assert (out.double() - torch.exp(-rate * torch.nn.functional.softplus(z + bias.double()))).abs().max() <= 4e-6
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("channels,col0,in_bias,act", [(1024, 0, False, True), (1027, 3, True, False), (516, 8, True, True)])
+def test_convolution_of_many_tokens_with_biases(channels, col0, in_bias, act, taps):
+    """Tiles of eight tokens, four channels a thread and one, over sequences of 1, 2, 1,300, 3 and 1,900 tokens, some behind
+    earlier inputs, some finished: the plain formulas to a few 32-bit roundings of sums of five terms."""
+    k = K()
+    lens, first = [1, 2, 1300, 3, 1900], [0, 5, 0, 1, 7]
+    t = sum(lens)
+    g = torch.Generator().manual_seed(taps)
+    proj = torch.randn(t, channels + col0 + 4 - (channels + col0) % 4, generator=g).to(DEV)
+    w, b, xb = (torch.randn(*s, generator=g).to(DEV) for s in ((channels, taps), (channels,), (channels,)))
+    state = torch.randn(5, 16 + channels * (taps - 1), generator=g).to(DEV)
+    pos = [p for n, p0 in zip(lens, first) for p in range(p0, p0 + n)]
+    slot = [s for s, n in enumerate(lens) for _ in range(n)]
+    pos[-4:] = [-1] * 4
+    out = torch.full((t, channels), 7.0, device=DEV)
+    k.conv_act(out, proj, col0, w, b, state, 16, i32(pos), i32(slot), t, channels, taps, in_bias=xb if in_bias else None,
+               activation="silu" if act else None)
+    cu = 0
+    for s, n in enumerate(lens):
+        live = n - 4 if s == len(lens) - 1 else n
+        x = torch.cat([state[s, 16:].view(channels, taps - 1).t(), proj[cu:cu + n, col0:col0 + channels]]).double()
+        if in_bias:                              # inputs before position 0 do not belong to a token
+            x[max(0, taps - 1 - first[s]):] += xb.double()
+        y = sum(x[j:j + n] * w[:, j].double() for j in range(taps)) + b.double()
+        y = y * torch.sigmoid(y) if act else y
+        assert rel(out[cu:cu + live], y[:live]) <= 2e-6
+        assert torch.equal(out[cu + live:cu + n], torch.full_like(out[cu + live:cu + n], 7.0))
+        cu += n
+
+
+@pytest.mark.parametrize("inner,vdim,parts", [(512, 64, 1), (520, 20, 2), (768, 4, 1), (96, 32, 3)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_state_space_output_norm(inner, vdim, parts, offset):
+    """Four channels a thread, and one by one where the gate's column is not on a 16-byte boundary: 32-bit results to a few
+    roundings."""
+    k = K()
+    t = 40
+    g = torch.Generator().manual_seed(inner)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    o, x, proj, d, w = rnd(t, inner), rnd(t, inner + 8), rnd(t, inner + 12), rnd(inner // vdim), rnd(inner)
+    y = torch.empty(t, inner, device=DEV)
+    k.ssm_out(y, o, x, proj, offset, d, w, 1e-5, i32(list(range(t))), t, inner, vdim, parts)
+    z = proj[:, offset:offset + inner].double()
+    u = (o.double() + d.double().repeat_interleave(vdim) * x[:, :inner].double()) * z * torch.sigmoid(z)
+    p = u.view(t, parts, -1)
+    want = (p * torch.rsqrt((p * p).mean(-1, keepdim=True) + 1e-5)).reshape(t, inner) * w.double()
+    assert rel(y, want) <= 2e-6
