@@ -1,5 +1,6 @@
 // Decode attention in bfloat16 with the cache pages streamed by TMA (head sizes 64 and 128,
-// up to 16 query heads a KV head).
+// up to 16 query heads a KV head; and rows of 256 values that are keys and values alike, which is
+// attention through a latent, any number of query heads in blocks of 16).
 //
 // One new token per sequence against its paged cache; the work is reading the sequence's keys
 // and values once.  A block owns (token, KV head, split): a whole number of cache pages (64 keys
@@ -28,14 +29,19 @@
 
 namespace ek {
 
-constexpr int kDtWarps = 4;                  // consumer warps
-constexpr int kDtThreads = (kDtWarps + 1) * 32;
+constexpr int kDtWarps = 4;                  // consumer warps of a page: 16 keys each
+// Rows of 256: two such sets of warps take the pages in turn.  One page is a serial chain of 64 matrix
+// instructions a warp, 0.93 us with one set; the queries' fragments, 64 registers, come from shared memory instead.
+template <int D>
+constexpr int kDtSets = D == 256 ? 2 : 1;
+template <int D>
+constexpr int kDtThreads = (kDtSets<D> * kDtWarps + 1) * 32;
 constexpr int kDtPortableSplits = 8;         // blocks of a cluster: the portable limit
 constexpr int kDtMaxSplits = 16;             // and the limit with the attribute for larger ones
 // floats a block can be sent by its cluster: every (head, dimension) pair once (dealt in runs of
-// ceil(pairs / splits), so up to one more a split), and (max, sum) of 16 heads from 16 splits
+// pairs / splits rounded up, by rows of 256 to whole fours: up to four more a split), and (max, sum) of 16 heads from 16 splits
 template <int D>
-constexpr int kDtRecvO = 16 * D + kDtMaxSplits;
+constexpr int kDtRecvO = 16 * D + (D == 256 ? 4 : 1) * kDtMaxSplits;
 constexpr int kDtRecvMl = kDtMaxSplits * 16 * 2;
 
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2,
@@ -61,47 +67,74 @@ __device__ __forceinline__ uint32_t pack2_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// grid (splits, kv heads, tokens); cluster (splits, 1, 1) when splits > 1
-template <int D, int STAGES>
-__global__ void __launch_bounds__(kDtThreads)
-attention_decode_tma_kernel(bf16* __restrict__ out, const bf16* q, int q_row_stride,
-                            const int* positions, const int* token_slot,
-                            const __grid_constant__ CUtensorMap map_k,
-                            const __grid_constant__ CUtensorMap map_v, const int* block_table,
-                            int table_stride, int n_kv_heads, int n_q_heads, float scale_log2,
-                            int window, int* status, float sink_log2, const float* __restrict__ sinks, int chunk,
-                            SoftCap cap) {
+// grid (splits, kv heads, tokens); cluster (splits, 1, 1) when splits > 1.  SHARED: the value rows
+// are the key rows, a stage holds them once, and grid.y counts blocks of 16 query heads of a KV head.
+// What bounds it is the latency of one block's pages, not the bytes: 8 tokens of 16 heads behind
+// 2,048 rows of 256 read 8 MB (1.3 us) and took the register kernel and its merge 24.8 us in a graph
+// (rows by plain loads, two or three rounds of them a warp, partial results through global memory); now 12.2.  A block
+// alone takes 0.86 us a page of 64 rows.
+template <int D, int STAGES, bool SHARED>
+__device__ __forceinline__ void
+attention_decode_tma_block(bf16* __restrict__ out, const bf16* q, int q_row_stride,
+                           const int* positions, const int* token_slot, const CUtensorMap& map_k,
+                           const CUtensorMap& map_v, const int* block_table,
+                           int table_stride, int n_kv_heads, int n_q_heads, float scale_log2,
+                           int window, int* status, float sink_log2, const float* __restrict__ sinks, int chunk,
+                           SoftCap cap, const bf16* __restrict__ gate, int gate_stride) {
   constexpr int DB = D / 64;                       // 64-wide (128-byte) blocks of the head dimension
   constexpr uint32_t kSub = EK_PAGE * 128;         // one [64 keys x 64 dims] sub-tile: 8 KB
-  constexpr uint32_t kStage = 2 * DB * kSub;       // K tile + V tile
+  constexpr uint32_t kStage = (SHARED ? 1 : 2) * DB * kSub;    // K tile (+ V tile)
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + STAGES * kStage);        // full[STAGES], empty[STAGES]
   // after the last page the ring is dead and holds, from its start: the warps' accumulators
-  // [4][16][OS] and their (max, sum) [4][16][2].
+  // [W][16][OS], their (max, sum) [W][16][2], the factors of the merge [W][16], and the heads' (max, sum).
   // A row of the accumulators is OS = D + 8 floats long, so that the rows a warp stores at once
   // (one per group of four lanes) lie on different banks.
   constexpr int OS = D + 8;
   float* o_s = (float*)smem;
-  float* ml_s = o_s + kDtWarps * 16 * OS;
-  static_assert((size_t)(kDtWarps * 16 * (OS + 2)) * 4 <= (size_t)STAGES * kStage,
+  constexpr int SETS = kDtSets<D>, W = SETS * kDtWarps, THREADS = kDtThreads<D>;
+  float* ml_s = o_s + W * 16 * OS;
+  float* factor_s = ml_s + W * 16 * 2;
+  float* head_s = factor_s + W * 16;
+  static_assert((size_t)(W * 16 * (OS + 3) + 32) * 4 <= (size_t)STAGES * kStage,
                 "merge buffers must fit the ring");
   // what the other blocks of the cluster send: [split][run] results, [split][head][2] (max, sum)
   float* recv_o = (float*)(bars + 2 * STAGES);
   float* recv_ml = recv_o + kDtRecvO<D>;
+  unsigned char* q_s = (unsigned char*)(recv_ml + kDtRecvMl);    // SHARED: [16 heads][D], 16-byte pieces swizzled
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
   const int split = blockIdx.x, n_splits = gridDim.x;
-  const int kv_head = blockIdx.y, t = blockIdx.z;
-  const int group = n_q_heads / n_kv_heads;
-  const int head0 = kv_head * group;
+  const int t = blockIdx.z;
+  const int heads = n_q_heads / n_kv_heads;                    // query heads of a KV head
+  const int row_blocks = SHARED ? (heads + 15) / 16 : 1;
+  const int kv_head = SHARED ? blockIdx.y / row_blocks : blockIdx.y;
+  const int row0 = SHARED ? 16 * (blockIdx.y % row_blocks) : 0;
+  const int group = SHARED ? min(16, heads - row0) : heads;
+  const int head0 = kv_head * heads + row0;
 
   pdl_launch_dependents();
-  if (tid == kDtWarps * 32) {
+  if (tid == W * 32) {
     tma_prefetch_map(&map_k);
-    tma_prefetch_map(&map_v);
+    if (!SHARED) tma_prefetch_map(&map_v);
   }
-  // Read before the wait: positions, slots and block tables must have been written by work that
+  const uint32_t bar0 = smem_u32(bars);
+  auto full = [&](int s) { return bar0 + 8u * s; };
+  auto empty = [&](int s) { return bar0 + 8u * (STAGES + s); };
+  auto init_barriers = [&] {
+    if (tid != 0) return;
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full(s), 1);
+      mbar_init(empty(s), kDtWarps);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  };
+  if constexpr (SHARED) {                        // (few pages a block: nothing is read ahead of the wait)
+    init_barriers();
+    pdl_wait();
+  }
+  // Otherwise read before the wait: positions, slots and block tables must have been written by work that
   // a plain (not programmatic) launch separates from this kernel.  A step's first kernel, the
   // embedding lookup, is such a launch, so the state advance of the step before is complete and
   // visible here, in a captured graph and in eager decoding alike.
@@ -118,16 +151,7 @@ attention_decode_tma_kernel(bf16* __restrict__ out, const bf16* q, int q_row_str
   const int n_pages = pg_last - pg_first + 1;                  // <= 0: nothing for this split
   const int new_page = pos >= 0 ? pos / EK_PAGE : -1;          // holds the key written just now
 
-  const uint32_t bar0 = smem_u32(bars);
-  auto full = [&](int s) { return bar0 + 8u * s; };
-  auto empty = [&](int s) { return bar0 + 8u * (STAGES + s); };
-  if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full(s), 1);
-      mbar_init(empty(s), kDtWarps);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
+  if constexpr (!SHARED) init_barriers();
   __syncthreads();
 
   bool ok = true;
@@ -136,10 +160,10 @@ attention_decode_tma_kernel(bf16* __restrict__ out, const bf16* q, int q_row_str
   for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};   // rows g and g + 8
 
-  if (tid == kDtWarps * 32) {
+  if (tid == W * 32) {
     // ------------------------------------------------------------------- TMA producer
     const int* table = block_table + (size_t)(pos >= 0 ? token_slot[t] : 0) * table_stride;
-    bool waited = false;
+    bool waited = SHARED;
     const uint64_t stream_policy = l2_policy_evict_first();   // a page is read once a step
     for (int i = 0; i < n_pages; ++i) {
       const int s = i % STAGES;
@@ -158,45 +182,60 @@ attention_decode_tma_kernel(bf16* __restrict__ out, const bf16* q, int q_row_str
 #pragma unroll
       for (int j = 0; j < DB; ++j) {
         tma_load_2d_hint(dst + j * kSub, &map_k, 64 * j, row, full(s), stream_policy);
-        tma_load_2d_hint(dst + (DB + j) * kSub, &map_v, 64 * j, row, full(s), stream_policy);
+        if (!SHARED) tma_load_2d_hint(dst + (DB + j) * kSub, &map_v, 64 * j, row, full(s), stream_policy);
       }
     }
-  } else if (warp < kDtWarps) {
+  } else if (warp < W) {
     // ------------------------------------------------------------------- consumers
     pdl_wait();                                  // the queries come from the kernel before
     if (n_pages > 0) {
       // Q fragments of m16n8k16 for every 16-wide step of the head dimension: rows g and g + 8
-      uint32_t qa[D / 16][4];
+      uint32_t qa[SHARED ? 1 : D / 16][4];
       const bf16* qrow = q + (size_t)t * q_row_stride + (size_t)head0 * D;
+      const int set = warp / kDtWarps, set_warp = warp % kDtWarps;
+      uint32_t q_addr = 0;
+      const int q_row = (lane & 7) + 8 * ((lane >> 3) & 1);
+      if constexpr (SHARED) {
+        for (int idx = tid; idx < 16 * (D / 8); idx += W * 32) {
+          const int r = idx / (D / 8), c = idx % (D / 8);
+          const uint4 v = r < group ? *reinterpret_cast<const uint4*>(qrow + (size_t)r * D + 8 * c) : make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(q_s + r * (2 * D) + ((c ^ (r & 7)) << 4)) = v;
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(W * 32) : "memory");
+        q_addr = smem_u32(q_s) + q_row * (2 * D);
+      } else {
 #pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks) {
-        const int d0 = 16 * ks + 2 * tq;
-        qa[ks][0] = g < group ? *reinterpret_cast<const uint32_t*>(qrow + (size_t)g * D + d0) : 0u;
-        qa[ks][1] = g + 8 < group ? *reinterpret_cast<const uint32_t*>(qrow + (size_t)(g + 8) * D + d0) : 0u;
-        qa[ks][2] = g < group ? *reinterpret_cast<const uint32_t*>(qrow + (size_t)g * D + d0 + 8) : 0u;
-        qa[ks][3] = g + 8 < group ? *reinterpret_cast<const uint32_t*>(qrow + (size_t)(g + 8) * D + d0 + 8) : 0u;
+        for (int ks = 0; ks < D / 16; ++ks) {
+          const int d0 = 16 * ks + 2 * tq;
+          qa[ks][0] = g < group ? *reinterpret_cast<const uint32_t*>(qrow + (size_t)g * D + d0) : 0u;
+          qa[ks][1] = g + 8 < group ? *reinterpret_cast<const uint32_t*>(qrow + (size_t)(g + 8) * D + d0) : 0u;
+          qa[ks][2] = g < group ? *reinterpret_cast<const uint32_t*>(qrow + (size_t)g * D + d0 + 8) : 0u;
+          qa[ks][3] = g + 8 < group ? *reinterpret_cast<const uint32_t*>(qrow + (size_t)(g + 8) * D + d0 + 8) : 0u;
+        }
       }
       // this lane's row and 16-byte column inside a [64 x 64] sub-tile for the two ldmatrix forms
-      const int k_row = 16 * warp + (lane & 7) + 8 * (lane >> 4), k_half = (lane >> 3) & 1;
-      const int v_row = 16 * warp + (lane & 7) + 8 * ((lane >> 3) & 1), v_half = lane >> 4;
-      for (int i = 0; i < n_pages; ++i) {
+      const int k_row = 16 * set_warp + (lane & 7) + 8 * (lane >> 4), k_half = (lane >> 3) & 1;
+      const int v_row = 16 * set_warp + (lane & 7) + 8 * ((lane >> 3) & 1), v_half = lane >> 4;
+      for (int i = set; i < n_pages; i += SETS) {
         const int s = i % STAGES;
         ok = mbar_wait(full(s), (i / STAGES) & 1, status, 42);
         if (!ok) break;
-        const int key0 = (pg_first + i) * EK_PAGE + 16 * warp;
+        const int key0 = (pg_first + i) * EK_PAGE + 16 * set_warp;
         if (key0 <= hi && key0 + 15 >= lo) {     // else none of this warp's 16 keys is visible
-          const uint32_t k_s = smem_u32(smem + s * kStage), v_s = k_s + DB * kSub;
+          const uint32_t k_s = smem_u32(smem + s * kStage), v_s = SHARED ? k_s : k_s + DB * kSub;
           float sc[2][4];
-          sc[0][0] = sc[0][1] = sc[0][2] = sc[0][3] = 0.f;
-          sc[1][0] = sc[1][1] = sc[1][2] = sc[1][3] = 0.f;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sc[0][e] = sc[1][e] = 0.f;
 #pragma unroll
           for (int ks = 0; ks < D / 16; ++ks) {
             const int chunk = 2 * ks + k_half;               // 16-byte column of the head dimension
             uint32_t b0, b1, b2, b3;
             ldsm_x4(k_s + (chunk >> 3) * kSub + k_row * 128 + (((chunk & 7) ^ (k_row & 7)) << 4), b0, b1,
                     b2, b3);
-            mma_bf16_16816(sc[0], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
-            mma_bf16_16816(sc[1], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b2, b3);
+            uint32_t* a = qa[SHARED ? 0 : ks];
+            if constexpr (SHARED) ldsm_x4(q_addr + (((2 * ks + (lane >> 4)) ^ (q_row & 7)) << 4), a[0], a[1], a[2], a[3]);
+            mma_bf16_16816(sc[0], a[0], a[1], a[2], a[3], b0, b1);
+            mma_bf16_16816(sc[1], a[0], a[1], a[2], a[3], b2, b3);
           }
           // sc[j][0..1]: row g, keys key0 + 8j + 2tq + {0,1}; sc[j][2..3]: row g + 8, same keys
           float mx[2] = {-INFINITY, -INFINITY};
@@ -254,7 +293,7 @@ attention_decode_tma_kernel(bf16* __restrict__ out, const bf16* q, int q_row_str
 
   // ------------------------------------------------------------ the warps' results, merged
   const int failed = __syncthreads_or(ok ? 0 : 1);  // every page consumed: the ring is dead
-  if (!failed && warp < kDtWarps) {
+  if (!failed && warp < W) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
@@ -284,37 +323,93 @@ attention_decode_tma_kernel(bf16* __restrict__ out, const bf16* q, int q_row_str
     }
   }
   __syncthreads();
+  // four results of a head with the sum l; a gated head's output is multiplied by the sigmoid of its gate
+  auto store4 = [&](bf16* to, float4 o, float l, int head) {
+    const float by = gate == nullptr ? 1.f : 1.f / (1.f + expf(-__bfloat162float(gate[(size_t)t * gate_stride + head])));
+    auto one = [&](float v) { return (l > 0.f ? v / l : 0.f) * by; };
+    *reinterpret_cast<uint2*>(to) = make_uint2(pack2_bf16(one(o.x), one(o.y)), pack2_bf16(one(o.z), one(o.w)));
+  };
   const int pairs = group * D;
-  const int run = (pairs + n_splits - 1) / n_splits;            // pairs a block of the cluster owns
-  if (!failed) {
-    // in warp order; a thread takes (row, dimension) pairs
-    for (int idx = tid; idx < pairs; idx += kDtThreads) {
-      const int r = idx / D, d = idx % D;
-      float m = -INFINITY;
+  const int per_block = (pairs + n_splits - 1) / n_splits;
+  const int run = SHARED ? (per_block + 3) & ~3 : per_block;    // pairs a block of the cluster owns (whole fours)
+  if constexpr (SHARED) {
+    if (!failed && tid < group) {                  // a thread a head: the warps' factors, its maximum and sum
+      float m = -INFINITY, l = 0.f;
 #pragma unroll
-      for (int w = 0; w < kDtWarps; ++w) m = fmaxf(m, ml_s[(w * 16 + r) * 2]);
-      float l = 0.f, o = 0.f;
+      for (int w = 0; w < W; ++w) m = fmaxf(m, ml_s[(w * 16 + tid) * 2]);
 #pragma unroll
-      for (int w = 0; w < kDtWarps; ++w) {
-        const float lw = ml_s[(w * 16 + r) * 2 + 1];
-        if (lw > 0.f) {
-          const float f = exp2f(ml_s[(w * 16 + r) * 2] - m);
-          l += lw * f;
-          o += o_s[((size_t)w * 16 + r) * OS + d] * f;
-        }
+      for (int w = 0; w < W; ++w) {
+        const float lw = ml_s[(w * 16 + tid) * 2 + 1];
+        const float f = lw > 0.f ? exp2f(ml_s[(w * 16 + tid) * 2] - m) : 0.f;
+        factor_s[w * 16 + tid] = f;
+        l += lw > 0.f ? lw * f : 0.f;
       }
       if (n_splits == 1) {
         // a sink: one more term exp(sink) in the denominator, with no value (-inf: none)
-        const float sk = sinks ? sinks[head0 + r] * 1.4426950408889634f : sink_log2;   // per head, if given
+        const float sk = sinks ? sinks[head0 + tid] * 1.4426950408889634f : sink_log2;     // per head, if given
         if (sk > -INFINITY && l > 0.f) l += exp2f(sk - m);
-        out[((size_t)t * n_q_heads + head0 + r) * D + d] = __float2bfloat16_rn(l > 0.f ? o / l : 0.f);
+        head_s[tid] = l;
       } else {
-        const int owner = idx / run;
-        st_cluster_f32(&recv_o[split * run + (idx - owner * run)], (unsigned)owner, o);
-        if (d == 0) {                            // every block needs this head's maximum and sum
-          for (int sp = 0; sp < n_splits; ++sp) {
-            st_cluster_f32(&recv_ml[(split * 16 + r) * 2], (unsigned)sp, m);
-            st_cluster_f32(&recv_ml[(split * 16 + r) * 2 + 1], (unsigned)sp, l);
+        for (int sp = 0; sp < n_splits; ++sp) {    // every block needs this head's maximum and sum
+          st_cluster_f32(&recv_ml[(split * 16 + tid) * 2], (unsigned)sp, m);
+          st_cluster_f32(&recv_ml[(split * 16 + tid) * 2 + 1], (unsigned)sp, l);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (!failed) {
+    if constexpr (SHARED) {
+      // in warp order; a thread takes four (row, dimension) pairs at a time
+      for (int idx = 4 * tid; idx < pairs; idx += 4 * THREADS) {
+        const int r = idx / D, d = idx % D;
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const float f = factor_s[w * 16 + r];
+          if (f > 0.f) {
+            const float4 v = *reinterpret_cast<const float4*>(o_s + ((size_t)w * 16 + r) * OS + d);
+            o.x += v.x * f; o.y += v.y * f; o.z += v.z * f; o.w += v.w * f;
+          }
+        }
+        if (n_splits == 1) {
+          const float l = head_s[r];
+          store4(out + ((size_t)t * n_q_heads + head0 + r) * D + d, o, l, head0 + r);
+        } else {
+          const int owner = idx / run;
+          st_cluster_f32x4(&recv_o[split * run + (idx - owner * run)], (unsigned)owner, o);
+        }
+      }
+    } else {
+      // in warp order; a thread takes (row, dimension) pairs
+      for (int idx = tid; idx < pairs; idx += THREADS) {
+        const int r = idx / D, d = idx % D;
+        float m = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < W; ++w) m = fmaxf(m, ml_s[(w * 16 + r) * 2]);
+        float l = 0.f, o = 0.f;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const float lw = ml_s[(w * 16 + r) * 2 + 1];
+          if (lw > 0.f) {
+            const float f = exp2f(ml_s[(w * 16 + r) * 2] - m);
+            l += lw * f;
+            o += o_s[((size_t)w * 16 + r) * OS + d] * f;
+          }
+        }
+        if (n_splits == 1) {
+          // a sink: one more term exp(sink) in the denominator, with no value (-inf: none)
+          const float sk = sinks ? sinks[head0 + r] * 1.4426950408889634f : sink_log2;   // per head, if given
+          if (sk > -INFINITY && l > 0.f) l += exp2f(sk - m);
+          out[((size_t)t * n_q_heads + head0 + r) * D + d] = __float2bfloat16_rn(l > 0.f ? o / l : 0.f);
+        } else {
+          const int owner = idx / run;
+          st_cluster_f32(&recv_o[split * run + (idx - owner * run)], (unsigned)owner, o);
+          if (d == 0) {                            // every block needs this head's maximum and sum
+            for (int sp = 0; sp < n_splits; ++sp) {
+              st_cluster_f32(&recv_ml[(split * 16 + r) * 2], (unsigned)sp, m);
+              st_cluster_f32(&recv_ml[(split * 16 + r) * 2 + 1], (unsigned)sp, l);
+            }
           }
         }
       }
@@ -327,46 +422,103 @@ attention_decode_tma_kernel(bf16* __restrict__ out, const bf16* q, int q_row_str
   // ------------------------------------------------------------ the splits, merged in order
   cluster_sync();                                // (every block gets here, whatever happened to it)
   if (!failed) {
-    for (int slot = tid; slot < run && split * run + slot < pairs; slot += kDtThreads) {
-      const int idx = split * run + slot;
-      const int r = idx / D;
-      float m = -INFINITY;
-      for (int sp = 0; sp < n_splits; ++sp) m = fmaxf(m, recv_ml[(sp * 16 + r) * 2]);
-      float l = 0.f, o = 0.f;
-      for (int sp = 0; sp < n_splits; ++sp) {
-        const float ls = recv_ml[(sp * 16 + r) * 2 + 1];
-        if (ls > 0.f) {
-          const float f = exp2f(recv_ml[(sp * 16 + r) * 2] - m);
-          l += ls * f;
-          o += recv_o[sp * run + slot] * f;
+    if constexpr (SHARED) {
+      for (int slot = 4 * tid; slot < run && split * run + slot < pairs; slot += 4 * THREADS) {
+        const int idx = split * run + slot;
+        const int r = idx / D;
+        float m = -INFINITY;
+        for (int sp = 0; sp < n_splits; ++sp) m = fmaxf(m, recv_ml[(sp * 16 + r) * 2]);
+        float l = 0.f;
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int sp = 0; sp < n_splits; ++sp) {
+          const float ls = recv_ml[(sp * 16 + r) * 2 + 1];
+          if (ls > 0.f) {
+            const float f = exp2f(recv_ml[(sp * 16 + r) * 2] - m);
+            const float4 v = *reinterpret_cast<const float4*>(recv_o + sp * run + slot);
+            l += ls * f;
+            o.x += v.x * f; o.y += v.y * f; o.z += v.z * f; o.w += v.w * f;
+          }
         }
+        const float sk = sinks ? sinks[head0 + r] * 1.4426950408889634f : sink_log2;
+        if (sk > -INFINITY && l > 0.f) l += exp2f(sk - m);      // the sink, counted once
+        store4(out + ((size_t)t * n_q_heads + head0) * D + idx, o, l, head0 + r);
       }
-      const float sk = sinks ? sinks[head0 + r] * 1.4426950408889634f : sink_log2;
-      if (sk > -INFINITY && l > 0.f) l += exp2f(sk - m);      // the sink, counted once
-      out[((size_t)t * n_q_heads + head0) * D + idx] = __float2bfloat16_rn(l > 0.f ? o / l : 0.f);
+    } else {
+      for (int slot = tid; slot < run && split * run + slot < pairs; slot += THREADS) {
+        const int idx = split * run + slot;
+        const int r = idx / D;
+        float m = -INFINITY;
+        for (int sp = 0; sp < n_splits; ++sp) m = fmaxf(m, recv_ml[(sp * 16 + r) * 2]);
+        float l = 0.f, o = 0.f;
+        for (int sp = 0; sp < n_splits; ++sp) {
+          const float ls = recv_ml[(sp * 16 + r) * 2 + 1];
+          if (ls > 0.f) {
+            const float f = exp2f(recv_ml[(sp * 16 + r) * 2] - m);
+            l += ls * f;
+            o += recv_o[sp * run + slot] * f;
+          }
+        }
+        const float sk = sinks ? sinks[head0 + r] * 1.4426950408889634f : sink_log2;
+        if (sk > -INFINITY && l > 0.f) l += exp2f(sk - m);      // the sink, counted once
+        out[((size_t)t * n_q_heads + head0) * D + idx] = __float2bfloat16_rn(l > 0.f ? o / l : 0.f);
+      }
     }
   }
 }
 
+template <int D, int STAGES>
+__global__ void __launch_bounds__(kDtThreads<D>)
+attention_decode_tma_kernel(bf16* __restrict__ out, const bf16* q, int q_row_stride,
+                            const int* positions, const int* token_slot,
+                            const __grid_constant__ CUtensorMap map_k,
+                            const __grid_constant__ CUtensorMap map_v, const int* block_table,
+                            int table_stride, int n_kv_heads, int n_q_heads, float scale_log2,
+                            int window, int* status, float sink_log2, const float* __restrict__ sinks, int chunk,
+                            SoftCap cap) {
+  attention_decode_tma_block<D, STAGES, false>(out, q, q_row_stride, positions, token_slot, map_k, map_v, block_table,
+                                               table_stride, n_kv_heads, n_q_heads, scale_log2, window, status, sink_log2,
+                                               sinks, chunk, cap, nullptr, 0);
+}
+
+// (a kernel of its own: the gate's two arguments and one map less)
+template <int D, int STAGES>
+__global__ void __launch_bounds__(kDtThreads<D>)
+attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_row_stride,
+                                   const int* positions, const int* token_slot,
+                                   const __grid_constant__ CUtensorMap map, const int* block_table,
+                                   int table_stride, int n_kv_heads, int n_q_heads, float scale_log2,
+                                   int window, int* status, float sink_log2, const float* __restrict__ sinks, int chunk,
+                                   SoftCap cap, const bf16* __restrict__ gate, int gate_stride) {
+  attention_decode_tma_block<D, STAGES, true>(out, q, q_row_stride, positions, token_slot, map, map, block_table,
+                                              table_stride, n_kv_heads, n_q_heads, scale_log2, window, status, sink_log2,
+                                              sinks, chunk, cap, gate, gate_stride);
+}
+
 // DEEP: a ring twice as deep (192 KB, one block an SM) for launches that leave SMs empty anyway, so
-// that more of a block's pages are on their way before the wait returns.
+// that more of a block's pages are on their way before the wait returns.  (Rows of 256 have the deep
+// ring only: two blocks' registers would not fit an SM.)
 template <int D, bool DEEP, bool QUERY = false>
 static int launch_dt(bf16* out, const bf16* q, int q_row_stride, const int* positions,
                      const int* token_slot, const void* k_pages, const void* v_pages,
                      long long page_rows, const int* block_table, int table_stride, int n_tokens,
                      int n_q_heads, int n_kv_heads, float scale, int window, int n_splits, int* status,
-                     float sink, const float* sinks, int chunk, float softcap, cudaStream_t stream) {
-  constexpr int STAGES = (D == 128 ? 3 : 6) * (DEEP ? 2 : 1);
+                     float sink, const float* sinks, int chunk, float softcap, const bf16* gate, int gate_stride, cudaStream_t stream) {
+  constexpr bool SHARED = D == 256;
+  static_assert(!SHARED || DEEP, "rows of 256: the deep ring only");
+  constexpr int STAGES = (D >= 128 ? 3 : 6) * (DEEP ? 2 : 1);
   constexpr int DB = D / 64;
-  constexpr size_t smem = 1024 + (size_t)STAGES * 2 * DB * EK_PAGE * 128 + 2 * STAGES * 8 +
-                          (size_t)(kDtRecvO<D> + kDtRecvMl) * 4;
+  constexpr size_t smem = 1024 + (size_t)STAGES * (SHARED ? 1 : 2) * DB * EK_PAGE * 128 + 2 * STAGES * 8 +
+                          (size_t)(kDtRecvO<D> + kDtRecvMl) * 4 + (SHARED ? 16 * D * 2 : 0);
   CUtensorMap mk, mv;
   int rc;
   if (!QUERY) {
     if ((rc = tensor_map(k_pages, page_rows, D, D, EK_PAGE, &mk))) return rc;
-    if ((rc = tensor_map(v_pages, page_rows, D, D, EK_PAGE, &mv))) return rc;
+    if (!SHARED && (rc = tensor_map(v_pages, page_rows, D, D, EK_PAGE, &mv))) return rc;
   }
-  auto kernel = attention_decode_tma_kernel<D, STAGES>;
+  const auto kernel = [] {
+    if constexpr (SHARED) return attention_decode_tma_shared_kernel<D, STAGES>;
+    else return attention_decode_tma_kernel<D, STAGES>;
+  }();
   static bool configured[kMaxDevices] = {};
   int device = 0;
   cudaError_t e = cudaGetDevice(&device);
@@ -375,18 +527,18 @@ static int launch_dt(bf16* out, const bf16* q, int q_row_stride, const int* posi
   if (!configured[device]) {
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    if (!DEEP) {                                 // clusters of 9 to 16 blocks (two blocks an SM only)
+    if (!DEEP || SHARED) {                       // clusters of 9 to 16 blocks
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
       if (e != cudaSuccess) return (int)e;
     }
     configured[device] = true;
   }
   prefer_carveout((const void*)kernel, 100);
-  dim3 grid(n_splits, n_kv_heads, n_tokens);
+  dim3 grid(n_splits, SHARED ? n_kv_heads * ((n_q_heads / n_kv_heads + 15) / 16) : n_kv_heads, n_tokens);
   if (QUERY) {                                   // can a cluster of 16 of these blocks run at all?
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kDtMaxSplits, 1, 1);
-    cfg.blockDim = dim3(kDtThreads);
+    cfg.blockDim = dim3(kDtThreads<D>);
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -400,16 +552,19 @@ static int launch_dt(bf16* out, const bf16* q, int q_row_stride, const int* posi
     if (e != cudaSuccess) { cudaGetLastError(); return 0; }
     return clusters;
   }
-  if (n_splits > 1)
-    return (int)launch_pdl_cluster_x(kernel, grid, dim3(kDtThreads), smem, stream, n_splits, out, q,
-                                     q_row_stride, positions, token_slot, mk, mv, block_table,
-                                     table_stride, n_kv_heads, n_q_heads,
-                                     scale * 1.4426950408889634f, window, status,
-                                     sink * 1.4426950408889634f, sinks, chunk, soft_cap(scale, softcap));
-  return (int)launch_pdl(kernel, grid, dim3(kDtThreads), smem, stream, out, q, q_row_stride, positions,
-                         token_slot, mk, mv, block_table, table_stride, n_kv_heads, n_q_heads,
-                         scale * 1.4426950408889634f, window, status, sink * 1.4426950408889634f, sinks, chunk,
-                         soft_cap(scale, softcap));
+  const float log2e = 1.4426950408889634f;
+  const SoftCap cap = soft_cap(scale, softcap);
+  auto launch = [&](auto... args) {
+    if (n_splits > 1)
+      return (int)launch_pdl_cluster_x(kernel, grid, dim3(kDtThreads<D>), smem, stream, n_splits, args...);
+    return (int)launch_pdl(kernel, grid, dim3(kDtThreads<D>), smem, stream, args...);
+  };
+  if constexpr (SHARED)
+    return launch(out, q, q_row_stride, positions, token_slot, mk, block_table, table_stride, n_kv_heads, n_q_heads,
+                  scale * log2e, window, status, sink * log2e, sinks, chunk, cap, gate, gate_stride);
+  else
+    return launch(out, q, q_row_stride, positions, token_slot, mk, mv, block_table, table_stride, n_kv_heads, n_q_heads,
+                  scale * log2e, window, status, sink * log2e, sinks, chunk, cap);
 }
 
 }  // namespace ek
@@ -421,35 +576,40 @@ EK_EXPORT int ek_attention_decode_tma_max_splits(int head_dim) {
   int clusters = 0;
   if (head_dim == 64)
     clusters = launch_dt<64, false, true>(nullptr, nullptr, 0, nullptr, nullptr, &clusters, &clusters, 64,
-                                          nullptr, 0, 1, 1, 1, 1.f, 0, 1, nullptr, -INFINITY, nullptr, 0, 0.f, nullptr);
+                                          nullptr, 0, 1, 1, 1, 1.f, 0, 1, nullptr, -INFINITY, nullptr, 0, 0.f, nullptr, 0, nullptr);
   else if (head_dim == 128)
     clusters = launch_dt<128, false, true>(nullptr, nullptr, 0, nullptr, nullptr, &clusters, &clusters, 64,
-                                           nullptr, 0, 1, 1, 1, 1.f, 0, 1, nullptr, -INFINITY, nullptr, 0, 0.f, nullptr);
+                                           nullptr, 0, 1, 1, 1, 1.f, 0, 1, nullptr, -INFINITY, nullptr, 0, 0.f, nullptr, 0, nullptr);
+  else if (head_dim == 256)
+    clusters = launch_dt<256, true, true>(nullptr, nullptr, 0, nullptr, nullptr, &clusters, &clusters, 64,
+                                          nullptr, 0, 1, 1, 1, 1.f, 0, 1, nullptr, -INFINITY, nullptr, 0, 0.f, nullptr, 0, nullptr);
   else
     return 0;
   return clusters >= 1 ? kDtMaxSplits : kDtPortableSplits;
 }
 
-// head_dim 64 or 128; at most 16 query heads a KV head; 1 to 16 splits (each takes whole pages of
+// head_dim 64 or 128 with at most 16 query heads a KV head, or 256 with k_pages == v_pages; 1 to 16 splits (each takes whole pages of
 // the token's visible range); q rows 4-byte aligned; n_pages = pages in k_pages / v_pages
 // ([pages, kv heads, 64, head_dim]); `status` is one int on the device.  `sink`: score of a key
 // without a value that every query also sees (one more term in the softmax denominator);
 // -INFINITY for none; `sinks` (may be null): one such score per query head, in place of `sink`.
 // `chunk` > 0 instead of a window: keys of the token's own chunk of positions only.
-// `softcap` > 0: scores become softcap tanh(score / softcap).
+// `softcap` > 0: scores become softcap tanh(score / softcap).  `gate` (null but for rows of 256): a value per token
+// and query head (rows `gate_stride` apart) whose sigmoid the head's output is multiplied by.
 EK_EXPORT int ek_attention_decode_tma(void* out, const void* q, int q_row_stride,
                                       const int* positions, const int* token_slot,
                                       const void* k_pages, const void* v_pages, int n_pages,
                                       const int* block_table, int table_stride, int n_tokens,
                                       int n_q_heads, int n_kv_heads, int head_dim, float scale,
                                       int window, int n_splits, int* status, float sink,
-                                      const float* sinks, int chunk, float softcap, cudaStream_t stream) {
+                                      const float* sinks, int chunk, float softcap, const void* gate,
+                                      int gate_stride, cudaStream_t stream) {
   using namespace ek;
   if (n_tokens <= 0) return 0;
   if (chunk < 0 || (chunk > 0 && window > 0)) return EK_ERR_ARG;
-  if ((head_dim != 64 && head_dim != 128) || n_kv_heads <= 0 || n_q_heads % n_kv_heads ||
-      n_q_heads / n_kv_heads > 16 || n_splits < 1 || n_splits > kDtMaxSplits || q_row_stride % 2 ||
-      ((uintptr_t)q & 3) || !status || n_kv_heads > 65535 || n_tokens > 65535 || n_pages <= 0)
+  if ((head_dim != 64 && head_dim != 128 && head_dim != 256) || n_kv_heads <= 0 || n_q_heads % n_kv_heads ||
+      (head_dim == 256 ? k_pages != v_pages || n_q_heads > 65535 : n_q_heads / n_kv_heads > 16) || n_splits < 1 || n_splits > kDtMaxSplits || q_row_stride % (head_dim == 256 ? 8 : 2) ||
+      ((uintptr_t)q & (head_dim == 256 ? 15 : 3)) || (head_dim == 256 ? ((uintptr_t)out & 7) != 0 : gate != nullptr) || !status || n_kv_heads > 65535 || n_tokens > 65535 || n_pages <= 0)
     return EK_ERR_ARG;
   const long long page_rows = (long long)n_pages * n_kv_heads * EK_PAGE;
   // one block an SM at most, and a cluster of the portable size (a deep ring is one block an SM)
@@ -458,7 +618,8 @@ EK_EXPORT int ek_attention_decode_tma(void* out, const void* q, int q_row_stride
   return launch_dt<D_, DEEP_>((bf16*)out, (const bf16*)q, q_row_stride, positions, token_slot,     \
                               k_pages, v_pages, page_rows, block_table, table_stride, n_tokens,   \
                               n_q_heads, n_kv_heads, scale, window, n_splits, status, sink, sinks,     \
-                              chunk, softcap, stream)
+                              chunk, softcap, (const bf16*)gate, gate_stride, stream)
+  if (head_dim == 256) EK_DT(256, true);
   if (head_dim == 64) {
     if (deep) EK_DT(64, true);
     EK_DT(64, false);

@@ -166,19 +166,9 @@ EK_EXPORT int ek_hc_broadcast(float* streams, const float* x, int n_tokens, int 
                                  (int)smem);                                                        \
       if (e != cudaSuccess) return (int)e;                                                          \
     }                                                                                               \
-    if (n <= 2)                                                                                     \
-      hc_step_kernel<T, 2><<<n_tokens, 256, smem, stream>>>(streams, (const T*)y, write_mix,        \
-                                                            write_out, read_in, u, n, width, gain,  \
-                                                            eps, (T*)normed);                       \
-    else if (n <= 4)                                                                                \
-      hc_step_kernel<T, 4><<<n_tokens, 256, smem, stream>>>(streams, (const T*)y, write_mix,        \
-                                                            write_out, read_in, u, n, width, gain,  \
-                                                            eps, (T*)normed);                       \
-    else                                                                                            \
-      hc_step_kernel<T, 8><<<n_tokens, 256, smem, stream>>>(streams, (const T*)y, write_mix,        \
-                                                            write_out, read_in, u, n, width, gain,  \
-                                                            eps, (T*)normed);                       \
-    EK_RETURN_LAUNCH_STATUS();                                                                      \
+    return (int)launch_pdl(n <= 2 ? hc_step_kernel<T, 2> : n <= 4 ? hc_step_kernel<T, 4> : hc_step_kernel<T, 8>, \
+                           dim3(n_tokens), dim3(256), smem, stream, streams, (const T*)y, write_mix, write_out,  \
+                           read_in, u, n, width, gain, eps, (T*)normed);                            \
   }
 
 EK_INSTANTIATE(f32, float)

@@ -779,7 +779,7 @@ def attention_decode_bf16(out, q, n_tokens, positions, token_slot, k_pages, v_pa
 
 _attn_decode_tma = Function("attention_decode_tma", "ek_attention_decode_tma",
                             [_P, _P, c_int, _P, _P, _P, _P, c_int, _P, c_int, c_int, c_int, c_int, c_int,
-                             c_float, c_int, c_int, _P, c_float, _P, c_int, c_float, _P])
+                             c_float, c_int, c_int, _P, c_float, _P, c_int, c_float, _P, c_int, _P])
 _attn_decode_tma_max = Function("attention_decode_tma", "ek_attention_decode_tma_max_splits", [c_int],
                                 check_status=False)
 DECODE_TMA_PORTABLE_SPLITS = 8
@@ -801,10 +801,16 @@ def attention_decode_tma_supported(dtype, head_dim, n_q_heads, n_kv_heads):
     return dtype == torch.bfloat16 and head_dim in (64, 128) and n_q_heads // n_kv_heads <= 16
 
 
+def attention_decode_tma_shared_supported(dtype, row):
+    """Rows that are keys and values alike (``v_pages`` is ``k_pages``), any number of query heads."""
+    return dtype == torch.bfloat16 and row == 256
+
+
 def attention_decode_tma(out, q, n_tokens, positions, token_slot, k_pages, v_pages, block_table,
                          n_q_heads, n_kv_heads, head_dim, scale, window=None, n_splits=1, sink=None, chunk=None,
-                         softcap=None, sinks=None):
-    """One new token per sequence (bfloat16, head size 64 or 128, at most 16 heads a group): the
+                         softcap=None, sinks=None, gate=None):
+    """One new token per sequence (bfloat16, head size 64 or 128, at most 16 heads a group, or
+    rows of 256 that are keys and values alike; ``gate`` [T, NQ]: see :func:`attention_decode_bf16`): the
     cache pages come by TMA, started before the kernel ahead has finished; ``n_splits`` (1 to 8)
     blocks (16 where :func:`decode_tma_max_splits` says so) share a token's pages and merge inside
     a thread-block cluster.
@@ -814,7 +820,8 @@ def attention_decode_tma(out, q, n_tokens, positions, token_slot, k_pages, v_pag
     step before) must be separated from this launch by a launch that is not programmatic:
     :func:`embed`, the first kernel of every step, is one."""
     _need_cuda(out, q, positions, token_slot, k_pages, v_pages, block_table)
-    _need(attention_decode_tma_supported(q.dtype, head_dim, n_q_heads, n_kv_heads),
+    shared = k_pages.data_ptr() == v_pages.data_ptr() and attention_decode_tma_shared_supported(q.dtype, head_dim)
+    _need(shared or attention_decode_tma_supported(q.dtype, head_dim, n_q_heads, n_kv_heads),
           "attention_decode_tma: bfloat16, head size 64 or 128, at most 16 query heads a KV head")
     _need(out.dtype == q.dtype == k_pages.dtype, "attention: one dtype for q, cache and out")
     _need(out.is_contiguous() and out.shape[-1] == n_q_heads * head_dim, "attention: out [T, NQ*D]")
@@ -830,7 +837,8 @@ def attention_decode_tma(out, q, n_tokens, positions, token_slot, k_pages, v_pag
                      _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table),
                      block_table.stride(0), n_tokens, n_q_heads, n_kv_heads, head_dim, float(scale),
                      int(window or 0), n_splits, _ptr(tc_status(q.device)), _sink(sink),
-                     _sinks(sinks, n_q_heads), int(chunk or 0), float(softcap or 0.0), _stream())
+                     _sinks(sinks, n_q_heads), int(chunk or 0), float(softcap or 0.0),
+                     *_gate_args(gate, q, n_q_heads), _stream())
 
 
 _attn_prefill_bf16 = Function("attention_prefill_bf16", "ek_attention_prefill_bf16",

@@ -210,6 +210,23 @@ class LatentAttention(Mixer):
             kernels.attention_prefill_f32(out, q, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
                                           pages, pages, table, nh, 1, row, self.scale, self.window, **common)
             return
+        if ctx.is_decode and t <= 65535 and kernels.attention_decode_tma_shared_supported(self.dtype, row):
+            blocks = t * -(-nh // 16)
+            pages = -(-visible // kernels.PAGE)
+            # One block an SM, and a cluster's blocks within one group of SMs: 8 blocks a token up to 96 in all, 16 up to
+            # 64, 2 or 4 up to the number of SMs.  Us behind 2,048 rows by blocks a token: 8 tokens 4: 12.4, 8: 10.0, 16 (a
+            # second wave): 17.1 (register-streaming kernel 26.3); 16 tokens 4: 13.0, 8: 19.8; 4 tokens 8: 9.2, 16: 8.3; 64
+            # behind 1,000 1: 16.4, 2: 13.7, 4: 19.8 (44.6); 256 1: 36.1, 2: 52.0 (54.3).  Behind 20 rows 6.2 (12.0).
+            most = max(1, kernels.sm_count(self.device) // blocks)
+            if most > 4 and 8 * blocks > 96:
+                most = 4
+            elif most > 8 and 16 * blocks > 64:
+                most = 8
+            splits = min(most, pages, kernels.decode_tma_max_splits(row, self.device))
+            splits = 1 << (splits.bit_length() - 1)
+            kernels.attention_decode_tma(out, q, t, ctx.positions, ctx.token_slot, entry.k_pages, entry.k_pages, table, nh, 1, row,
+                                         self.scale, self.window, splits, **common)
+            return
         fast = ctx.is_decode and kernels.attention_decode_supported(self.dtype, row)
         if fast:
             blocks = t * -(-nh // 16)

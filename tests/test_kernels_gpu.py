@@ -327,6 +327,37 @@ def test_attention_decode_bf16(nq, nkv, d):
             assert rel(out[i], want) <= TOL[dtype], (window, splits, i)
 
 
+@pytest.mark.parametrize("nq,window,softcap", [(1, None, None), (16, None, None), (17, 100, None), (20, None, 30.0), (40, 1, None)])
+def test_attention_decode_tma_rows_that_are_keys_and_values(nq, window, softcap):
+    """Rows of 256 read once for both uses by the TMA-fed kernel: blocks of 16 heads, 1 to 16 splits (more than a short
+    sequence has pages), gates in wider rows, a sink per head, finished rows; against the register-streaming kernel,
+    which the tests hold against plain arithmetic."""
+    k, d = K(), 256
+    lens = [1, 64, 65, 1100, 130]
+    pages = Pages(len(lens), max(lens), 1, d, torch.bfloat16, seed=6)
+    for s, n in enumerate(lens):
+        pages.fill(s, rnd(n, 1, d, dtype=torch.bfloat16, seed=40 + s), rnd(n, 1, d, dtype=torch.bfloat16, seed=50 + s))
+    positions = torch.tensor([n - 1 for n in lens] + [-1, 1023], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([0, 1, 2, 3, 4, 0, 3], dtype=torch.int32, device=DEV)
+    t = len(positions)
+    q = rnd(t, nq * d, dtype=torch.bfloat16, seed=60)
+    q[3, :d] = (pages.k.float().abs().max() + 1).to(torch.bfloat16) * q[3, :d].sign()      # one query with large scores
+    gate = rnd(t, nq + 3, dtype=torch.bfloat16, seed=61)
+    sinks = rnd(nq, seed=62)
+    args = (positions, slots, pages.k, pages.k, pages.table, nq, 1, d, d ** -0.5, window)
+    for kw in (dict(), dict(gate=gate, sinks=sinks)):
+        want = torch.empty((t, nq * d), dtype=torch.bfloat16, device=DEV)
+        k.attention_decode_bf16(want, q, t, *args, softcap=softcap, **kw)
+        for splits in (1, 2, 5, 8, 16):
+            if splits > k.decode_tma_max_splits(d, q.device):
+                continue
+            out = torch.full((t, nq * d), 7.0, dtype=torch.bfloat16, device=DEV)
+            k.attention_decode_tma(out, q, t, *args, splits, softcap=softcap, **kw)
+            assert out[5].abs().max().item() == 0
+            assert rel(out, want) <= TOL[torch.bfloat16], (splits, list(kw))
+    k.check_tc_status(q.device)
+
+
 @pytest.mark.parametrize("nq,nkv,d", [(6, 3, 64), (32, 8, 128), (5, 5, 64), (16, 1, 128), (40, 4, 128),
                                       (3, 1, 64)])
 def test_attention_decode_tma(nq, nkv, d):

@@ -120,6 +120,14 @@ def test_products_per_head(dtype, heads, n_in, n_out, r, rot, tokens):
         assert out[..., n_out + r:].abs().sum().item() == 0
 
 
+@pytest.mark.parametrize("heads,n_in,n_out,r,rot,tokens", [(16, 128, 192, 64, 64, 8), (5, 48, 72, 16, 16, 9), (3, 16, 8, 8, 4, 1),
+                                                           (4, 192, 128, 0, 0, 64), (2, 400, 40, 0, 0, 17)])
+def test_products_per_head_of_whole_steps(heads, n_in, n_out, r, rot, tokens):
+    """Few rows whose inputs are whole steps of 16 and whose outputs are whole pieces of 8: edges of the output tiles of 32
+    and the token tiles of 8, inputs in wider rows, the tail of a block of its own."""
+    test_products_per_head(torch.bfloat16, heads, n_in, n_out, r, rot, tokens)
+
+
 def _delta_inputs(t, heads, kv_heads, dim, vdim, seed):
     g = torch.Generator().manual_seed(seed)
     q = plain.unit(torch.randn(t, kv_heads, dim, generator=g, dtype=torch.float64)) * dim ** -0.5
