@@ -333,7 +333,7 @@ constexpr int kScanLanes = 8;        // lanes that share a column
 constexpr int kScanChunk = 16;       // tokens fetched into shared memory at a time
 constexpr int kScanThreads = kScanCols * kScanLanes;
 
-// grid (sequences, heads, column tiles); 128 threads = 16 columns x 8 lanes (small blocks: the scan is a
+// a block per (sequence, head, column tile), tiles fastest; 128 threads = 16 columns x 8 lanes (small blocks: the scan is a
 // chain of latencies, and more blocks put it on more SMs); a lane holds RPL
 // consecutive rows of its column.  The tokens' q, k, decays, v and beta come in chunks of 16 through
 // two shared-memory buffers: while a chunk is worked through, the next one is on its way from global
@@ -361,12 +361,14 @@ delta_scan_kernel(float* __restrict__ out, const float* __restrict__ qn, const f
   float* o_s = b_s + 2 * kScanChunk;            // [chunk][cols]
   pdl_launch_dependents();
   pdl_wait();
-  const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+  // sequences slowest, so that the blocks of the longest one spread over the SMs
+  const int tiles = (sh.vdim + kScanCols - 1) / kScanCols, tile = blockIdx.x % tiles;
+  const int b = blockIdx.x / tiles / sh.heads, h = blockIdx.x / tiles % sh.heads, tid = threadIdx.x;
   const int start = cu_seqlens[b], n = cu_seqlens[b + 1] - start;
   if (n <= 0 || positions[start] < 0) return;
   const int slot = token_slot[start];
   const int cl = tid / kScanLanes, lr = tid % kScanLanes;
-  const int col = blockIdx.z * kScanCols + cl;
+  const int col = tile * kScanCols + cl;
   const bool live = col < sh.vdim;
   const int kvh = h / (sh.heads / sh.kv_heads);
   const int cq = sh.cq(), cv = sh.cv(), nd = sh.heads * sh.dim;
@@ -394,7 +396,7 @@ delta_scan_kernel(float* __restrict__ out, const float* __restrict__ qn, const f
 #pragma unroll
     for (int i = 0; i < PERV; ++i) {
       const int idx = tid + i * kScanThreads, tt = idx / kScanCols, c = idx % kScanCols;
-      const int gc = blockIdx.z * kScanCols + c;
+      const int gc = tile * kScanCols + c;
       rv[i] = (tt < nt && gc < sh.vdim) ? vc[(size_t)(start + c0 + tt) * cv + (size_t)h * sh.vdim + gc] : 0.f;
     }
     if (tid < kScanChunk) rb = tid < nt ? beta[(size_t)(start + c0 + tid) * sh.heads + h] : 0.f;
@@ -463,7 +465,7 @@ delta_scan_kernel(float* __restrict__ out, const float* __restrict__ qn, const f
     __syncthreads();
     for (int idx = tid; idx < nt * kScanCols; idx += kScanThreads) {
       const int tt = idx / kScanCols, c = idx % kScanCols;
-      const int gc = blockIdx.z * kScanCols + c;
+      const int gc = tile * kScanCols + c;
       if (gc < sh.vdim) out[(size_t)(start + c0 + tt) * cv + (size_t)h * sh.vdim + gc] = o_s[idx];
     }
     __syncthreads();                            // o_s is written again in the next chunk
@@ -487,9 +489,8 @@ static cudaError_t launch_scan(dim3 grid, cudaStream_t stream, float* out, const
     cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  delta_scan_kernel<RPL><<<grid, kScanThreads, smem, stream>>>(out, qn, kn, vc, beta, decay, state, slot_stride,
-                                                              cu_seqlens, positions, token_slot, sh, decay_per_head);
-  return cudaGetLastError();
+  return launch_pdl(delta_scan_kernel<RPL>, grid, dim3(kScanThreads), smem, stream, out, qn, kn, vc, beta, decay, state,
+                    slot_stride, cu_seqlens, positions, token_slot, sh, decay_per_head);
 }
 
 // grid: tokens.  y[t, h, j] = o[t, h, j] / rms_j(o[t, h, :]) * w[j] * f(gate[t, h, j]); gate rows are
@@ -558,9 +559,8 @@ EK_EXPORT int ek_delta_low_rank(float* out, const float* proj, int proj_stride, 
     if (e != cudaSuccess) return (int)e;
   }
   const int wide = four ? 512 : 128;
-  kernel<<<dim3(token_tiles, (channels + wide - 1) / wide), 128, smem, stream>>>(
-      out, proj, proj_stride, offset, rank, w2t, bias, a_log, dim, channels, n_tokens, mode);
-  EK_RETURN_LAUNCH_STATUS();
+  return (int)launch_pdl(kernel, dim3(token_tiles, (channels + wide - 1) / wide), dim3(128), smem, stream, out, proj, proj_stride,
+                         offset, rank, w2t, bias, a_log, dim, channels, n_tokens, mode);
 }
 
 EK_EXPORT int ek_delta_prepare(float* qn, float* kn, float* vc, float* beta,
@@ -578,10 +578,8 @@ EK_EXPORT int ek_delta_prepare(float* qn, float* kn, float* vc, float* beta,
       (long long)(n_tokens / kPrepTokens) * units >= 2 * sm_count()) {
     const dim3 grid((n_tokens + kPrepTokens - 1) / kPrepTokens, units);
     auto kernel = taps == 2 ? delta_prepare_tile_kernel<2> : taps == 3 ? delta_prepare_tile_kernel<3> : delta_prepare_tile_kernel<4>;
-    kernel<<<grid, (widest + 31) / 32 * 32, 0, stream>>>(qn, kn, vc, beta, proj, proj_stride, conv_w, state,
-                                                         (size_t)slot_stride, (size_t)tail_offset, positions, token_slot,
-                                                         n_tokens, sh);
-    EK_RETURN_LAUNCH_STATUS();
+    return (int)launch_pdl(kernel, grid, dim3((widest + 31) / 32 * 32), 0, stream, qn, kn, vc, beta, proj, proj_stride, conv_w,
+                           state, (size_t)slot_stride, (size_t)tail_offset, positions, token_slot, n_tokens, sh);
   }
   if (n_tokens >= 512) {
     const size_t smem = (size_t)(2 * sh.cq()) * sizeof(float);
@@ -591,17 +589,13 @@ EK_EXPORT int ek_delta_prepare(float* qn, float* kn, float* vc, float* beta,
                                            (int)smem);
       if (e != cudaSuccess) return (int)e;
     }
-    delta_prepare_token_kernel<<<n_tokens, 256, smem, stream>>>(qn, kn, vc, beta, proj, proj_stride, conv_w, state,
-                                                                (size_t)slot_stride, (size_t)tail_offset, positions,
-                                                                token_slot, sh);
-    EK_RETURN_LAUNCH_STATUS();
+    return (int)launch_pdl(delta_prepare_token_kernel, dim3(n_tokens), dim3(256), smem, stream, qn, kn, vc, beta, proj,
+                           proj_stride, conv_w, state, (size_t)slot_stride, (size_t)tail_offset, positions, token_slot, sh);
   }
   const size_t smem = (size_t)(2 * dim) * sizeof(float);
   if (smem > 40 * 1024 || kv_heads > 65535) return EK_ERR_ARG;
-  delta_prepare_kernel<<<dim3(n_tokens, kv_heads), 128, smem, stream>>>(qn, kn, vc, beta, proj, proj_stride, conv_w,
-                                                                       state, (size_t)slot_stride,
-                                                                       (size_t)tail_offset, positions, token_slot, sh);
-  EK_RETURN_LAUNCH_STATUS();
+  return (int)launch_pdl(delta_prepare_kernel, dim3(n_tokens, kv_heads), dim3(128), smem, stream, qn, kn, vc, beta, proj,
+                         proj_stride, conv_w, state, (size_t)slot_stride, (size_t)tail_offset, positions, token_slot, sh);
 }
 
 EK_EXPORT int ek_delta_conv_tail(float* state, long long slot_stride, long long tail_offset,
@@ -611,10 +605,8 @@ EK_EXPORT int ek_delta_conv_tail(float* state, long long slot_stride, long long 
   if (n_seqs <= 0 || taps <= 1) return 0;
   if (channels <= 0 || proj_stride < channels) return EK_ERR_ARG;
   dim3 grid(n_seqs, (channels + 255) / 256 > 64 ? 64 : (channels + 255) / 256);
-  ek::delta_conv_tail_kernel<<<grid, 256, 0, stream>>>(state, (size_t)slot_stride, (size_t)tail_offset,
-                                                         proj, proj_stride, cu_seqlens, positions,
-                                                         token_slot, channels, taps);
-  EK_RETURN_LAUNCH_STATUS();
+  return (int)ek::launch_pdl(ek::delta_conv_tail_kernel, grid, dim3(256), 0, stream, state, (size_t)slot_stride,
+                             (size_t)tail_offset, proj, proj_stride, cu_seqlens, positions, token_slot, channels, taps);
 }
 
 EK_EXPORT int ek_delta_scan(float* out, const float* qn, const float* kn, const float* vc,
@@ -627,8 +619,9 @@ EK_EXPORT int ek_delta_scan(float* out, const float* qn, const float* kn, const 
   DeltaShape sh{heads, kv_heads, dim, vdim, 1, 1, 1};
   // S is read and written four values at a time: every slot's S must start on a 16-byte boundary
   if (!shape_ok(sh) || slot_stride % 4 || ((uintptr_t)state & 15)) return EK_ERR_ARG;
-  dim3 grid(n_seqs, heads, (vdim + kScanCols - 1) / kScanCols);
-  if (grid.z > 65535) return EK_ERR_ARG;
+  const long long blocks = (long long)n_seqs * heads * ((vdim + kScanCols - 1) / kScanCols);
+  if (blocks > 0x7fffffffLL || heads > 65535 || vdim > 65535 * kScanCols) return EK_ERR_ARG;
+  const dim3 grid((unsigned)blocks);
   const int rows = ek_delta_state_rows(dim);
 #define EK_SCAN(RPL)                                                                                 \
   return (int)launch_scan<RPL>(grid, stream, out, qn, kn, vc, beta, decay, state, (size_t)slot_stride, \
@@ -654,9 +647,8 @@ EK_EXPORT int ek_delta_scan(float* out, const float* qn, const float* kn, const 
     if (n_tokens <= 0) return 0;                                                                     \
     DeltaShape sh{heads, kv_heads, dim, vdim, taps, rank_a, rank_g};                                 \
     if (!shape_ok(sh) || gate_stride < sh.cv() || gate_act < 0 || gate_act > 1) return EK_ERR_ARG;   \
-    delta_out_norm_kernel<T><<<n_tokens, 256, 0, stream>>>((T*)y, o, gate, w, eps, positions, sh,    \
-                                                           gate_stride, gate_act);                   \
-    EK_RETURN_LAUNCH_STATUS();                                                                       \
+    return (int)launch_pdl(delta_out_norm_kernel<T>, dim3(n_tokens), dim3(256), 0, stream, (T*)y, o, gate, w, eps, \
+                           positions, sh, gate_stride, gate_act);                                    \
   }
 
 EK_INSTANTIATE(f32, float)

@@ -275,7 +275,7 @@ __host__ __device__ constexpr size_t chunk_scan_smem() {
                                   (2 * 2 + 1) * kChunk * kChunkCols + 2 * D);
 }
 
-// grid (sequences, heads, tiles of 16 columns).
+// a block per (sequence, head, tile of 16 columns), tiles fastest.
 template <int D>
 __global__ void __launch_bounds__(kChunkThreads)
 delta_chunk_scan_kernel(float* __restrict__ o, const float* __restrict__ w, const float* __restrict__ qp,
@@ -292,12 +292,14 @@ delta_chunk_scan_kernel(float* __restrict__ o, const float* __restrict__ w, cons
   float* gam_s = u_s + kChunk * kChunkCols;    // [2][D]
   pdl_launch_dependents();
   pdl_wait();
-  const int tid = threadIdx.x, b = blockIdx.x, h = blockIdx.y;
+  // sequences slowest, so that the blocks of the longest one spread over the SMs
+  const int tiles = (sh.vdim + kChunkCols - 1) / kChunkCols, tile = blockIdx.x % tiles;
+  const int tid = threadIdx.x, b = blockIdx.x / tiles / sh.heads, h = blockIdx.x / tiles % sh.heads;
   const int start = cu_seqlens[b], n = cu_seqlens[b + 1] - start;
   if (n <= 0 || positions[start] < 0) return;
   int chunk0 = 0;                              // the sequence's first chunk among all
   for (int i = 0; i < b; ++i) chunk0 += (cu_seqlens[i + 1] - cu_seqlens[i] + kChunk - 1) / kChunk;
-  const int E = sh.vdim, col0 = blockIdx.z * kChunkCols, cols = min(kChunkCols, E - col0);
+  const int E = sh.vdim, col0 = tile * kChunkCols, cols = min(kChunkCols, E - col0);
   float* S = state + (size_t)token_slot[start] * slot_stride + ((size_t)h * E + col0) * D;
 
   auto copy16 = [&](float* dst, const float* src, bool ok) {
@@ -439,7 +441,9 @@ static int launch_chunks(float* o, float* w, float* qp, float* kh, float* v, flo
   e = launch_pdl(prepare, dim3(chunks, sh.heads), dim3(kChunkThreads), smem, stream, w, qp, kh, v, o, gam, qn, kn, decay,
                  beta, cu_seqlens, n_seqs, positions, sh, decay_per_head);
   if (e != cudaSuccess) return (int)e;
-  return (int)launch_pdl(scan, dim3(n_seqs, sh.heads, (sh.vdim + kChunkCols - 1) / kChunkCols), dim3(kChunkThreads),
+  const long long blocks = (long long)n_seqs * sh.heads * ((sh.vdim + kChunkCols - 1) / kChunkCols);
+  if (blocks > 0x7fffffffLL || sh.heads > 65535 || sh.vdim > 65535 * kChunkCols) return EK_ERR_ARG;
+  return (int)launch_pdl(scan, dim3((unsigned)blocks), dim3(kChunkThreads),
                          chunk_scan_smem<D>(), stream, o, w, qp, kh, v, gam, state, slot_stride, cu_seqlens, positions,
                          token_slot, sh);
 }

@@ -28,6 +28,8 @@
 //   lru_gates        both gates from block-diagonal products, the decay and the gated input
 //   lru_scan         S_t = a_t S_(t-1) + x_t per channel, times the GELU of a side branch
 // Everything here is 32-bit; only the two output kernels round, once, to the activation type.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace ek {
@@ -526,9 +528,32 @@ xgate_scan_kernel(float* __restrict__ a, float* __restrict__ b, float* __restric
   if (write_state && threadIdx.x == 0) *m_state = m_in;
 }
 
-constexpr int kScanCols = 16;        // columns of S a block takes (twice as many with two a lane)
-constexpr int kScanLanes = 8;        // lanes that share a column
-constexpr int kScanThreads = kScanCols * kScanLanes;
+constexpr int kScanCols = 16;        // columns of S a block takes (as many times more as a lane takes)
+// Lanes that share a column: 8; with four columns a lane and 64 or 256 rows 16 (64 rows, 16 heads, prompts of 1,500 and 500: 61 us
+// against 69; 256 rows, a prompt of 2,048: 561 us, two columns on 8 lanes 664, and four there do not fit the registers;
+// but 128 rows: 541 us against 515 for the four prompts below).
+template <int DK, int CPL>
+constexpr int kScanLanes = CPL == 4 && DK != 128 ? 16 : 8;
+template <int DK, int CPL>
+constexpr int kScanThreads = kScanCols * kScanLanes<DK, CPL>;
+
+// Two 32-bit FMAs (products) in one instruction, each rounded as fmaf (the product) rounds: what a long walk is short of
+// is issue slots.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+        "l"(reinterpret_cast<const unsigned long long&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return d;
+}
 constexpr int kScanFloats = 2048;    // values of keys (and of queries) fetched into shared memory at a time
 
 // Long prompts of few sequences leave most of the machine empty when every sequence is walked by one block a head and
@@ -542,40 +567,51 @@ constexpr int kScanFloats = 2048;    // values of keys (and of queries) fetched 
 struct ScanSegments {
   float* carry;
   float* prods;
-  int count;                 // segments of the longest sequence (grid.x = sequences * count)
+  int count;                 // segments of the longest sequence
   int len;
 };
 
-// grid (sequences, heads, column tiles).  RPL rows of a column a lane: lane l holds rows 32 g + 4 l + c
-// (g < RPL / 4, c < 4), so that the 8 lanes of a column read 128 neighbouring bytes of a key at a time.
+// One block per (sequence, segment, head, column tile), in that order, tiles fastest: the blocks of the longest sequence
+// spread over the SMs.  (With sequences fastest, four of them and 148 SMs, every fourth SM had nothing but the longest
+// sequence's blocks.)  RPL rows of a column a lane: lane l holds rows 32 g + 4 l + c
+// (g < RPL / 4, c < 4; of 16 lanes 64 g + 4 l + c), so that a column's lanes read neighbouring bytes of a key at a time.
 // S of a slot: state[((h * C + j) * DK + i], DK = 8 RPL rows (keys padded with zeros), C = dv + ones_col columns.
 // `ab_stride`: values of a (and b) from token to token - the heads, or 0 where they are the same for every token.
-// CPL columns a lane (j and j + 16): with two, a key fetched from shared memory - what bounds a long walk - serves two
-// columns; single tokens take one, for the shorter walk through S.
+// CPL columns a lane (j, j + 16, ..): a key fetched from shared memory - what bounds a long walk, since a warp's 16-byte
+// load takes four cycles - serves that many columns; single tokens take one, for the shorter walk through S.
+// Eight tokens at a time S is kept divided by the product P_t of the group's decays so far: S / P_t needs one FMA a value,
+// S + (b_t v_t / P_t) k_t, instead of a product and an FMA, and the group ends with S = P_8 (S / P_8).  Where a P_t is not
+// within 2^-40 .. 2^40 (a decay of zero, say) the group is walked token by token.
+// Measured, prompts of 1,500, 1,103, 817 and 404 tokens, 32 heads of 128 x 128: 552 us with sequences fastest, two columns
+// a lane and the product in every token; 461 now in one walk, 400 in segments.  One of 2,048: 372, now 240.
 // Column dv (with ones_col) has v = 1: it carries n_t = a n + b k and gives n.q.
 // Tokens come 2048 / DK at a time: while one portion is worked through from shared memory, the next one's
 // keys, queries, values and gates are already on their way into registers.
-template <int RPL, int MODE, int CPL>
-__global__ void __launch_bounds__(kScanThreads)
+template <int DK, int MODE, int CPL>
+__global__ void __launch_bounds__(kScanThreads<DK, CPL>)
 decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restrict__ q, int q_stride,
                   const float* __restrict__ k, int k_stride, const float* __restrict__ v, int v_stride,
                   const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ state,
                   size_t slot_stride, const int* __restrict__ cu_seqlens, const int* __restrict__ positions,
                   const int* __restrict__ token_slot, int heads, int kv_heads, int dk, int dv, int ones_col,
                   int write_state, int ab_stride, ScanSegments seg) {
-  constexpr int DK = 8 * RPL, G4 = RPL / 4, DK4 = DK / 4, COLS = kScanCols * CPL;
+  constexpr int LANES = kScanLanes<DK, CPL>, THREADS = kScanThreads<DK, CPL>, RPL = DK / LANES, G4 = RPL / 4, DK4 = DK / 4, COLS = kScanCols * CPL;
   constexpr int CH = kScanFloats / DK;                       // tokens a portion: 64, 32, 16 or 8
-  constexpr int NV4 = kScanFloats / 4 / kScanThreads;        // float4 of keys (of queries) a thread fetches
-  constexpr int NV = CH * COLS / kScanThreads;               // values a thread fetches
-  static_assert(CH <= kScanThreads && CH * COLS % kScanThreads == 0, "portion sizes");
+  constexpr int NV4 = kScanFloats / 4 / THREADS;        // float4 of keys (of queries) a thread fetches
+  constexpr int NV = CH * COLS / THREADS;               // values a thread fetches
+  static_assert(CH <= THREADS && CH * COLS % THREADS == 0, "portion sizes");
   __shared__ __align__(16) float k_s[CH][DK];
   __shared__ __align__(16) float q_s[CH][DK];
   __shared__ float v_s[CH][COLS];
   __shared__ float a_s[CH], b_s[CH];
+  __shared__ float p_s[CH], bp_s[CH];                        // P_t and b_t / P_t
+  __shared__ int good_s[CH / 8];                             // groups of eight that may be walked so
   pdl_launch_dependents();
   pdl_wait();
-  const int seq = MODE == 0 ? blockIdx.x : blockIdx.x / seg.count, part = MODE == 0 ? 0 : blockIdx.x % seg.count;
-  const int h = blockIdx.y, col0 = blockIdx.z * COLS;
+  const int C = dv + ones_col, tiles = (C + COLS - 1) / COLS;
+  const int walk = blockIdx.x / tiles / heads, h = blockIdx.x / tiles % heads, tile = blockIdx.x % tiles;
+  const int seq = MODE == 0 ? walk : walk / seg.count, part = MODE == 0 ? 0 : walk % seg.count;
+  const int col0 = tile * COLS;
   int start = cu_seqlens[seq], n = cu_seqlens[seq + 1] - start;
   if (n <= 0 || positions[start] < 0) return;
   const int slot = token_slot[start];
@@ -588,8 +624,7 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
     start += part * seg.len;
     n = min(seg.len, n - part * seg.len);
   }
-  const int tid = threadIdx.x, col = tid / kScanLanes, lane = tid % kScanLanes;
-  const int C = dv + ones_col;
+  const int tid = threadIdx.x, col = tid / LANES, lane = tid % LANES;
   int j[CPL];
   bool live[CPL];
 #pragma unroll
@@ -603,7 +638,7 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
                    (((uintptr_t)q | (uintptr_t)k) & 15) == 0;
   float* sp = state + (size_t)slot * slot_stride;
   auto carry_at = [&](int slot_of) { return seg.carry + ((size_t)seq * seg.count + slot_of) * heads * C * DK; };
-  auto place = [&](int c, int g) { return ((size_t)h * C + j[c]) * DK + 32 * g + 4 * lane; };     // of S within a slot
+  auto place = [&](int c, int g) { return ((size_t)h * C + j[c]) * DK + 4 * LANES * g + 4 * lane; };     // of S within a slot
   auto load = [&](const float* from, int c, int g) { return *reinterpret_cast<const float4*>(from + place(c, g)); };
   auto store = [&](float* to, int c, int g, float4 v) { *reinterpret_cast<float4*>(to + place(c, g)) = v; };
   float4 S[CPL][G4];
@@ -657,7 +692,7 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
     const int nc = min(CH, n - c0);
 #pragma unroll
     for (int m = 0; m < NV4; ++m) {
-      const int f = tid + m * kScanThreads, tt = f / DK4, i = (f % DK4) * 4;
+      const int f = tid + m * THREADS, tt = f / DK4, i = (f % DK4) * 4;
       k_r[m] = q_r[m] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (tt < nc) {
         row4(k_r[m], k, (size_t)start + c0 + tt, k_stride, i);
@@ -666,7 +701,7 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
     }
 #pragma unroll
     for (int m = 0; m < NV; ++m) {
-      const int f = tid + m * kScanThreads, tt = f / COLS, jj = col0 + f % COLS;
+      const int f = tid + m * THREADS, tt = f / COLS, jj = col0 + f % COLS;
       v_r[m] = jj >= dv && jj < C ? 1.f : 0.f;
       if (tt < nc && jj < dv) v_r[m] = v[((size_t)start + c0 + tt) * v_stride + (size_t)h * dv + jj];
     }
@@ -682,26 +717,67 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
     __syncthreads();                             // the portion before is worked through
 #pragma unroll
     for (int m = 0; m < NV4; ++m) {
-      const int f = tid + m * kScanThreads;
+      const int f = tid + m * THREADS;
       reinterpret_cast<float4*>(&k_s[0][0])[f] = k_r[m];
       if (MODE != 1) reinterpret_cast<float4*>(&q_s[0][0])[f] = q_r[m];
     }
 #pragma unroll
-    for (int m = 0; m < NV; ++m) (&v_s[0][0])[tid + m * kScanThreads] = v_r[m];
-    if (tid < CH) { a_s[tid] = a_r; b_s[tid] = b_r; }
+    for (int m = 0; m < NV; ++m) (&v_s[0][0])[tid + m * THREADS] = v_r[m];
+    if (tid < (CH < 32 ? 32 : CH)) {             // (whole warps; past the portion a is 1 and b is 0)
+      float prefix = a_r;
+#pragma unroll
+      for (int by = 1; by < 8; by *= 2) {
+        const float before = __shfl_up_sync(0xffffffffu, prefix, by, 8);
+        if ((tid & 7) >= by) prefix *= before;
+      }
+      const unsigned good = __ballot_sync(0xffffffffu, prefix > 0x1p-40f && prefix < 0x1p40f);
+      if (tid < CH) {
+        a_s[tid] = a_r;
+        b_s[tid] = b_r;
+        p_s[tid] = prefix;
+        bp_s[tid] = b_r / prefix;
+        if ((tid & 7) == 0) good_s[tid / 8] = (good >> (tid & 24) & 0xffu) == 0xffu;
+      }
+    }
     __syncthreads();
     if (c0 + CH < n) fetch(c0 + CH);
-    auto token = [&](int tt, float* sums) {      // S <- a S + b v k; sums: this lane's parts of S^T q
-      const float aa = a_s[tt];
+    // S <- a S + b v k, or S / P_t <- S / P_(t-1) + (b / P_t) v k; sums: this lane's parts of S^T q
+    auto token = [&](int tt, float* sums, auto form) {
+      constexpr bool divided = decltype(form)::value;
       float bv[CPL];
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) bv[c] = (divided ? bp_s[tt] : b_s[tt]) * v_s[tt][col + c * kScanCols];
+      if constexpr (divided) {
+        float2 part[CPL];
+#pragma unroll
+        for (int g = 0; g < G4; ++g) {
+          const float4 kk = *reinterpret_cast<const float4*>(&k_s[tt][4 * LANES * g + 4 * lane]);
+          float4 qq;
+          if (MODE != 1) qq = *reinterpret_cast<const float4*>(&q_s[tt][4 * LANES * g + 4 * lane]);
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) {
+            const float2 b2 = make_float2(bv[c], bv[c]);
+            float2* s2 = reinterpret_cast<float2*>(&S[c][g]);
+            s2[0] = fma2(b2, make_float2(kk.x, kk.y), s2[0]);
+            s2[1] = fma2(b2, make_float2(kk.z, kk.w), s2[1]);
+            if (MODE != 1) {
+              part[c] = g == 0 ? mul2(s2[0], make_float2(qq.x, qq.y)) : fma2(s2[0], make_float2(qq.x, qq.y), part[c]);
+              part[c] = fma2(s2[1], make_float2(qq.z, qq.w), part[c]);
+            }
+          }
+        }
+        if (MODE == 1) return;
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) sums[c] = (part[c].x + part[c].y) * p_s[tt];
+        return;
+      }
+      const float aa = a_s[tt];
       float acc[CPL][G4];
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) bv[c] = b_s[tt] * v_s[tt][col + c * kScanCols];
-#pragma unroll
       for (int g = 0; g < G4; ++g) {
-        const float4 kk = *reinterpret_cast<const float4*>(&k_s[tt][32 * g + 4 * lane]);
+        const float4 kk = *reinterpret_cast<const float4*>(&k_s[tt][4 * LANES * g + 4 * lane]);
         float4 qq;
-        if (MODE != 1) qq = *reinterpret_cast<const float4*>(&q_s[tt][32 * g + 4 * lane]);
+        if (MODE != 1) qq = *reinterpret_cast<const float4*>(&q_s[tt][4 * LANES * g + 4 * lane]);
 #pragma unroll
         for (int c = 0; c < CPL; ++c) {
           float4& s4 = S[c][g];
@@ -712,7 +788,7 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
           if (MODE != 1) acc[c][g] = fmaf(s4.w, qq.w, fmaf(s4.z, qq.z, fmaf(s4.y, qq.y, s4.x * qq.x)));
         }
       }
-      if (MODE == 1) { prod *= aa; return; }
+      if (MODE == 1) return;
 #pragma unroll
       for (int c = 0; c < CPL; ++c) {
         sums[c] = acc[c][0];
@@ -720,52 +796,87 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
         for (int g = 1; g < G4; ++g) sums[c] += acc[c][g];
       }
     };
+    auto group_end = [&](float p) {              // S / P_8 -> S
+#pragma unroll
+      for (int c = 0; c < CPL; ++c)
+#pragma unroll
+        for (int g = 0; g < G4; ++g) {
+          float2* s2 = reinterpret_cast<float2*>(&S[c][g]);
+          s2[0] = mul2(s2[0], make_float2(p, p));
+          s2[1] = mul2(s2[1], make_float2(p, p));
+        }
+      if (MODE == 1) prod *= p;
+    };
     int tt = 0;
     if (MODE == 1) {
-#pragma unroll 4
-      for (; tt < nc; ++tt) token(tt, nullptr);
+      while (tt < nc) {
+        if (tt % 8 == 0 && tt + 8 <= nc && good_s[tt / 8]) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) token(tt + u, nullptr, std::true_type());
+          group_end(p_s[tt + 7]);
+          tt += 8;
+        } else {
+          token(tt, nullptr, std::false_type());
+          prod *= a_s[tt++];
+        }
+      }
       continue;
     }
     // eight tokens at a time: their partial sums are exchanged so that lane l ends with token l's total
     // (7 shuffles in 3 levels for 8 tokens instead of 24 in 24)
-    for (; tt + 8 <= nc; tt += 8) {
-      float p8[8][CPL];
+    for (; tt < nc;) {
+      if (tt % 8 == 0 && tt + 8 <= nc && good_s[tt / 8]) {
+        float p8[8][CPL];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) token(tt + u, p8[u]);
+        for (int u = 0; u < 8; ++u) token(tt + u, p8[u], std::true_type());
+        group_end(p_s[tt + 7]);
+        if constexpr (LANES == 16) {             // the halves of the lanes take two of the four columns each
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) {
-        float p[8];
+          for (int c = 0; c < CPL / 2; ++c)
 #pragma unroll
-        for (int u = 0; u < 8; ++u) p[u] = p8[u][c];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float send = (lane & 4) ? p[u] : p[u + 4], keep = (lane & 4) ? p[u + 4] : p[u];
-          p[u] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+            for (int u = 0; u < 8; ++u) {
+              const float low = p8[u][c], high = p8[u][c + CPL / 2];
+              p8[u][c] = ((lane & 8) ? high : low) + __shfl_xor_sync(0xffffffffu, (lane & 8) ? low : high, 8);
+            }
         }
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const float send = (lane & 2) ? p[u] : p[u + 2], keep = (lane & 2) ? p[u + 2] : p[u];
-          p[u] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+        for (int c = 0; c < (LANES == 16 ? CPL / 2 : CPL); ++c) {
+          float p[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) p[u] = p8[u][c];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float send = (lane & 4) ? p[u] : p[u + 4], keep = (lane & 4) ? p[u + 4] : p[u];
+            p[u] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const float send = (lane & 2) ? p[u] : p[u + 2], keep = (lane & 2) ? p[u + 2] : p[u];
+            p[u] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+          }
+          const float send = (lane & 1) ? p[0] : p[1], keep = (lane & 1) ? p[1] : p[0];
+          const float total = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+          const int jc = col0 + col + (LANES == 16 && (lane & 8) ? c + CPL / 2 : c) * kScanCols;
+          if (jc < C) out[(size_t)(start + c0 + tt + (lane & 7)) * out_stride + (size_t)h * C + jc] = total;
         }
-        const float send = (lane & 1) ? p[0] : p[1], keep = (lane & 1) ? p[1] : p[0];
-        const float total = keep + __shfl_xor_sync(0xffffffffu, send, 1);
-        if (live[c]) out[(size_t)(start + c0 + tt + lane) * out_stride + (size_t)h * C + j[c]] = total;
+        tt += 8;
+        continue;
       }
-    }
-    for (; tt < nc; ++tt) {
       float sums[CPL];
-      token(tt, sums);
+      token(tt, sums, std::false_type());
 #pragma unroll
       for (int c = 0; c < CPL; ++c) {
         float sum = sums[c];
+        if (LANES == 16) sum += __shfl_xor_sync(0xffffffffu, sum, 8);
         sum += __shfl_xor_sync(0xffffffffu, sum, 4);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         if (lane == 0 && live[c]) out[(size_t)(start + c0 + tt) * out_stride + (size_t)h * C + j[c]] = sum;
       }
+      ++tt;
     }
   }
-  if (MODE == 1 && tid == 0 && blockIdx.z == 0) seg.prods[((size_t)seq * seg.count + part) * heads + h] = prod;
+  if (MODE == 1 && tid == 0 && tile == 0) seg.prods[((size_t)seq * seg.count + part) * heads + h] = prod;
   if (MODE == 1 || write_state) {
     float* to = MODE == 1 ? carry_at(part + 1) : sp;
 #pragma unroll
@@ -1051,7 +1162,7 @@ EK_EXPORT int ek_decay_scan(float* out, int out_stride, const float* q, int q_st
                             long long slot_stride, const int* cu_seqlens, const int* positions,
                             const int* token_slot, int n_seqs, int heads, int kv_heads, int dk, int dv,
                             int ones_col, int write_state, int ab_stride, float* carry, float* prods,
-                            int segments, int seg_len, int wide, cudaStream_t stream) {
+                            int segments, int seg_len, int lane_cols, cudaStream_t stream) {
   using namespace ek;
   if (n_seqs <= 0) return 0;
   if (segments > 1 && (!carry || !prods || seg_len <= 0 || ((uintptr_t)carry & 15))) return EK_ERR_ARG;
@@ -1062,14 +1173,18 @@ EK_EXPORT int ek_decay_scan(float* out, int out_stride, const float* q, int q_st
     return EK_ERR_ARG;
   const int C = dv + (ones_col ? 1 : 0);
   const bool cut = segments > 1;
-  const int cols = kScanCols * (wide ? 2 : 1);
-  dim3 grid(n_seqs * (cut ? segments : 1), heads, (C + cols - 1) / cols);
+  if (lane_cols != 1 && lane_cols != 2 && (lane_cols != 4 || rows < 64)) return EK_ERR_ARG;
+  const int cols = kScanCols * lane_cols;
+  const long long blocks = (long long)n_seqs * (cut ? segments : 1) * heads * ((C + cols - 1) / cols);
+  if (blocks > 0x7fffffffLL) return EK_ERR_ARG;
+  const dim3 grid((unsigned)blocks);
   const ScanSegments seg{carry, prods, segments, seg_len};
 #define EK_SCAN_ROWS(MODE_, CPL_)                                                                               \
-  (rows == 32 ? decay_scan_kernel<4, MODE_, CPL_> : rows == 64 ? decay_scan_kernel<8, MODE_, CPL_>              \
-   : rows == 128 ? decay_scan_kernel<16, MODE_, CPL_> : decay_scan_kernel<32, MODE_, CPL_>)
+  (rows == 32 ? decay_scan_kernel<32, MODE_, CPL_ == 4 ? 2 : CPL_> : rows == 64 ? decay_scan_kernel<64, MODE_, CPL_> \
+   : rows == 128 ? decay_scan_kernel<128, MODE_, CPL_> : decay_scan_kernel<256, MODE_, CPL_>)
 #define EK_SCAN(MODE_)                                                                                          \
-  (int)launch_pdl(wide ? EK_SCAN_ROWS(MODE_, 2) : EK_SCAN_ROWS(MODE_, 1), grid, dim3(kScanThreads), 0, stream,  \
+  (int)launch_pdl(lane_cols == 4 ? EK_SCAN_ROWS(MODE_, 4) : lane_cols == 2 ? EK_SCAN_ROWS(MODE_, 2)             \
+                  : EK_SCAN_ROWS(MODE_, 1), grid, dim3(kScanCols * (lane_cols == 4 && rows != 128 ? 16 : 8)), 0, stream, \
                   out, out_stride, q, q_stride, k, k_stride, v, v_stride, a, b, state, (size_t)slot_stride,     \
                   cu_seqlens, positions, token_slot, heads, kv_heads, dk, dv, ones_col ? 1 : 0, write_state,    \
                   ab_stride, seg)

@@ -1884,24 +1884,34 @@ def xgate_scan(a, b, m_run, proj, col_i, col_f, bias_i, bias_f, cap, state, m_of
                 _ptr(token_slot), n_seqs, heads, 1 if write_state else 0, _stream())
 
 
-SCAN_COLUMNS = 16           # columns of S a block of the decay scan takes, one a lane; twice as many with two
-SCAN_WIDE_TOKENS = 64       # sequences of at least this many tokens take two columns a lane
+SCAN_COLUMNS = 16           # columns of S a block of the decay scan takes, one a lane; two or four times as many with more
+SCAN_WIDE_TOKENS = 64       # sequences of at least this many tokens take two or four columns a lane
 SCAN_BLOCKS_PER_SM = 6      # what a cut of long prompts into segments aims at
 SCAN_MIN_SEGMENT = 128      # tokens
 SCAN_MIN_SEGMENTS = 4       # (the walk of the states costs two thirds of a walk: two or three segments gain nothing)
 
 
-def decay_scan_wide(columns, max_new) -> bool:
-    """Whether a lane of :func:`decay_scan` takes two columns (long walks of enough columns)."""
-    return max_new >= SCAN_WIDE_TOKENS and columns > SCAN_COLUMNS
+def decay_scan_lane_columns(columns, max_new, dim=DECAY_SCAN_MAX_KEY_DIM) -> int:
+    """Columns that a lane of :func:`decay_scan` takes: one in short walks, four where there are enough columns and
+    16 lanes a column have four rows each, else two."""
+    if max_new < SCAN_WIDE_TOKENS or columns <= SCAN_COLUMNS:
+        return 1
+    return 4 if columns > 2 * SCAN_COLUMNS and dim > 32 else 2
 
 
-def decay_scan_segments(n_seqs, heads, columns, max_new, device=None):
+def decay_scan_segments(n_seqs, heads, columns, max_new, device=None, n_tokens=0):
     """(segments of the longest sequence, tokens a segment) that :func:`decay_scan` cuts a step's sequences into; one
-    segment where the sequences, heads and columns fill the machine, or the sequences are short."""
-    tile = SCAN_COLUMNS * (2 if decay_scan_wide(columns, max_new) else 1)
-    blocks = n_seqs * heads * -(-columns // tile)
-    want = min(SCAN_BLOCKS_PER_SM * sm_count(device) // blocks, max_new // SCAN_MIN_SEGMENT)
+    segment where the sequences, heads and columns fill the machine, or the sequences are short.  ``n_tokens`` (of all
+    sequences, if known) tells a ragged batch, whose longest sequence is left alone at the end, from an even one."""
+    lane_columns = decay_scan_lane_columns(columns, max_new)
+    blocks = n_seqs * heads * -(-columns // (SCAN_COLUMNS * lane_columns))
+    most, sms = -(-max_new // SCAN_MIN_SEGMENT), sm_count(device)
+    want = min(SCAN_BLOCKS_PER_SM * sms // blocks, most)
+    # Uncut, a step takes as long as its longest sequence, 0.30 us a token with two blocks an SM; cut, 0.24 us a token and
+    # block of each SM's share (both walks).  32 heads of 128, prompts of 1,500, 1,103, 817, 404: 461 us uncut, 400 in 6
+    # segments; 40 heads (more blocks): 471 and 495.
+    if want < SCAN_MIN_SEGMENTS and lane_columns == 4 and n_tokens * (blocks // n_seqs) * 0.81 < max_new * sms and n_tokens:
+        want = min(2 * SCAN_BLOCKS_PER_SM * sms // blocks, most)
     if want < SCAN_MIN_SEGMENTS:
         return 1, max_new
     length = -(-(-(-max_new // want)) // 64) * 64
@@ -1909,13 +1919,15 @@ def decay_scan_segments(n_seqs, heads, columns, max_new, device=None):
 
 
 def decay_scan(out, q, k, v, a, b, state, cu_seqlens, positions, token_slot, n_seqs, heads, kv_heads, dim, vdim,
-               ones_column=False, write_state=True, n_tokens=0, max_new=0, workspace=None, segments=None):
+               ones_column=False, write_state=True, n_tokens=0, max_new=0, workspace=None, segments=None,
+               lane_columns=None):
     """S_t = a_t S_(t-1) + b_t k_t v_t^T, out_t = S_t^T q_t per head over every sequence's tokens, S
     ([heads, columns, rows] at the start of a slot's state, 32-bit) read and written back.  ``q``, ``k``
     [T, >= kv_heads * dim] (head h reads key head h // (heads / kv_heads)), ``v`` [T, >= heads * vdim],
     ``a``, ``b`` [T, heads], or [heads] where they are the same for every token.  ``ones_column``: one more column whose v is 1 (it carries a n + b k and
     gives n . q); out is [T, heads * columns].  With ``workspace`` and ``max_new`` (tokens of the longest sequence) long
-    sequences are cut into segments that run side by side (:func:`decay_scan_segments`, or ``segments`` as given)."""
+    sequences are cut into segments that run side by side (:func:`decay_scan_segments`, or ``segments`` as given); ``lane_columns`` (1, 2 or 4):
+    :func:`decay_scan_lane_columns` unless given."""
     _need_cuda(out, q, k, v, a, b, state, cu_seqlens, positions, token_slot)
     _need_f32("decay_scan", out, q, k, v, a, b, state)
     cols = vdim + (1 if ones_column else 0)
@@ -1929,7 +1941,7 @@ def decay_scan(out, q, k, v, a, b, state, cu_seqlens, positions, token_slot, n_s
                      flops=4 * n_tokens * heads * dim * cols)
     parts, length, carry, prods = 1, 0, None, None
     if workspace is not None and max_new > 1:
-        parts, length = segments or decay_scan_segments(n_seqs, heads, cols, max_new, out.device)
+        parts, length = segments or decay_scan_segments(n_seqs, heads, cols, max_new, out.device, n_tokens)
         _need(length >= 1 and parts * length >= max_new, "decay_scan: the segments cover the longest sequence")
         if parts > 1:
             carry = workspace.get("scan_carry", (n_seqs, parts, heads * cols * decay_scan_rows(dim)), torch.float32)
@@ -1938,7 +1950,7 @@ def decay_scan(out, q, k, v, a, b, state, cu_seqlens, positions, token_slot, n_s
                 _ptr(a), _ptr(b), _ptr(state), state.stride(0), _ptr(cu_seqlens), _ptr(positions), _ptr(token_slot),
                 n_seqs, heads, kv_heads, dim, vdim, 1 if ones_column else 0, 1 if write_state else 0,
                 heads if a.dim() > 1 else 0, _ptr(carry), _ptr(prods), parts, length,
-                1 if decay_scan_wide(cols, max_new) else 0, _stream())
+                lane_columns or decay_scan_lane_columns(cols, max_new, dim), _stream())
     if parts > 1:
         count_extra_launches()
 

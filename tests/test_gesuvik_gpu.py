@@ -263,6 +263,44 @@ def test_scan_in_segments_is_the_scan(heads, kv_heads, dim, vdim, ones):
             assert torch.equal(keep, start)
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,ones", [(2, 1, 128, 130, False), (3, 3, 60, 64, True), (2, 2, 20, 33, False), (1, 1, 200, 40, False)])
+def test_decay_scan_columns_a_lane(heads, kv_heads, dim, vdim, ones):
+    """One, two and four columns a lane: groups of eight tokens whose decays' product is within the range that is walked
+    divided by it, at its edge, beyond it on both sides and zero; sequences of 1, 7, 8, 9 and 150 tokens."""
+    from enginekernel_b200.parts.base import Workspace
+    k = K()
+    lens, slots = [150, 1, 9, 7, 8], [1, 0, 2, 4, 3]
+    n, cols, rows = sum(lens), vdim + int(ones), k.decay_scan_rows(dim)
+    cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    tok_slots = [s for s, ln in zip(slots, lens) for _ in range(ln)]
+    pos = [3 + j for ln in lens for j in range(ln)]
+    q, kk, v = rnd(n, kv_heads * dim, seed=1), rnd(n, kv_heads * dim, seed=2, scale=0.5), rnd(n, heads * vdim, seed=3)
+    start = torch.zeros(5, heads, cols, rows, device=DEV)
+    start[..., :dim] = rnd(5, heads, cols, dim, seed=4)
+    start = start.view(5, -1)
+    a, b = 0.3 + 0.7 * torch.rand(n, heads, generator=torch.Generator().manual_seed(5)), torch.randn(n, heads, generator=torch.Generator().manual_seed(6))
+    a[8:16], a[16:24], a[24:32], a[32:40], a[45] = 2.0 ** -5, 2.0 ** -4.99, 2.0 ** -12, 1.5, 0.0
+    a, b = a.to(DEV), b.to(DEV)
+    want, ends = torch.empty(n, heads, cols, dtype=F64), {}
+    for s, (ln, slot) in enumerate(zip(lens, slots)):
+        S = start[slot].double().cpu().view(heads, cols, rows)[..., :dim].clone()
+        for t in range(cu[s], cu[s + 1]):
+            kt, qt = (x[t].double().cpu().view(kv_heads, dim).repeat_interleave(heads // kv_heads, 0) for x in (kk, q))
+            vt = torch.cat([v[t].double().cpu().view(heads, vdim), torch.ones(heads, int(ones), dtype=F64)], 1)
+            S = a[t].double().cpu()[:, None, None] * S + (b[t].double().cpu()[:, None] * vt)[:, :, None] * kt[:, None, :]
+            want[t] = (S * qt[:, None, :]).sum(-1)
+        ends[slot] = S
+    for lane_columns in (1, 2, 4) if dim > 32 else (1, 2):
+        for segments in ((1, 150), (3, 50)):
+            state, out = start.clone(), torch.full((n, heads * cols), 7.0, device=DEV)
+            k.decay_scan(out, q, kk, v, a, b, state, i32(cu), i32(pos), i32(tok_slots), 5, heads, kv_heads, dim, vdim,
+                         ones_column=ones, n_tokens=n, max_new=150, workspace=Workspace(DEV), segments=segments,
+                         lane_columns=lane_columns)
+            assert rel(out.view(n, heads, cols), want) <= 1e-5, (lane_columns, segments)
+            for slot, S in ends.items():
+                assert rel(state[slot].view(heads, cols, rows)[..., :dim], S) <= 1e-5, (lane_columns, segments, slot)
+
+
 def test_how_a_step_is_cut_into_segments():
     k = K()
     for n_seqs, heads, cols, longest in ((1, 16, 128, 2048), (1, 2, 16, 130), (8, 16, 128, 2048), (1, 16, 128, 1), (3, 1, 20, 100000)):
