@@ -583,7 +583,7 @@ struct ScanSegments {
 // S + (b_t v_t / P_t) k_t, instead of a product and an FMA, and the group ends with S = P_8 (S / P_8).  Where a P_t is not
 // within 2^-40 .. 2^40 (a decay of zero, say) the group is walked token by token.
 // Measured, prompts of 1,500, 1,103, 817 and 404 tokens, 32 heads of 128 x 128: 552 us with sequences fastest, two columns
-// a lane and the product in every token; 461 now in one walk, 400 in segments.  One of 2,048: 372, now 240.
+// a lane and the product in every token; 461 now in one walk, 406 in segments.  One of 2,048: 372, now 242.
 // Column dv (with ones_col) has v = 1: it carries n_t = a n + b k and gives n.q.
 // Tokens come 2048 / DK at a time: while one portion is worked through from shared memory, the next one's
 // keys, queries, values and gates are already on their way into registers.
@@ -724,18 +724,30 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
 #pragma unroll
     for (int m = 0; m < NV; ++m) (&v_s[0][0])[tid + m * THREADS] = v_r[m];
     if (tid < (CH < 32 ? 32 : CH)) {             // (whole warps; past the portion a is 1 and b is 0)
-      float prefix = a_r;
+      // P_t and b_t / P_t correctly rounded, but for a last place: the product is carried as a sum of two floats (a
+      // rounding of P_8 is the same for all of S and would add up from group to group)
+      float prefix = a_r, rest = 0.f;
 #pragma unroll
       for (int by = 1; by < 8; by *= 2) {
         const float before = __shfl_up_sync(0xffffffffu, prefix, by, 8);
-        if ((tid & 7) >= by) prefix *= before;
+        const float before_rest = __shfl_up_sync(0xffffffffu, rest, by, 8);
+        if ((tid & 7) >= by) {
+          const float product = prefix * before;
+          rest = fmaf(rest, before, fmaf(prefix, before_rest, fmaf(prefix, before, -product)));
+          prefix = product;
+        }
       }
+      const float rounded = prefix + rest;
+      rest -= rounded - prefix;
+      prefix = rounded;
+      float quotient = b_r / prefix;
+      quotient += fmaf(-quotient, rest, fmaf(-quotient, prefix, b_r)) / prefix;
       const unsigned good = __ballot_sync(0xffffffffu, prefix > 0x1p-40f && prefix < 0x1p40f);
       if (tid < CH) {
         a_s[tid] = a_r;
         b_s[tid] = b_r;
         p_s[tid] = prefix;
-        bp_s[tid] = b_r / prefix;
+        bp_s[tid] = quotient;
         if ((tid & 7) == 0) good_s[tid / 8] = (good >> (tid & 24) & 0xffu) == 0xffu;
       }
     }

@@ -1908,7 +1908,7 @@ def decay_scan_segments(n_seqs, heads, columns, max_new, device=None, n_tokens=0
     most, sms = -(-max_new // SCAN_MIN_SEGMENT), sm_count(device)
     want = min(SCAN_BLOCKS_PER_SM * sms // blocks, most)
     # Uncut, a step takes as long as its longest sequence, 0.30 us a token with two blocks an SM; cut, 0.24 us a token and
-    # block of each SM's share (both walks).  32 heads of 128, prompts of 1,500, 1,103, 817, 404: 461 us uncut, 400 in 6
+    # block of each SM's share (both walks).  32 heads of 128, prompts of 1,500, 1,103, 817, 404: 461 us uncut, 406 in 6
     # segments; 40 heads (more blocks): 471 and 495.
     if want < SCAN_MIN_SEGMENTS and lane_columns == 4 and n_tokens * (blocks // n_seqs) * 0.81 < max_new * sms and n_tokens:
         want = min(2 * SCAN_BLOCKS_PER_SM * sms // blocks, most)
