@@ -582,6 +582,8 @@ struct ScanSegments {
 // Eight tokens at a time S is kept divided by the product P_t of the group's decays so far: S / P_t needs one FMA a value,
 // S + (b_t v_t / P_t) k_t, instead of a product and an FMA, and the group ends with S = P_8 (S / P_8).  Where a P_t is not
 // within 2^-40 .. 2^40 (a decay of zero, say) the group is walked token by token.
+// Errors against 64 bits (1,500 tokens, decays of 0.5 to 1; 0.95 to 1): outputs 1.0e-7; 1.5e-7, S 5.4e-8; 1.2e-7; with the
+// product in every token 0.9e-7; 1.4e-7 and 5.3e-8; 1.2e-7.
 // Measured, prompts of 1,500, 1,103, 817 and 404 tokens, 32 heads of 128 x 128: 552 us with sequences fastest, two columns
 // a lane and the product in every token; 461 now in one walk, 406 in segments.  One of 2,048: 372, now 242.
 // Column dv (with ones_col) has v = 1: it carries n_t = a n + b k and gives n.q.
