@@ -22,7 +22,7 @@
 // that sees the query rows as [tokens][heads][head size].  A block's fixed costs count here (half
 // the time of a 2,048-token prompt went to them when Q was fetched with plain loads and all
 // setup stood behind the wait for the kernel ahead), so everything that does not read that
-// kernel's results - tile search, barriers, the TMEM allocation - is done before the wait.  Shared memory
+// step's results - barriers, the TMEM allocation - is done before the wait.  Shared memory
 // holds Q, three stages of K (the scores of page t+1 need their K two softmax steps ahead of
 // time, or the softmax warps wait for it) and two of V - 112 KB at head size 128 - and TMEM 256
 // columns (S, S, O): two blocks an SM.  Every wait is bounded and reports through `status`.
@@ -119,13 +119,6 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
   // (SHARED: not before the tensor memory is ours - a block of the next kernel that took part of it meanwhile would
   // wait for this one)
   if (!SHARED) pdl_launch_dependents();
-  // The tile's tokens, position and slot come from a table made once per step (sequence bounds,
-  // positions and slots were uploaded before the step's first kernel, and the table is made
-  // before its first attention kernel): one 16-byte load instead of a search through the
-  // sequences and two more dependent loads in every block of every layer.
-  const int4 tile = __ldg(&tiles[blockIdx.y]);     // first token, tokens, position of the first, slot
-  const int t_first = tile.x, n_tok = tile.y;
-  if (n_tok <= 0) return;                          // the table is padded to the grid's size
   if (tid == 128) {
     tma_prefetch_map(&map_q);
     tma_prefetch_map(&map_k);
@@ -143,13 +136,19 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   if (SHARED) pdl_launch_dependents();
+  pdl_wait();                                      // the table, Q and the newest keys and values
+  // The tile's tokens, position and slot come from a table made once per step: one 16-byte load instead of a
+  // search through the sequences and two more dependent loads in every block of every layer.  It is read behind
+  // the wait: every kernel between the one that makes it and this one may be a programmatic launch that lets its
+  // successor start at its top, and then nothing else says that the table is complete.
+  const int4 tile = __ldg(&tiles[blockIdx.y]);     // first token, tokens, position of the first, slot
+  const int t_first = tile.x, n_tok = tile.y;      // (no tokens: the table is padded to the grid's size)
   const int n_rows = n_tok * group;
   const bool misplaced = (smem_u32(smem) & 1023u) != 0;   // never seen; the swizzled tiles would be wrong
-  const int pos0 = misplaced ? -1 : tile.z;
+  const int pos0 = misplaced || n_tok <= 0 ? -1 : tile.z;
   if (pos0 < 0) {                                  // rows of a finished sequence: zeros
     if (misplaced && tid == 0) atomicCAS(status, 0, 19);
     if (!misplaced) {
-      pdl_wait();                                  // the rows may still be read by a kernel ahead
       for (int i = tid; i < n_rows * D; i += kFaThreads) {
         const int r = i / D, d = i % D;
         out[((size_t)(t_first + r / group) * n_q_heads + kv_head * group + r % group) * D + d] =
@@ -169,7 +168,6 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
   const int n_first = KEEP && keep_first > 0 ? min((keep_first + kFaKeys - 1) / kFaKeys, kt_lo) : 0;
   const int n_iter = n_first + kt_hi - kt_lo + 1;
   auto page_of = [&](int it) { return KEEP && it < n_first ? it : kt_lo + it - n_first; };
-  pdl_wait();                                      // Q and the newest keys and values: the kernel ahead
 
   bool ok = true;
   if (tid == 128) {

@@ -982,9 +982,8 @@ def attention_prefill_tiles(tiles, n_tokens, positions, token_slot, cu_seqlens, 
     tokens, position of the first, slot) per tile; the sequences in bands whose keys and values fit
     L2 together (longest context first), inside a band the longest key ranges first; padded with
     empty tiles.
-    It is read by the attention kernels before they wait for the kernel ahead of them, so it has
-    to be made before the step's first kernel (:func:`embed`, a plain launch), not just before the
-    attention; returns the number of entries to pass on."""
+    The attention kernels read it behind their wait for the kernel ahead of them, so any earlier place on the
+    stream will do; returns the number of entries to pass on."""
     _need_cuda(tiles, positions, token_slot, cu_seqlens)
     tok_per_tile = PREFILL_TC_ROWS // (n_q_heads // n_kv_heads)
     need = -(-n_tokens // tok_per_tile) + n_seqs
@@ -1005,9 +1004,8 @@ def attention_prefill_tc(out, q, n_tokens, positions, token_slot, cu_seqlens, n_
     that divide 128): TMA-fed pages, scores and P.V in TMEM.  With ``v_cols``, rows of 256 values that are keys and
     values alike (``v_pages`` is ``k_pages``, one KV head, up to 128 query heads): only the first ``v_cols`` values of a
     head's result are written.  ``tiles`` / ``n_tiles``: the table
-    :func:`attention_prefill_tiles` made for this step (made once, before the step's first
-    kernel, and used by every layer); without it the table is made here and the stream is
-    waited for, which suits a single call, not a model's step."""
+    :func:`attention_prefill_tiles` made for this step (made once and used by every layer); without it the
+    table is made here."""
     _need_cuda(out, q, positions, token_slot, cu_seqlens, k_pages, v_pages, block_table, tiles)
     if v_cols is not None:
         _need(attention_prefill_shared_supported(q.dtype, head_dim, n_q_heads) and n_kv_heads == 1
@@ -1027,7 +1025,6 @@ def attention_prefill_tc(out, q, n_tokens, positions, token_slot, cu_seqlens, n_
         tiles = torch.empty((-(-n_tokens // tok_per_tile) + n_seqs, 4), dtype=torch.int32, device=q.device)
         n_tiles = attention_prefill_tiles(tiles, n_tokens, positions, token_slot, cu_seqlens, n_seqs,
                                           n_q_heads, n_kv_heads, head_dim)
-        torch.cuda.current_stream().synchronize()
     _need(tiles.dtype == torch.int32 and tiles.numel() >= 4 * n_tiles and tiles.data_ptr() % 16 == 0,
           "attention_prefill_tc: the table of tiles")
     _attention_cost(q, n_tokens, positions, n_q_heads, n_kv_heads, head_dim, window, True, chunk)

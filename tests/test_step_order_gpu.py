@@ -1,0 +1,86 @@
+"""What a layer's kernels read of a step - its table of tiles, positions, slots - is that step's, not an earlier one's."""
+
+import pytest
+import torch
+
+from tests import helpers
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+H, EPS = 256, 1e-5
+
+
+def layer(kind, heads=4):
+    """A layer with weights of its own, small enough for every launch of a short prompt to be a programmatic one."""
+    from enginekernel_b200.parts.spec import PartSpec
+    from enginekernel_b200.registry import lookup_part
+    g = torch.Generator().manual_seed(11)
+    rand = lambda *s: (torch.randn(*s, generator=g) * 0.1).to(torch.bfloat16).to(DEV)
+    rope = lambda d: PartSpec("rope_neox", dict(head_dim=d, theta=10000.0, rotary_dim=d))
+    if kind == "latent":
+        d, r, e, c, a = 32, 64, 32, 192, 64
+        p = dict(hidden_size=H, num_heads=heads, head_dim=d, rot_dim=r, v_dim=e, q_rank=a, kv_rank=c,
+                 scale=(d + r) ** -0.5, eps=EPS, position=rope(r))
+        w = dict(dq=rand(a, H), dq_norm=rand(a), uq=rand(heads * (d + r), a), dkv=rand(c + r, H), dkv_norm=rand(c),
+                 uk=rand(heads * d, c), uv=rand(heads * e, c), o=rand(H, heads * e))
+        kind = "latent_attention"
+    else:
+        d, kv = 64, heads // 2
+        p = dict(hidden_size=H, num_heads=heads, num_kv_heads=kv, head_dim=d, scale=d ** -0.5, qk_norm_eps=EPS,
+                 window=None, position=rope(d))
+        w = dict(q=rand(heads * d, H), k=rand(kv * d, H), v=rand(kv * d, H), o=rand(H, heads * d), q_norm=rand(d),
+                 k_norm=rand(d))
+        if kind == "window":
+            p.update(window=70, keep_first=3, head_gate=True, keep_all_keys=True)
+            w["gate"] = rand(heads, H)
+        kind = "attention"
+    part = lookup_part("mixer", kind)(PartSpec(kind, p, {n: n for n in w}), torch.bfloat16, DEV)
+    part.load(w)
+    part.prepare(512)
+    return part
+
+
+def prompts(part, lens, seed):
+    """A step of prompts of these lengths with a cache of its own: (input rows, context, entry)."""
+    from enginekernel_b200.cache import SequenceCache
+    cache = SequenceCache([part.cache_spec()], torch.bfloat16, DEV, max_tokens=64 * sum(-(-n // 64) for n in lens),
+                          max_slots=len(lens))
+    slots = [cache.open() for _ in lens]
+    for s, n in zip(slots, lens):
+        cache.reserve(s, n)
+    cache.upload_tables()
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    ctx = helpers.make_context(torch.bfloat16, DEV, [i for n in lens for i in range(n)],
+                               [s for s, n in zip(slots, lens) for _ in range(n)], cu)
+    x = torch.randn(cu[-1], H, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16).to(DEV)
+    return x, ctx, cache.entry(0)
+
+
+@pytest.mark.parametrize("kind", ["attention", "window", "latent"])
+def test_a_layer_driven_alone_reads_its_own_steps_table(kind):
+    """``begin_step`` and ``forward`` with nothing in between and one workspace for steps of unequal sequences, none
+    waited for: every result is the one of the step alone in a workspace of its own, with the table waited for."""
+    from enginekernel_b200.parts.base import Workspace
+    part = layer(kind)
+    steps = [prompts(part, lens, i) for i, lens in enumerate([[9], [3, 13], [1, 2, 5, 1], [130, 40], [2, 14]])]
+    wants = []
+    for x, ctx, entry in steps:
+        ctx.workspace = Workspace(torch.device(DEV))
+        ctx.shared = {}
+        part.begin_step(ctx)
+        torch.cuda.synchronize()
+        wants.append(part.forward(x, ctx, entry, True).clone())
+        torch.cuda.synchronize()
+    shared = Workspace(torch.device(DEV))
+    got = []
+    for _ in range(4):
+        for x, ctx, entry in steps:
+            ctx.workspace, ctx.shared = shared, {}
+            part.begin_step(ctx)
+            got.append(part.forward(x, ctx, entry, True).clone())
+    torch.cuda.synchronize()
+    for i, y in enumerate(got):
+        assert torch.equal(y, wants[i % len(steps)]), (i // len(steps), i % len(steps))
