@@ -136,9 +136,10 @@ attention_decode_tma_block(bf16* __restrict__ out, const bf16* q, int q_row_stri
   }
   // Otherwise read before the wait: positions, slots and block tables must have been written by work that
   // a plain (not programmatic) launch separates from this kernel.  A step's first kernel, the
-  // embedding lookup, is such a launch, so the state advance of the step before is complete and
-  // visible here, in a captured graph and in eager decoding alike.
-  const int pos = positions[t];
+  // embedding lookup, is such a launch, so the state advance of the step before is complete here, in a
+  // captured graph and in eager decoding alike.  Past L1, which may hold the step before's (common.cuh).
+  const int pos = load_past_l1(positions + t);
+  const int slot_t = load_past_l1(token_slot + t);
   int lo = 0, hi = -1, pg_first = 0, pg_last = -1;
   if (pos >= 0) {
     lo = first_key(pos, window, chunk);
@@ -160,30 +161,36 @@ attention_decode_tma_block(bf16* __restrict__ out, const bf16* q, int q_row_stri
   for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};   // rows g and g + 8
 
-  if (tid == W * 32) {
-    // ------------------------------------------------------------------- TMA producer
-    const int* table = block_table + (size_t)(pos >= 0 ? token_slot[t] : 0) * table_stride;
+  if (warp == W) {
+    // ------------------------------------------------------------------- TMA producer: one thread, for which the
+    // warp's lanes fetch 32 entries of the block table at a time
+    const int* table = block_table + (size_t)(pos >= 0 ? slot_t : 0) * table_stride + pg_first;
     bool waited = SHARED;
     const uint64_t stream_policy = l2_policy_evict_first();   // a page is read once a step
+    int entry = 0;
     for (int i = 0; i < n_pages; ++i) {
-      const int s = i % STAGES;
-      const int pg = pg_first + i;
-      if (i >= STAGES) {
-        ok = mbar_wait(empty(s), ((i / STAGES) & 1) ^ 1, status, 41);
-        if (!ok) break;
-      }
-      if (pg == new_page && !waited) {           // this page was written to by the kernel before
-        pdl_wait();
-        waited = true;
-      }
-      const int row = (table[pg] * n_kv_heads + kv_head) * EK_PAGE;
-      const uint32_t dst = smem_u32(smem + s * kStage);
-      mbar_expect_tx(full(s), kStage);
+      if (i % 32 == 0 && i + lane < n_pages) entry = load_past_l1(table + i + lane);
+      const int page = __shfl_sync(0xffffffffu, entry, i % 32);
+      if (lane == 0) {
+        const int s = i % STAGES;
+        if (i >= STAGES) ok = mbar_wait(empty(s), ((i / STAGES) & 1) ^ 1, status, 41);
+        if (pg_first + i == new_page && !waited) {   // this page was written to by the kernel before
+          pdl_wait();
+          waited = true;
+        }
+        if (ok) {
+          const int row = (page * n_kv_heads + kv_head) * EK_PAGE;
+          const uint32_t dst = smem_u32(smem + s * kStage);
+          mbar_expect_tx(full(s), kStage);
 #pragma unroll
-      for (int j = 0; j < DB; ++j) {
-        tma_load_2d_hint(dst + j * kSub, &map_k, 64 * j, row, full(s), stream_policy);
-        if (!SHARED) tma_load_2d_hint(dst + (DB + j) * kSub, &map_v, 64 * j, row, full(s), stream_policy);
+          for (int j = 0; j < DB; ++j) {
+            tma_load_2d_hint(dst + j * kSub, &map_k, 64 * j, row, full(s), stream_policy);
+            if (!SHARED) tma_load_2d_hint(dst + (DB + j) * kSub, &map_v, 64 * j, row, full(s), stream_policy);
+          }
+        }
       }
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      if (!ok) break;
     }
   } else if (warp < W) {
     // ------------------------------------------------------------------- consumers

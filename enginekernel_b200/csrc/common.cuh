@@ -148,9 +148,19 @@ __device__ __forceinline__ float capped_log2(float s, SoftCap cap) {
 // reads anything that kernel wrote or writes anything that kernel reads (only constants -
 // weights, tables - may be touched earlier), and calls `pdl_launch_dependents()` at its top
 // so that its own successor can be set up early.  Both are no-ops in a plain launch.
+// The wait is also what makes the writes of kernels before it visible to ordinary loads.  Ahead of it an
+// SM's L1 may still hold a line from an earlier step, although the kernel that wrote the value since has
+// long finished: a captured step of a small model that looked up its positions ahead of the wait by plain
+// loads found those of the step before.  What changes from step to step and has to be read ahead of the
+// wait is read by `load_past_l1`, and only where a plain launch stands between its writer and the reader.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ int load_past_l1(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
 }
 
 // Split of an SM's 256 KB between L1 and shared memory that a kernel wants, in percent of

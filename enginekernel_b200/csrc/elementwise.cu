@@ -522,8 +522,8 @@ using namespace ek;
     if (n_tokens <= 0) return 0;                                                                \
     if (pos_table && (!positions || max_positions <= 0)) return EK_ERR_ARG;                     \
     /* A plain launch, on purpose: the first kernel of a step starts only when everything   */ \
-    /* before it on the stream has finished and is visible.  The kernels behind it may then */ \
-    /* read per-step state (positions, slots) before their own griddepcontrol.wait even     */ \
+    /* before it on the stream has finished.  The kernels behind it may then read per-step  */ \
+    /* state (positions, slots; by load_past_l1) before their own griddepcontrol.wait even   */ \
     /* when the step before was not a graph launch of its own (eager decode).               */ \
     embed_kernel<T><<<dim3(n_tokens), dim3(256), 0, stream>>>(resid, (const T*)table, ids,     \
                                                                hidden, vocab, scale,            \

@@ -28,8 +28,8 @@ namespace ek {
 //
 // What bounds it, with few tokens, is the chain of loads that wait for one another.  The gains are fetched before the wait
 // for the kernel ahead; behind it the row comes into registers while the token's place and its angles are looked up, and
-// both norms are one reduction.  (Reading positions before the wait as well gained nothing, and a captured step then
-// generated other tokens than an eager one.)
+// both norms are one reduction.  (Positions stand behind the wait: ahead of it an ordinary load may find the step before's,
+// see common.cuh, and reading them there gained nothing.)
 // 8 tokens of 768 + 192 + 64 values in a captured step: 6.2 us with every load in its place, now 2.1.
 constexpr int kPrepKeep = 8;         // values of the first part a thread keeps, and of the latent a quarter of that
 template <typename T>

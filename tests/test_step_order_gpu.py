@@ -84,3 +84,56 @@ def test_a_layer_driven_alone_reads_its_own_steps_table(kind):
     torch.cuda.synchronize()
     for i, y in enumerate(got):
         assert torch.equal(y, wants[i % len(steps)]), (i // len(steps), i % len(steps))
+
+
+@pytest.mark.parametrize("d,n_splits", [(64, 1), (64, 4), (128, 2), (256, 1), (256, 4)])
+def test_a_captured_decode_step_reads_this_steps_places(d, n_splits):
+    """Positions, slots and pages that change from step to step, looked up ahead of the wait: in a captured step of few
+    blocks, replayed back to back, every step's attention is the one of its own places (taken eagerly, the device idle)."""
+    from enginekernel_b200.ops import kernels as k
+    nq, nkv, past = 4, (1 if d == 256 else 2), 190
+    g = torch.Generator().manual_seed(3)
+    rand = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16).to(DEV)
+    pages = rand(9, nkv, 64, d)
+    values = pages if d == 256 else rand(9, nkv, 64, d)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    table = i32([[0, 2, 4, 6], [1, 3, 5, 7]])
+    positions, slots = i32([past, past - 70]), i32([0, 1])
+    q, out = rand(2, nq * d), torch.zeros(2, nq * d, dtype=torch.bfloat16, device=DEV)
+    stream, ids, vocab = torch.zeros(2, 64, device=DEV), i32([3, 5]), rand(8, 64)
+    normed, gain = torch.zeros(2, 64, dtype=torch.bfloat16, device=DEV), torch.ones(64, device=DEV)
+
+    def attend(to):
+        k.attention_decode_tma(to, q, 2, positions, slots, pages, values, table, nq, nkv, d, d ** -0.5, n_splits=n_splits)
+
+    def step():
+        positions.add_(1)                      # plain launches: what a step's state advance leaves behind
+        slots.copy_(1 - slots)
+        table.copy_(table.roll(1, 0))
+        k.embed(stream, vocab, ids, 2)         # the step's first kernel, a plain launch; the next are programmatic
+        k.rmsnorm(normed, stream, gain, 1e-5, n_rows=2)
+        attend(out)
+
+    at = lambda: [t.clone() for t in (positions, slots, table)]
+    start = at()
+    step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    for t, s in zip((positions, slots, table), start):
+        t.copy_(s)
+    got, places = [], []
+    for _ in range(12):
+        graph.replay()
+        got.append(out.clone())
+        places.append(at())
+    torch.cuda.synchronize()
+    for y, place in zip(got, places):
+        for t, s in zip((positions, slots, table), place):
+            t.copy_(s)
+        torch.cuda.synchronize()
+        want = torch.zeros_like(out)
+        attend(want)
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
