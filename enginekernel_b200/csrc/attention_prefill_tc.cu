@@ -82,10 +82,33 @@ constexpr float kBoundedCap = 40.f * 1.4426950408889634f;
 // Measured against the mma.sync kernel that took these prompts before: three of 2,500, 965 and 755 tokens under a
 // window of 1,024 with 4 kept, 16 heads of 128 on 8, gated: 215 -> 42 us; one of 2,048 tokens, 16 heads on rows of 256
 // (192 wanted): 216 -> 40 us (850 TFLOP/s of its 34 GFLOP).
+//
+// Without a table a block finds its tile in `seqs`: the tiles of a sequence from the last to the first, the sequences in
+// the order of the step.  The search costs a layer's pass 0 to 1 us (1,500 to 4,096 tokens); the table costs the step a
+// launch of 4 us and a call of the host, and is worth that where several layers read it or its order matters.
+struct FaSequences {
+  const int* cu_seqlens;
+  const int* positions;
+  const int* token_slot;
+  int count;
+};
+__device__ __forceinline__ int4 fa_find_tile(const FaSequences& seqs, int idx, int tok_per_tile) {
+  for (int b = 0; b < seqs.count; ++b) {
+    const int first = seqs.cu_seqlens[b], n = seqs.cu_seqlens[b + 1] - first;
+    const int tiles = (n + tok_per_tile - 1) / tok_per_tile;
+    if (idx < tiles) {
+      const int at = (tiles - 1 - idx) * tok_per_tile;       // long key ranges first
+      return make_int4(first + at, min(tok_per_tile, n - at), seqs.positions[first + at], seqs.token_slot[first + at]);
+    }
+    idx -= tiles;
+  }
+  return make_int4(0, 0, -1, 0);
+}
+
 template <int D, bool CAP, bool KEEP, bool SHARED>
 __global__ void __launch_bounds__(kFaThreads, SHARED ? 1 : 2)
 attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUtensorMap map_q,
-                            const int4* __restrict__ tiles,
+                            const int4* __restrict__ tiles, const FaSequences seqs,
                             const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const int* block_table,
                             int table_stride, int n_kv_heads, int n_q_heads, float scale_log2,
@@ -141,7 +164,8 @@ attention_prefill_tc_kernel(bf16* __restrict__ out, const __grid_constant__ CUte
   // search through the sequences and two more dependent loads in every block of every layer.  It is read behind
   // the wait: every kernel between the one that makes it and this one may be a programmatic launch that lets its
   // successor start at its top, and then nothing else says that the table is complete.
-  const int4 tile = __ldg(&tiles[blockIdx.y]);     // first token, tokens, position of the first, slot
+  // (first token, tokens, position of the first, slot)
+  const int4 tile = tiles != nullptr ? __ldg(&tiles[blockIdx.y]) : fa_find_tile(seqs, blockIdx.y, tok_per_tile);
   const int t_first = tile.x, n_tok = tile.y;      // (no tokens: the table is padded to the grid's size)
   const int n_rows = n_tok * group;
   const bool misplaced = (smem_u32(smem) & 1023u) != 0;   // never seen; the swizzled tiles would be wrong
@@ -505,7 +529,7 @@ attention_prefill_tiles_kernel(int4* tiles, int max_tiles, const int* cu_seqlens
 }
 
 template <int D, bool CAP, bool KEEP, bool SHARED>
-static int launch_fa(bf16* out, const bf16* q, int q_row_stride, const int4* tiles, int n_tiles, int n_tokens,
+static int launch_fa(bf16* out, const bf16* q, int q_row_stride, const int4* tiles, FaSequences seqs, int n_tiles, int n_tokens,
                      const void* k_pages, const void* v_pages, long long page_rows,
                      const int* block_table, int table_stride, int n_q_heads, int n_kv_heads,
                      float scale, int window, int* status, float sink, const float* sinks, int chunk,
@@ -535,7 +559,7 @@ static int launch_fa(bf16* out, const bf16* q, int q_row_stride, const int4* til
   prefer_carveout((const void*)kernel, 100);
   if (n_tiles > 65535) return EK_ERR_ARG;
   dim3 grid(n_kv_heads, n_tiles);
-  return (int)launch_pdl(kernel, grid, dim3(kFaThreads), smem, stream, out, mq, tiles, mk, mv, block_table,
+  return (int)launch_pdl(kernel, grid, dim3(kFaThreads), smem, stream, out, mq, tiles, seqs, mk, mv, block_table,
                          table_stride, n_kv_heads, n_q_heads, scale * 1.4426950408889634f,
                          window, tok_per_tile, status, sink * 1.4426950408889634f, sinks, chunk,
                          soft_cap(scale, softcap), keep_first, gate, gate_stride, v_cols);
@@ -560,7 +584,8 @@ EK_EXPORT int ek_attention_prefill_tiles(int* tiles, int max_tiles, const int* c
 
 // head_dim 64 or 128; the group (query heads per KV head) must divide 128; q rows 16-byte
 // aligned; n_pages = number of pages in k_pages / v_pages ([pages, kv heads, 64, head_dim]);
-// `tiles` / n_tiles: the table ek_attention_prefill_tiles made for this step and group size.
+// `tiles` / n_tiles: the table ek_attention_prefill_tiles made for this step and group size; null: blocks find their tiles in
+// cu_seqlens, positions and token_slot (n_seqs sequences), n_tiles then being a bound on their number.
 // `sink`: score of a key without a value that every query also sees (one more term in the softmax
 // denominator); -INFINITY for none.  `chunk` > 0 instead of a window: keys of a token's own chunk only.
 // `softcap` > 0: scores become softcap tanh(score / softcap).  `keep_first` > 0 (with a window): the sequence's first
@@ -568,6 +593,7 @@ EK_EXPORT int ek_attention_prefill_tiles(int* tiles, int max_tiles, const int* c
 // head's result.  head_dim 256 with one KV head: attention over rows that are keys and values alike (v_pages is
 // k_pages), any group up to 128, and only the first `v_cols` values (rounded up to 16) of every head are written.
 EK_EXPORT int ek_attention_prefill_tc(void* out, const void* q, int q_row_stride, const int* tiles,
+                                      const int* cu_seqlens, const int* positions, const int* token_slot, int n_seqs,
                                       int n_tiles, int n_tokens,
                                       const void* k_pages, const void* v_pages, int n_pages,
                                       const int* block_table, int table_stride, int n_q_heads,
@@ -581,15 +607,17 @@ EK_EXPORT int ek_attention_prefill_tc(void* out, const void* q, int q_row_stride
   const bool shared = head_dim == 256;
   if ((head_dim != 64 && head_dim != 128 && !shared) || n_kv_heads <= 0 || n_q_heads % n_kv_heads ||
       n_q_heads / n_kv_heads > kFaRows || (!shared && kFaRows % (n_q_heads / n_kv_heads)) || q_row_stride % 8 ||
-      ((uintptr_t)q & 15) || !status || !(scale > 0.f) || n_pages <= 0 || !tiles || ((uintptr_t)tiles & 15) ||
+      ((uintptr_t)q & 15) || !status || !(scale > 0.f) || n_pages <= 0 || ((uintptr_t)tiles & 15) ||
+      (!tiles && (!cu_seqlens || !positions || !token_slot || n_seqs <= 0)) ||
       (shared && (n_kv_heads != 1 || v_pages != k_pages || v_cols <= 0 || v_cols > head_dim || softcap > 0.f)))
     return EK_ERR_ARG;
   const long long page_rows = (long long)n_pages * n_kv_heads * EK_PAGE;
+  const FaSequences seqs{cu_seqlens, positions, token_slot, n_seqs};
   if (window <= 0) keep_first = 0;
   const bool keep = keep_first > 0 || gate != nullptr;
   v_cols = (v_cols + 15) / 16 * 16;
 #define EK_FA(D_, CAP_, KEEP_, SHARED_)                                                                  \
-  return launch_fa<D_, CAP_, KEEP_, SHARED_>((bf16*)out, (const bf16*)q, q_row_stride, (const int4*)tiles, n_tiles, \
+  return launch_fa<D_, CAP_, KEEP_, SHARED_>((bf16*)out, (const bf16*)q, q_row_stride, (const int4*)tiles, seqs, n_tiles, \
                              n_tokens, k_pages, v_pages, page_rows, block_table, table_stride, n_q_heads, \
                              n_kv_heads, scale, window, status, sink, sinks, chunk, softcap, keep_first, \
                              (const bf16*)gate, gate_stride, v_cols, stream)

@@ -923,7 +923,7 @@ def attention_prefill_f32(out, q, n_tokens, positions, token_slot, cu_seqlens, n
 
 
 _attn_prefill_tc = Function("attention_prefill_tc", "ek_attention_prefill_tc",
-                            [_P, _P, c_int, _P, c_int, c_int, _P, _P, c_int, _P, c_int, c_int,
+                            [_P, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, _P, _P, c_int, _P, c_int, c_int,
                              c_int, c_int, c_float, c_int, _P, c_float, _P, c_int, c_float, c_int, _P, c_int, c_int, _P])
 _attn_prefill_tiles = Function("attention_prefill_tc", "ek_attention_prefill_tiles",
                                [_P, c_int, _P, _P, _P, c_int, c_int, c_int, _P])
@@ -959,6 +959,18 @@ def attention_prefill_tc_supported(dtype, head_dim, n_q_heads, n_kv_heads):
 def attention_prefill_shared_supported(dtype, row, n_q_heads):
     """Rows that are keys and values alike (attention through a latent): 256 values, up to 128 heads on one."""
     return dtype == torch.bfloat16 and row == 256 and n_q_heads <= PREFILL_TC_ROWS
+
+
+def attention_prefill_tiles_pay(n_tokens, n_seqs, n_q_heads, n_kv_heads, device=None) -> bool:
+    """Whether a step's prompts are worth a table of tiles (:func:`attention_prefill_tiles`) to a layer that would be the
+    only one to use it: a call of the host and 4 us of the device, against blocks that look their tiles up in the step's
+    order.  From two and a half fillings of the machine on (two blocks an SM) by several sequences, whose tiles the
+    order mixes: a windowed layer's pass over 8 prompts, 16 heads of 128 on 8, 6,467 tokens (2.9 fillings): 270 us without,
+    264 with; 5,070 tokens (2.4): 203 both; 2,174 tokens (1.1): 92 without, 96 with; one prompt of 4,096: 188 and 191.
+    Short prompts wait for the host: 9 tokens 87 us a pass without, 100 with.  (Attention over latents, whose group is all
+    heads, makes none: 84 against 88 us for 1,500 tokens, 255 against 261 for 6,467 in 8 prompts.)"""
+    blocks = (n_tokens // (PREFILL_TC_ROWS // (n_q_heads // n_kv_heads)) + n_seqs) * n_kv_heads
+    return n_seqs > 1 and blocks > 5 * sm_count(device)
 
 
 _l2_bytes = {}
@@ -1004,36 +1016,40 @@ def attention_prefill_tc(out, q, n_tokens, positions, token_slot, cu_seqlens, n_
     that divide 128): TMA-fed pages, scores and P.V in TMEM.  With ``v_cols``, rows of 256 values that are keys and
     values alike (``v_pages`` is ``k_pages``, one KV head, up to 128 query heads): only the first ``v_cols`` values of a
     head's result are written.  ``tiles`` / ``n_tiles``: the table
-    :func:`attention_prefill_tiles` made for this step (made once and used by every layer); without it the
-    table is made here."""
+    :func:`attention_prefill_tiles` made for this step (made once and used by every layer); without it every
+    block looks its tile up in ``cu_seqlens``, in the step's order.  The results are the same either way."""
     _need_cuda(out, q, positions, token_slot, cu_seqlens, k_pages, v_pages, block_table, tiles)
+    dtype, q_stride, q_at, group = q.dtype, q.stride(0), q.data_ptr(), n_q_heads // n_kv_heads
+    k_at, v_at = k_pages.data_ptr(), v_pages.data_ptr()
     if v_cols is not None:
-        _need(attention_prefill_shared_supported(q.dtype, head_dim, n_q_heads) and n_kv_heads == 1
-              and v_pages.data_ptr() == k_pages.data_ptr() and 0 < v_cols <= head_dim and not softcap,
+        _need(attention_prefill_shared_supported(dtype, head_dim, n_q_heads) and n_kv_heads == 1
+              and v_at == k_at and 0 < v_cols <= head_dim and not softcap,
               "attention_prefill_tc: shared rows are 256 bfloat16 values of one KV head, without a soft cap")
     else:
-        _need(attention_prefill_tc_supported(q.dtype, head_dim, n_q_heads, n_kv_heads),
+        _need(attention_prefill_tc_supported(dtype, head_dim, n_q_heads, n_kv_heads),
               "attention_prefill_tc: bfloat16, head size 64 or 128, a group size that divides 128")
-    _need(out.dtype == q.dtype == k_pages.dtype, "attention: one dtype for q, cache and out")
+    _need(out.dtype == dtype == k_pages.dtype, "attention: one dtype for q, cache and out")
     _need(out.is_contiguous() and out.shape[-1] == n_q_heads * head_dim, "attention: out [T, NQ*D]")
-    _need(q.stride(-1) == 1 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0,
-          "attention: dense, 16-byte aligned q rows")
-    _need(k_pages.is_contiguous() and v_pages.is_contiguous() and k_pages.dim() == 4
-          and k_pages.shape[1:] == (n_kv_heads, PAGE, head_dim), "attention: pages [P, NKV, 64, D]")
+    _need(q.stride(-1) == 1 and q_stride % 8 == 0 and q_at % 16 == 0, "attention: dense, 16-byte aligned q rows")
+    n_pages, *page = k_pages.shape
+    _need(k_pages.is_contiguous() and (v_pages is k_pages or v_pages.is_contiguous()) and page == [n_kv_heads, PAGE, head_dim],
+          "attention: pages [P, NKV, 64, D]")
     if tiles is None:
-        tok_per_tile = PREFILL_TC_ROWS // (n_q_heads // n_kv_heads)
-        tiles = torch.empty((-(-n_tokens // tok_per_tile) + n_seqs, 4), dtype=torch.int32, device=q.device)
-        n_tiles = attention_prefill_tiles(tiles, n_tokens, positions, token_slot, cu_seqlens, n_seqs,
-                                          n_q_heads, n_kv_heads, head_dim)
-    _need(tiles.dtype == torch.int32 and tiles.numel() >= 4 * n_tiles and tiles.data_ptr() % 16 == 0,
-          "attention_prefill_tc: the table of tiles")
-    _attention_cost(q, n_tokens, positions, n_q_heads, n_kv_heads, head_dim, window, True, chunk)
-    _attn_prefill_tc(_ptr(out), _ptr(q), q.stride(0), _ptr(tiles), n_tiles, n_tokens, _ptr(k_pages),
-                     _ptr(v_pages), k_pages.shape[0], _ptr(block_table), block_table.stride(0), n_q_heads,
-                     n_kv_heads, head_dim, float(scale), int(window or 0),
-                     _ptr(tc_status(q.device)), _sink(sink), _sinks(sinks, n_q_heads), int(chunk or 0),
-                     float(softcap or 0.0), int(keep_first or 0), *_gate_args(gate, q, n_q_heads), int(v_cols or 0),
-                     _stream())
+        _need(n_seqs <= PREFILL_TC_MAX_SEQS, "attention_prefill_tc: at most 1024 sequences a step")
+        _need(cu_seqlens.dtype == torch.int32 and cu_seqlens.numel() > n_seqs, "attention: cu_seqlens")
+        tiles_at, n_tiles = None, n_tokens // (PREFILL_TC_ROWS // group) + n_seqs
+    else:
+        tiles_at = tiles.data_ptr()
+        _need(tiles.dtype == torch.int32 and tiles.numel() >= 4 * n_tiles and tiles_at % 16 == 0,
+              "attention_prefill_tc: the table of tiles")
+    if lib.recording():
+        _attention_cost(q, n_tokens, positions, n_q_heads, n_kv_heads, head_dim, window, True, chunk)
+    gate_at, gate_stride = (None, 0) if gate is None else _gate_args(gate, q, n_q_heads)
+    _attn_prefill_tc(out.data_ptr(), q_at, q_stride, tiles_at, cu_seqlens.data_ptr(), positions.data_ptr(),
+                     token_slot.data_ptr(), n_seqs, n_tiles, n_tokens, k_at, v_at, n_pages, block_table.data_ptr(),
+                     block_table.stride(0), n_q_heads, n_kv_heads, head_dim, float(scale), int(window or 0),
+                     tc_status(q.device).data_ptr(), _sink(sink), _sinks(sinks, n_q_heads), int(chunk or 0),
+                     float(softcap or 0.0), int(keep_first or 0), gate_at, gate_stride, int(v_cols or 0), _stream())
 
 
 # ------------------------------------------------------------------ matrix products
@@ -1067,10 +1083,11 @@ _sm_counts = {}
 
 def sm_count(device=None) -> int:
     """Streaming multiprocessors of ``device`` (the current one if None), asked once."""
-    if not torch.cuda.is_available():
+    if not _sm_counts and not torch.cuda.is_available():
         return B200_SM_COUNT
-    index = torch.cuda.current_device() if device is None or torch.device(device).index is None \
-        else torch.device(device).index
+    index = None if device is None else device.index if type(device) is torch.device else torch.device(device).index
+    if index is None:
+        index = _raw_device() if _sm_counts and _raw_device is not None else torch.cuda.current_device()
     if index not in _sm_counts:
         _sm_counts[index] = int(torch.cuda.get_device_properties(index).multi_processor_count)
     return _sm_counts[index]
@@ -1101,10 +1118,13 @@ TC_SWAP_MAX_ROWS = 64
 
 def tc_status(device):
     """One int per device that the tensor-core GEMM sets when a barrier wait times out."""
-    key = str(torch.device(device))
-    if key not in _tc_status:
-        _tc_status[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _tc_status[key]
+    status = _tc_status.get(device)              # (by the torch.device that launches hand over)
+    if status is None:
+        key = torch.device(device)
+        if key not in _tc_status:
+            _tc_status[key] = torch.zeros(1, dtype=torch.int32, device=device)
+        status = _tc_status[key]
+    return status
 
 
 def check_tc_status(device):

@@ -81,7 +81,7 @@ def make_prefill_tiles(ctx, key, num_heads, num_kv_heads, head_dim):
 
 
 def prefill_tiles(ctx, key):
-    """The table made for this step as arguments of the kernel (a part driven alone has none)."""
+    """The table made for this step as arguments of the kernel (none, where it does not pay or a part is driven alone)."""
     made = ctx.shared.get(key)
     return {} if made is None else dict(tiles=made[0], n_tiles=made[1])
 
@@ -186,6 +186,10 @@ class Attention(Mixer):
             kernels.check_head_dim(self.padded_dim)
             # (this path takes normalised activations and returns a plain tensor)
             self.takes_deferred_norm = self.defers_norm = False
+        #: whether prompts run on the tcgen05 kernel, and the key of their table of tiles
+        self.prompts_on_tc = self.scale > 0 and kernels.attention_prefill_tc_supported(
+            dtype, self.padded_dim, self.num_heads, self.num_kv_heads)
+        self._tiles_key = ("prefill_tc_tiles", self.num_heads // self.num_kv_heads, self.num_kv_heads * self.padded_dim)
         if self.output_biased:                   # (the product alone is not the result yet)
             self.defers_norm = False
         pos = spec.params.get("position")
@@ -204,18 +208,16 @@ class Attention(Mixer):
         if self.position is not None:
             self.position.prepare(max_positions)
 
-    def _tiles_key(self):
-        return ("prefill_tc_tiles", self.num_heads // self.num_kv_heads, self.num_kv_heads * self.padded_dim)
-
     def _on_prefill_tc(self, ctx):
         """Whether a prompt of this step runs on the tcgen05 kernel."""
-        return (not ctx.is_decode and ctx.n_seqs <= kernels.PREFILL_TC_MAX_SEQS and self.scale > 0
-                and kernels.attention_prefill_tc_supported(self.dtype, self.padded_dim, self.num_heads, self.num_kv_heads))
+        return self.prompts_on_tc and not ctx.is_decode and ctx.n_seqs <= kernels.PREFILL_TC_MAX_SEQS
 
     def begin_step(self, ctx):
-        """The table of tiles of the tcgen05 prompt attention, once per step and shape of the heads."""
-        if self._on_prefill_tc(ctx):
-            make_prefill_tiles(ctx, self._tiles_key(), self.num_heads, self.num_kv_heads, self.padded_dim)
+        """The table of tiles of the tcgen05 prompt attention, once per step and shape of the heads.  (``general`` layers
+        make none for short prompts, which the ``mma.sync`` kernel took without one before.)"""
+        if self._on_prefill_tc(ctx) and (not self.general or kernels.attention_prefill_tiles_pay(
+                ctx.n_tokens, ctx.n_seqs, self.num_heads, self.num_kv_heads, device=self.device)):
+            make_prefill_tiles(ctx, self._tiles_key, self.num_heads, self.num_kv_heads, self.padded_dim)
 
     def _by_head(self, t, n, reorder):
         """[n * size, ...] -> [n * padded_dim, ...]: a head's values in the kernels' order (``reorder``: they turn
@@ -299,7 +301,7 @@ class Attention(Mixer):
             kernels.attention_prefill_tc(out, rows, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
                                          entry.k_pages, entry.v_pages, entry.block_table, nh, nkv, big, self.scale,
                                          self.window, keep_first=self.keep_first, gate=gate, **mask,
-                                         **prefill_tiles(ctx, self._tiles_key()))
+                                         **prefill_tiles(ctx, self._tiles_key))
             return self._project(out, ctx, None, leave_bias)
         if not ctx.is_decode and kernels.attention_prefill_supported(self.dtype, big, nh, nkv):
             kernels.attention_prefill_bf16(out, rows, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
@@ -495,7 +497,7 @@ class Attention(Mixer):
                 self.dtype, self.head_dim, self.num_heads, self.num_kv_heads):
             prefill, extra = kernels.attention_prefill_bf16, {}
             if self._on_prefill_tc(ctx):
-                prefill, extra = kernels.attention_prefill_tc, prefill_tiles(ctx, self._tiles_key())   # tcgen05
+                prefill, extra = kernels.attention_prefill_tc, prefill_tiles(ctx, self._tiles_key)   # tcgen05
             prefill(
                 out, qkv, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
                 entry.k_pages, entry.v_pages, entry.block_table, self.num_heads, self.num_kv_heads,

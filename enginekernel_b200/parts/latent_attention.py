@@ -43,7 +43,6 @@ import torch
 from ..ops import kernels
 from ..ops.linear import linear
 from ..registry import lookup_part, register_part
-from .attention import make_prefill_tiles, prefill_tiles
 from .base import Mixer
 from .rope import neighbours_to_halves
 from .spec import CacheSpec, TensorSpec
@@ -97,6 +96,8 @@ class LatentAttention(Mixer):
         if self.row > kernels.GENERIC_MAX_HEAD_DIM:
             raise kernels.KernelError(f"latent_attention: a cached row of {self.row} values (kv_rank + rot_dim) exceeds "
                                       f"the attention kernels' limit of {kernels.GENERIC_MAX_HEAD_DIM}")
+        #: whether prompts run on the tcgen05 kernel
+        self.prompts_on_tc = self.scale > 0 and kernels.attention_prefill_shared_supported(dtype, self.row, self.num_heads)
         #: values of a row's first part: the query latent, or the plain queries (and gates behind them) up to a
         #: multiple of 64
         self.front = self.q_rank if self.q_rank is not None else \
@@ -112,15 +113,7 @@ class LatentAttention(Mixer):
             self.position.prepare(max_positions)
 
     def _on_prefill_tc(self, ctx):
-        return (not ctx.is_decode and ctx.n_seqs <= kernels.PREFILL_TC_MAX_SEQS and self.scale > 0
-                and kernels.attention_prefill_shared_supported(self.dtype, self.row, self.num_heads))
-
-    def _tiles_key(self):
-        return ("prefill_tc_tiles", self.num_heads, self.row)
-
-    def begin_step(self, ctx):
-        if self._on_prefill_tc(ctx):
-            make_prefill_tiles(ctx, self._tiles_key(), self.num_heads, 1, self.row)
+        return self.prompts_on_tc and not ctx.is_decode and ctx.n_seqs <= kernels.PREFILL_TC_MAX_SEQS
 
     def load(self, tensors):
         w = self.spec.weights
@@ -199,7 +192,7 @@ class LatentAttention(Mixer):
         if self._on_prefill_tc(ctx):
             kernels.attention_prefill_tc(out, q, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,
                                          pages, pages, table, nh, 1, row, self.scale, self.window, v_cols=self.kv_rank,
-                                         **common, **prefill_tiles(ctx, self._tiles_key()))
+                                         **common)
             return
         if not ctx.is_decode and kernels.attention_prefill_supported(self.dtype, row, nh, 1):
             kernels.attention_prefill_bf16(out, q, t, ctx.positions, ctx.token_slot, ctx.cu_seqlens, ctx.n_seqs,

@@ -27,6 +27,15 @@ def test_the_benchmark_shape_gets_the_splits_the_profiles_name():
     assert kernels.swap_k_split(2560, 9728, kernels.EPI_BF16) == 8      # down
 
 
+def test_short_prompts_of_general_layers_make_no_table_of_tiles():
+    """The rule at its line: several sequences, and more than two and a half fillings of the machine with two blocks an SM."""
+    sms = kernels.sm_count()
+    pays = lambda tokens, seqs: kernels.attention_prefill_tiles_pay(tokens, seqs, 16, 8)      # 64 tokens a tile, 8 key heads
+    line = 5 * sms // 8 + 1                                 # tiles (of 8 blocks each) from which it pays
+    assert not pays(9, 1) and not pays(36, 8) and not pays(512, 3) and not pays(64 * (line - 3), 2)
+    assert pays(64 * (line - 2), 2) and pays(64 * line, 8) and not pays(1 << 20, 1)
+
+
 def test_launch_record_groups_costs_and_issues_again():
     """The record behind the per-kernel tables, without a GPU: entries keep their order, are named
     with their label, sum their costs by name, and are issued again by name."""

@@ -86,6 +86,18 @@ def test_a_layer_driven_alone_reads_its_own_steps_table(kind):
         assert torch.equal(y, wants[i % len(steps)]), (i // len(steps), i % len(steps))
 
 
+@pytest.mark.parametrize("kind", ["attention", "window"])
+def test_tiles_found_by_the_blocks_are_those_of_the_table(kind):
+    """A step with a table of tiles and without one: the same results, for sequences of one token to several tiles."""
+    from enginekernel_b200.parts.attention import make_prefill_tiles
+    part = layer(kind)
+    x, ctx, entry = prompts(part, [1, 300, 64, 65, 17, 128, 2], 5)
+    ctx.shared = {}
+    alone = part.forward(x, ctx, entry, True).clone()
+    make_prefill_tiles(ctx, part._tiles_key, part.num_heads, part.num_kv_heads, part.padded_dim)
+    assert torch.equal(part.forward(x, ctx, entry, True), alone)
+
+
 @pytest.mark.parametrize("d,n_splits", [(64, 1), (64, 4), (128, 2), (256, 1), (256, 4)])
 def test_a_captured_decode_step_reads_this_steps_places(d, n_splits):
     """Positions, slots and pages that change from step to step, looked up ahead of the wait: in a captured step of few
