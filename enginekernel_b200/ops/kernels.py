@@ -1916,11 +1916,13 @@ def decay_scan_lane_columns(columns, max_new, dim=DECAY_SCAN_MAX_KEY_DIM) -> int
     return 4 if columns > 2 * SCAN_COLUMNS and dim > 32 else 2
 
 
-def decay_scan_segments(n_seqs, heads, columns, max_new, device=None, n_tokens=0):
+def decay_scan_segments(n_seqs, heads, columns, max_new, device=None, n_tokens=0, lane_columns=None):
     """(segments of the longest sequence, tokens a segment) that :func:`decay_scan` cuts a step's sequences into; one
     segment where the sequences, heads and columns fill the machine, or the sequences are short.  ``n_tokens`` (of all
-    sequences, if known) tells a ragged batch, whose longest sequence is left alone at the end, from an even one."""
-    lane_columns = decay_scan_lane_columns(columns, max_new)
+    sequences, if known) tells a ragged batch, whose longest sequence is left alone at the end, from an even one.
+    ``lane_columns``: what the launch takes (:func:`decay_scan_lane_columns` for the widest keys, unless given)."""
+    if lane_columns is None:
+        lane_columns = decay_scan_lane_columns(columns, max_new)
     blocks = n_seqs * heads * -(-columns // (SCAN_COLUMNS * lane_columns))
     most, sms = -(-max_new // SCAN_MIN_SEGMENT), sm_count(device)
     want = min(SCAN_BLOCKS_PER_SM * sms // blocks, most)
@@ -1957,8 +1959,9 @@ def decay_scan(out, q, k, v, a, b, state, cu_seqlens, positions, token_slot, n_s
                                 + 2 * n_seqs * heads * cols * decay_scan_rows(dim)),
                      flops=4 * n_tokens * heads * dim * cols)
     parts, length, carry, prods = 1, 0, None, None
+    lane_columns = lane_columns or decay_scan_lane_columns(cols, max_new, dim)
     if workspace is not None and max_new > 1:
-        parts, length = segments or decay_scan_segments(n_seqs, heads, cols, max_new, out.device, n_tokens)
+        parts, length = segments or decay_scan_segments(n_seqs, heads, cols, max_new, out.device, n_tokens, lane_columns)
         _need(length >= 1 and parts * length >= max_new, "decay_scan: the segments cover the longest sequence")
         if parts > 1:
             carry = workspace.get("scan_carry", (n_seqs, parts, heads * cols * decay_scan_rows(dim)), torch.float32)
@@ -1967,7 +1970,7 @@ def decay_scan(out, q, k, v, a, b, state, cu_seqlens, positions, token_slot, n_s
                 _ptr(a), _ptr(b), _ptr(state), state.stride(0), _ptr(cu_seqlens), _ptr(positions), _ptr(token_slot),
                 n_seqs, heads, kv_heads, dim, vdim, 1 if ones_column else 0, 1 if write_state else 0,
                 heads if a.dim() > 1 else 0, _ptr(carry), _ptr(prods), parts, length,
-                lane_columns or decay_scan_lane_columns(cols, max_new, dim), _stream())
+                lane_columns, _stream())
     if parts > 1:
         count_extra_launches()
 

@@ -1,8 +1,10 @@
 """Host-side choices of how a product is cut into blocks (no GPU needed)."""
 
 import pytest
+import torch
 
 from enginekernel_b200.ops import kernels
+from enginekernel_b200.parts.base import Workspace
 
 
 @pytest.mark.parametrize("n_out,k,epi", [
@@ -34,6 +36,28 @@ def test_short_prompts_of_general_layers_make_no_table_of_tiles():
     line = 5 * sms // 8 + 1                                 # tiles (of 8 blocks each) from which it pays
     assert not pays(9, 1) and not pays(36, 8) and not pays(512, 3) and not pays(64 * (line - 3), 2)
     assert pays(64 * (line - 2), 2) and pays(64 * line, 8) and not pays(1 << 20, 1)
+
+
+@pytest.mark.parametrize("dim,lane_columns", [(20, 2), (32, 2), (33, 4), (128, 4)])
+def test_segments_are_planned_with_the_columns_that_the_scan_takes(dim, lane_columns, monkeypatch):
+    """64 columns: keys of up to 32 values are walked two columns a lane, wider ones four; the scan is cut for the blocks
+    that it launches, and its launch gets the same number."""
+    assert kernels.decay_scan_lane_columns(64, 2048, dim) == lane_columns
+    blocks = 64 * 64 // (kernels.SCAN_COLUMNS * lane_columns)
+    want = min(kernels.SCAN_BLOCKS_PER_SM * kernels.sm_count() // blocks, 2048 // kernels.SCAN_MIN_SEGMENT)
+    length = -(-(-(-2048 // want)) // 64) * 64
+    plan = (-(-2048 // length), length)
+    assert kernels.decay_scan_segments(1, 64, 64, 2048, lane_columns=lane_columns) == plan
+    launched = []
+    monkeypatch.setattr(kernels, "_need_cuda", lambda *tensors: None)
+    monkeypatch.setattr(kernels, "_decay_scan", lambda *args: launched.append(args))
+    monkeypatch.setattr(kernels, "_stream", lambda: 0)
+    rows = kernels.decay_scan_rows(dim)
+    f32, i32 = (lambda *s: torch.zeros(*s)), (lambda n: torch.zeros(n, dtype=torch.int32))
+    kernels.decay_scan(f32(2048, 64 * 64), f32(2048, dim), f32(2048, dim), f32(2048, 64 * 64), f32(2048, 64),
+                       f32(2048, 64), f32(1, 64 * 64 * rows), i32(2), i32(2048), i32(2048), 1, 64, 1, dim, 64, n_tokens=2048,
+                       max_new=2048, workspace=Workspace(torch.device("cpu")))
+    assert launched[0][-4:-1] == (*plan, lane_columns)
 
 
 def test_launch_record_groups_costs_and_issues_again():
