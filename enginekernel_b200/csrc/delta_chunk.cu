@@ -450,8 +450,6 @@ static int launch_chunks(float* o, float* w, float* qp, float* kh, float* v, flo
 
 }  // namespace ek
 
-EK_EXPORT int ek_delta_chunk_tokens() { return ek::kChunk; }
-
 // The recurrence of ek_delta_scan for key sizes 64 and 128 and value sizes in steps of 4 up to twice that, by chunks.
 // `v` [T, heads vdim] is overwritten; `decay` too, unless `kh` is memory of its own (decay_per_head needs that).
 // w, qp, kh: [T, heads dim] of scratch; gam: [chunks, heads, dim], chunks = the sequences' tokens / 32 rounded up, summed.

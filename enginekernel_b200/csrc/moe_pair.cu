@@ -326,10 +326,6 @@ static bool moe_pair_args(const void* x, const void* w, int N, int K, int n_expe
 
 }  // namespace ek
 
-// The most pairs of a tile, and what tiles are rounded up to (the plan's tile_rows and even).
-EK_EXPORT int ek_moe_pair_tile_rows() { return ek::kMoeTile; }
-EK_EXPORT int ek_moe_pair_even() { return ek::kMoeEven; }
-
 // `gathered`: x holds a row per pair in the plan's order (n_rows pairs) instead of one per token (n_rows tokens).
 EK_EXPORT int ek_moe_pair_up(void* out, const void* x, const void* w, const int* tiles, const int* n_tiles,
                              const int* sorted_pair, int n_rows, int gathered, int n_experts, int max_tiles, int top, int N, int K,

@@ -43,15 +43,6 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
       ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
-__device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
-}
-
 // One stage of the pair's product in one piece of PTX: ask the NEXT stage's barrier (test_wait: it
 // answers at once and never suspends the thread, unlike try_wait), issue this stage's four MMAs (K = 16 each, 32 bytes further along the swizzled row), commit them to this stage's "empty"
 // barrier in both blocks, and only then look at the barrier's answer - the thread does not wait for it

@@ -878,7 +878,7 @@ def attention_prefill_bf16(out, q, n_tokens, positions, token_slot, cu_seqlens, 
 _attn_prefill_f32 = Function("attention_prefill_f32", "ek_attention_prefill_f32",
                              [_P, _P, c_int, _P, _P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, c_int, c_int,
                               c_float, c_int, c_float, _P, c_int, _P, c_int, c_int, c_float, _P])
-PREFILL_F32_ROWS = 64           # tokens a block of attention_prefill_f32 takes
+PREFILL_F32_ROWS = 64           # tokens a block of attention_prefill_f32 takes; must equal kF32Rows there
 PREFILL_F32_ROUND = 1024        # (see attention_prefill_f32_wins)
 
 
@@ -947,7 +947,7 @@ def attention_prefill_cross_bf16(parts, q, n_tokens, positions, token_slot, cu_s
                         n_kv_heads, head_dim, float(scale), int(window or 0), int(keep_first or 0), _stream())
 
 
-PREFILL_TC_ROWS = 128       # (token, query head of a group) rows a block of attention_prefill_tc owns
+PREFILL_TC_ROWS = 128       # (token, query head of a group) rows a block of attention_prefill_tc owns; must equal kFaRows there
 PREFILL_TC_MAX_SEQS = 1024
 
 
@@ -1901,7 +1901,8 @@ def xgate_scan(a, b, m_run, proj, col_i, col_f, bias_i, bias_f, cap, state, m_of
                 _ptr(token_slot), n_seqs, heads, 1 if write_state else 0, _stream())
 
 
-SCAN_COLUMNS = 16           # columns of S a block of the decay scan takes, one a lane; two or four times as many with more
+SCAN_COLUMNS = 16           # columns of S a block of the decay scan takes, one a lane; two or four times as many with more;
+                            # must equal kScanCols in csrc/recurrent.cu
 SCAN_WIDE_TOKENS = 64       # sequences of at least this many tokens take two or four columns a lane
 SCAN_BLOCKS_PER_SM = 6      # what a cut of long prompts into segments aims at
 SCAN_MIN_SEGMENT = 128      # tokens

@@ -1,9 +1,12 @@
 """Host-side choices of how a product is cut into blocks (no GPU needed)."""
 
+import os
+import re
+
 import pytest
 import torch
 
-from enginekernel_b200.ops import kernels
+from enginekernel_b200.ops import build, kernels
 from enginekernel_b200.parts.base import Workspace
 
 
@@ -58,6 +61,18 @@ def test_segments_are_planned_with_the_columns_that_the_scan_takes(dim, lane_col
                        f32(2048, 64), f32(1, 64 * 64 * rows), i32(2), i32(2048), i32(2048), 1, 64, 1, dim, 64, n_tokens=2048,
                        max_new=2048, workspace=Workspace(torch.device("cpu")))
     assert launched[0][-4:-1] == (*plan, lane_columns)
+
+
+@pytest.mark.parametrize("name,source,constant", [
+    ("DELTA_CHUNK", "delta_chunk.cu", "kChunk"), ("MOE_TILE_ROWS", "moe.cu", "kTileRows"),
+    ("MOE_PAIR_TILE_ROWS", "moe_pair.cu", "kMoeTile"), ("MOE_PAIR_EVEN", "moe_pair.cu", "kMoeEven"),
+    ("PREFILL_F32_ROWS", "attention_prefill_f32.cu", "kF32Rows"), ("PREFILL_TC_ROWS", "attention_prefill_tc.cu", "kFaRows"),
+    ("SCAN_COLUMNS", "recurrent.cu", "kScanCols")])
+def test_sizes_that_host_and_kernels_share(name, source, constant):
+    """What the host sizes grids and scratch by is what the kernels are built with."""
+    with open(os.path.join(build.CSRC, source)) as f:
+        (value,) = re.findall(rf"constexpr int {constant} = (\d+)", f.read())
+    assert getattr(kernels, name) == int(value)
 
 
 def test_launch_record_groups_costs_and_issues_again():
