@@ -66,6 +66,9 @@ class RoutedExperts(FeedForward):
         super().__init__(spec, dtype, device)
         g = lambda n: int(self.param(n))
         self.hidden, self.inter, self.experts, self.top = g("hidden_size"), g("intermediate_size"), g("experts"), g("top")
+        #: the experts' size that the kernels see: whole 16-byte pieces, which their form on pairs of SMs takes (the values
+        #: behind the last are zero rows of ``up`` and zero columns of ``down``)
+        self.inner = -(-self.inter // 8) * 8 if dtype == torch.bfloat16 else self.inter
         self.groups = int(spec.params.get("groups") or 1)
         self.keep = int(spec.params.get("keep") or self.groups)
         self.scale = float(spec.params.get("scale", 1.0))
@@ -106,12 +109,16 @@ class RoutedExperts(FeedForward):
         self.w_router = torch.cat([router, router.new_zeros((-self.routed % 16, self.hidden))], 0).to(self.dtype).contiguous()
         if self.corrected:
             self.correction = tensors[w["correction"]].to(torch.float32).contiguous()
+        more = self.inner - self.inter
         ups = [tensors[w[f"up_{e}"]] for e in range(self.experts)]
         if self.gated:               # rows gate_0, up_0, gate_1, up_1, ... of every expert
             ups = [torch.stack([tensors[w[f"gate_{e}"]], up], 1).reshape(2 * self.inter, self.hidden)
                    for e, up in enumerate(ups)]
-        self.w_up = torch.stack(ups).to(self.dtype).contiguous()
-        self.w_down = torch.stack([tensors[w[f"down_{e}"]] for e in range(self.experts)]).to(self.dtype).contiguous()
+        w_up, w_down = torch.stack(ups), torch.stack([tensors[w[f"down_{e}"]] for e in range(self.experts)])
+        if more:
+            w_up = torch.nn.functional.pad(w_up, (0, 0, 0, 2 * more if self.gated else more))
+            w_down = torch.nn.functional.pad(w_down, (0, more))
+        self.w_up, self.w_down = w_up.to(self.dtype).contiguous(), w_down.to(self.dtype).contiguous()
 
     def bytes_read_per_step(self, n_tokens):
         """The router and the experts that ``n_tokens`` tokens can reach at most."""
@@ -133,7 +140,7 @@ class RoutedExperts(FeedForward):
         tiles = ws.get("moe_tiles", (kernels.moe_max_tiles(pairs, self.experts, wide), 3), torch.int32)
         n_tiles = ws.get("moe_n_tiles", (1,), torch.int32)
         kernels.moe_plan(sorted_pair, tiles, n_tiles, chosen, pairs, self.experts, wide=wide)
-        act = ws.get("moe_act", (pairs, self.inter), self.dtype)
+        act = ws.get("moe_act", (pairs, self.inner), self.dtype)
         pair_out = ws.get("moe_pair_out", (pairs, self.hidden), torch.float32)      # (free until the down product)
         kernels.moe_expert_up(act, x, self.w_up, tiles, n_tiles, sorted_pair, pairs, top, self.activation,
                               gated=self.gated, limit=self.limit, input_weight=weight if self.weigh_input else None, wide=wide,

@@ -75,6 +75,31 @@ def test_sizes_that_host_and_kernels_share(name, source, constant):
     assert getattr(kernels, name) == int(value)
 
 
+@pytest.mark.parametrize("inter,gated", [(20, True), (20, False), (9, True), (24, True)])
+def test_experts_of_any_size_run_on_pairs_of_sms(inter, gated):
+    """bfloat16 experts whose size is no whole number of 16-byte pieces: laid out so that both products take the form on
+    pairs of SMs, with zeros behind the last value; in 32-bit as they are."""
+    from enginekernel_b200.parts.spec import PartSpec
+    from enginekernel_b200.registry import lookup_part
+    h, n = 32, 3
+    g = torch.Generator().manual_seed(1)
+    w = {"router": torch.randn(n, h, generator=g)}
+    for e in range(n):
+        w.update({f"gate_{e}": torch.randn(inter, h, generator=g), f"up_{e}": torch.randn(inter, h, generator=g),
+                  f"down_{e}": torch.randn(h, inter, generator=g)})
+    params = dict(hidden_size=h, intermediate_size=inter, experts=n, top=2, activation="silu", gated=gated)
+    for dtype in (torch.bfloat16, torch.float32):
+        part = lookup_part("feed_forward", "routed_experts")(PartSpec("routed_experts", params, {k: k for k in w}), dtype, "cpu")
+        part.load(w)
+        if dtype == torch.bfloat16:
+            assert kernels.moe_on_pairs(torch.zeros(5, h, dtype=dtype), part.w_up, part.w_down)
+        for e in range(n):
+            rows = part.w_up[e, :2 * inter].view(inter, 2, h) if gated else part.w_up[e, :inter].view(inter, 1, h)
+            assert torch.equal(rows[:, -1], w[f"up_{e}"].to(dtype)) and torch.equal(rows[:, 0], w[f"gate_{e}" if gated else f"up_{e}"].to(dtype))
+            assert torch.equal(part.w_down[e, :, :inter], w[f"down_{e}"].to(dtype))
+        assert not part.w_up[:, (2 if gated else 1) * inter:].any() and not part.w_down[:, :, inter:].any()
+
+
 def test_launch_record_groups_costs_and_issues_again():
     """The record behind the per-kernel tables, without a GPU: entries keep their order, are named
     with their label, sum their costs by name, and are issued again by name."""
