@@ -893,10 +893,11 @@ def attention_prefill_f32_wins(n_tokens, n_seqs, n_q_heads, visible, device):
     600,000 (token, head, key, dimension) products a microsecond once it fills the GPU.  Both grow with the keys
     and the head size alike, which leaves the rows: 1,024 (token, head) rows for every round of blocks (heads of
     128, keys before the prompt: 32 tokens x 16 heads 118 us here against 215, 64 x 32 1,565 against 780).  Below
-    two pages of keys what a block fetches first decides (64 tokens x 16 heads alone: 15 us against 22)."""
-    blocks = (n_tokens // PREFILL_F32_ROWS + n_seqs) * n_q_heads
-    rounds = -(-blocks // (2 * sm_count(device)))
-    return visible >= 2 * PAGE and n_tokens * n_q_heads >= PREFILL_F32_ROUND * rounds
+    two pages of keys what a block fetches first decides (64 tokens x 16 heads alone: 15 us against 22).  (More tiles
+    than a grid's second axis holds, 4.2 million tokens, stay with the general kernel.)"""
+    tiles = n_tokens // PREFILL_F32_ROWS + n_seqs
+    rounds = -(-tiles * n_q_heads // (2 * sm_count(device)))
+    return tiles <= 65535 and visible >= 2 * PAGE and n_tokens * n_q_heads >= PREFILL_F32_ROUND * rounds
 
 
 def attention_prefill_f32(out, q, n_tokens, positions, token_slot, cu_seqlens, n_seqs, k_pages, v_pages,

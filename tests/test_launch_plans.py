@@ -100,6 +100,24 @@ def test_experts_of_any_size_run_on_pairs_of_sms(inter, gated):
         assert not part.w_up[:, (2 if gated else 1) * inter:].any() and not part.w_down[:, :, inter:].any()
 
 
+def test_the_delta_rule_goes_by_chunks_from_96_tokens_a_sequence():
+    by = kernels.delta_by_chunks
+    assert by(96, 1, 128, 128) and not by(95, 1, 128, 128) and by(4 * 96, 4, 64, 4) and not by(4 * 96 - 1, 4, 64, 4)
+    assert by(500, 1, 64, 128) and not by(500, 1, 64, 132) and not by(500, 1, 128, 130)      # values up to twice the keys, whole fours
+    assert not by(500, 1, 32, 32) and not by(500, 1, 256, 128) and not by(1, 1, 128, 128)    # keys of 64 and 128
+
+
+def test_where_32_bit_prompt_attention_takes_blocks_of_64_tokens():
+    """From two pages of keys and 1,024 (token, head) rows a round of blocks, two an SM, on; never beyond what its grid holds."""
+    sms = kernels.sm_count()
+    wins = lambda tokens, seqs, heads, visible: kernels.attention_prefill_f32_wins(tokens, seqs, heads, visible, None)
+    assert wins(64, 1, 16, 128) and not wins(64, 1, 16, 127) and not wins(63, 1, 16, 128)
+    heads = 2 * sms // 2                                       # two blocks a head (64 tokens, one sequence): one round
+    assert wins(64, 1, heads, 128)
+    assert (64 * (heads + 1) >= 2 * kernels.PREFILL_F32_ROUND) == wins(64, 1, heads + 1, 128)     # a second round for one head
+    assert wins(64 * 65534, 1, 16, 10**6) and not wins(64 * 65535, 1, 16, 10**6)
+
+
 def test_launch_record_groups_costs_and_issues_again():
     """The record behind the per-kernel tables, without a GPU: entries keep their order, are named
     with their label, sum their costs by name, and are issued again by name."""
