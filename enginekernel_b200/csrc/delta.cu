@@ -18,6 +18,8 @@
 // State of a slot (32-bit): [heads][e][DP] for S (DP = d rounded up to the scan's row count), then
 // [channels][taps-1] convolution inputs.  A fresh slot is all zeros.
 // Everything that enters the recurrence is computed and kept in 32-bit.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace ek {
@@ -72,11 +74,11 @@ delta_low_rank_kernel(float* __restrict__ out, const float* __restrict__ proj, i
   for (int tt = 0; tt < kRankTokens; ++tt)
 #pragma unroll
     for (int p = 0; p < PER; ++p) acc[tt][p] = bias ? b[p] : 0.f;
-  for (int r = 0; r < rank; r += 4) {           // four rows of weights, then one 16-byte read of a token's four inputs
+  auto rows = [&](int r, auto all) {            // four rows of weights, then one 16-byte read of a token's four inputs
     float w[4][PER];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      if (r + j < rank) fetch(w[j], w2t + (size_t)(r + j) * channels + c);
+      if (decltype(all)::value || r + j < rank) fetch(w[j], w2t + (size_t)(r + j) * channels + c);
       else
 #pragma unroll
         for (int p = 0; p < PER; ++p) w[j][p] = 0.f;
@@ -88,7 +90,12 @@ delta_low_rank_kernel(float* __restrict__ out, const float* __restrict__ proj, i
       for (int p = 0; p < PER; ++p)
         acc[tt][p] = fmaf(w[3][p], x.w, fmaf(w[2][p], x.z, fmaf(w[1][p], x.y, fmaf(w[0][p], x.x, acc[tt][p]))));
     }
-  }
+  };
+  constexpr int kAhead = PER == 1 ? 4 : 1;      // rounds unrolled: with few tokens a block waits for its weights
+  int r = 0;
+#pragma unroll kAhead
+  for (; r + 4 <= rank; r += 4) rows(r, std::true_type());
+  if (r < rank) rows(r, std::false_type());
   float rate[PER];
 #pragma unroll
   for (int p = 0; p < PER; ++p) rate[p] = mode == 0 ? expf(a_log[(c + p) / dim]) : 0.f;
