@@ -97,6 +97,53 @@ def test_delta_rule_by_chunks(heads, kv_heads, dim, vdim, decays):
     assert torch.equal(spoilt[keep], out[keep])
 
 
+@pytest.mark.parametrize("per_head", [False, True])
+def test_a_sequence_alone_in_company_and_in_portions(per_head):
+    """The form of the recurrence goes by a step's tokens a sequence, and chunks start at a step's first token: one sequence
+    of 300 tokens alone (chunks), beside five of 9 tokens (token by token), beside one of 200 (chunks), and in portions of
+    130, 70 and 100 tokens.  What differs is the order of 32-bit sums: each run is within 2e-7 (2-norm) of 64 bits, so two
+    runs are within 1e-6 of one another."""
+    from enginekernel_b200.parts.base import Workspace
+    k, heads, kv_heads, dim, vdim, n = K(), 4, 2, 128, 128, 300
+    g_ = torch.Generator().manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=g_)
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    t = n + 200
+    q, kk, v = unit(rnd(t, kv_heads, dim)) * dim ** -0.5, unit(rnd(t, kv_heads, dim)), rnd(t, heads, vdim)
+    beta, decay = torch.rand(t, heads, generator=g_), torch.rand(t, heads, 1 if per_head else dim, generator=g_) ** 0.1
+    q, kk, v, beta, decay = (x.reshape(t, -1).to(DEV) for x in (q, kk, v, beta, decay))
+    start = (rnd(8, heads * vdim * dim) * 0.3).to(DEV)
+
+    def run(lens, first, state):
+        """A step of sequences of these tokens, the first one's from ``first`` on, the others' behind token 300."""
+        rows, at = list(range(first, first + lens[0])), n
+        for m in lens[1:]:
+            rows += range(at, at + m)
+            at += m
+        cu, slot, pos = [0], [], []
+        for b, m in enumerate(lens):
+            cu.append(cu[-1] + m)
+            slot += [b] * m
+            pos += [j + (first if b == 0 else 0) for j in range(m)]
+        out = torch.empty(len(rows), heads * vdim, device=DEV)
+        args = [x[rows].contiguous() for x in (q, kk, v, beta, decay)]
+        k.delta_scan(out, *args, state, i32(cu), i32(pos), i32(slot), len(lens), heads, kv_heads, dim, vdim, n_tokens=len(rows),
+                     decay_per_head=per_head, workspace=Workspace(torch.device(DEV)))
+        return out[:lens[0]]
+
+    runs = []
+    for steps in ([[n]], [[n] + [9] * 5], [[n, 200]], [[130], [70], [100]]):
+        state, first, outs = start.clone(), 0, []
+        for lens in steps:
+            outs.append(run(lens, first, state))
+            first += lens[0]
+        runs.append((torch.cat(outs), state[0]))
+    assert k.delta_by_chunks(n, 1, dim, vdim) and not k.delta_by_chunks(n + 45, 6, dim, vdim) and k.delta_by_chunks(t, 2, dim, vdim)
+    far = lambda got, want: ((got.double() - want.double()).norm() / want.double().norm()).item()
+    for out, state in runs[1:]:
+        assert far(out, runs[0][0]) <= 1e-6 and far(state, runs[0][1]) <= 1e-6
+
+
 @pytest.mark.parametrize("taps", [2, 3, 4])
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(8, 8, 40, 24), (12, 4, 64, 100)])
 def test_convolution_and_unit_vectors_of_many_tokens(heads, kv_heads, dim, vdim, taps):

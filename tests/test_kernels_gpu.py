@@ -1092,3 +1092,42 @@ def test_attention_prefill_tc_over_rows_that_are_keys_and_values(heads, v_cols, 
         g, w = got.view(t, heads, 256), want.view(t, heads, 256)
         assert rel(g[..., :v_cols], w[..., :v_cols]) <= 2 ** -7
         assert (g[..., written:] == 7.0).all()
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("nq,nkv,d,keep", [(4, 2, 128, 5), (4, 2, 64, 0), (16, 1, 256, 0)])
+def test_attention_prefill_tc_a_bad_value_stays_with_the_tiles_that_read_its_page(nq, nkv, d, keep, bad):
+    """An infinite value or one that is no number, in a row that a window of 70 hides from most tokens: those that see it
+    get it, and the tiles that do not read its page - those before it, behind its window, of other sequences - are what
+    they were, bit for bit.  (Within a tile that reads the page a weight of 0 times such a value is no number either.)"""
+    k = K()
+    lens, window, key = [400, 130], 70, 150
+    t, dtype, per_tile = sum(lens), torch.bfloat16, 128 // (nq // nkv)
+    pages = Pages(2, 400, nkv, d, dtype, seed=3)
+    for s, n in enumerate(lens):
+        rows = rnd(n, nkv, d, dtype=dtype, seed=10 + s)
+        pages.fill(s, rows, rnd(n, nkv, d, dtype=dtype, seed=20 + s))
+    shared = d == 256
+    values = pages.k if shared else pages.v
+    q = rnd(t, nq * d + 8 * nq, dtype=dtype, seed=30)
+    pos, slots, cu = _prompt_rows(lens, [0, 0])
+    kw = dict(v_cols=192) if shared else dict(keep_first=keep, gate=q[:, nq * d:])
+
+    def run():
+        out = torch.zeros(t, nq * d, dtype=dtype, device=DEV)
+        k.attention_prefill_tc(out, q[:, :nq * d], t, pos, slots, cu, 2, pages.k, values, pages.table, nq, nkv, d, d ** -0.5,
+                               window, **kw)
+        return out.view(t, nq, d)[..., :192 if shared else d]
+
+    clean = run()
+    values[int(pages.table[0, key // 64]), :, key % 64, 3] = bad
+    spoilt = run()
+    k.check_tc_status(DEV)
+    assert clean.isfinite().all() and not spoilt[key:key + window, :, 3].isfinite().any()
+    untouched = torch.ones(t, dtype=torch.bool, device=DEV)
+    for first in range(0, lens[0], per_tile):
+        last = min(first + per_tile, lens[0]) - 1
+        if max(0, first - window + 1) // 64 <= key // 64 <= last // 64:
+            untouched[first:last + 1] = False
+    assert untouched[:key - 150 % 64 - per_tile].all() and untouched[lens[0]:].all() and untouched[key + 64 + window + per_tile:].all()
+    assert torch.equal(spoilt[untouched], clean[untouched])
