@@ -4,8 +4,8 @@
 // consecutive tokens of one sequence and one query head, and every key page serves all of them.
 //
 // Bound by the FMA pipes and the shared-memory reads that feed them (as the 32-bit product,
-// gemm_f32.cu).  128 threads: 8 rows x 4 keys a thread for the scores, the same 8 rows x an eighth of
-// the head a thread... for the weighted sum of values, so that a row's maximum and sum stay with the 16
+// gemm_f32.cu).  128 threads: 8 rows x 4 keys a thread for the scores, the same 8 rows x a sixteenth of
+// the head a thread for the weighted sum of values, so that a row's maximum and sum stay with the 16
 // lanes that hold its scores and its result.  Keys and values of a page take turns in one buffer (the
 // values are on their way while the softmax runs): two blocks fit an SM, and one computes while the
 // other waits.  Pages are aligned to the sequence, so what a token adds up, and in which order, does
