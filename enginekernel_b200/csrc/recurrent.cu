@@ -6,9 +6,9 @@
 // running maximum m_t = max(f + m_(t-1), i) and capped gate pre-activations; its normaliser
 // n_t = a n + b k is one more column of S whose v is 1.
 //
-// A column of S never meets another, so the scan runs one column per group of 8 lanes, the column's
-// rows in the lanes' registers, sequentially over a sequence's tokens and in parallel over sequences,
-// heads and columns.  All kernels take packed rows of several sequences (prompts, portions, single
+// A column of S never meets another, so the scan runs columns side by side: one to four columns per group
+// of 8 or 16 lanes, the columns' rows in the lanes' registers, sequentially over a sequence's tokens (or
+// a segment's) and in parallel over sequences, heads and columns.  All kernels take packed rows of several sequences (prompts, portions, single
 // tokens); rows whose position is negative belong to finished sequences and are skipped.
 //
 //   conv_silu        causal convolution per channel with bias, then SiLU; predecessors are found in the
@@ -28,8 +28,6 @@
 //   lru_gates        both gates from block-diagonal products, the decay and the gated input
 //   lru_scan         S_t = a_t S_(t-1) + x_t per channel, times the GELU of a side branch
 // Everything here is 32-bit; only the two output kernels round, once, to the activation type.
-#include <type_traits>
-
 #include "common.cuh"
 
 namespace ek {
@@ -547,6 +545,13 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
         "l"(reinterpret_cast<const unsigned long long&>(c)));
   return d;
 }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return d;
+}
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   float2 d;
   asm("mul.rn.f32x2 %0, %1, %2;"
@@ -575,17 +580,24 @@ struct ScanSegments {
 // spread over the SMs.  (With sequences fastest, four of them and 148 SMs, every fourth SM had nothing but the longest
 // sequence's blocks.)  RPL rows of a column a lane: lane l holds rows 32 g + 4 l + c
 // (g < RPL / 4, c < 4; of 16 lanes 64 g + 4 l + c), so that a column's lanes read neighbouring bytes of a key at a time.
-// S of a slot: state[((h * C + j) * DK + i], DK = 8 RPL rows (keys padded with zeros), C = dv + ones_col columns.
+// S of a slot: state[((h * C + j) * DK + i], DK = LANES RPL rows (keys padded with zeros), C = dv + ones_col columns.
 // `ab_stride`: values of a (and b) from token to token - the heads, or 0 where they are the same for every token.
 // CPL columns a lane (j, j + 16, ..): a key fetched from shared memory - what bounds a long walk, since a warp's 16-byte
 // load takes four cycles - serves that many columns; single tokens take one, for the shorter walk through S.
-// Eight tokens at a time S is kept divided by the product P_t of the group's decays so far: S / P_t needs one FMA a value,
-// S + (b_t v_t / P_t) k_t, instead of a product and an FMA, and the group ends with S = P_8 (S / P_8).  Where a P_t is not
+// Eight tokens at a time S is scaled to the group's last token: with G_t the product of the group's decays behind token t
+// and P that of all eight, G_t S_t needs one FMA a value and token, G_t S_t = G_(t-1) S_(t-1) + (b_t G_t v_t) k_t, after a
+// first one that scales S_0 by P; the last token's S is S itself.  Outputs are divided by G_t.  Where P or a G_t is not
 // within 2^-40 .. 2^40 (a decay of zero, say) the group is walked token by token.
-// Errors against 64 bits (1,500 tokens, decays of 0.5 to 1; 0.95 to 1): outputs 1.0e-7; 1.5e-7, S 5.4e-8; 1.2e-7; with the
-// product in every token 0.9e-7; 1.4e-7 and 5.3e-8; 1.2e-7.
-// Measured, prompts of 1,500, 1,103, 817 and 404 tokens, 32 heads of 128 x 128: 552 us with sequences fastest, two columns
-// a lane and the product in every token; 461 now in one walk, 406 in segments.  One of 2,048: 372, now 242.
+// (One and two columns a lane, which single tokens and short walks take: a product and an FMA a value and token.  The form
+// in eights needs registers - one column 139 instead of 107, a block an SM less: 49 sequences' single tokens, 32 heads, 77 us
+// instead of 60 - and its scalings are a chain of their own in every portion: 150 tokens of 32 heads 41 us against 36.)
+// The roundings are no more than token by token: P, b_t G_t and 1 / G_t are sums of two floats (a rounding of P is the same for
+// all of S and would add up from group to group), the last sum of an output and its division are rounded together.
+// Errors against 64 bits (1,500 tokens, decays of 0.5 to 1; 0.95 to 1): outputs 8.7e-8; 1.37e-7, S 4.6e-8; 1.15e-7; token by
+// token 9.1e-8; 1.40e-7 and 5.3e-8; 1.17e-7.  (S / P_t with P_t the product so far gave 1.01e-7; 1.53e-7 and 5.4e-8; 1.24e-7,
+// in 242 us where this takes 266.)
+// Measured, prompts of 1,500, 1,103, 817 and 404 tokens, 32 heads of 128 x 128: 548 us token by token with sequences fastest
+// and two columns a lane, now 448 in segments.  One of 2,048: 371, now 266.
 // Column dv (with ones_col) has v = 1: it carries n_t = a n + b k and gives n.q.
 // Tokens come 2048 / DK at a time: while one portion is worked through from shared memory, the next one's
 // keys, queries, values and gates are already on their way into registers.
@@ -599,6 +611,7 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
                   int write_state, int ab_stride, ScanSegments seg) {
   constexpr int LANES = kScanLanes<DK, CPL>, THREADS = kScanThreads<DK, CPL>, RPL = DK / LANES, G4 = RPL / 4, DK4 = DK / 4, COLS = kScanCols * CPL;
   constexpr int CH = kScanFloats / DK;                       // tokens a portion: 64, 32, 16 or 8
+  constexpr bool GROUPS = CPL == 4;
   constexpr int NV4 = kScanFloats / 4 / THREADS;        // float4 of keys (of queries) a thread fetches
   constexpr int NV = CH * COLS / THREADS;               // values a thread fetches
   static_assert(CH <= THREADS && CH * COLS % THREADS == 0, "portion sizes");
@@ -606,7 +619,7 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
   __shared__ __align__(16) float q_s[CH][DK];
   __shared__ float v_s[CH][COLS];
   __shared__ float a_s[CH], b_s[CH];
-  __shared__ float p_s[CH], bp_s[CH];                        // P_t and b_t / P_t
+  __shared__ float2 bg_s[CH], inv_s[CH], p_s[CH / 8];        // b_t G_t, 1 / G_t and P, each a sum of two floats
   __shared__ int good_s[CH / 8];                             // groups of eight that may be walked so
   pdl_launch_dependents();
   pdl_wait();
@@ -725,66 +738,94 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
     }
 #pragma unroll
     for (int m = 0; m < NV; ++m) (&v_s[0][0])[tid + m * THREADS] = v_r[m];
-    if (tid < (CH < 32 ? 32 : CH)) {             // (whole warps; past the portion a is 1 and b is 0)
-      // P_t and b_t / P_t correctly rounded, but for a last place: the product is carried as a sum of two floats (a
-      // rounding of P_8 is the same for all of S and would add up from group to group)
-      float prefix = a_r, rest = 0.f;
+    if (!GROUPS) {
+      if (tid < CH) { a_s[tid] = a_r; b_s[tid] = b_r; }
+    } else if (tid < (CH < 32 ? 32 : CH)) {      // (whole warps; past the portion a is 1 and b is 0)
+      // products of the decays from the token on, as sums of two floats
+      float product = a_r, rest = 0.f;
 #pragma unroll
       for (int by = 1; by < 8; by *= 2) {
-        const float before = __shfl_up_sync(0xffffffffu, prefix, by, 8);
-        const float before_rest = __shfl_up_sync(0xffffffffu, rest, by, 8);
-        if ((tid & 7) >= by) {
-          const float product = prefix * before;
-          rest = fmaf(rest, before, fmaf(prefix, before_rest, fmaf(prefix, before, -product)));
-          prefix = product;
+        const float behind = __shfl_down_sync(0xffffffffu, product, by, 8);
+        const float behind_rest = __shfl_down_sync(0xffffffffu, rest, by, 8);
+        if ((tid & 7) + by < 8) {
+          const float both = product * behind;
+          rest = fmaf(rest, behind, fmaf(product, behind_rest, fmaf(product, behind, -both)));
+          product = both;
         }
       }
-      const float rounded = prefix + rest;
-      rest -= rounded - prefix;
-      prefix = rounded;
-      float quotient = b_r / prefix;
-      quotient += fmaf(-quotient, rest, fmaf(-quotient, prefix, b_r)) / prefix;
-      const unsigned good = __ballot_sync(0xffffffffu, prefix > 0x1p-40f && prefix < 0x1p40f);
+      // P and b_t G_t as a float no larger than the product and one of the same sign behind it, never zero: an infinite S or
+      // value stays what it is
+      const float high = __fadd_rd(product, rest), low = fmaxf((product - high) + rest, 0x1p-126f);
+      float g = __shfl_down_sync(0xffffffffu, product, 1, 8), g_rest = __shfl_down_sync(0xffffffffu, rest, 1, 8);
+      if ((tid & 7) == 7) g = 1.f, g_rest = 0.f;
+      const float inv = 1.f / g;
+      const unsigned good = __ballot_sync(0xffffffffu, product > 0x1p-40f && product < 0x1p40f);
       if (tid < CH) {
         a_s[tid] = a_r;
         b_s[tid] = b_r;
-        p_s[tid] = prefix;
-        bp_s[tid] = quotient;
-        if ((tid & 7) == 0) good_s[tid / 8] = (good >> (tid & 24) & 0xffu) == 0xffu;
+        float bg = __fmul_rz(b_r, g), bg_rest = fmaf(b_r, g, -bg) + b_r * g_rest;
+        if (bg != 0.f) {
+          if (bg_rest * bg < 0.f) {
+            const float nearer = __int_as_float(__float_as_int(bg) - 1);
+            bg_rest += bg - nearer;
+            bg = nearer;
+          }
+          bg_rest = copysignf(fmaxf(fabsf(bg_rest), 0x1p-126f), bg);
+        }
+        bg_s[tid] = make_float2(bg, bg_rest);
+        inv_s[tid] = make_float2(inv, fmaf(-g_rest, inv, fmaf(-g, inv, 1.f)) * inv);
+        if ((tid & 7) == 0) {
+          p_s[tid / 8] = make_float2(high, low);
+          good_s[tid / 8] = (good >> (tid & 24) & 0xffu) == 0xffu;
+        }
       }
     }
     __syncthreads();
     if (c0 + CH < n) fetch(c0 + CH);
-    // S <- a S + b v k, or S / P_t <- S / P_(t-1) + (b / P_t) v k; sums: this lane's parts of S^T q
-    auto token = [&](int tt, float* sums, auto form) {
-      constexpr bool divided = decltype(form)::value;
+    // S <- a S + b v k, or (a group's token u) G_t S_t from G_(t-1) S_(t-1); sums: this lane's parts of S^T q
+    auto grouped = [&](int tt, int u, float* sums) {
       float bv[CPL];
+      float2 part[CPL][2], high, low;
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) bv[c] = (divided ? bp_s[tt] : b_s[tt]) * v_s[tt][col + c * kScanCols];
-      if constexpr (divided) {
-        float2 part[CPL];
+      for (int c = 0; c < CPL; ++c) {
+        const float value = v_s[tt][col + c * kScanCols];
+        bv[c] = fmaf(bg_s[tt].x, value, bg_s[tt].y * value);
+      }
+      if (u == 0) {
+        const float2 p = p_s[tt / 8];
+        high = make_float2(p.x, p.x), low = make_float2(p.y, p.y);
+      }
 #pragma unroll
-        for (int g = 0; g < G4; ++g) {
-          const float4 kk = *reinterpret_cast<const float4*>(&k_s[tt][4 * LANES * g + 4 * lane]);
-          float4 qq;
-          if (MODE != 1) qq = *reinterpret_cast<const float4*>(&q_s[tt][4 * LANES * g + 4 * lane]);
+      for (int g = 0; g < G4; ++g) {
+        const float4 kk = *reinterpret_cast<const float4*>(&k_s[tt][4 * LANES * g + 4 * lane]);
+        float4 qq;
+        if (MODE != 1) qq = *reinterpret_cast<const float4*>(&q_s[tt][4 * LANES * g + 4 * lane]);
+        const float2 k2[2] = {make_float2(kk.x, kk.y), make_float2(kk.z, kk.w)};
 #pragma unroll
-          for (int c = 0; c < CPL; ++c) {
-            const float2 b2 = make_float2(bv[c], bv[c]);
-            float2* s2 = reinterpret_cast<float2*>(&S[c][g]);
-            s2[0] = fma2(b2, make_float2(kk.x, kk.y), s2[0]);
-            s2[1] = fma2(b2, make_float2(kk.z, kk.w), s2[1]);
-            if (MODE != 1) {
-              part[c] = g == 0 ? mul2(s2[0], make_float2(qq.x, qq.y)) : fma2(s2[0], make_float2(qq.x, qq.y), part[c]);
-              part[c] = fma2(s2[1], make_float2(qq.z, qq.w), part[c]);
-            }
+        for (int c = 0; c < CPL; ++c) {
+          const float2 b2 = make_float2(bv[c], bv[c]);
+          float2* s2 = reinterpret_cast<float2*>(&S[c][g]);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) s2[e] = u == 0 ? fma2(s2[e], high, fma2(s2[e], low, mul2(b2, k2[e]))) : fma2(b2, k2[e], s2[e]);
+          if (MODE != 1) {                       // two sums (four values a float2: four products each for 16 rows)
+            constexpr int HALF = (G4 + 1) / 2;
+            float2& x = part[c][g / HALF];
+            x = g % HALF == 0 ? mul2(s2[0], make_float2(qq.x, qq.y)) : fma2(s2[0], make_float2(qq.x, qq.y), x);
+            x = fma2(s2[1], make_float2(qq.z, qq.w), x);
           }
         }
-        if (MODE == 1) return;
-#pragma unroll
-        for (int c = 0; c < CPL; ++c) sums[c] = (part[c].x + part[c].y) * p_s[tt];
-        return;
       }
+      if (MODE == 1) return;
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        const float2 x = G4 > 1 ? add2(part[c][0], part[c][1]) : part[c][0];
+        sums[c] = x.x + x.y;
+      }
+    };
+    auto token = [&](int tt, float* sums) {
+      float bv[CPL];
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) bv[c] = b_s[tt] * v_s[tt][col + c * kScanCols];
       const float aa = a_s[tt];
       float acc[CPL][G4];
 #pragma unroll
@@ -810,27 +851,19 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
         for (int g = 1; g < G4; ++g) sums[c] += acc[c][g];
       }
     };
-    auto group_end = [&](float p) {              // S / P_8 -> S
-#pragma unroll
-      for (int c = 0; c < CPL; ++c)
-#pragma unroll
-        for (int g = 0; g < G4; ++g) {
-          float2* s2 = reinterpret_cast<float2*>(&S[c][g]);
-          s2[0] = mul2(s2[0], make_float2(p, p));
-          s2[1] = mul2(s2[1], make_float2(p, p));
-        }
-      if (MODE == 1) prod *= p;
-    };
+    // a group may end behind the portion's last token (a is 1, b 0 and the rows are zero there): three tokens so take less
+    // time than one by one
+    auto group_at = [&](int tt) { return GROUPS && tt % 8 == 0 && nc - tt >= 3 && good_s[tt / 8]; };
     int tt = 0;
     if (MODE == 1) {
       while (tt < nc) {
-        if (tt % 8 == 0 && tt + 8 <= nc && good_s[tt / 8]) {
+        if (group_at(tt)) {
 #pragma unroll
-          for (int u = 0; u < 8; ++u) token(tt + u, nullptr, std::true_type());
-          group_end(p_s[tt + 7]);
+          for (int u = 0; u < 8; ++u) grouped(tt + u, u, nullptr);
+          prod *= p_s[tt / 8].x + p_s[tt / 8].y;
           tt += 8;
         } else {
-          token(tt, nullptr, std::false_type());
+          token(tt, nullptr);
           prod *= a_s[tt++];
         }
       }
@@ -839,11 +872,13 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
     // eight tokens at a time: their partial sums are exchanged so that lane l ends with token l's total
     // (7 shuffles in 3 levels for 8 tokens instead of 24 in 24)
     for (; tt < nc;) {
-      if (tt % 8 == 0 && tt + 8 <= nc && good_s[tt / 8]) {
+      if (group_at(tt) || (!GROUPS && tt + 8 <= nc)) {
         float p8[8][CPL];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) token(tt + u, p8[u], std::true_type());
-        group_end(p_s[tt + 7]);
+        for (int u = 0; u < 8; ++u) {
+          if constexpr (GROUPS) grouped(tt + u, u, p8[u]);
+          else token(tt + u, p8[u]);
+        }
         if constexpr (LANES == 16) {             // the halves of the lanes take two of the four columns each
 #pragma unroll
           for (int c = 0; c < CPL / 2; ++c)
@@ -869,15 +904,22 @@ decay_scan_kernel(float* __restrict__ out, int out_stride, const float* __restri
             p[u] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
           }
           const float send = (lane & 1) ? p[0] : p[1], keep = (lane & 1) ? p[1] : p[0];
-          const float total = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+          const float got = __shfl_xor_sync(0xffffffffu, send, 1), sum = keep + got;
+          float total = sum;
+          if constexpr (GROUPS) {                // (keep + got) / G_t, rounded once: what the sum's rounding loses joins
+            const float2 inv = inv_s[tt + (lane & 7)];                                   // behind the quotient
+            const float back = sum - keep, lost = (keep - (sum - back)) + (got - back);
+            const float rest = fmaf(sum, inv.y, lost * inv.x);
+            total = rest == rest ? fmaf(sum, inv.x, rest) : sum * inv.x;                 // (infinite sums have no rest)
+          }
           const int jc = col0 + col + (LANES == 16 && (lane & 8) ? c + CPL / 2 : c) * kScanCols;
-          if (jc < C) out[(size_t)(start + c0 + tt + (lane & 7)) * out_stride + (size_t)h * C + jc] = total;
+          if (jc < C && tt + (lane & 7) < nc) out[(size_t)(start + c0 + tt + (lane & 7)) * out_stride + (size_t)h * C + jc] = total;
         }
         tt += 8;
         continue;
       }
       float sums[CPL];
-      token(tt, sums, std::false_type());
+      token(tt, sums);
 #pragma unroll
       for (int c = 0; c < CPL; ++c) {
         float sum = sums[c];

@@ -1905,16 +1905,21 @@ def xgate_scan(a, b, m_run, proj, col_i, col_f, bias_i, bias_f, cap, state, m_of
 SCAN_COLUMNS = 16           # columns of S a block of the decay scan takes, one a lane; two or four times as many with more;
                             # must equal kScanCols in csrc/recurrent.cu
 SCAN_WIDE_TOKENS = 64       # sequences of at least this many tokens take two or four columns a lane
+SCAN_FEW_TOKENS = 224       # (see decay_scan_lane_columns)
 SCAN_BLOCKS_PER_SM = 6      # what a cut of long prompts into segments aims at
 SCAN_MIN_SEGMENT = 128      # tokens
 SCAN_MIN_SEGMENTS = 4       # (the walk of the states costs two thirds of a walk: two or three segments gain nothing)
 
 
-def decay_scan_lane_columns(columns, max_new, dim=DECAY_SCAN_MAX_KEY_DIM) -> int:
+def decay_scan_lane_columns(columns, max_new, dim=DECAY_SCAN_MAX_KEY_DIM, walks=None, device=None) -> int:
     """Columns that a lane of :func:`decay_scan` takes: one in short walks, four where there are enough columns and
-    16 lanes a column have four rows each, else two."""
+    16 lanes a column have four rows each, else two.  ``walks`` (sequences times heads, if known): walks of less than 224
+    tokens that leave an SM to every block of two columns take two (32 heads of 128 x 128, two columns against four: 100
+    tokens 23 us and 26, 150 tokens 36 and 41, 200 tokens 52 and 53, 300 tokens 79 and 66; three prompts of 128: 46 both)."""
     if max_new < SCAN_WIDE_TOKENS or columns <= SCAN_COLUMNS:
         return 1
+    if walks is not None and max_new < SCAN_FEW_TOKENS and walks * -(-columns // (2 * SCAN_COLUMNS)) <= sm_count(device):
+        return 2
     return 4 if columns > 2 * SCAN_COLUMNS and dim > 32 else 2
 
 
@@ -1924,13 +1929,14 @@ def decay_scan_segments(n_seqs, heads, columns, max_new, device=None, n_tokens=0
     sequences, if known) tells a ragged batch, whose longest sequence is left alone at the end, from an even one.
     ``lane_columns``: what the launch takes (:func:`decay_scan_lane_columns` for the widest keys, unless given)."""
     if lane_columns is None:
-        lane_columns = decay_scan_lane_columns(columns, max_new)
+        lane_columns = decay_scan_lane_columns(columns, max_new, walks=n_seqs * heads, device=device)
     blocks = n_seqs * heads * -(-columns // (SCAN_COLUMNS * lane_columns))
     most, sms = -(-max_new // SCAN_MIN_SEGMENT), sm_count(device)
     want = min(SCAN_BLOCKS_PER_SM * sms // blocks, most)
-    # Uncut, a step takes as long as its longest sequence, 0.30 us a token with two blocks an SM; cut, 0.24 us a token and
-    # block of each SM's share (both walks).  32 heads of 128, prompts of 1,500, 1,103, 817, 404: 461 us uncut, 406 in 6
-    # segments; 40 heads (more blocks): 471 and 495.
+    # Uncut, a step takes as long as its longest sequence, 0.33 us a token with two blocks an SM; cut, 0.265 us a token and
+    # block of each SM's share (both walks).  Us uncut and in segments (32 heads of 128 unless said): prompts of 1,500, 1,103, 817
+    # and 404 tokens 498 / 438, of 1,000 and three of 60 317 / 160, of 700, 500, 300 208 / 183 (all cut by the rule); four of 600
+    # 210 / 277 and 40 heads of the first 508 / 539 (left whole).
     if want < SCAN_MIN_SEGMENTS and lane_columns == 4 and n_tokens * (blocks // n_seqs) * 0.81 < max_new * sms and n_tokens:
         want = min(2 * SCAN_BLOCKS_PER_SM * sms // blocks, most)
     if want < SCAN_MIN_SEGMENTS:
@@ -1961,7 +1967,7 @@ def decay_scan(out, q, k, v, a, b, state, cu_seqlens, positions, token_slot, n_s
                                 + 2 * n_seqs * heads * cols * decay_scan_rows(dim)),
                      flops=4 * n_tokens * heads * dim * cols)
     parts, length, carry, prods = 1, 0, None, None
-    lane_columns = lane_columns or decay_scan_lane_columns(cols, max_new, dim)
+    lane_columns = lane_columns or decay_scan_lane_columns(cols, max_new, dim, n_seqs * heads, out.device)
     if workspace is not None and max_new > 1:
         parts, length = segments or decay_scan_segments(n_seqs, heads, cols, max_new, out.device, n_tokens, lane_columns)
         _need(length >= 1 and parts * length >= max_new, "decay_scan: the segments cover the longest sequence")
