@@ -13,7 +13,7 @@
 //                      by TMA and is used as it lies (rows = keys, i.e. an MN-major operand)
 // The scores of page t+2 overwrite an S buffer only after the P.V of page t, which reads its P
 // from there, is done: the S issuer waits for that page's pv_done barrier.
-// The running maximum is lazy: exponentials are taken against a reference that is raised (and O
+// The running maximum is lazy (but for the KEEP and SHARED forms below): exponentials are taken against a reference that is raised (and O
 // and the running sum rescaled, by tcgen05.ld/st of the row) only when a page's maximum exceeds
 // it by more than 2^8, which keeps every probability finite in bfloat16 and skips the rescale
 // of almost every page.  O is divided by the sum once, at the end.
