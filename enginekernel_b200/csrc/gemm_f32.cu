@@ -1,47 +1,42 @@
-// C[M,N] = A[M,K] . W[N,K]^T in true 32-bit: FFMA on the CUDA cores, no tensor-core
-// mode of reduced precision anywhere.  The reference runs its 32-bit path through a
-// library product with TF32 switched off (engine/engine.py:190-192); this kernel makes
-// the precision a property of the code instead of a global flag.
+// C[M,N] = A[M,K] . W[N,K]^T in true 32-bit.  The reference runs its 32-bit path through a library product
+// with TF32 switched off (engine/engine.py:190-192); here the precision is a property of the code.
 //
-// One order of summation for every output, whatever M is and whichever form below runs: the K
-// products of a run of 64 (kRun) are summed in ascending k from zero, and the runs' sums are added
-// in ascending order.  A row's result therefore does not depend, bit for bit, on which other rows
-// share the launch, and few rows can spread K over many lanes.
+// A row's result does not depend, bit for bit, on which other rows share the launch: every form that a layout and K
+// can take sums in one order, whatever M is.
 //
-//   few rows (M <= 16)  bound by the weight stream.  A lane takes a few columns and one run of K: their
-//                       weights straight from memory, 32 bytes a load, the rows' x from L1; it leaves the
-//                       run's sums in shared memory, where one thread an output adds them in order.
-//                       Measured (us, the 16 x 128 tiles over all of K before): 4 x 4096 x 1024 (M x N x K)
-//                       111 -> 12.3, 4 x 1024 x 3072 311 -> 18.8, 1 x 151936 x 1024 347 -> 113 (5.5 TB/s).
-//   more rows           bound by the FMA pipes and the shared-memory reads that feed them: 8 x 8 outputs a
-//                       thread read 16 values of 4 steps of K by 16-byte loads for 256 FMAs, which takes
-//                       shared memory as long as the FMAs take (a warp's 16-byte load returns 512 bytes at
-//                       128 a cycle).  Operands arrive by cp.async, 16 of K a step, four stages.  64 x 64
-//                       tiles of two warps: 4096^3 5.69 -> 3.17 ms (43 TFLOP/s), 1129 x 1024 x 3072
-//                       515 -> 217 us.  128 x 128 tiles gave 41 TFLOP/s and leave narrow outputs with too
-//                       few blocks; packed pairs of FMAs need moves to double one operand and gave 40.
-#include "common.cuh"
+// Rows of whole 32-byte pieces (K and both strides multiples of 8): tcgen05.  A 32-bit value is the sum of three
+// bfloat16 terms exactly, and the products of two terms are exact in 32 bits.  Of the nine products of two values'
+// terms the three smallest (2^-24 of the value and less) are left out; weights that came from 16 bits have one term,
+// and then nothing is.  The tensor cores cut a sum at its last place instead of rounding it, so no more than 32 of K go
+// into one accumulator: chunks of 32 are added in 32-bit registers, rounded, to spans of 256, and the spans to the result.
+// Relative error against 64 bits (normal values, K = 1,024; this and FFMA in chains of 64): 0.9e-7 and 1.6e-7.
+//   up to 64 rows   bound by the weight stream.  TMA brings 32-bit values, 16 warps write their terms for the MMA,
+//                   the weights on its 128-row side; blocks take tile after tile, or a cluster shares K of one and
+//                   every block sends its spans' sums to the one that adds them up.  us, FFMA before: 4 x 1024 x 3072
+//                   (M x N x K) 22.6 -> 17.4, 16 x 151936 x 1024 248 -> 118 (5.3 TB/s), 13 x 6144 x 2560 78 -> 30,
+//                   64 x 6144 x 2560 163 -> 42.  One row of a narrow product is the exception: 1 x 4096 x 1024 11.3 ->
+//                   15.4, the chain from copy to conversion, MMA and sum being longer than FFMA's.  Loads into registers or
+//                   cp.async instead of TMA ran at half this rate (long chains in every converting warp).
+//   more rows       a kernel of its own writes both operands' terms as the tiles that the MMA reads, so that a value is
+//                   converted once and not by every block that needs it (which took half as long again); the product
+//                   streams these tiles.  128 x 128 outputs a tile read 64 KB of operands for 64 of K, which L2 supplies
+//                   at about the rate of the MMAs.  1129 x 6144 x 1024 360 -> 87 us, 1129 x 1024 x 3072 219 -> 56,
+//                   4096^3 3,165 -> 515 (267 TFLOP/s).  The three terms of x side by side in one MMA of 192 columns
+//                   read less shared memory but more L2 (128 x 64 tiles): 820 us.
+// Other rows: FFMA, chains of 64 (kRun) whose sums are added in ascending order.
+//   few rows (M <= 16)  a lane takes a few columns and one run of K; one thread an output adds the runs' sums in order.
+//   more rows           8 x 8 outputs a thread from tiles in shared memory.
+#include "tc_common.cuh"
 
 namespace ek {
 
+constexpr int kSms = 148;              // of a B200: how many blocks a launch should at least have
 constexpr int kRun = 64;              // products summed in one chain
 
-// 8 values of a row from column k on (zeros from K on).  VEC: the 32 bytes are aligned and whole.
-template <bool VEC>
+// 8 values of a row from column k on (zeros from K on).
 __device__ __forceinline__ void load8(float (&v)[8], const float* row, int k, int K) {
-  if (VEC) {
-    if (k < K) {
-      asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                   : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-                   : "l"(row + k));
-      return;
-    }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = 0.f;
-  } else {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = k + j < K ? row[k + j] : 0.f;
-  }
+  for (int j = 0; j < 8; ++j) v[j] = k + j < K ? row[k + j] : 0.f;
 }
 
 // ------------------------------------------------------------------------------- few rows
@@ -50,7 +45,7 @@ __host__ __device__ constexpr int few_cols(int mr) { return mr == 1 ? 1 : mr <= 
 __host__ __device__ constexpr int few_warps(int mr) { return mr <= 8 ? 8 : 4; }      // (the runs' sums fit 48 KB)
 
 // MR rows (M <= MR).  Lane = 8 groups of columns x 4 runs; a warp takes 4 runs at a time.
-template <int MR, bool VEC>
+template <int MR>
 __global__ void __launch_bounds__(few_warps(MR) * 32)
 sgemm_few_rows_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
                       int M, int N, int K, int lda, int ldw, int ldc) {
@@ -80,13 +75,13 @@ sgemm_few_rows_kernel(float* __restrict__ C, const float* __restrict__ A, const 
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i)
 #pragma unroll
-          for (int c = 0; c < CPL; ++c) load8<VEC>(w[c][i], w_row[c], k0 + 8 * (i0 + i), K);
+          for (int c = 0; c < CPL; ++c) load8(w[c][i], w_row[c], k0 + 8 * (i0 + i), K);
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i)
 #pragma unroll
           for (int m = 0; m < MR; ++m) {
             float x[8];
-            load8<VEC>(x, A + (size_t)min(m, M - 1) * lda, k0 + 8 * (i0 + i), K);
+            load8(x, A + (size_t)min(m, M - 1) * lda, k0 + 8 * (i0 + i), K);
 #pragma unroll
             for (int c = 0; c < CPL; ++c)
 #pragma unroll
@@ -116,7 +111,7 @@ constexpr int kStepK = 16, kStepLd = kStepK + 4, kStages = 4;
 __host__ __device__ constexpr int tile_smem(int bm, int bn) { return kStages * (bm + bn) * kStepLd * 4; }
 
 // 8 x 8 outputs a thread: rows ty + i TY, columns tx + j TX.
-template <int BM, int BN, bool VEC>
+template <int BM, int BN>
 __global__ void __launch_bounds__(BM / 8 * (BN / 8))
 sgemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
                   int M, int N, int K, int lda, int ldw, int ldc) {
@@ -140,17 +135,9 @@ sgemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const floa
       const bool ok = r < (is_a ? M : N);
       const float* src = is_a ? A + (size_t)(ok ? r : 0) * lda : W + (size_t)(ok ? r : 0) * ldw;
       float* dst = to + row * kStepLd + piece % (kStepK / 4) * 4;
-      if (VEC) {
-        const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-        const int bytes = ok && k < K ? 16 : 0;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(bytes ? src + k : src), "r"(bytes)
-                     : "memory");
-      } else {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dst[j] = ok && k + j < K ? src[k + j] : 0.f;
-      }
+      for (int j = 0; j < 4; ++j) dst[j] = ok && k + j < K ? src[k + j] : 0.f;
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
   float acc[8][8], total[8][8];
@@ -163,13 +150,10 @@ sgemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const floa
 #pragma unroll
   for (int s = 0; s < kStages - 1; ++s) {
     if (s < steps) copy(s);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
   }
   for (int s = 0; s < steps; ++s) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
     __syncthreads();                           // the step's operands are there, and the stage refilled below is free
     if (s + kStages - 1 < steps) copy(s + kStages - 1);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
     const float* a_s = ring + (size_t)(s % kStages) * (BM + BN) * kStepLd + ty * kStepLd;
     const float* w_s = ring + (size_t)(s % kStages) * (BM + BN) * kStepLd + (BM + tx) * kStepLd;
 #pragma unroll
@@ -210,21 +194,19 @@ sgemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const floa
   }
 }
 
-template <int BM, int BN, bool VEC>
+template <int BM, int BN>
 static int launch_tile(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc,
                        cudaStream_t stream) {
   const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   if (grid.y > 65535) return EK_ERR_ARG;
-  auto kernel = sgemm_tile_kernel<BM, BN, VEC>;
+  auto kernel = sgemm_tile_kernel<BM, BN>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem(BM, BN));
   if (e != cudaSuccess) return (int)e;
   kernel<<<grid, BM / 8 * (BN / 8), tile_smem(BM, BN), stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
   return (int)cudaGetLastError();
 }
 
-template <bool VEC>
-static int launch_sgemm(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc,
-                        cudaStream_t stream) {
+static int launch_ffma(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
   // 5 to 16 rows of many columns: x is read often enough for the few-row form to be bound by L1, and there
   // are columns enough for tiles (16 x 151936 x 1024: 425 us against 248; 12 x 40000 x 1024: 114 against 87;
   // but 16 x 6144 x 1024: 30 against 74)
@@ -232,23 +214,793 @@ static int launch_sgemm(float* C, const float* A, const float* W, int M, int N, 
     const int mr = M == 1 ? 1 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
     const int threads = 32 * min(few_warps(mr), (K + 4 * kRun - 1) / (4 * kRun));
     const dim3 grid((N + 8 * few_cols(mr) - 1) / (8 * few_cols(mr)));
-    if (mr == 1) sgemm_few_rows_kernel<1, VEC><<<grid, threads, 0, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
-    else if (mr == 4) sgemm_few_rows_kernel<4, VEC><<<grid, threads, 0, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
-    else if (mr == 8) sgemm_few_rows_kernel<8, VEC><<<grid, threads, 0, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
-    else sgemm_few_rows_kernel<16, VEC><<<grid, threads, 0, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
+    if (mr == 1) sgemm_few_rows_kernel<1><<<grid, threads, 0, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
+    else if (mr == 4) sgemm_few_rows_kernel<4><<<grid, threads, 0, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
+    else if (mr == 8) sgemm_few_rows_kernel<8><<<grid, threads, 0, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
+    else sgemm_few_rows_kernel<16><<<grid, threads, 0, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
     return (int)cudaGetLastError();
   }
-  if (M <= 16) return launch_tile<16, 128, VEC>(C, A, W, M, N, K, lda, ldw, ldc, stream);
-  return launch_tile<64, 64, VEC>(C, A, W, M, N, K, lda, ldw, ldc, stream);
+  if (M <= 16) return launch_tile<16, 128>(C, A, W, M, N, K, lda, ldw, ldc, stream);
+  return launch_tile<64, 64>(C, A, W, M, N, K, lda, ldw, ldc, stream);
+}
+
+// ------------------------------------------------------------------------- on the tensor cores
+constexpr int kSpan = 256;            // of K: a span's sum is that of its chunks of 32, a result that of its spans
+constexpr int kStepSpan = kSpan / 64;
+constexpr int kTermTile = 128 * 128;  // bytes of one term of 128 rows, 64 of K
+
+// 8 values as sums of three bfloat16 terms each, exactly: x = hi + mid + lo, every term the nearest to what the ones
+// before it leave.  `largest` gathers the largest magnitude of either half: where it is an infinity or a NaN the terms
+// say nothing.
+__device__ __forceinline__ uint32_t two_bf16(float a, float b) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
+__device__ __forceinline__ uint4 first_terms(const float (&v)[8], uint32_t& largest) {
+  uint32_t h[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    h[i] = two_bf16(v[2 * i], v[2 * i + 1]);
+    asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(largest) : "r"(largest), "r"(h[i]));
+  }
+  return make_uint4(h[0], h[1], h[2], h[3]);
+}
+__device__ __forceinline__ void other_terms(const float (&v)[8], const uint4& hi, uint4& mid, uint4& lo) {
+  const uint32_t h[4] = {hi.x, hi.y, hi.z, hi.w};
+  uint32_t m[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float a = v[2 * i] - __uint_as_float(h[i] << 16), b = v[2 * i + 1] - __uint_as_float(h[i] & 0xffff0000u);
+    m[i] = two_bf16(a, b);
+    l[i] = two_bf16(a - __uint_as_float(m[i] << 16), b - __uint_as_float(m[i] & 0xffff0000u));
+  }
+  mid = make_uint4(m[0], m[1], m[2], m[3]);
+  lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+__device__ __forceinline__ bool is_odd(uint32_t largest) {
+  return (largest & 0x7f80u) == 0x7f80u || (largest & 0x7f800000u) == 0x7f800000u;
+}
+__device__ __forceinline__ void load_row8(float (&v)[8], const float* from, bool there) {
+  if (there) {
+    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(from));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.f;
+  }
+}
+__device__ __forceinline__ void st_shared_16(uint32_t at, uint4 v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+// The value of one output over columns [k0, k1) of K by FFMA, in the order of chunks and spans, where its rows hold an
+// infinity or a NaN (a term of theirs times a zero would make a NaN of an infinity) or a value that rounds to an
+// infinity in 16 bits.
+__device__ __noinline__ void plain_if_odd(float* out, const float* a, const float* w, int k0, int k1) {
+  bool odd = false;
+  float total = 0.f;
+  for (int s = k0; s < k1; s += kSpan) {
+    float span = 0.f;
+    for (int c = s; c < min(k1, s + kSpan); c += 32) {
+      float chunk = 0.f;
+      for (int k = c; k < min(k1, c + 32); ++k) {
+        odd |= !(fabsf(a[k]) < 0x1.ffp127f) || !(fabsf(w[k]) < 0x1.ffp127f);
+        chunk = fmaf(a[k], w[k], chunk);
+      }
+      span += chunk;
+    }
+    total += span;
+  }
+  if (odd) *out = total;
+}
+
+// The MMAs of one chunk of 32 (c: the stage's first or second) into the NT columns from `acc` on; tile(i) is where
+// term i (0-2 the weights', 3-5 x's) of the stage begins.  `more`: the weights have second or third terms.  The
+// smallest products come first: the tensor cores cut a sum, rather than round it, at the last place it holds (a
+// chain of 64 by 4.5e-8 of it on average, of 1,024 by 8e-7).
+template <int NT, typename Tile>
+__device__ __forceinline__ void chunk_mmas(uint32_t acc, Tile tile, int c, bool more) {
+  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+  auto product = [&](int w, int x, uint32_t add) {
+    const uint64_t wd = smem_desc_k_sw128(tile(w)) + 4 * c, xd = smem_desc_k_sw128(tile(3 + x)) + 4 * c;
+    tc_mma(acc, wd, xd, idesc, add);
+    tc_mma(acc, wd + 2, xd + 2, idesc, 1u);
+  };
+  if (more) {
+    product(2, 0, 0);
+    product(1, 1, 1);
+    product(0, 2, 1);
+    product(1, 0, 1);
+  } else {
+    product(0, 2, 0);
+  }
+  product(0, 1, 1);
+  product(0, 0, 1);
+}
+
+// ------------------------------------------------------------- few rows: operands converted on their way in
+constexpr int kConvWarps = 16, kAddWarps = 4, kFewThreads = (kConvWarps + kAddWarps + 3) * 32;
+// Shared memory of a block: two stages of first terms of the weights and all of x's, the weights' other terms (of one
+// stage where K is split: those blocks are short and want their values early), `depth` stages of values as they are,
+// sums that other blocks send.
+constexpr int kTermStages = 2;
+__host__ __device__ constexpr int few_terms(int nt) { return kTermTile + 3 * nt * 128; }
+__host__ __device__ constexpr int few_low(bool split) { return (split ? 1 : kTermStages) * 2 * kTermTile; }
+__host__ __device__ constexpr int few_raw(int nt) { return (128 + nt) * 256; }
+constexpr int kFewDepth = 4;
+__host__ __device__ constexpr int few_fixed(int nt, bool split) {           // (barriers; a 1024-byte border)
+  return kTermStages * few_terms(nt) + few_low(split) + 512 + 1024;
+}
+constexpr int kMaxSmem = 227 * 1024;
+
+__device__ __forceinline__ void read_16(float* v, uint32_t at) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(at) : "memory");
+}
+
+// C tiles of 128 columns (weight rows, the MMA's M) x NT rows (tokens, its N).  SPLIT: the blocks of a cluster
+// share K of one tile, whole spans each; otherwise a block takes tile after tile.
+template <int NT, bool SPLIT>
+__global__ void __launch_bounds__(kFewThreads, 1)
+sgemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                 float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
+                 int M, int N, int K, int lda, int ldw, int ldc, int spans_a_block,
+                 int depth, int* status) {
+  constexpr int CW = kConvWarps, AW = kAddWarps;
+  constexpr uint32_t kStage = few_terms(NT), kRaw = few_raw(NT), kXTile = NT * 128;
+  extern __shared__ unsigned char raw[];
+  unsigned char* ring = raw + ((1024 - (smem_u32(raw) & 1023)) & 1023);
+  const uint32_t terms0 = smem_u32(ring), low0 = terms0 + kTermStages * kStage, raw0 = low0 + few_low(SPLIT);
+  unsigned char* tail = ring + kTermStages * kStage + few_low(SPLIT) + depth * kRaw;
+  uint64_t* bars = (uint64_t*)tail;                     // full[2], summed[2], taken[2], done, received, here[4], read[4]
+  uint32_t* tmem_slot = (uint32_t*)(bars + 16);
+  volatile int* any_odd = (int*)(tmem_slot + 1);
+  unsigned char* more_terms = (unsigned char*)(tmem_slot + 4);     // [stage][CW]: the weights have second or third terms
+  float* received = (float*)(tail + 512);               // [span][token of this block][128]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int m0 = blockIdx.z * NT, tiles_n = (N + 127) / 128;
+  const int k_begin = SPLIT ? blockIdx.y * spans_a_block * kSpan : 0;
+  const int k_end = SPLIT ? min(K, k_begin + spans_a_block * kSpan) : K;
+  const int stages = k_end > k_begin ? (k_end - k_begin + 63) / 64 : 0;
+  const int tiles = SPLIT ? 1 : (tiles_n - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int total = tiles * stages;
+  const uint32_t full0 = smem_u32(bars), summed0 = full0 + 16, taken0 = full0 + 32, done = full0 + 48,
+                 received0 = full0 + 56, here0 = full0 + 64, read0 = full0 + 96;
+  // split: block r of the cluster adds up the tokens r, r + ranks, ...
+  const int rank = SPLIT ? blockIdx.y : 0, ranks = SPLIT ? gridDim.y : 1, rows = min(NT, M - m0);
+  const int slots = (rows + ranks - 1) / ranks, mine = rows > rank ? (rows - rank + ranks - 1) / ranks : 0;
+  const int all_spans = (K + kSpan - 1) / kSpan;
+
+  // The copying thread has its own barriers ready and the first weights on their way before anything else, and
+  // before the kernel ahead has ended: weights do not depend on it.
+  const uint64_t once = l2_policy_evict_first();
+  auto raw_at = [&](int slot) { return raw0 + (uint32_t)slot * kRaw; };
+  auto copy_w = [&](int slot, int tile, int s) {
+    mbar_expect_tx(here0 + 8 * slot, kRaw);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      tma_load_2d_hint(raw_at(slot) + h * (128 * 128), &map_w, k_begin + s * 64 + h * 32, tile * 128, here0 + 8 * slot, once);
+  };
+  auto copy_x = [&](int slot, int s) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      tma_load_2d(raw_at(slot) + 128 * 256 + h * (NT * 128), &map_x, k_begin + s * 64 + h * 32, m0, here0 + 8 * slot);
+  };
+  pdl_launch_dependents();
+  if (tid == (AW + CW) * 32) {
+    tma_prefetch_map(&map_w);
+    tma_prefetch_map(&map_x);
+    for (int i = 0; i < depth; ++i) {
+      mbar_init(here0 + 8 * i, 1);
+      mbar_init(read0 + 8 * i, CW);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int q = 0; q < min(depth, total); ++q) copy_w(q, blockIdx.x + q / stages * gridDim.x, q % stages);
+  }
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(full0 + 8 * i, CW);
+      mbar_init(summed0 + 8 * i, 2);
+      mbar_init(taken0 + 8 * i, AW);
+    }
+    mbar_init(done, 2);
+    mbar_init(received0, 1);
+    *any_odd = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (SPLIT && mine > 0) mbar_expect_tx(received0, (uint32_t)(all_spans * mine * 512));
+  }
+  // (that barrier exists in every block before a store from another one reaches it: arrive here, wait before the
+  // first such store)
+  __syncwarp();
+  if (SPLIT) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  if (warp == AW + CW) tmem_alloc(smem_u32(tmem_slot), 8 * NT);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t lanes = tmem + ((uint32_t)(warp * 32) << 16);
+  bool ok = true;
+  if (warp < AW) pdl_wait();                               // before anything is written
+
+  if (warp < AW) {
+    // ------------------------------------------------------------------ chunk sums out of TMEM, added in 32 bits
+    float span[NT];
+    int s = 0, tile = blockIdx.x;
+    if (SPLIT) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+#pragma unroll 1
+    for (int q = 0; q < total; ++q) {
+      if (!(ok = mbar_wait(summed0 + 8 * (q & 1), (q >> 1) & 1, status, 33))) break;
+      tc_fence_after();
+      const bool fresh = s % kStepSpan == 0;
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int t = 0; t < NT; t += 16) {
+          float v[16];
+          tmem_ld16(lanes + (uint32_t)((2 * (q & 1) + c) * NT + t), v);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) span[t + j] = c == 0 && fresh ? v[j] : span[t + j] + v[j];
+        }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(taken0 + 8 * (q & 1));
+      const bool last = ++s == stages;
+      if (s % kStepSpan != 0 && !last) continue;
+      const int span_of = (s - 1) / kStepSpan;
+      if constexpr (SPLIT) {
+        // every token's sum to the block that adds it up
+        const int n = tile * 128 + tid, k0 = k_begin + span_of * kSpan;
+        const bool odd = *any_odd != 0;
+        int to = 0, slot = 0;
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+          if (t < rows) {
+            float v = span[t];
+            if (odd && n < N) plain_if_odd(&v, A + (size_t)(m0 + t) * lda, W + (size_t)n * ldw, k0, min(k_end, k0 + kSpan));
+            st_async_f32(&received[((size_t)(k0 / kSpan) * slots + slot) * 128 + tid], (unsigned)to, v, received0);
+            if (++to == ranks) {
+              to = 0;
+              ++slot;
+            }
+          }
+      } else {
+        // the total of the spans so far waits in tensor memory
+#pragma unroll
+        for (int t = 0; t < NT; t += 16) {
+          if (span_of > 0) {
+            float v[16];
+            tmem_ld16(lanes + (uint32_t)(4 * NT + t), v);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) span[t + j] = v[j] + span[t + j];
+          }
+          if (!last) {
+            uint32_t v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(span[t + j]);
+            tmem_st16(lanes + (uint32_t)(4 * NT + t), v);
+          }
+        }
+        tmem_st_wait();
+        if (last) {
+          s = 0;
+          const int n = tile * 128 + tid;
+#pragma unroll
+          for (int t = 0; t < NT; ++t)
+            if (n < N && t < rows) C[(size_t)(m0 + t) * ldc + n] = span[t];
+          if (*any_odd && n < N)
+            for (int m = m0; m < m0 + rows; ++m)
+              plain_if_odd(C + (size_t)m * ldc + n, A + (size_t)m * lda, W + (size_t)n * ldw, 0, K);
+          tile += gridDim.x;
+        }
+      }
+    }
+    if (SPLIT && ok && mine > 0) {
+      ok = mbar_wait(received0, 0, status, 39);
+      const int n = blockIdx.x * 128 + tid;
+      if (ok && n < N)
+        for (int i = 0; i < mine; ++i) {
+          float sum = 0.f;
+#pragma unroll 4
+          for (int j = 0; j < all_spans; ++j) {
+            const float v = received[((size_t)j * slots + i) * 128 + tid];
+            sum = j > 0 ? sum + v : v;
+          }
+          C[(size_t)(m0 + rank + i * ranks) * ldc + n] = sum;
+        }
+    }
+  } else if (warp < AW + CW) {
+    // ------------------------------------------------------------------- three terms of each value to shared memory
+    // A pass is 8 rows x 32 of K, 8 values a lane; a warp takes two of the weights and where there are some left one
+    // of x.  Neighbouring fours of lanes take rows r and r ^ 5: 16-byte accesses to the swizzled rows of either side
+    // then touch every bank once.
+    // Weights that came from 16 bits have a first term only: the others are written where they are not zero, or
+    // where such were before.
+    const int cw = warp - AW, i8 = lane >> 2, r8 = (i8 >> 1) ^ (i8 & 1 ? 5 : 0), k4 = lane & 3;
+    const bool has_x = cw < NT / 4;
+    const uint32_t even = (uint32_t)(((2 * k4) ^ r8) << 4), odd = even ^ 16u;
+    uint32_t to_w[2];                                     // where a pass's first terms go, from the stage's start on
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const int n = cw + p * CW;
+      to_w[p] = (8 * (n >> 1) + r8) * 128 + (((4 * (n & 1) + k4) ^ r8) << 4);
+      for (int i = 0; i < (SPLIT ? 2 : 4); ++i) st_shared_16(low0 + i * kTermTile + to_w[p], make_uint4(0, 0, 0, 0));
+    }
+    const uint32_t to_x = kTermTile + (8 * (cw >> 1) + r8) * 128 + (((4 * (cw & 1) + k4) ^ r8) << 4);
+    uint32_t stale = 0;                                   // a bit each place of other terms: it holds some that are not zero
+    int slot = 0, phase = 0;
+#pragma unroll 1
+    for (int q = 0; q < total; ++q) {
+      if (!(ok = mbar_wait(here0 + 8 * slot, phase, status, 37))) break;
+      const uint32_t from = raw0 + (uint32_t)slot * kRaw, at = terms0 + (q & 1) * kStage;
+      float w[2][8], x[8];
+      uint32_t low = 0, largest = 0;
+      // pass n: half n & 1 of the stage's K, rows 8 (n >> 1) ..
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const int n = cw + p * CW;
+        const uint32_t in = from + (n & 1) * (128 * 128) + (8 * (n >> 1) + r8) * 128;
+        read_16(w[p], in + even);
+        read_16(w[p] + 4, in + odd);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) low |= __float_as_uint(w[p][j]);
+      }
+      if (has_x) {
+        const uint32_t in = from + 128 * 256 + (cw & 1) * (NT * 128) + (8 * (cw >> 1) + r8) * 128;
+        read_16(x, in + even);
+        read_16(x + 4, in + odd);
+      }
+      uint4 hi[2], x_hi;
+#pragma unroll
+      for (int p = 0; p < 2; ++p) hi[p] = first_terms(w[p], largest);
+      if (has_x) x_hi = first_terms(x, largest);
+      if (is_odd(largest)) *any_odd = 1;
+      // (every lane has used what it read when the vote is over: the place may be filled again)
+      const bool more = __any_sync(0xffffffffu, (low & 0xffffu) != 0);
+      if (lane == 0) mbar_arrive(read0 + 8 * slot);
+      if (q >= kTermStages && !(ok = mbar_wait(summed0 + 8 * (q & 1), ((q >> 1) & 1) ^ 1, status, 31))) break;
+#pragma unroll
+      for (int p = 0; p < 2; ++p) st_shared_16(at + to_w[p], hi[p]);
+      const int place = SPLIT ? 0 : q & 1;
+      if (more || (stale >> place & 1)) {
+        // (one place for both stages: the MMAs of the stage before have to be done)
+        if (SPLIT && q > 0 && !(ok = mbar_wait(summed0 + 8 * ((q - 1) & 1), ((q - 1) >> 1) & 1, status, 31))) break;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          uint4 mid, lo;
+          other_terms(w[p], hi[p], mid, lo);
+          st_shared_16(low0 + place * 2 * kTermTile + to_w[p], mid);
+          st_shared_16(low0 + place * 2 * kTermTile + to_w[p] + kTermTile, lo);
+        }
+      }
+      stale = (stale & ~(1u << place)) | ((more ? 1u : 0u) << place);
+      if (has_x) {
+        uint4 mid, lo;
+        st_shared_16(at + to_x, x_hi);
+        other_terms(x, x_hi, mid, lo);
+        st_shared_16(at + to_x + kXTile, mid);
+        st_shared_16(at + to_x + 2 * kXTile, lo);
+      }
+      if (lane == 0) more_terms[(q & 1) * CW + cw] = more;
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full0 + 8 * (q & 1));
+      if (++slot == depth) {
+        slot = 0;
+        phase ^= 1;
+      }
+    }
+  } else if (warp == AW + CW) {
+    // ------------------------------------------------------------------------------ the values, DEPTH stages ahead
+    if (lane == 0) {
+      pdl_wait();
+      int asked = min(depth, total), s = 0, tile = blockIdx.x, slot = 0, phase = 1;
+#pragma unroll 1
+      for (int q = 0; q < total; ++q) {
+        if (q >= depth) {
+          if (!(ok = mbar_wait(read0 + 8 * slot, phase, status, 38))) break;
+          copy_w(slot, tile, s);
+        }
+        copy_x(slot, s);
+        asked = max(asked, q + 1);
+        if (++s == stages) {
+          s = 0;
+          tile += gridDim.x;
+        }
+        if (++slot == depth) {
+          slot = 0;
+          phase ^= 1;
+        }
+      }
+      if (!ok)                                            // copies in flight land before the block leaves
+        for (int q = max(0, asked - depth); q < asked; ++q) mbar_wait(here0 + 8 * (q % depth), (q / depth) & 1, status, 36);
+    }
+  } else if (lane == 0) {
+    // ------------------------------------------------------------------------------------------- the MMAs
+    // (two threads, a chunk of every stage each: a thread's barriers and commits take longer than its MMAs)
+    const int c = warp - AW - CW - 1;
+#pragma unroll 1
+    for (int q = 0; q < total; ++q) {
+      if (!(ok = mbar_wait(full0 + 8 * (q & 1), (q >> 1) & 1, status, 32))) break;
+      if (q >= 2 && !(ok = mbar_wait(taken0 + 8 * (q & 1), ((q >> 1) & 1) ^ 1, status, 34))) break;
+      tc_fence_after();
+      uint4 more;
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(more.x), "=r"(more.y), "=r"(more.z), "=r"(more.w)
+                   : "r"(smem_u32(more_terms + (q & 1) * CW)) : "memory");
+      const uint32_t base = terms0 + (q & 1) * kStage, low = low0 + (SPLIT ? 0 : (q & 1) * 2 * kTermTile);
+      chunk_mmas<NT>(tmem + (uint32_t)((2 * (q & 1) + c) * NT),
+                     [&](int i) { return i == 0 ? base : i < 3 ? low + (i - 1) * kTermTile : base + kTermTile + (i - 3) * kXTile; },
+                     c, (more.x | more.y | more.z | more.w) != 0);
+      tc_commit(summed0 + 8 * (q & 1));                    // with the other one's: the sums are there, and the stage may be filled again
+    }
+    tc_commit(done);                                      // every MMA that was issued has ended
+    mbar_wait(done, 0, status, 35);
+  }
+  if (SPLIT) {
+    // no block leaves while a sum may still be on its way to it, or before all have one that they wait for
+    __syncwarp();
+    if (warp >= AW) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == AW + CW) tmem_dealloc(tmem, 8 * NT);
+  if (SPLIT) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Rows of 32-bit values, boxes of 32 x box_rows, 128-byte swizzle, zeros outside.
+static bool tensor_map_f32(const float* rows, int n, int k, int ld, int box_rows, CUtensorMap* out) {
+  const EncodeTiledFn fn = encode_fn();
+  const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)n}, strides[1] = {(cuuint64_t)ld * 4};
+  const cuuint32_t box[2] = {32, (cuuint32_t)box_rows}, step[2] = {1, 1};
+  return fn != nullptr && fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(rows), dims, strides, box, step,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// How many clusters of b blocks run at a time (a GPU part's SMs are no multiple of b): asked once.
+template <int NT>
+static int clusters_at_once(int b) {
+  static int counts[9];
+  static std::once_flag once;
+  std::call_once(once, [] {
+    auto kernel = sgemm_tc_few_kernel<NT, true>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess) return;
+    for (int n = 2; n <= 8; ++n) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(1, n, 1);
+      cfg.blockDim = dim3(kFewThreads);
+      cfg.dynamicSmemBytes = kMaxSmem;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 1;
+      attr[0].val.clusterDim.y = n;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&counts[n], kernel, &cfg) != cudaSuccess) counts[n] = 0;
+    }
+    cudaGetLastError();
+  });
+  return counts[b];
+}
+
+template <int NT>
+static int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int* status,
+                      cudaStream_t stream) {
+  const int tiles_n = (N + 127) / 128, tiles_m = (M + NT - 1) / NT, spans = (K + kSpan - 1) / kSpan;
+  if (tiles_m > 65535) return EK_ERR_ARG;
+  // K over the blocks of a cluster where the tiles alone leave SMs idle: the fewest rounds of blocks, a block's cost
+  // taken as its spans and one and a half for its start and end
+  int blocks = 1, each = spans, kept = 0;
+  const long long tiles = (long long)tiles_n * tiles_m;
+  long long best = (tiles + kSms - 1) / kSms * (2 * spans) + 3;
+  for (int b = 2; b <= 8 && b <= spans; ++b) {
+    const int e = (spans + b - 1) / b, at_once = clusters_at_once<NT>(b);
+    const long long sums = (long long)spans * ((min(NT, M) + b - 1) / b) * 512;
+    if (at_once <= 0 || (b - 1) * e >= spans || sums > kMaxSmem - few_fixed(NT, true) - 2 * few_raw(NT)) continue;
+    const long long cost = (tiles + at_once - 1) / at_once * (2 * e + 3);
+    if (cost < best) {
+      best = cost;
+      blocks = b;
+      each = e;
+      kept = (int)sums;
+    }
+  }
+  const bool split = blocks > 1;
+  const int fits = (kMaxSmem - few_fixed(NT, split) - kept) / few_raw(NT), depth = fits < kFewDepth ? fits : kFewDepth;
+  const int smem = few_fixed(NT, split) + kept + depth * few_raw(NT);
+  auto kernel = split ? sgemm_tc_few_kernel<NT, true> : sgemm_tc_few_kernel<NT, false>;
+  CUtensorMap map_w, map_x;
+  if (!tensor_map_f32(W, N, K, ldw, 128, &map_w) || !tensor_map_f32(A, M, K, lda, NT, &map_x)) return EK_ERR_ARG;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+  if (e != cudaSuccess) return (int)e;
+  const dim3 grid(split ? tiles_n : min(tiles_n, max(1, kSms / tiles_m)), blocks, tiles_m);
+  e = split ? launch_pdl_cluster(kernel, grid, dim3(kFewThreads), smem, stream, blocks, map_w, map_x, C, A, W, M, N, K, lda, ldw, ldc,
+                                 each, depth, status)
+            : launch_pdl(kernel, grid, dim3(kFewThreads), smem, stream, map_w, map_x, C, A, W, M, N, K, lda, ldw, ldc, each, depth, status);
+  return (int)(e != cudaSuccess ? e : cudaGetLastError());
+}
+
+// ------------------------------------------------------------------ many rows: operands converted ahead
+// Images: [row block of 128][64 of K][term] tiles of 16 KB as the MMA reads them (K-major, 128-byte swizzle), and
+// one word a (row block, 64 of K): bit 0 - there are second or third terms, bit 1 - a value is infinite or NaN.
+
+__global__ void __launch_bounds__(256)
+sgemm_terms_kernel(uint4* __restrict__ images, uint32_t* __restrict__ flags, const float* __restrict__ A, const float* __restrict__ W,
+                   int M, int N, int K, int lda, int ldw, int w_blocks) {
+  const int tid = threadIdx.x, piece = tid & 7, row = tid >> 3, kb = blockIdx.x, rb = blockIdx.y;
+  const bool is_w = rb < w_blocks;
+  pdl_launch_dependents();
+  const int r0 = (is_w ? rb : rb - w_blocks) * 128, limit = is_w ? N : M, k = kb * 64 + 8 * piece;
+  const float* from = is_w ? W : A;
+  const size_t ld = is_w ? ldw : lda;
+  float v[4][8];
+  uint32_t low = 0, largest = 0;
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    load_row8(v[p], from + (size_t)(r0 + row + 32 * p) * ld + k, r0 + row + 32 * p < limit && k < K);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) low |= __float_as_uint(v[p][j]);
+  }
+  const int more = __syncthreads_or((low & 0xffffu) != 0);
+  uint4* to = images + ((size_t)rb * gridDim.x + kb) * (3 * kTermTile / 16) + row * 8 + (piece ^ (row & 7));
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const uint4 hi = first_terms(v[p], largest);
+    to[p * 256] = hi;
+    if (more) {
+      uint4 mid, lo;
+      other_terms(v[p], hi, mid, lo);
+      to[p * 256 + kTermTile / 16] = mid;
+      to[p * 256 + 2 * kTermTile / 16] = lo;
+    }
+  }
+  const int odd = __syncthreads_or(is_odd(largest));
+  if (tid == 0) flags[(size_t)rb * gridDim.x + kb] = (more ? 1u : 0u) | (odd ? 2u : 0u);
+}
+
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+constexpr int kManyThreads = 352;     // 8 warps that add, one that copies, two that issue MMAs
+constexpr int kManyRing = 13;         // tiles of 16 KB: 3 stages of weights in one term, 2 in three
+constexpr int kManySlots = 4;         // stages that barriers are kept for
+constexpr int kManySmem = kManyRing * kTermTile + 512 + 1024;
+
+// C tiles of 128 columns x NT rows; a block takes tile after tile.  A stage takes the tiles of the ring that it needs:
+// the weights' first term or all three, then the three terms of x.
+template <int NT>
+__global__ void __launch_bounds__(kManyThreads, 1)
+sgemm_tc_many_kernel(float* __restrict__ C, const unsigned char* __restrict__ images, const uint32_t* __restrict__ flags,
+                  const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K, int lda, int ldw, int ldc,
+                  int w_blocks, int* status) {
+  constexpr int COLS = NT / 2;                          // tokens an adding thread takes
+  extern __shared__ unsigned char raw[];
+  unsigned char* ring = raw + ((1024 - (smem_u32(raw) & 1023)) & 1023);
+  uint64_t* bars = (uint64_t*)(ring + kManyRing * kTermTile);   // full[4], freed[4], summed[2], taken[2], done
+  uint32_t* tmem_slot = (uint32_t*)(bars + 14);
+  volatile int* any_odd = (int*)(tmem_slot + 1);
+  volatile int* more_terms = (int*)(tmem_slot + 2);     // of the stage behind each barrier
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int stages = (K + 63) / 64, all_tiles = w_blocks * ((M + NT - 1) / NT);
+  const int tiles = (all_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x, total = tiles * stages;
+  const uint32_t full0 = smem_u32(bars), freed0 = full0 + 32, summed0 = full0 + 64, taken0 = full0 + 80, done = full0 + 96;
+  if (tid == 0) {
+    for (int i = 0; i < kManySlots; ++i) {
+      mbar_init(full0 + 8 * i, 1);
+      mbar_init(freed0 + 8 * i, 2);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(summed0 + 8 * i, 2);
+      mbar_init(taken0 + 8 * i, 8);
+    }
+    mbar_init(done, 2);
+    *any_odd = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 9) tmem_alloc(smem_u32(tmem_slot), 4 * NT);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  bool ok = true;
+  if (warp <= 8) pdl_wait();                              // before images are read and anything is written
+
+  if (warp < 8) {
+    const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * COLS);
+    float span[COLS], sum[COLS];
+    int s = 0, tile = blockIdx.x;
+#pragma unroll 1
+    for (int q = 0; q < total; ++q) {
+      if (!(ok = mbar_wait(summed0 + 8 * (q & 1), (q >> 1) & 1, status, 33))) break;
+      tc_fence_after();
+      const bool fresh = s % kStepSpan == 0;
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int t = 0; t < COLS; t += 16) {
+          float v[16];
+          tmem_ld16(lanes + (uint32_t)((2 * (q & 1) + c) * NT + t), v);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) span[t + j] = c == 0 && fresh ? v[j] : span[t + j] + v[j];
+        }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(taken0 + 8 * (q & 1));
+      const bool last = s + 1 == stages;
+      if (s % kStepSpan == kStepSpan - 1 || last) {
+#pragma unroll
+        for (int t = 0; t < COLS; ++t) sum[t] = s < kStepSpan ? span[t] : sum[t] + span[t];
+      }
+      if (!last) { ++s; continue; }
+      s = 0;
+      const int n = tile % w_blocks * 128 + (warp & 3) * 32 + lane, m0 = tile / w_blocks * NT + (warp >> 2) * COLS;
+#pragma unroll
+      for (int t = 0; t < COLS; ++t)
+        if (n < N && m0 + t < M) C[(size_t)(m0 + t) * ldc + n] = sum[t];
+      if (*any_odd && n < N)
+        for (int m = m0; m < min(M, m0 + COLS); ++m)
+          plain_if_odd(C + (size_t)m * ldc + n, A + (size_t)m * lda, W + (size_t)n * ldw, 0, K);
+      tile += gridDim.x;
+    }
+  } else if (warp == 8) {
+    if (lane == 0) {
+      int s = 0, tile = blockIdx.x, at = 0, room = kManyRing, oldest = 0, asked = 0;
+      uint32_t sizes = 0;                               // tiles of the stages in flight, 8 bits each, the oldest lowest
+      size_t wi = (size_t)(tile % w_blocks) * stages, xi = (size_t)(w_blocks + tile / w_blocks * NT / 128) * stages;
+      uint32_t w_flag = total > 0 ? flags[wi] : 0, x_flag = total > 0 ? flags[xi] : 0;
+#pragma unroll 1
+      for (int q = 0; q < total; ++q) {
+        const bool more = w_flag & 1u;
+        if ((w_flag | x_flag) & 2u) *any_odd = 1;
+        const int need = more ? 6 : 4, slot = q % kManySlots;
+        while (ok && (room < need || q - oldest >= kManySlots)) {
+          ok = mbar_wait(freed0 + 8 * (oldest % kManySlots), (oldest / kManySlots) & 1, status, 31);
+          room += sizes & 255;
+          sizes >>= 8;
+          ++oldest;
+        }
+        if (!ok) break;
+        const unsigned char *w_from = images + wi * (3 * kTermTile),
+                            *x_from = images + xi * (3 * kTermTile) + (tile / w_blocks * NT & 127) * 128;
+        more_terms[slot] = more;
+        const uint32_t bar = full0 + 8 * slot;
+        mbar_expect_tx(bar, (uint32_t)((need - 3) * kTermTile + 3 * NT * 128));
+        for (int i = 0; i < need - 3; ++i) {
+          bulk_load(smem_u32(ring) + at * kTermTile, w_from + i * kTermTile, kTermTile, bar);
+          at = at + 1 == kManyRing ? 0 : at + 1;
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          bulk_load(smem_u32(ring) + at * kTermTile, x_from + i * kTermTile, NT * 128, bar);
+          at = at + 1 == kManyRing ? 0 : at + 1;
+        }
+        sizes |= (uint32_t)need << (8 * (q - oldest));
+        room -= need;
+        asked = q + 1;
+        ++wi;
+        ++xi;
+        if (++s == stages) {
+          s = 0;
+          tile += gridDim.x;
+          wi = (size_t)(tile % w_blocks) * stages;
+          xi = (size_t)(w_blocks + tile / w_blocks * NT / 128) * stages;
+        }
+        if (q + 1 < total) {                            // (their latency passes behind the next wait)
+          w_flag = flags[wi];
+          x_flag = flags[xi];
+        }
+      }
+      if (!ok)                                          // copies in flight land before the block leaves
+        for (int q = oldest; q < asked; ++q) mbar_wait(full0 + 8 * (q % kManySlots), (q / kManySlots) & 1, status, 36);
+    }
+  } else if (lane == 0) {
+    // (two threads, a chunk of every stage each: a thread's barriers and commits take longer than its MMAs)
+    const int c = warp - 9;
+    int at = 0;
+#pragma unroll 1
+    for (int q = 0; q < total; ++q) {
+      const int slot = q % kManySlots;
+      if (!(ok = mbar_wait(full0 + 8 * slot, (q / kManySlots) & 1, status, 32))) break;
+      if (q >= 2 && !(ok = mbar_wait(taken0 + 8 * (q & 1), ((q >> 1) & 1) ^ 1, status, 34))) break;
+      tc_fence_after();
+      const bool more = more_terms[slot] != 0;
+      const int w_tiles = more ? 3 : 1;
+      chunk_mmas<NT>(tmem + (uint32_t)((2 * (q & 1) + c) * NT),
+                     [&](int i) {
+                       const int j = at + (i < 3 ? i : w_tiles + i - 3);
+                       return smem_u32(ring) + (uint32_t)(j >= kManyRing ? j - kManyRing : j) * kTermTile;
+                     }, c, more);
+      tc_commit(freed0 + 8 * slot);
+      tc_commit(summed0 + 8 * (q & 1));
+      at += w_tiles + 3;
+      if (at >= kManyRing) at -= kManyRing;
+    }
+    tc_commit(done);
+    mbar_wait(done, 0, status, 35);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 9) {
+    __syncwarp();
+    tmem_dealloc(tmem, 4 * NT);
+  }
+}
+
+// Bytes of images and flags for `rows` rows of x or of weights.
+static size_t terms_bytes(int rows, int K) {
+  return (size_t)((rows + 127) / 128) * ((K + 63) / 64) * (3 * kTermTile + 4);
+}
+
+template <int NT>
+static int launch_many(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, unsigned char* scratch,
+                       int* status, cudaStream_t stream) {
+  const int w_blocks = (N + 127) / 128, x_blocks = (M + 127) / 128, stages = (K + 63) / 64;
+  uint32_t* flags = (uint32_t*)(scratch + (size_t)(w_blocks + x_blocks) * stages * (3 * kTermTile));
+  if (w_blocks + x_blocks > 65535) return EK_ERR_ARG;
+  sgemm_terms_kernel<<<dim3(stages, w_blocks + x_blocks), 256, 0, stream>>>((uint4*)scratch, flags, A, W, M, N, K, lda, ldw, w_blocks);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return (int)e;
+  auto kernel = sgemm_tc_many_kernel<NT>;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kManySmem);
+  if (e != cudaSuccess) return (int)e;
+  const int tiles = w_blocks * ((M + NT - 1) / NT);
+  return (int)launch_pdl(kernel, dim3(min(tiles, kSms)), dim3(kManyThreads), kManySmem, stream, C, (const unsigned char*)scratch,
+                         (const uint32_t*)flags, A, W, M, N, K, lda, ldw, ldc, w_blocks, status);
+}
+
+constexpr int kFewRows = 64;          // up to here operands are converted on their way in
+constexpr long long kImageBytes = 128ll << 20;    // of weights, and of rows of x, that are converted at a time
+
+// Rows whose images are made at a time: equal parts, whole blocks.
+static int image_rows(int rows, int K) {
+  const long long block = (long long)((K + 63) / 64) * (3 * kTermTile + 4), blocks = (rows + 127) / 128;
+  const long long most = kImageBytes / block > 1 ? kImageBytes / block : 1, parts = (blocks + most - 1) / most;
+  return (int)((blocks + parts - 1) / parts * 128);
+}
+
+static int launch_tc(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc,
+                           unsigned char* scratch, int* status, cudaStream_t stream) {
+  if (M > kFewRows) {
+    if (scratch == nullptr) return EK_ERR_ARG;
+    const int rows_m = min(M, image_rows(M, K)), rows_n = min(N, image_rows(N, K));
+    // 64 rows a tile cost three quarters of what 128 do
+    auto rounds = [&](int nt) { return ((long long)((rows_n + 127) / 128) * ((rows_m + nt - 1) / nt) + kSms - 1) / kSms; };
+    const bool wide = 4 * rounds(128) <= 3 * rounds(64);
+    for (int n = 0; n < N; n += rows_n)
+      for (int m = 0; m < M; m += rows_m) {
+        float* c = C + (size_t)m * ldc + n;
+        const float *a = A + (size_t)m * lda, *w = W + (size_t)n * ldw;
+        const int mm = min(rows_m, M - m), nn = min(rows_n, N - n);
+        const int rc = wide ? launch_many<128>(c, a, w, mm, nn, K, lda, ldw, ldc, scratch, status, stream)
+                            : launch_many<64>(c, a, w, mm, nn, K, lda, ldw, ldc, scratch, status, stream);
+        if (rc != 0) return rc;
+      }
+    return 0;
+  }
+  return M > 16 ? launch_few<32>(C, A, W, M, N, K, lda, ldw, ldc, status, stream)
+                : launch_few<16>(C, A, W, M, N, K, lda, ldw, ldc, status, stream);
 }
 
 }  // namespace ek
 
+// Bytes that a product of these sizes wants for its operands' terms (0: none).
+EK_EXPORT int ek_gemm_f32_scratch(int M, int N, int K) {
+  if (M <= ek::kFewRows || N <= 0 || K <= 0 || K % 8 != 0) return 0;
+  return (int)(ek::terms_bytes(ek::image_rows(M, K), K) + ek::terms_bytes(ek::image_rows(N, K), K));
+}
+
 EK_EXPORT int ek_gemm_nt_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda,
-                             int ldw, int ldc, cudaStream_t stream) {
+                             int ldw, int ldc, void* scratch, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || lda < K || ldw < K || ldc < N) return EK_ERR_ARG;
+  // (a rule on the layout and K, not on M: a row's result does not depend on the rows beside it)
   const bool vec = K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && ((uintptr_t)A & 31) == 0 && ((uintptr_t)W & 31) == 0;
-  return vec ? ek::launch_sgemm<true>(C, A, W, M, N, K, lda, ldw, ldc, stream)
-             : ek::launch_sgemm<false>(C, A, W, M, N, K, lda, ldw, ldc, stream);
+  return vec ? ek::launch_tc(C, A, W, M, N, K, lda, ldw, ldc, (unsigned char*)scratch, status, stream)
+             : ek::launch_ffma(C, A, W, M, N, K, lda, ldw, ldc, stream);
 }

@@ -1055,7 +1055,8 @@ def attention_prefill_tc(out, q, n_tokens, positions, token_slot, cu_seqlens, n_
 
 # ------------------------------------------------------------------ matrix products
 _gemm_f32 = Function("gemm_f32", "ek_gemm_nt_f32",
-                     [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P])
+                     [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P, _P])
+_gemm_f32_scratch = Function("gemm_f32", "ek_gemm_f32_scratch", [c_int, c_int, c_int], check_status=False)
 EPI_BF16, EPI_F32, EPI_SWIGLU, EPI_GEGLU = 0, 1, 2, 3      # GEGLU: the gate is the tanh form of GELU
 # ("clamped" is EPI_SWIGLU with a gate_limit)
 GATED_EPILOGUES = {"silu": EPI_SWIGLU, "gelu_tanh": EPI_GEGLU, "clamped": EPI_SWIGLU}
@@ -1075,7 +1076,11 @@ def gemm_f32(out, x, w, n_rows=None):
     _need(x.shape[-1] == k and out.shape[-1] == n and out.shape[0] >= m, "gemm_f32: shapes disagree")
     if lib.recording():
         lib.annotate(bytes=4 * (n * k + m * k + m * n), flops=2 * m * n * k)
-    _gemm_f32(_ptr(out), _ptr(x), _ptr(w), m, n, k, x.stride(0), w.stride(0), out.stride(0), _stream())
+    # many rows: the operands' bfloat16 terms, in memory of the current stream
+    room = _gemm_f32_scratch(m, n, k)
+    scratch = torch.empty(room, dtype=torch.uint8, device=x.device) if room else None
+    _gemm_f32(_ptr(out), _ptr(x), _ptr(w), m, n, k, x.stride(0), w.stride(0), out.stride(0),
+              _ptr(scratch), tc_status(x.device).data_ptr(), _stream())
 
 
 B200_SM_COUNT = 148        # used only where no device can be asked (launch plans worked out on a CPU box)

@@ -1,6 +1,7 @@
 """y = x . W^T for the engine's two precisions.
 
-* float32: the hand-written FFMA kernel (no tensor-core mode of reduced precision).
+* float32: hand-written kernels that are exact to 32 bits (products of three bfloat16 terms a value on the
+  tensor cores, FFMA where rows are not whole 32-byte pieces; no mode of reduced precision).
 * bfloat16, at most 64 rows (decode): the tcgen05 kernel in its swapped form - weights on the
   128-row side of the MMA, TMA-streamed, K split over blocks.
 * bfloat16, more rows (prefill): the tcgen05 kernel on pairs of SMs (256 x 256 tiles, a

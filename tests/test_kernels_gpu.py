@@ -491,6 +491,58 @@ def test_gemm_f32_forms_sum_in_one_order(m, n, k_, pad):
         assert torch.equal(one[0], out[r])
 
 
+@pytest.mark.parametrize("m,n,k_,pad", [(1, 130, 8, 0), (16, 128, 264, 8), (4, 1000, 2560, 0), (9, 24584, 72, 0), (17, 257, 1032, 0),
+                                        (33, 640, 4104, 0), (64, 300, 512, 16), (65, 300, 512, 0), (129, 1283, 40, 0),
+                                        (200, 2600, 1096, 8), (130, 700, 32768, 0)])
+@pytest.mark.parametrize("weights", ["16", "32", "some"])
+def test_gemm_f32_on_tensor_cores(m, n, k_, pad, weights):
+    """Edges of the tiles (128 columns, 16, 32, 64 and 128 rows), of a stage (64 of K) and a span (256), K shared by a
+    cluster or not, images in parts; weights of one term, of three, and of three in one block of K and rows only.  Every
+    row equals the one-row product bit for bit.  Against 64 bits: a chunk of 32 is cut by about 3e-8 of it, two levels
+    of up to K / 256 and 8 rounded sums of random terms add sqrt(K / 512) 2.5e-8 each: below 4e-7 up to K = 32,768."""
+    k = K()
+    xs, ws = rnd(m, k_ + pad, seed=1).to(DEV), rnd(n, k_ + pad, seed=2).to(DEV)
+    if weights != "32":
+        full = ws.clone()
+        ws = ws.bfloat16().float()
+        if weights == "some":
+            ws[n // 2, k_ // 2:k_ // 2 + 9] = full[n // 2, k_ // 2:k_ // 2 + 9]
+    x, w = xs[:, :k_], ws[:, :k_]
+    out = torch.full((m, n + 3), float("nan"), device=DEV)
+    k.gemm_f32(out[:, :n], x, w)
+    want = x.double() @ w.double().t()
+    assert (out[:, :n].double() - want).norm() <= 4e-7 * want.norm() and out[:, n:].isnan().all()
+    for r in {0, m // 2, m - 1}:
+        one = torch.empty(1, n, device=DEV)
+        k.gemm_f32(one, x[r:r + 1], w)
+        assert torch.equal(one[0], out[r, :n])
+    k.check_tc_status(DEV)
+
+
+@pytest.mark.parametrize("m,n,k_", [(5, 140, 1024), (40, 200, 320), (150, 140, 136)])
+def test_gemm_f32_on_tensor_cores_with_infinities(m, n, k_):
+    """Infinities, NaN and the largest values reach the outputs of their rows as multiplication and addition bring them
+    there, and no other row."""
+    k = K()
+    x, w = rnd(m, k_, seed=1).to(DEV), rnd(n, k_, seed=2).to(DEV)
+    clean = torch.empty(m, n, device=DEV)
+    k.gemm_f32(clean, x, w)
+    w[3, k_ - 1], w[130, 0] = float("inf"), 0.0
+    x[1, 0], x[2, 5], x[4, 7], x[4, 9] = float("inf"), float("nan"), float("inf"), float("-inf")
+    x[3] *= 1e-6
+    x[3, 2], w[7, 2] = 3.4e38, 1e-30
+    out = torch.empty(m, n, device=DEV)
+    k.gemm_f32(out, x, w)
+    want = x.double() @ w.double().t()
+    assert torch.equal(out.isnan(), want.isnan())
+    big = want.abs() > 3.4028235e38                              # (infinite, or beyond what 32 bits hold)
+    near = (want.abs() > 3.39e38) & (want.abs() < 3.42e38)
+    assert torch.equal(out.isinf() & ~near, big & ~near)
+    assert torch.equal(out[5:, 8:130], clean[5:, 8:130])
+    assert abs(out[3, 7].item() - want[3, 7].item()) <= 1e-6 * abs(want[3, 7].item())
+    k.check_tc_status(DEV)
+
+
 @pytest.mark.parametrize("m,n,k_", [(17, 256, 128), (64, 2560, 4096), (33, 1000, 1000), (1, 128, 64),
                                     (48, 331 * 2, 80), (64, 6144, 2560), (24, 1280, 2560),
                                     (24, 20012, 2560)])
