@@ -33,15 +33,20 @@ class EntryView:
         self.spec = spec
         self._group = group
         self._i = index_in_group
+        # (made once: the group's storage stays where it is, and a view costs the host 2 us)
+        pages, data = group.pages, group.data
+        self._k_pages = None if pages is None else pages[index_in_group, 0]
+        self._v_pages = None if pages is None else pages[index_in_group, pages.shape[1] - 1]
+        self._state = None if data is None else data[index_in_group]
 
     @property
     def k_pages(self):
-        return self._group.pages[self._i, 0]
+        return self._k_pages
 
     @property
     def v_pages(self):
         """The value pages; with one plane per token (``CacheSpec.planes == 1``) the key pages again."""
-        return self._group.pages[self._i, self._group.pages.shape[1] - 1]
+        return self._v_pages
 
     @property
     def block_table(self):
@@ -50,7 +55,7 @@ class EntryView:
     @property
     def state(self):
         """[slots, *shape] for ``state`` entries."""
-        return self._group.data[self._i]
+        return self._state
 
 
 class GroupStorage:

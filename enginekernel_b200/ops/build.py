@@ -18,11 +18,12 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
 from concurrent.futures import ThreadPoolExecutor
-from typing import Dict, Iterable, List
+from typing import Dict, Iterable, List, Optional
 
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "csrc")
 CSRC = os.path.normpath(CSRC)
@@ -145,9 +146,43 @@ def ensure_built(module: str) -> str:
     return out
 
 
+HOST_FLAGS = ["-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden"]
+
+
+def host_library() -> Optional[str]:
+    """Path of the built ``csrc/hostcall.cc`` (a Python extension, for this interpreter), compiling it if needed;
+    None where there is no C++ compiler or the interpreter has no headers: the callers then do without it."""
+    src = os.path.join(CSRC, "hostcall.cc")
+    h = hashlib.sha256((" ".join(HOST_FLAGS) + (sysconfig.get_config_var("EXT_SUFFIX") or "")).encode())
+    with open(src, "rb") as f:
+        h.update(f.read())
+    out = os.path.join(build_dir(), f"ek_hostcall.{h.hexdigest()[:16]}.so")
+    include = sysconfig.get_paths()["include"]
+    cxx = shutil.which("g++") or shutil.which("c++")
+    with _lock:
+        if os.path.exists(out):
+            return out
+        if cxx is None or not os.path.exists(os.path.join(include, "Python.h")):
+            return None
+        fd, tmp = tempfile.mkstemp(prefix="ek_hostcall.", suffix=".so.tmp", dir=os.path.dirname(out))
+        os.close(fd)
+        try:
+            done = subprocess.run([cxx] + HOST_FLAGS + ["-I", include, "-o", tmp, src], stdout=subprocess.PIPE,
+                                  stderr=subprocess.STDOUT, text=True)
+            if done.returncode != 0:
+                _say(f"{cxx} failed on hostcall.cc (kernels are called through ctypes):\n{done.stdout}")
+                return None
+            os.replace(tmp, out)
+        finally:
+            if os.path.exists(tmp):
+                os.unlink(tmp)
+    return out
+
+
 def build_all(names: Iterable[str] = None, jobs: int = None) -> Dict[str, str]:
     """Compile every module (or ``names``) in parallel; returns module -> library path."""
     names = list(names) if names is not None else modules()
+    host_library()
     jobs = jobs or min(len(names), os.cpu_count() or 1) or 1
     with ThreadPoolExecutor(max_workers=jobs) as pool:
         paths = list(pool.map(ensure_built, names))

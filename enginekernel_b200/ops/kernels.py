@@ -34,10 +34,6 @@ def _suffix(dtype) -> str:
         raise KernelError(f"kernels exist for float32 and bfloat16, not {dtype}") from None
 
 
-def _ptr(t):
-    return None if t is None else t.data_ptr()
-
-
 def _slow_stream():
     return torch.cuda.current_stream().cuda_stream
 
@@ -123,8 +119,8 @@ def embed(resid, table, ids, n_tokens, scale=1.0, pos_table=None, positions=None
     if lib.recording():
         lib.annotate(bytes=n_tokens * hidden * (table.element_size() * (2 if pos_table is not None else 1)
                                                 + (8 if accumulate else 4)))
-    _embed[table.dtype](_ptr(resid), _ptr(table), _ptr(ids), n_tokens, hidden, vocab, float(scale),
-                        _ptr(pos_table), _ptr(positions), max_positions, 1 if accumulate else 0, _stream())
+    _embed[table.dtype](resid, table, ids, n_tokens, hidden, vocab, float(scale),
+                        pos_table, positions, max_positions, 1 if accumulate else 0, _stream())
 
 
 def scale_(x, scale, n=None):
@@ -134,7 +130,7 @@ def scale_(x, scale, n=None):
     count = x.numel() if n is None else n
     if lib.recording():
         lib.annotate(bytes=8 * count)
-    _scale_f32(_ptr(x), count, float(scale), _stream())
+    _scale_f32(x, count, float(scale), _stream())
 
 
 def scale_cap_(x, scale, cap, n=None):
@@ -144,7 +140,7 @@ def scale_cap_(x, scale, cap, n=None):
     count = x.numel() if n is None else n
     if lib.recording():
         lib.annotate(bytes=8 * count)
-    _scale_cap_f32(_ptr(x), count, float(scale), float(cap), _stream())
+    _scale_cap_f32(x, count, float(scale), float(cap), _stream())
 
 
 def rmsnorm(y, resid, gain, eps, add=None, rows=None, n_rows=None, write_back=True):
@@ -163,7 +159,7 @@ def rmsnorm(y, resid, gain, eps, add=None, rows=None, n_rows=None, write_back=Tr
     if lib.recording():
         per_value = 4 + y.element_size() + ((y.element_size() + (4 if write_back else 0)) if add is not None else 0)
         lib.annotate(bytes=n_rows * hidden * per_value)
-    _rmsnorm[y.dtype](_ptr(y), _ptr(resid), _ptr(add), _ptr(gain), _ptr(rows), float(eps),
+    _rmsnorm[y.dtype](y, resid, add, gain, rows, float(eps),
                       n_rows, hidden, 1 if write_back else 0, _stream())
 
 
@@ -194,8 +190,8 @@ def rmsnorm_scaled_sum(y, resid, a, gain, eps, scale_a=None, b=None, scale_b=Non
     if lib.recording():
         lib.annotate(bytes=n_rows * hidden * (4 + (4 if write_back else 0)
                                               + y.element_size() * (2 if b is None else 3)))
-    _rmsnorm_scaled_sum[y.dtype](_ptr(y), _ptr(resid), _ptr(a), _ptr(scale_a), _ptr(b), _ptr(scale_b), _ptr(gain),
-                                 _ptr(rows), float(eps), n_rows, hidden, 1 if write_back else 0, _stream())
+    _rmsnorm_scaled_sum[y.dtype](y, resid, a, scale_a, b, scale_b, gain,
+                                 rows, float(eps), n_rows, hidden, 1 if write_back else 0, _stream())
 
 
 _add_scaled = _per_dtype("elementwise", "ek_add_scaled", [_P, _P, _P, _P, _P, c_longlong, c_int, _P])
@@ -215,14 +211,14 @@ def add_scaled(resid, a, scale_a=None, b=None, scale_b=None, n_rows=None):
     n = (n_rows if n_rows is not None else resid.shape[0]) * hidden
     if lib.recording():
         lib.annotate(bytes=n * (8 + a.element_size() * (1 if b is None else 2)))
-    _add_scaled[a.dtype](_ptr(resid), _ptr(a), _ptr(scale_a), _ptr(b), _ptr(scale_b), n, hidden, _stream())
+    _add_scaled[a.dtype](resid, a, scale_a, b, scale_b, n, hidden, _stream())
 
 
 def add_residual(resid, x, n_rows=None):
     _need_cuda(resid, x)
     n = (n_rows if n_rows is not None else resid.shape[0]) * resid.shape[-1]
     _need(resid.dtype == torch.float32 and x.shape[-1] == resid.shape[-1], "add_residual: shapes")
-    _add_residual[x.dtype](_ptr(resid), _ptr(x), n, _stream())
+    _add_residual[x.dtype](resid, x, n, _stream())
 
 
 def silu_mul(out, gu, n_rows=None):
@@ -246,7 +242,7 @@ def act_mul(out, gu, activation="silu", n_rows=None, limit=0.0):
         lib.annotate(bytes=3 * rows * inter * gu.element_size())
     for r0 in range(0, rows, 65535):
         r1 = min(rows, r0 + 65535)
-        _act_mul[gu.dtype](_ptr(out[r0:]), _ptr(gu[r0:]), r1 - r0, inter, GATE_ACTIVATIONS[activation],
+        _act_mul[gu.dtype](out[r0:], gu[r0:], r1 - r0, inter, GATE_ACTIVATIONS[activation],
                            float(limit), _stream())
 
 
@@ -272,7 +268,7 @@ def embed_pair(resid, table, ids, positions, token_slot, before, n_tokens, bucke
           and token_slot.dtype == torch.int32, "embed_pair: int32 indices and previous tokens")
     if lib.recording():
         lib.annotate(bytes=n_tokens * hidden * (table.element_size() + 8))
-    _embed_pair[table.dtype](_ptr(resid), _ptr(table), _ptr(ids), _ptr(positions), _ptr(token_slot), _ptr(before),
+    _embed_pair[table.dtype](resid, table, ids, positions, token_slot, before,
                              before.stride(0), n_tokens, hidden, int(buckets), int(mul_prev), int(mul_cur), _stream())
 
 
@@ -280,7 +276,7 @@ def keep_last_token(before, ids, positions, token_slot, n_tokens):
     """before[slot] = the last token each sequence of the step brought."""
     _need_cuda(before, ids, positions, token_slot)
     _need(before.dtype == torch.int32, "keep_last_token: int32 state")
-    _keep_last_token(_ptr(before), before.stride(0), _ptr(ids), _ptr(positions), _ptr(token_slot), n_tokens, _stream())
+    _keep_last_token(before, before.stride(0), ids, positions, token_slot, n_tokens, _stream())
 
 
 def cast_columns(dst, col0, src, n_rows):
@@ -291,7 +287,7 @@ def cast_columns(dst, col0, src, n_rows):
           and col0 + width <= dst.shape[-1], "cast_columns: 32-bit source rows that fit the destination's")
     if lib.recording():
         lib.annotate(bytes=n_rows * width * (4 + dst.element_size()))
-    _cast_columns[dst.dtype](_ptr(dst), dst.stride(0), col0, _ptr(src), width, n_rows, _stream())
+    _cast_columns[dst.dtype](dst, dst.stride(0), col0, src, width, n_rows, _stream())
 
 
 def rmsnorm_post_add(y, resid, a, gain_post, eps_post, gain=None, eps=0.0, weight_a=1.0, b=None, weight_b=1.0,
@@ -312,8 +308,8 @@ def rmsnorm_post_add(y, resid, a, gain_post, eps_post, gain=None, eps=0.0, weigh
     n = n_rows if n_rows is not None else resid.shape[0]
     if lib.recording():
         lib.annotate(bytes=n * hidden * (8 + a.element_size() * ((1 if b is None else 2) + (0 if y is None else 1))))
-    _rmsnorm_post_add[a.dtype](_ptr(y), _ptr(resid), _ptr(a), float(weight_a), _ptr(b), float(weight_b), _ptr(bias),
-                               _ptr(gain_post), float(eps_post), _ptr(gain), float(eps), n, hidden, _stream())
+    _rmsnorm_post_add[a.dtype](y, resid, a, float(weight_a), b, float(weight_b), bias,
+                               gain_post, float(eps_post), gain, float(eps), n, hidden, _stream())
 
 
 def bias_act(out, x, bias=None, activation=None, col0=0, n_rows=None):
@@ -328,7 +324,7 @@ def bias_act(out, x, bias=None, activation=None, col0=0, n_rows=None):
     n = n_rows if n_rows is not None else out.shape[0]
     if lib.recording():
         lib.annotate(bytes=n * width * (x.element_size() + out.element_size()))
-    _bias_act[out.dtype](_ptr(out), _ptr(x), 1 if x.dtype == torch.float32 else 0, x.stride(0), col0, _ptr(bias),
+    _bias_act[out.dtype](out, x, 1 if x.dtype == torch.float32 else 0, x.stride(0), col0, bias,
                          width, n, ROW_ACTIVATIONS[activation], _stream())
 
 
@@ -350,7 +346,7 @@ def _tanh_norm_args(y, norm, hidden, name):
     for t, n in ((alpha, 1), (w, hidden), (b, hidden)):
         _need(t.dtype == torch.float32 and t.is_contiguous() and t.numel() == n,
               f"{name}: 32-bit alpha [1], weight and shift of the stream's width")
-    return [_ptr(t) for t in (y, alpha, w, b)]
+    return [t for t in (y, alpha, w, b)]
 
 
 def dynamic_tanh(y, stream, norm, second=None, second_norm=None, add=None, rows=None, n_rows=None, write_back=True):
@@ -368,8 +364,8 @@ def dynamic_tanh(y, stream, norm, second=None, second_norm=None, add=None, rows=
         lib.annotate(bytes=n * hidden * (4 + y.element_size() * ((1 if second is None else 2) + (0 if add is None else 1))
                                          + (4 if add is not None and write_back else 0)))
     _dynamic_tanh[y.dtype](*_tanh_norm_args(y, norm, hidden, "dynamic_tanh"),
-                           *_tanh_norm_args(second, second_norm, hidden, "dynamic_tanh"), _ptr(stream), _ptr(add),
-                           _ptr(rows), n, hidden, 1 if write_back else 0, _stream())
+                           *_tanh_norm_args(second, second_norm, hidden, "dynamic_tanh"), stream, add,
+                           rows, n, hidden, 1 if write_back else 0, _stream())
 
 
 def depth_join(x_next, x, first, kept, n, depth, mult, a, gate_a, f=None, gate_f=None, bias_a=None, pair=None,
@@ -408,10 +404,10 @@ def depth_join(x_next, x, first, kept, n, depth, mult, a, gate_a, f=None, gate_f
         streams = (0 if x.data_ptr() == first.data_ptr() else 1) + n + 1 + (1 if keep else 0)
         narrow = sum(1 for t in (a, b, za, f, zf, y1, y2) if t is not None)
         lib.annotate(bytes=rows * hidden * (4 * streams + a.element_size() * narrow))
-    _depth_join[a.dtype](_ptr(x), _ptr(x_next), _ptr(first), _ptr(kept),
-                         kept.stride(0) if kept is not None else 0, _ptr(depth), n, 1 if keep else 0, float(mult), _ptr(a),
-                         _ptr(bias_a), _ptr(b), _ptr(gain_a), _ptr(gain_b), float(eps), float(weight), _ptr(za), _ptr(ba),
-                         _ptr(f), _ptr(zf), _ptr(bf), *_tanh_norm_args(y1, norm1, hidden, "depth_join"),
+    _depth_join[a.dtype](x, x_next, first, kept,
+                         kept.stride(0) if kept is not None else 0, depth, n, 1 if keep else 0, float(mult), a,
+                         bias_a, b, gain_a, gain_b, float(eps), float(weight), za, ba,
+                         f, zf, bf, *_tanh_norm_args(y1, norm1, hidden, "depth_join"),
                          *_tanh_norm_args(y2, norm2, hidden, "depth_join"), rows, hidden, _stream())
 
 
@@ -461,11 +457,11 @@ def qk_prepare_kv(qkv, n_tokens, q_gain, k_gain, cos, sin, rot_dim, positions, t
     _need(every >= 1, "qk_prepare_kv: the temperature's step must be at least one position")
     if lib.recording():
         lib.annotate(bytes=n_tokens * head_dim * qkv.element_size() * (2 * n_q_heads + 3 * n_kv_heads))
-    _qk_prepare[qkv.dtype](_ptr(qkv), qkv.stride(0), _ptr(q_gain), _ptr(k_gain), _ptr(cos), _ptr(sin),
-                           rot_dim, _ptr(positions), _ptr(token_slot), _ptr(k_pages), _ptr(v_pages),
-                           _ptr(block_table), block_table.stride(0), n_tokens, n_q_heads, n_kv_heads,
-                           head_dim, float(eps), 1 if write_kv else 0, _ptr(q_bias), _ptr(k_bias),
-                           _ptr(v_bias), coef, every, 1 if values_from_keys else 0, _stream())
+    _qk_prepare[qkv.dtype](qkv, qkv.stride(0), q_gain, k_gain, cos, sin,
+                           rot_dim, positions, token_slot, k_pages, v_pages,
+                           block_table, block_table.stride(0), n_tokens, n_q_heads, n_kv_heads,
+                           head_dim, float(eps), 1 if write_kv else 0, q_bias, k_bias,
+                           v_bias, coef, every, 1 if values_from_keys else 0, _stream())
 
 
 _qk_prepare_padded = _per_dtype("rope_kv", "ek_qk_prepare_padded_kv",
@@ -494,11 +490,11 @@ def qk_prepare_padded_kv(qkv, n_tokens, q_gain, k_gain, cos, sin, rot_dim, posit
               "qk_prepare_padded_kv: biases are 32-bit [heads * D]")
     if lib.recording():
         lib.annotate(bytes=n_tokens * head_dim * qkv.element_size() * (2 * n_q_heads + 3 * n_kv_heads))
-    _qk_prepare_padded[qkv.dtype](_ptr(qkv), qkv.stride(0), _ptr(q_gain), _ptr(k_gain), _ptr(cos), _ptr(sin),
-                                  rot_dim, _ptr(positions), _ptr(token_slot), _ptr(k_pages), _ptr(v_pages),
-                                  _ptr(block_table), block_table.stride(0), n_tokens, n_q_heads, n_kv_heads,
-                                  head_dim, float(eps), 1 if write_kv else 0, _ptr(q_bias), _ptr(k_bias),
-                                  _ptr(v_bias), int(norm_dim), 1 if value_unit_eps is not None else 0,
+    _qk_prepare_padded[qkv.dtype](qkv, qkv.stride(0), q_gain, k_gain, cos, sin,
+                                  rot_dim, positions, token_slot, k_pages, v_pages,
+                                  block_table, block_table.stride(0), n_tokens, n_q_heads, n_kv_heads,
+                                  head_dim, float(eps), 1 if write_kv else 0, q_bias, k_bias,
+                                  v_bias, int(norm_dim), 1 if value_unit_eps is not None else 0,
                                   int(value_dim or head_dim), float(value_unit_eps or 0.0), _stream())
 
 
@@ -520,9 +516,9 @@ def qk_norm_rope_kv(qkv, n_tokens, q_gain, k_gain, cos, sin, rot_dim, positions,
         _need(g is None or (g.dtype == torch.float32 and g.numel() == head_dim), "qk gains: 32-bit [D]")
     if lib.recording():
         lib.annotate(bytes=n_tokens * head_dim * qkv.element_size() * (2 * n_q_heads + 3 * n_kv_heads))
-    _rope_kv[qkv.dtype](_ptr(qkv), qkv.stride(0), _ptr(q_gain), _ptr(k_gain), _ptr(cos), _ptr(sin),
-                        rot_dim, _ptr(positions), _ptr(token_slot), _ptr(k_pages), _ptr(v_pages),
-                        _ptr(block_table), block_table.stride(0), n_tokens, n_q_heads, n_kv_heads,
+    _rope_kv[qkv.dtype](qkv, qkv.stride(0), q_gain, k_gain, cos, sin,
+                        rot_dim, positions, token_slot, k_pages, v_pages,
+                        block_table, block_table.stride(0), n_tokens, n_q_heads, n_kv_heads,
                         head_dim, float(eps), 1 if write_kv else 0, _stream())
 
 
@@ -554,8 +550,8 @@ def qk_whole_norm_kv(rows, n_tokens, q_gain, k_gain, cos, sin, rot_dim, position
               "qk_whole_norm_kv: gains are 32-bit [heads * D]")
     if lib.recording():
         lib.annotate(bytes=n_tokens * head_dim * rows.element_size() * (2 * n_q_heads + (4 * n_kv_heads if write_kv else 0)))
-    _whole_norm_kv[rows.dtype](_ptr(rows), rows.stride(0), _ptr(q_gain), _ptr(k_gain), _ptr(cos), _ptr(sin), rot_dim,
-                               _ptr(positions), _ptr(token_slot), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
+    _whole_norm_kv[rows.dtype](rows, rows.stride(0), q_gain, k_gain, cos, sin, rot_dim,
+                               positions, token_slot, k_pages, v_pages, block_table,
                                block_table.stride(0), n_tokens, n_q_heads, n_kv_heads, head_dim,
                                int(norm_dim or head_dim), float(eps), 1 if write_kv else 0, _stream())
 
@@ -584,8 +580,8 @@ def qk_rope_unit_kv(rows, n_tokens, k_col, v_col, cos, sin, rot_dim, positions, 
           and token_slot.dtype == torch.int32, "qk_rope_unit_kv: int32 indices")
     if lib.recording():
         lib.annotate(bytes=n_tokens * head_dim * rows.element_size() * (2 * n_q_heads + (4 * n_kv_heads if write_kv else 0)))
-    _rope_unit_kv[rows.dtype](_ptr(rows), rows.stride(0), k_col, v_col, _ptr(cos), _ptr(sin), rot_dim,
-                              _ptr(positions), _ptr(token_slot), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
+    _rope_unit_kv[rows.dtype](rows, rows.stride(0), k_col, v_col, cos, sin, rot_dim,
+                              positions, token_slot, k_pages, v_pages, block_table,
                               block_table.stride(0), n_tokens, n_q_heads, n_kv_heads, head_dim, norm_dim,
                               float(eps), 1 if unit else 0, 1 if write_kv else 0, _stream())
 
@@ -642,12 +638,12 @@ def attention_generic(out, q, n_tokens, positions, token_slot, k_pages, v_pages,
               and part_acc.numel() >= n_tokens * n_q_heads * n_splits * head_dim
               and part_ml.numel() >= n_tokens * n_q_heads * n_splits * 2, "attention: split buffers")
     _attention_cost(q, n_tokens, positions, n_q_heads, n_kv_heads, head_dim, window, False, chunk)
-    _attn_generic[q.dtype](_ptr(out), _ptr(q), q.stride(0), _ptr(positions), _ptr(token_slot),
-                           _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.stride(0),
+    _attn_generic[q.dtype](out, q, q.stride(0), positions, token_slot,
+                           k_pages, v_pages, block_table, block_table.stride(0),
                            n_tokens, n_q_heads, n_kv_heads, head_dim, float(scale),
-                           int(window or 0), n_splits, keys_per_split, _ptr(part_acc),
-                           _ptr(part_ml), _sink(sink), _sinks(sinks, n_q_heads), int(keep_first or 0),
-                           _ptr(gate), gate.stride(0) if gate is not None else 0, int(chunk or 0),
+                           int(window or 0), n_splits, keys_per_split, part_acc,
+                           part_ml, _sink(sink), _sinks(sinks, n_q_heads), int(keep_first or 0),
+                           gate, gate.stride(0) if gate is not None else 0, int(chunk or 0),
                            float(softcap or 0.0), _stream())
     if n_splits > 1:
         count_extra_launches()               # the merge kernel
@@ -677,10 +673,10 @@ def attention_generic_cross(parts, q, n_tokens, positions, token_slot, k_pages, 
               and part_acc.numel() >= n_tokens * n_q_heads * n_kv_heads * n_splits * head_dim
               and part_ml.numel() >= n_tokens * n_q_heads * n_kv_heads * n_splits * 2, "attention: split buffers")
     _attention_cost(q, n_tokens, positions, n_q_heads * n_kv_heads, n_kv_heads, head_dim, window, False)
-    _attn_generic_cross[q.dtype](_ptr(parts), _ptr(q), q.stride(0), _ptr(positions), _ptr(token_slot),
-                                 _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.stride(0),
+    _attn_generic_cross[q.dtype](parts, q, q.stride(0), positions, token_slot,
+                                 k_pages, v_pages, block_table, block_table.stride(0),
                                  n_tokens, n_q_heads, n_kv_heads, head_dim, float(scale), int(window or 0),
-                                 n_splits, keys_per_split, _ptr(part_acc), _ptr(part_ml), int(keep_first or 0),
+                                 n_splits, keys_per_split, part_acc, part_ml, int(keep_first or 0),
                                  _stream())
     if n_splits > 1:
         count_extra_launches()
@@ -698,8 +694,8 @@ def mix_heads(out, parts, mix, positions, n_tokens, n_q_heads, n_kv_heads, head_
     if lib.recording():
         lib.annotate(bytes=n_tokens * n_q_heads * (4 * n_kv_heads * head_dim + 2 * value_dim * out.element_size()),
                      flops=2 * n_tokens * n_q_heads * n_q_heads * value_dim)
-    _mix_heads[out.dtype](_ptr(out), _ptr(parts), _ptr(mix), _ptr(gate), gate.stride(0) if gate is not None else 0,
-                          _ptr(positions), n_tokens, n_q_heads, n_kv_heads, head_dim, value_dim, _stream())
+    _mix_heads[out.dtype](out, parts, mix, gate, gate.stride(0) if gate is not None else 0,
+                          positions, n_tokens, n_q_heads, n_kv_heads, head_dim, value_dim, _stream())
 
 
 _attn_decode_bf16 = Function("attention_decode_bf16", "ek_attention_decode_bf16",
@@ -728,10 +724,10 @@ def attention_decode_cross_bf16(parts, q, n_tokens, positions, token_slot, k_pag
               and part_acc.numel() >= n_tokens * n_q_heads * n_kv_heads * n_splits * head_dim
               and part_ml.numel() >= n_tokens * n_q_heads * n_kv_heads * n_splits * 2, "attention: split buffers")
     _attention_cost(q, n_tokens, positions, n_q_heads * n_kv_heads, n_kv_heads, head_dim, window, False)
-    _attn_decode_cross(_ptr(parts), _ptr(q), q.stride(0), _ptr(positions), _ptr(token_slot), _ptr(k_pages),
-                       _ptr(v_pages), _ptr(block_table), block_table.stride(0), n_tokens, n_q_heads, n_kv_heads,
-                       head_dim, float(scale), int(window or 0), n_splits, keys_per_split, _ptr(part_acc),
-                       _ptr(part_ml), int(keep_first or 0), _stream())
+    _attn_decode_cross(parts, q, q.stride(0), positions, token_slot, k_pages,
+                       v_pages, block_table, block_table.stride(0), n_tokens, n_q_heads, n_kv_heads,
+                       head_dim, float(scale), int(window or 0), n_splits, keys_per_split, part_acc,
+                       part_ml, int(keep_first or 0), _stream())
     if n_splits > 1:
         count_extra_launches()
 
@@ -741,7 +737,7 @@ def _gate_args(gate, q, n_q_heads):
     _need(gate is None or (gate.is_cuda and gate.dtype == q.dtype and gate.stride(-1) == 1
                            and gate.shape[-1] >= n_q_heads),
           "attention: the gate holds one value per token and query head, in q's dtype")
-    return _ptr(gate), (gate.stride(0) if gate is not None else 0)
+    return gate, (gate.stride(0) if gate is not None else 0)
 
 
 def attention_decode_supported(dtype, head_dim):
@@ -767,10 +763,10 @@ def attention_decode_bf16(out, q, n_tokens, positions, token_slot, k_pages, v_pa
               and part_acc.numel() >= n_tokens * n_q_heads * n_splits * head_dim
               and part_ml.numel() >= n_tokens * n_q_heads * n_splits * 2, "attention: split buffers")
     _attention_cost(q, n_tokens, positions, n_q_heads, n_kv_heads, head_dim, window, False, chunk)
-    _attn_decode_bf16(_ptr(out), _ptr(q), q.stride(0), _ptr(positions), _ptr(token_slot),
-                      _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.stride(0),
+    _attn_decode_bf16(out, q, q.stride(0), positions, token_slot,
+                      k_pages, v_pages, block_table, block_table.stride(0),
                       n_tokens, n_q_heads, n_kv_heads, head_dim, float(scale), int(window or 0),
-                      n_splits, keys_per_split, _ptr(part_acc), _ptr(part_ml), _sink(sink),
+                      n_splits, keys_per_split, part_acc, part_ml, _sink(sink),
                       _sinks(sinks, n_q_heads), int(keep_first or 0), *_gate_args(gate, q, n_q_heads),
                       int(chunk or 0), float(softcap or 0.0), _stream())
     if n_splits > 1:
@@ -833,10 +829,10 @@ def attention_decode_tma(out, q, n_tokens, positions, token_slot, k_pages, v_pag
           f"attention_decode_tma: 1 to {decode_tma_max_splits(head_dim, q.device)} splits on this device")
     _need(n_tokens <= 65535, "attention_decode_tma: at most 65535 tokens a call")
     _attention_cost(q, n_tokens, positions, n_q_heads, n_kv_heads, head_dim, window, False, chunk)
-    _attn_decode_tma(_ptr(out), _ptr(q), q.stride(0), _ptr(positions), _ptr(token_slot),
-                     _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table),
+    _attn_decode_tma(out, q, q.stride(0), positions, token_slot,
+                     k_pages, v_pages, k_pages.shape[0], block_table,
                      block_table.stride(0), n_tokens, n_q_heads, n_kv_heads, head_dim, float(scale),
-                     int(window or 0), n_splits, _ptr(tc_status(q.device)), _sink(sink),
+                     int(window or 0), n_splits, tc_status(q.device), _sink(sink),
                      _sinks(sinks, n_q_heads), int(chunk or 0), float(softcap or 0.0),
                      *_gate_args(gate, q, n_q_heads), _stream())
 
@@ -867,9 +863,9 @@ def attention_prefill_bf16(out, q, n_tokens, positions, token_slot, cu_seqlens, 
     _need(q.stride(-1) == 1 and q.stride(0) % 8 == 0, "attention: dense, 16-byte aligned q rows")
     _need(cu_seqlens.dtype == torch.int32 and cu_seqlens.numel() >= n_seqs + 1, "attention: cu_seqlens")
     _attention_cost(q, n_tokens, positions, n_q_heads, n_kv_heads, head_dim, window, True, chunk)
-    _attn_prefill_bf16(_ptr(out), _ptr(q), q.stride(0), _ptr(positions), _ptr(token_slot),
-                       _ptr(cu_seqlens), n_seqs, n_tokens, _ptr(k_pages), _ptr(v_pages),
-                       _ptr(block_table), block_table.stride(0), n_q_heads, n_kv_heads, head_dim,
+    _attn_prefill_bf16(out, q, q.stride(0), positions, token_slot,
+                       cu_seqlens, n_seqs, n_tokens, k_pages, v_pages,
+                       block_table, block_table.stride(0), n_q_heads, n_kv_heads, head_dim,
                        float(scale), int(window or 0), _sink(sink), _sinks(sinks, n_q_heads),
                        int(keep_first or 0), *_gate_args(gate, q, n_q_heads), int(chunk or 0),
                        float(softcap or 0.0), _stream())
@@ -916,10 +912,10 @@ def attention_prefill_f32(out, q, n_tokens, positions, token_slot, cu_seqlens, n
           "attention: the gate holds one value per token and query head, in q's dtype")
     _need(cu_seqlens.dtype == torch.int32 and cu_seqlens.numel() >= n_seqs + 1, "attention: cu_seqlens")
     _attention_cost(q, n_tokens, positions, n_q_heads, n_kv_heads, head_dim, window, True, chunk)
-    _attn_prefill_f32(_ptr(out), _ptr(q), q.stride(0), _ptr(positions), _ptr(token_slot), _ptr(cu_seqlens), n_seqs,
-                      n_tokens, _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.stride(0), n_q_heads,
+    _attn_prefill_f32(out, q, q.stride(0), positions, token_slot, cu_seqlens, n_seqs,
+                      n_tokens, k_pages, v_pages, block_table, block_table.stride(0), n_q_heads,
                       n_kv_heads, head_dim, float(scale), int(window or 0), _sink(sink), _sinks(sinks, n_q_heads),
-                      int(keep_first or 0), _ptr(gate), gate.stride(0) if gate is not None else 0, int(chunk or 0),
+                      int(keep_first or 0), gate, gate.stride(0) if gate is not None else 0, int(chunk or 0),
                       float(softcap or 0.0), _stream())
 
 
@@ -943,8 +939,8 @@ def attention_prefill_cross_bf16(parts, q, n_tokens, positions, token_slot, cu_s
           and parts.numel() >= n_tokens * n_q_heads * n_kv_heads * head_dim and q.stride(-1) == 1
           and q.stride(0) % 8 == 0, "attention_prefill_cross_bf16: parts [T, NQ, NKV, D] in 32-bit")
     _attention_cost(q, n_tokens, positions, n_q_heads * n_kv_heads, n_kv_heads, head_dim, window, True)
-    _attn_prefill_cross(_ptr(parts), _ptr(q), q.stride(0), _ptr(positions), _ptr(token_slot), _ptr(cu_seqlens), n_seqs,
-                        n_tokens, _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.stride(0), n_q_heads,
+    _attn_prefill_cross(parts, q, q.stride(0), positions, token_slot, cu_seqlens, n_seqs,
+                        n_tokens, k_pages, v_pages, block_table, block_table.stride(0), n_q_heads,
                         n_kv_heads, head_dim, float(scale), int(window or 0), int(keep_first or 0), _stream())
 
 
@@ -981,8 +977,9 @@ PREFILL_BAND_L2_SHARE = 0.5
 def prefill_band_tokens(n_kv_heads, head_dim, device=None) -> int:
     """Tokens of context whose 16-bit keys and values of one layer fill ``PREFILL_BAND_L2_SHARE`` of
     the device's L2: the sequences that the prompt attention works on together."""
-    index = torch.cuda.current_device() if device is None or torch.device(device).index is None \
-        else torch.device(device).index
+    index = None if device is None else device.index if type(device) is torch.device else torch.device(device).index
+    if index is None:
+        index = torch.cuda.current_device()
     if index not in _l2_bytes:
         _l2_bytes[index] = int(torch.cuda.get_device_properties(index).L2_cache_size)
     return max(1, int(_l2_bytes[index] * PREFILL_BAND_L2_SHARE) // (4 * n_kv_heads * head_dim))
@@ -1004,7 +1001,7 @@ def attention_prefill_tiles(tiles, n_tokens, positions, token_slot, cu_seqlens, 
           and tiles.data_ptr() % 16 == 0, "attention_prefill_tiles: int32 [tiles, 4], 16-byte aligned")
     _need(n_seqs <= PREFILL_TC_MAX_SEQS, f"attention_prefill_tc: at most {PREFILL_TC_MAX_SEQS} sequences a step")
     _need(cu_seqlens.dtype == torch.int32 and cu_seqlens.numel() >= n_seqs + 1, "attention: cu_seqlens")
-    _attn_prefill_tiles(_ptr(tiles), need, _ptr(cu_seqlens), _ptr(positions), _ptr(token_slot), n_seqs,
+    _attn_prefill_tiles(tiles, need, cu_seqlens, positions, token_slot, n_seqs,
                         tok_per_tile, prefill_band_tokens(n_kv_heads, head_dim, tiles.device), _stream())
     return need
 
@@ -1079,8 +1076,8 @@ def gemm_f32(out, x, w, n_rows=None):
     # many rows: the operands' bfloat16 terms, in memory of the current stream
     room = _gemm_f32_scratch(m, n, k)
     scratch = torch.empty(room, dtype=torch.uint8, device=x.device) if room else None
-    _gemm_f32(_ptr(out), _ptr(x), _ptr(w), m, n, k, x.stride(0), w.stride(0), out.stride(0),
-              _ptr(scratch), tc_status(x.device).data_ptr(), _stream())
+    _gemm_f32(out, x, w, m, n, k, x.stride(0), w.stride(0), out.stride(0),
+              scratch, tc_status(x.device).data_ptr(), _stream())
 
 
 B200_SM_COUNT = 148        # used only where no device can be asked (launch plans worked out on a CPU box)
@@ -1108,11 +1105,14 @@ def split_scratch(device):
     """Per-device scratch of products whose K is split over more blocks than a cluster holds:
     partial tiles and zeroed tickets.  Created on first use; create it before capturing a graph
     (``ModelRunner`` does)."""
-    key = str(torch.device(device))
-    if key not in _split_scratch:
-        _split_scratch[key] = (torch.empty(_SPLIT_PARTIAL_FLOATS, dtype=torch.float32, device=device),
-                               torch.zeros(_SPLIT_TICKETS, dtype=torch.int32, device=device))
-    return _split_scratch[key]
+    made = _split_scratch.get(device)            # (by the torch.device that launches hand over)
+    if made is None:
+        key = torch.device(device)
+        if key not in _split_scratch:
+            _split_scratch[key] = (torch.empty(_SPLIT_PARTIAL_FLOATS, dtype=torch.float32, device=device),
+                                   torch.zeros(_SPLIT_TICKETS, dtype=torch.int32, device=device))
+        made = _split_scratch[key]
+    return made
 
 
 _gemm_tc = Function("gemm_tc_bf16", "ek_gemm_tc_bf16",
@@ -1152,7 +1152,7 @@ def wait_that_runs_out(device, code=77, limit=4096):
     records ``code`` in the device's status word - what a kernel does when a wait of its own runs
     out.  The kernel ends by itself; :func:`check_tc_status` then raises."""
     with torch.cuda.device(device):
-        _wait_that_runs_out(_ptr(tc_status(device)), int(code), int(limit), _stream())
+        _wait_that_runs_out(tc_status(device), int(code), int(limit), _stream())
 
 
 TC_MAX_CLUSTER = 8          # blocks of a thread-block cluster (the portable limit)
@@ -1229,10 +1229,10 @@ def gemm_tc_bf16(out, x, w, epilogue=EPI_BF16, n_rows=None, swap=None, k_split=N
     if lib.recording():
         moved = 2 * (n * k + m * k) + m * n_out * out.element_size() + (8 * m * n if residual is not None else 0)
         lib.annotate(bytes=moved, flops=2 * m * n * k, label=f"{n}x{k}")
-    _gemm_tc(_ptr(out), _ptr(x), _ptr(w), m, n, k, x.stride(0), w.stride(0), out.stride(0),
-             epilogue, 1 if swap else 0, k_split, 1 if cluster else 0, _ptr(partials), _ptr(tickets),
-             _SPLIT_PARTIAL_FLOATS, _SPLIT_TICKETS, _ptr(ss_in), ss_tiles, int(size), float(eps),
-             _ptr(stream), ld_stream, _ptr(gain), _ptr(ss_out), float(gate_limit), _ptr(tc_status(x.device)),
+    _gemm_tc(out, x, w, m, n, k, x.stride(0), w.stride(0), out.stride(0),
+             epilogue, 1 if swap else 0, k_split, 1 if cluster else 0, partials, tickets,
+             _SPLIT_PARTIAL_FLOATS, _SPLIT_TICKETS, ss_in, ss_tiles, int(size), float(eps),
+             stream, ld_stream, gain, ss_out, float(gate_limit), tc_status(x.device),
              _stream())
 
 
@@ -1271,8 +1271,8 @@ def gemm_pair_bf16(out, x, w, epilogue=PAIR_EPI_BF16, n_rows=None, gate_limit=0.
     if lib.recording():
         moved = 2 * (n * k + m * k) + m * n_out * (8 if epilogue == PAIR_EPI_ADD_F32 else 2)
         lib.annotate(bytes=moved, flops=2 * m * n * k, label=f"{n}x{k}")
-    _gemm_pair(_ptr(out), _ptr(x), _ptr(w), m, n, k, x.stride(0), w.stride(0), out.stride(0), epilogue,
-               float(gate_limit), _ptr(tc_status(x.device)), _stream())
+    _gemm_pair(out, x, w, m, n, k, x.stride(0), w.stride(0), out.stride(0), epilogue,
+               float(gate_limit), tc_status(x.device), _stream())
 
 
 _gemm_tc_qkv = Function("gemm_tc_bf16", "ek_gemm_tc_qkv_rope",
@@ -1319,11 +1319,11 @@ def gemm_tc_qkv_rope(qkv, x, w, n_rows, q_gain, k_gain, qk_eps, cos, sin, positi
         k_split = swap_k_split(n, k, EPI_BF16)
     if lib.recording():
         lib.annotate(bytes=2 * (n * k + m * k + m * n), flops=2 * m * n * k)
-    _gemm_tc_qkv(_ptr(qkv), _ptr(x), _ptr(w), m, k, x.stride(0), w.stride(0), qkv.stride(0), k_split,
-                 _ptr(ss_in), ss_tiles, int(size), float(eps), _ptr(q_gain), _ptr(k_gain), float(qk_eps),
-                 _ptr(cos), _ptr(sin), _ptr(positions), _ptr(token_slot), _ptr(k_pages), _ptr(v_pages),
-                 _ptr(block_table), block_table.stride(0), n_q_heads, n_kv_heads, 1 if write_kv else 0,
-                 _ptr(tc_status(x.device)), _stream())
+    _gemm_tc_qkv(qkv, x, w, m, k, x.stride(0), w.stride(0), qkv.stride(0), k_split,
+                 ss_in, ss_tiles, int(size), float(eps), q_gain, k_gain, float(qk_eps),
+                 cos, sin, positions, token_slot, k_pages, v_pages,
+                 block_table, block_table.stride(0), n_q_heads, n_kv_heads, 1 if write_kv else 0,
+                 tc_status(x.device), _stream())
 
 
 _gemm_tc_qkv_prepare = Function("gemm_tc_bf16", "ek_gemm_tc_qkv_prepare",
@@ -1379,12 +1379,12 @@ def gemm_tc_qkv_prepare(qkv, x, w, n_rows, q_gain, k_gain, qk_eps, cos, sin, pos
         k_split = swap_k_split(n, k, EPI_BF16)
     if lib.recording():
         lib.annotate(bytes=2 * (n * k + m * k + m * n), flops=2 * m * n * k)
-    _gemm_tc_qkv_prepare(_ptr(qkv), _ptr(x), _ptr(w), m, k, x.stride(0), w.stride(0), qkv.stride(0), k_split,
-                         _ptr(ss_in), ss_tiles, int(size), float(eps), _ptr(q_gain), _ptr(k_gain), float(qk_eps),
-                         _ptr(cos), _ptr(sin), _ptr(positions), _ptr(token_slot), _ptr(k_pages), _ptr(v_pages),
-                         _ptr(block_table), block_table.stride(0), n_q_heads, n_kv_heads, 1 if write_kv else 0,
-                         _ptr(q_bias), _ptr(k_bias), _ptr(v_bias), coef, every, 1 if values_from_keys else 0,
-                         _ptr(tc_status(x.device)), _stream())
+    _gemm_tc_qkv_prepare(qkv, x, w, m, k, x.stride(0), w.stride(0), qkv.stride(0), k_split,
+                         ss_in, ss_tiles, int(size), float(eps), q_gain, k_gain, float(qk_eps),
+                         cos, sin, positions, token_slot, k_pages, v_pages,
+                         block_table, block_table.stride(0), n_q_heads, n_kv_heads, 1 if write_kv else 0,
+                         q_bias, k_bias, v_bias, coef, every, 1 if values_from_keys else 0,
+                         tc_status(x.device), _stream())
 
 
 _gemm_pair_qkv = Function("gemm_pair_bf16", "ek_gemm_pair_qkv_rope",
@@ -1418,10 +1418,10 @@ def gemm_pair_qkv_rope(qkv, x, w, n_rows, q_gain, k_gain, qk_eps, cos, sin, posi
           "gemm_pair_qkv_rope: int32 indices, one per row")
     if lib.recording():
         lib.annotate(bytes=2 * (n * k + m * k + m * n), flops=2 * m * n * k, label=f"{n}x{k}")
-    _gemm_pair_qkv(_ptr(qkv), _ptr(x), _ptr(w), m, k, x.stride(0), w.stride(0), qkv.stride(0),
-                   _ptr(q_gain), _ptr(k_gain), float(qk_eps), _ptr(cos), _ptr(sin), _ptr(positions),
-                   _ptr(token_slot), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.stride(0),
-                   n_q_heads, n_kv_heads, 1 if write_kv else 0, _ptr(tc_status(x.device)), _stream())
+    _gemm_pair_qkv(qkv, x, w, m, k, x.stride(0), w.stride(0), qkv.stride(0),
+                   q_gain, k_gain, float(qk_eps), cos, sin, positions,
+                   token_slot, k_pages, v_pages, block_table, block_table.stride(0),
+                   n_q_heads, n_kv_heads, 1 if write_kv else 0, tc_status(x.device), _stream())
 
 
 # ------------------------------------------------------------------ sampling and decode state
@@ -1455,9 +1455,9 @@ def sample(out_token, logits, temperature, top_k, seed, streams=None, draws=None
     rows = n_rows if n_rows is not None else logits.shape[0]
     if lib.recording():
         lib.annotate(bytes=4 * rows * logits.shape[-1])
-    _sample(_ptr(out_token), _ptr(logits), logits.stride(0), rows, logits.shape[-1],
-            float(temperature), int(top_k), int(seed) & 0xFFFFFFFFFFFFFFFF, _ptr(streams),
-            _ptr(draws), _ptr(active), _ptr(dyn), _stream())
+    _sample(out_token, logits, logits.stride(0), rows, logits.shape[-1],
+            float(temperature), int(top_k), int(seed) & 0xFFFFFFFFFFFFFFFF, streams,
+            draws, active, dyn, _stream())
 
 
 SAMPLE_SEGMENTS = 32
@@ -1478,9 +1478,9 @@ def sample_cluster(out_token, logits, temperature, top_k, seed, streams=None, dr
     rows = n_rows if n_rows is not None else logits.shape[0]
     if lib.recording():
         lib.annotate(bytes=4 * rows * logits.shape[-1])
-    _sample_cluster(_ptr(out_token), _ptr(logits), logits.stride(0), rows, logits.shape[-1],
-                    float(temperature), int(top_k), int(seed) & 0xFFFFFFFFFFFFFFFF, _ptr(streams),
-                    _ptr(draws), _ptr(active), _ptr(dyn), _stream())
+    _sample_cluster(out_token, logits, logits.stride(0), rows, logits.shape[-1],
+                    float(temperature), int(top_k), int(seed) & 0xFFFFFFFFFFFFFFFF, streams,
+                    draws, active, dyn, _stream())
 
 
 def sample_wide(out_token, logits, temperature, seed, part_score, part_index, streams=None,
@@ -1495,9 +1495,9 @@ def sample_wide(out_token, logits, temperature, seed, part_score, part_index, st
           and part_index.numel() >= rows * SAMPLE_SEGMENTS, "sample_wide: partial buffers")
     if lib.recording():
         lib.annotate(bytes=4 * rows * logits.shape[-1])
-    _sample_wide(_ptr(out_token), _ptr(logits), logits.stride(0), rows, logits.shape[-1],
-                 float(temperature), int(seed) & 0xFFFFFFFFFFFFFFFF, _ptr(streams), _ptr(draws),
-                 _ptr(active), _ptr(dyn), _ptr(part_score), _ptr(part_index), SAMPLE_SEGMENTS,
+    _sample_wide(out_token, logits, logits.stride(0), rows, logits.shape[-1],
+                 float(temperature), int(seed) & 0xFFFFFFFFFFFFFFFF, streams, draws,
+                 active, dyn, part_score, part_index, SAMPLE_SEGMENTS,
                  _stream())
     count_extra_launches()                   # partial kernel + final kernel
 
@@ -1508,8 +1508,8 @@ def decode_advance(sampled, token_ids, positions, draws, remaining, out_tokens, 
     for t in (sampled, token_ids, positions, draws, remaining, out_tokens, step_index):
         _need(t.dtype == torch.int32, "decode_advance: int32 state")
     _need(out_tokens.shape[-1] == batch, "decode_advance: out_tokens [steps, batch]")
-    _decode_advance(_ptr(sampled), _ptr(token_ids), _ptr(positions), _ptr(draws), _ptr(remaining),
-                    _ptr(out_tokens), _ptr(step_index), _ptr(stop_ids), n_stop, batch,
+    _decode_advance(sampled, token_ids, positions, draws, remaining,
+                    out_tokens, step_index, stop_ids, n_stop, batch,
                     out_tokens.shape[0], _stream())
 
 
@@ -1527,7 +1527,7 @@ def hc_broadcast(streams, x, n_tokens):
     n, width = streams.shape[1], streams.shape[2]
     if lib.recording():
         lib.annotate(bytes=4 * n_tokens * width * (n + 1))
-    _hc_broadcast(_ptr(streams), _ptr(x), n_tokens, n, width, _stream())
+    _hc_broadcast(streams, x, n_tokens, n, width, _stream())
 
 
 def hc_step(streams, n_tokens, y=None, write_mix=None, write_out=None, read_in=None, u=None, norm=None):
@@ -1557,8 +1557,8 @@ def hc_step(streams, n_tokens, y=None, write_mix=None, write_out=None, read_in=N
                                                + (y.element_size() if y is not None else 0)
                                                + (4 if u is not None else 0)
                                                + (normed.element_size() if normed is not None else 0)))
-    _hc_step[dtype](_ptr(streams), _ptr(y), _ptr(write_mix), _ptr(write_out), _ptr(read_in), _ptr(u),
-                    n_tokens, n, width, _ptr(gain), float(eps), _ptr(normed), _stream())
+    _hc_step[dtype](streams, y, write_mix, write_out, read_in, u,
+                    n_tokens, n, width, gain, float(eps), normed, _stream())
 
 
 # ------------------------------------------------------------------ latent attention
@@ -1590,9 +1590,9 @@ def latent_prepare(cq, proj, n_tokens, gain_q, gain_kv, eps, cos, sin, rot_dims,
     d = pages.shape[-1]
     if lib.recording():
         lib.annotate(bytes=n_tokens * (4 * (q_rank + kv_rank + rot_dim) + pages.element_size() * (q_rank + d)))
-    _latent_prepare[pages.dtype](_ptr(cq), _ptr(proj), proj.stride(0), _ptr(gain_q), _ptr(gain_kv), float(eps),
-                                 _ptr(cos), _ptr(sin), rot_dims, _ptr(positions), _ptr(token_slot), _ptr(pages),
-                                 _ptr(block_table), block_table.stride(0), n_tokens, q_rank, kv_rank, rot_dim, d,
+    _latent_prepare[pages.dtype](cq, proj, proj.stride(0), gain_q, gain_kv, float(eps),
+                                 cos, sin, rot_dims, positions, token_slot, pages,
+                                 block_table, block_table.stride(0), n_tokens, q_rank, kv_rank, rot_dim, d,
                                  1 if write_cache else 0, _stream())
 
 
@@ -1631,9 +1631,9 @@ def head_linear(out, x, w, n_tokens, heads, n_in, n_out, rot=None):
         lib.annotate(bytes=x.element_size() * ((0 if by_library else heads * n_in * n_out)
                                                + n_tokens * heads * (n_in + n_out + 2 * r)),
                      flops=0 if by_library else 2 * n_tokens * heads * n_in * n_out)
-    _head_linear[x.dtype](_ptr(out), out.stride(0), out.stride(1), _ptr(x), x.stride(0), x.stride(1),
-                          None if by_library else _ptr(w),
-                          n_tokens, heads, n_in, n_out, r, rot_dims, _ptr(cos), _ptr(sin), _ptr(positions),
+    _head_linear[x.dtype](out, out.stride(0), out.stride(1), x, x.stride(0), x.stride(1),
+                          None if by_library else w,
+                          n_tokens, heads, n_in, n_out, r, rot_dims, cos, sin, positions,
                           _stream())
 
 
@@ -1675,7 +1675,7 @@ def delta_low_rank(out, proj, n_tokens, offset, w2t, bias=None, a_log=None, dim=
     _need(w2t.is_contiguous() and out.is_contiguous() and out.shape[-1] == channels, "delta_low_rank: w2t [rank, channels]")
     if lib.recording():
         lib.annotate(bytes=4 * (n_tokens * (rank + channels) + rank * channels), flops=2 * n_tokens * rank * channels)
-    _delta_low_rank(_ptr(out), _ptr(proj), proj.stride(0), offset, rank, _ptr(w2t), _ptr(bias), _ptr(a_log), dim,
+    _delta_low_rank(out, proj, proj.stride(0), offset, rank, w2t, bias, a_log, dim,
                     channels, n_tokens, 0 if a_log is not None else 1, _stream())
 
 
@@ -1688,16 +1688,16 @@ def delta_prepare(qn, kn, vc, beta, proj, n_tokens, conv_w, state, tail_offset, 
         _need(t.dtype == torch.float32 and t.stride(-1) == 1, "delta_prepare: 32-bit tensors")
     if lib.recording():
         lib.annotate(bytes=4 * n_tokens * (proj.shape[-1] + 2 * qn.shape[-1] + vc.shape[-1]))
-    _delta_prepare(_ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(proj), proj.stride(0),
-                   _ptr(conv_w), _ptr(state), state.stride(0),
-                   tail_offset, _ptr(positions), _ptr(token_slot), n_tokens, *[int(v) for v in shape], _stream())
+    _delta_prepare(qn, kn, vc, beta, proj, proj.stride(0),
+                   conv_w, state, state.stride(0),
+                   tail_offset, positions, token_slot, n_tokens, *[int(v) for v in shape], _stream())
 
 
 def delta_conv_tail(state, tail_offset, proj, cu_seqlens, positions, token_slot, n_seqs, channels, taps):
     """The last ``taps - 1`` convolution inputs of every sequence of the step go to its state."""
     _need_cuda(state, proj, cu_seqlens, positions, token_slot)
-    _delta_conv_tail(_ptr(state), state.stride(0), tail_offset, _ptr(proj), proj.stride(0), _ptr(cu_seqlens),
-                     _ptr(positions), _ptr(token_slot), n_seqs, channels, taps, _stream())
+    _delta_conv_tail(state, state.stride(0), tail_offset, proj, proj.stride(0), cu_seqlens,
+                     positions, token_slot, n_seqs, channels, taps, _stream())
 
 
 _delta_chunks = Function("delta_chunk", "ek_delta_chunks",
@@ -1735,13 +1735,13 @@ def delta_scan(out, qn, kn, vc, beta, decay, state, cu_seqlens, positions, token
         qp = workspace.get("delta_chunk_q", (n_tokens, heads * dim), torch.float32)
         kh = workspace.get("delta_chunk_k", (n_tokens, heads * dim), torch.float32) if decay_per_head else decay
         gam = workspace.get("delta_chunk_decay", (chunks, heads, dim), torch.float32)
-        _delta_chunks(_ptr(out), _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(decay), _ptr(w), _ptr(qp), _ptr(kh), _ptr(gam),
-                      _ptr(state), state.stride(0), _ptr(cu_seqlens), _ptr(positions), _ptr(token_slot), n_seqs, chunks,
+        _delta_chunks(out, qn, kn, vc, beta, decay, w, qp, kh, gam,
+                      state, state.stride(0), cu_seqlens, positions, token_slot, n_seqs, chunks,
                       heads, kv_heads, dim, vdim, 1 if decay_per_head else 0, _stream())
         count_extra_launches()
         return
-    _delta_scan(_ptr(out), _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(decay), _ptr(state), state.stride(0),
-                _ptr(cu_seqlens), _ptr(positions), _ptr(token_slot), n_seqs, heads, kv_heads, dim, vdim,
+    _delta_scan(out, qn, kn, vc, beta, decay, state, state.stride(0),
+                cu_seqlens, positions, token_slot, n_seqs, heads, kv_heads, dim, vdim,
                 1 if decay_per_head else 0, _stream())
 
 
@@ -1754,8 +1754,8 @@ def delta_out_norm(y, o, gate, w, eps, positions, n_tokens, shape, gate_activati
           and gate.stride(-1) == 1, "delta_out_norm: 32-bit inputs")
     if lib.recording():
         lib.annotate(bytes=n_tokens * o.shape[-1] * (8 + y.element_size()))
-    _delta_out_norm[y.dtype](_ptr(y), _ptr(o), _ptr(gate), _ptr(w), float(eps),
-                             _ptr(positions), n_tokens, *[int(v) for v in shape], gate.stride(0),
+    _delta_out_norm[y.dtype](y, o, gate, w, float(eps),
+                             positions, n_tokens, *[int(v) for v in shape], gate.stride(0),
                              1 if gate_activation == "silu" else 0, _stream())
 
 
@@ -1808,8 +1808,8 @@ def conv_silu(out, proj, col0, conv_w, conv_b, state, tail_offset, positions, to
           and col0 + channels <= proj.shape[-1], "conv_silu: weights [channels, taps], columns within the rows")
     if lib.recording():
         lib.annotate(bytes=8 * n_tokens * channels)
-    _conv_silu(_ptr(out), out.stride(0), _ptr(proj), proj.stride(0), col0, _ptr(conv_w), _ptr(conv_b), _ptr(state),
-               state.stride(0), tail_offset, _ptr(positions), _ptr(token_slot), n_tokens, channels, taps, _stream())
+    _conv_silu(out, out.stride(0), proj, proj.stride(0), col0, conv_w, conv_b, state,
+               state.stride(0), tail_offset, positions, token_slot, n_tokens, channels, taps, _stream())
 
 
 _conv_act = Function("recurrent", "ek_conv_act",
@@ -1833,9 +1833,9 @@ def conv_act(out, proj, col0, conv_w, conv_b, state, tail_offset, positions, tok
           and col0 + channels <= proj.shape[-1], "conv_act: weights [channels, taps], columns within the rows")
     if lib.recording():
         lib.annotate(bytes=8 * n_tokens * channels)
-    _conv_act(_ptr(out), out.stride(0), _ptr(proj), proj.stride(0), col0, _ptr(conv_w), _ptr(conv_b), _ptr(in_bias),
-              1 if activation == "silu" else 0, _ptr(state), state.stride(0), tail_offset, _ptr(positions),
-              _ptr(token_slot), n_tokens, channels, taps, _stream())
+    _conv_act(out, out.stride(0), proj, proj.stride(0), col0, conv_w, conv_b, in_bias,
+              1 if activation == "silu" else 0, state, state.stride(0), tail_offset, positions,
+              token_slot, n_tokens, channels, taps, _stream())
 
 
 def lru_gates(a, x, u, w_a, b_a, w_i, b_i, lam, rate, n_tokens, parts, size, w_a_rows=None, w_i_rows=None):
@@ -1853,8 +1853,8 @@ def lru_gates(a, x, u, w_a, b_a, w_i, b_i, lam, rate, n_tokens, parts, size, w_a
           and lam.numel() == width, "lru_gates: a, x [T, parts * size]; weights [parts, size, size]")
     if lib.recording():
         lib.annotate(bytes=4 * (3 * n_tokens * width + 2 * parts * size * size), flops=4 * n_tokens * width * size)
-    _lru_gates(_ptr(a), _ptr(x), _ptr(u), u.stride(0), _ptr(w_a), _ptr(b_a), _ptr(w_i), _ptr(b_i), _ptr(w_a_rows),
-               _ptr(w_i_rows), _ptr(lam), float(rate), n_tokens, parts, size, _stream())
+    _lru_gates(a, x, u, u.stride(0), w_a, b_a, w_i, b_i, w_a_rows,
+               w_i_rows, lam, float(rate), n_tokens, parts, size, _stream())
 
 
 def lru_scan(out, a, x, side, side_col, side_bias, state, cu_seqlens, positions, token_slot, n_seqs, channels,
@@ -1870,8 +1870,8 @@ def lru_scan(out, a, x, side, side_col, side_bias, state, cu_seqlens, positions,
           "lru_scan: out, a, x [T, channels]")
     if lib.recording():
         lib.annotate(bytes=n_tokens * channels * (12 + out.element_size()) + 8 * n_seqs * channels)
-    _lru_scan[out.dtype](_ptr(out), _ptr(a), _ptr(x), _ptr(side), side.stride(0), side_col, _ptr(side_bias),
-                         _ptr(state), state.stride(0), _ptr(cu_seqlens), _ptr(positions), _ptr(token_slot), n_seqs,
+    _lru_scan[out.dtype](out, a, x, side, side.stride(0), side_col, side_bias,
+                         state, state.stride(0), cu_seqlens, positions, token_slot, n_seqs,
                          channels, 1 if write_state else 0, int(max_new), _stream())
 
 
@@ -1879,8 +1879,8 @@ def conv_tail(state, tail_offset, proj, col0, cu_seqlens, positions, token_slot,
     """The last ``taps - 1`` convolution inputs of every sequence of the step go to its state."""
     _need_cuda(state, proj, cu_seqlens, positions, token_slot)
     _need_f32("conv_tail", state, proj)
-    _conv_tail(_ptr(state), state.stride(0), tail_offset, _ptr(proj), proj.stride(0), col0, _ptr(cu_seqlens),
-               _ptr(positions), _ptr(token_slot), n_seqs, channels, taps, _stream())
+    _conv_tail(state, state.stride(0), tail_offset, proj, proj.stride(0), col0, cu_seqlens,
+               positions, token_slot, n_seqs, channels, taps, _stream())
 
 
 def ssm_gates(a, b, proj, col0, dt_bias, a_log, n_tokens, heads):
@@ -1889,7 +1889,7 @@ def ssm_gates(a, b, proj, col0, dt_bias, a_log, n_tokens, heads):
     _need_f32("ssm_gates", a, b, proj, dt_bias, a_log)
     _need(a.is_contiguous() and b.is_contiguous() and a.shape[-1] == heads == b.shape[-1]
           and dt_bias.numel() == heads == a_log.numel(), "ssm_gates: one value per head")
-    _ssm_gates(_ptr(a), _ptr(b), _ptr(proj), proj.stride(0), col0, _ptr(dt_bias), _ptr(a_log), n_tokens, heads,
+    _ssm_gates(a, b, proj, proj.stride(0), col0, dt_bias, a_log, n_tokens, heads,
                _stream())
 
 
@@ -1902,9 +1902,9 @@ def xgate_scan(a, b, m_run, proj, col_i, col_f, bias_i, bias_f, cap, state, m_of
     _need_f32("xgate_scan", a, b, m_run, proj, bias_i, bias_f, state)
     _need(a.is_contiguous() and b.is_contiguous() and m_run.is_contiguous() and a.shape[-1] == heads,
           "xgate_scan: a, b, m [T, heads]")
-    _xgate_scan(_ptr(a), _ptr(b), _ptr(m_run), _ptr(proj), proj.stride(0), col_i, col_f, _ptr(bias_i), _ptr(bias_f),
-                float(cap), _ptr(state), state.stride(0), m_offset, _ptr(cu_seqlens), _ptr(positions),
-                _ptr(token_slot), n_seqs, heads, 1 if write_state else 0, _stream())
+    _xgate_scan(a, b, m_run, proj, proj.stride(0), col_i, col_f, bias_i, bias_f,
+                float(cap), state, state.stride(0), m_offset, cu_seqlens, positions,
+                token_slot, n_seqs, heads, 1 if write_state else 0, _stream())
 
 
 SCAN_COLUMNS = 16           # columns of S a block of the decay scan takes, one a lane; two or four times as many with more;
@@ -1979,10 +1979,10 @@ def decay_scan(out, q, k, v, a, b, state, cu_seqlens, positions, token_slot, n_s
         if parts > 1:
             carry = workspace.get("scan_carry", (n_seqs, parts, heads * cols * decay_scan_rows(dim)), torch.float32)
             prods = workspace.get("scan_prods", (n_seqs, parts, heads), torch.float32)
-    _decay_scan(_ptr(out), out.stride(0), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0),
-                _ptr(a), _ptr(b), _ptr(state), state.stride(0), _ptr(cu_seqlens), _ptr(positions), _ptr(token_slot),
+    _decay_scan(out, out.stride(0), q, q.stride(0), k, k.stride(0), v, v.stride(0),
+                a, b, state, state.stride(0), cu_seqlens, positions, token_slot,
                 n_seqs, heads, kv_heads, dim, vdim, 1 if ones_column else 0, 1 if write_state else 0,
-                heads if a.dim() > 1 else 0, _ptr(carry), _ptr(prods), parts, length,
+                heads if a.dim() > 1 else 0, carry, prods, parts, length,
                 lane_columns, _stream())
     if parts > 1:
         count_extra_launches()
@@ -1997,8 +1997,8 @@ def ssm_out(y, o, x, proj, col_z, d_skip, w, eps, positions, n_tokens, inner, vd
           "ssm_out: y, o [T, inner]")
     if lib.recording():
         lib.annotate(bytes=n_tokens * inner * (12 + y.element_size()))
-    _ssm_out[y.dtype](_ptr(y), _ptr(o), _ptr(x), x.stride(0), _ptr(proj), proj.stride(0), col_z, _ptr(d_skip),
-                      _ptr(w), float(eps), _ptr(positions), n_tokens, inner, vdim, parts, _stream())
+    _ssm_out[y.dtype](y, o, x, x.stride(0), proj, proj.stride(0), col_z, d_skip,
+                      w, float(eps), positions, n_tokens, inner, vdim, parts, _stream())
 
 
 _norm_gate_out = _per_dtype("recurrent", "ek_norm_gate_out",
@@ -2015,7 +2015,7 @@ def norm_gate_out(y, o, proj, col_g, w, eps, positions, n_tokens):
           and col_g + inner <= proj.shape[-1], "norm_gate_out: y, o, w of one width, the gate within the rows")
     if lib.recording():
         lib.annotate(bytes=n_tokens * inner * (8 + y.element_size()))
-    _norm_gate_out[y.dtype](_ptr(y), _ptr(o), _ptr(proj), proj.stride(0), col_g, _ptr(w), float(eps), _ptr(positions),
+    _norm_gate_out[y.dtype](y, o, proj, proj.stride(0), col_g, w, float(eps), positions,
                             n_tokens, inner, _stream())
 
 
@@ -2031,7 +2031,7 @@ def rotate_heads(x, col0, heads, dim, rot_dims, cos, sin, positions, n_tokens):
         return
     if lib.recording():
         lib.annotate(bytes=8 * n_tokens * heads * rot_dims)
-    _rotate_heads(_ptr(x), x.stride(0), col0, heads, dim, rot_dims, _ptr(cos), _ptr(sin), _ptr(positions), n_tokens,
+    _rotate_heads(x, x.stride(0), col0, heads, dim, rot_dims, cos, sin, positions, n_tokens,
                   _stream())
 
 
@@ -2046,8 +2046,8 @@ def head_norm_gate_out(y, o, proj, col_g, w, eps, positions, n_tokens, heads, vd
           "head_norm_gate_out: y, o, w of one width, the gate within the rows")
     if lib.recording():
         lib.annotate(bytes=n_tokens * heads * vdim * (8 + y.element_size()))
-    _head_norm_gate_out[y.dtype](_ptr(y), _ptr(o), _ptr(proj), proj.stride(0), col_g, _ptr(w), float(eps),
-                                 1 if gate_activation == "silu" else 0, _ptr(positions), n_tokens, heads, vdim,
+    _head_norm_gate_out[y.dtype](y, o, proj, proj.stride(0), col_g, w, float(eps),
+                                 1 if gate_activation == "silu" else 0, positions, n_tokens, heads, vdim,
                                  _stream())
 
 
@@ -2061,8 +2061,8 @@ def xlstm_out(y, o, m_run, proj, col_g, w, eps, q_scale, positions, n_tokens, he
           and o.shape[-1] == heads * (vdim + 1) and w.numel() == heads * vdim, "xlstm_out: shapes")
     if lib.recording():
         lib.annotate(bytes=n_tokens * heads * vdim * (8 + y.element_size()))
-    _xlstm_out[y.dtype](_ptr(y), _ptr(o), _ptr(m_run), _ptr(proj), proj.stride(0), col_g, _ptr(w), float(eps),
-                        float(q_scale), _ptr(positions), n_tokens, heads, vdim, _stream())
+    _xlstm_out[y.dtype](y, o, m_run, proj, proj.stride(0), col_g, w, float(eps),
+                        float(q_scale), positions, n_tokens, heads, vdim, _stream())
 
 
 # ------------------------------------------------------------------ routed experts
@@ -2123,15 +2123,15 @@ def moe_route(sel_expert, sel_weight, logits, n_tokens, n_groups, keep, top, sca
     _need(weights in ROUTE_WEIGHTS, f"moe_route: no weights {weights!r}")
     _need(logits.dtype == torch.float32 and logits.stride(-1) == 1 and sel_expert.dtype == torch.int32
           and sel_weight.dtype == torch.float32, "moe_route: 32-bit logits and weights, int32 choices")
-    _moe_route(_ptr(sel_expert), _ptr(sel_weight), _ptr(logits), logits.stride(0), n_tokens, logits.shape[-1], n_groups, keep,
-               top, float(scale), ROUTE_WEIGHTS[weights], _ptr(correction), _stream())
+    _moe_route(sel_expert, sel_weight, logits, logits.stride(0), n_tokens, logits.shape[-1], n_groups, keep,
+               top, float(scale), ROUTE_WEIGHTS[weights], correction, _stream())
 
 
 def moe_plan(sorted_pair, tiles, n_tiles, sel_expert, n_pairs, n_experts, wide=False):
     """Sort the pairs by expert and cut every expert's stretch into row tiles: of 64, or (``wide``) into equal
     ones of up to 256."""
     _need_cuda(sorted_pair, tiles, n_tiles, sel_expert)
-    _moe_plan(_ptr(sorted_pair), _ptr(tiles), _ptr(n_tiles), _ptr(sel_expert), n_pairs, n_experts,
+    _moe_plan(sorted_pair, tiles, n_tiles, sel_expert, n_pairs, n_experts,
               *((MOE_PAIR_TILE_ROWS, MOE_PAIR_EVEN) if wide else (MOE_TILE_ROWS, 0)), _stream())
 
 
@@ -2160,15 +2160,15 @@ def moe_expert_up(out, x, w, tiles, n_tiles, sorted_pair, n_pairs, top, activati
             _need_cuda(scratch)
             _need(scratch.is_contiguous() and scratch.data_ptr() % 16 == 0
                   and scratch.numel() * scratch.element_size() >= n_pairs * k * x.element_size(), "moe_expert_up: scratch")
-            _moe_gather(_ptr(scratch), _ptr(x), _ptr(sorted_pair), _ptr(tiles), _ptr(n_tiles), n_pairs, top, k, _stream())
+            _moe_gather(scratch, x, sorted_pair, tiles, n_tiles, n_pairs, top, k, _stream())
             x, rows, gathered = scratch, n_pairs, 1
-        _moe_up_pair(_ptr(out), _ptr(x), _ptr(w), _ptr(tiles), _ptr(n_tiles), _ptr(sorted_pair), rows, gathered, e,
+        _moe_up_pair(out, x, w, tiles, n_tiles, sorted_pair, rows, gathered, e,
                      moe_max_tiles(n_pairs, e, True), top, n, k, EXPERT_ACTIVATIONS[activation], 1 if gated else 0,
-                     float(limit), _ptr(input_weight), _ptr(tc_status(w.device)), _stream())
+                     float(limit), input_weight, tc_status(w.device), _stream())
         return
-    _moe_up[x.dtype](_ptr(out), _ptr(x), _ptr(w), _ptr(tiles), _ptr(n_tiles), _ptr(sorted_pair),
+    _moe_up[x.dtype](out, x, w, tiles, n_tiles, sorted_pair,
                      moe_max_tiles(n_pairs, e), top, n, k, EXPERT_ACTIVATIONS[activation], 1 if gated else 0,
-                     float(limit), _ptr(input_weight), _stream())
+                     float(limit), input_weight, _stream())
 
 
 def moe_expert_down(pair_out, a, w, tiles, n_tiles, sorted_pair, pair_weight, n_pairs, wide=False):
@@ -2184,11 +2184,11 @@ def moe_expert_down(pair_out, a, w, tiles, n_tiles, sorted_pair, pair_weight, n_
     if wide:
         _need(_moe_on_pairs(a, w) and a.shape[0] >= n_pairs, "moe_expert_down: a wide plan takes bfloat16 rows "
               "that can be read 16 bytes at a time")
-        _moe_down_pair(_ptr(pair_out), _ptr(a), _ptr(w), _ptr(tiles), _ptr(n_tiles), _ptr(sorted_pair), _ptr(pair_weight),
-                       n_pairs, e, moe_max_tiles(n_pairs, e, True), n, k, _ptr(tc_status(a.device)), _stream())
+        _moe_down_pair(pair_out, a, w, tiles, n_tiles, sorted_pair, pair_weight,
+                       n_pairs, e, moe_max_tiles(n_pairs, e, True), n, k, tc_status(a.device), _stream())
         return
-    _moe_down[a.dtype](_ptr(pair_out), _ptr(a), _ptr(w), _ptr(tiles), _ptr(n_tiles), _ptr(sorted_pair),
-                       _ptr(pair_weight), moe_max_tiles(n_pairs, e), n, k, _stream())
+    _moe_down[a.dtype](pair_out, a, w, tiles, n_tiles, sorted_pair,
+                       pair_weight, moe_max_tiles(n_pairs, e), n, k, _stream())
 
 
 def moe_combine(out, pair_out, n_tokens, top, add=None, identity=None):
@@ -2207,8 +2207,8 @@ def moe_combine(out, pair_out, n_tokens, top, add=None, identity=None):
           "moe_combine: identity experts take the input's rows in out's type, choices and 32-bit weights")
     if lib.recording():
         lib.annotate(bytes=n_tokens * width * (4 * top + out.element_size() * (1 + (add is not None) + (x is not None))))
-    _moe_combine[out.dtype](_ptr(out), _ptr(pair_out), n_tokens, top, width, _ptr(add), _ptr(chosen), _ptr(weight),
-                            _ptr(x), e, _stream())
+    _moe_combine[out.dtype](out, pair_out, n_tokens, top, width, add, chosen, weight,
+                            x, e, _stream())
 
 
 def build_all():

@@ -3,6 +3,8 @@
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import threading
 from typing import Dict
 
@@ -139,8 +141,30 @@ def check(status: int, what: str) -> None:
                       f" ({_cuda_error_names.get(status, 'see cudaError_t')})")
 
 
+_host = None               # the module of csrc/hostcall.cc; False where it cannot be had
+_KINDS = {ctypes.c_void_p: "p", ctypes.c_int: "i", ctypes.c_uint: "i", ctypes.c_longlong: "i", ctypes.c_ulonglong: "i",
+          ctypes.c_float: "f"}
+
+
+def _host_module():
+    global _host
+    if _host is None:
+        try:
+            path = build.host_library()
+            if path is None:
+                raise ImportError
+            loader = importlib.machinery.ExtensionFileLoader("ek_hostcall", path)
+            host = importlib.util.module_from_spec(importlib.util.spec_from_loader("ek_hostcall", loader))
+            loader.exec_module(host)
+            _host = host
+        except (ImportError, OSError, build.BuildError):
+            _host = False
+    return _host
+
+
 class Function:
-    """A C entry point with its argument types bound once."""
+    """A C entry point with its argument types bound once (csrc/hostcall.cc calls it, where that can be built and takes
+    the signature, else ctypes).  An address is an int, None, or a tensor, which stands for its ``data_ptr()``."""
 
     def __init__(self, module: str, name: str, argtypes, check_status: bool = True):
         """``check_status`` False: the entry point launches nothing and returns a value, not a status."""
@@ -156,8 +180,10 @@ class Function:
             raise KernelError(f"{lib._name} has no entry point {self.name}") from None
         fn.argtypes = self.argtypes
         fn.restype = ctypes.c_int
-        self._fn = fn
-        return fn
+        host, kinds = _host_module(), [_KINDS.get(t) for t in self.argtypes]
+        bound = host.bind(ctypes.cast(fn, ctypes.c_void_p).value, "".join(kinds)) if host and None not in kinds else None
+        self._fn = bound or (lambda *args: fn(*[a.data_ptr() if hasattr(a, "data_ptr") else a for a in args]))
+        return self._fn
 
     def __call__(self, *args):
         global _launch_calls
@@ -170,4 +196,6 @@ class Function:
             head, cost, _pending_cost = args[:-1], _pending_cost or {}, None
             name = f"{self.name}[{cost['label']}]" if cost.get("label") else self.name
             _recorder.append((name, lambda stream: check(fn(*head, stream), self.name), cost))
-        check(fn(*args), self.name)
+        status = fn(*args)
+        if status:
+            check(status, self.name)

@@ -113,7 +113,7 @@ def linear(x, w, ctx, name: str, n_rows=None, out_dtype=None, defer=None, image=
             if pair_product_wins(stream, x, w, m, kernels.PAIR_EPI_ADD_F32):
                 kernels.gemm_pair_bf16(stream, x, w, kernels.PAIR_EPI_ADD_F32, n_rows=m)
             else:
-                _library_product_add(stream[:m], x[:m], w)
+                _library_product_add(_first(stream, m), _first(x, m), w)
             return None
     if row_scale is not None and not (w.dtype == torch.bfloat16 and m <= SMALL_ROWS and tc_takes(x, w)):
         raise kernels.KernelError("a deferred norm reached a product that cannot scale its rows")
@@ -130,20 +130,24 @@ def linear(x, w, ctx, name: str, n_rows=None, out_dtype=None, defer=None, image=
         if want_f32:
             _library_product(x[:m].float(), w.float(), out)
         else:
-            _library_product(x[:m], w, out)
+            _library_product(_first(x, m), w, out)
         return out
     if m <= SMALL_ROWS:
         kernels.gemm_tc_bf16(out, x, w, epi if want_f32 else epi_bf16, n_rows=m, swap=True, row_scale=row_scale)
     elif want_f32 and wide_f32 == "library":
-        _library_product_f32(x[:m], w, out)
+        _library_product_f32(_first(x, m), w, out)
     elif want_f32:
         # 32-bit logits for many rows: 128 x 128 tiles with the accumulator stored as it is
         kernels.gemm_tc_bf16(out, x, w, epi, n_rows=m, swap=False)
     elif pair_product_wins(out, x, w, m, kernels.PAIR_EPI_BF16):
         kernels.gemm_pair_bf16(out, x, w, kernels.PAIR_EPI_BF16, n_rows=m)
     else:
-        _library_product(x[:m], w, out)
+        _library_product(_first(x, m), w, out)
     return out
+
+
+def _first(x, m):
+    return x if x.shape[0] == m else x[:m]       # (a slice costs the host 1.2 us)
 
 
 def _library_product_add(stream, x, w):
@@ -160,7 +164,7 @@ def _library_product_add(stream, x, w):
 
 def _library_product_f32(x, w, out):
     """out (32-bit) = x . w^T for bfloat16 operands by the library: 32-bit accumulators, not rounded."""
-    torch.mm(x, w.t(), out_dtype=torch.float32, out=out[:x.shape[0]])
+    torch.mm(x, w.t(), out_dtype=torch.float32, out=_first(out, x.shape[0]))
     if lib.recording():
         m, k = x.shape
         n = w.shape[0]
@@ -172,10 +176,10 @@ def _library_product_f32(x, w, out):
 def _library_product(x, w, out):
     """out = x . w^T by the library (cuBLAS through torch), as the reference does for prompts
     (engine/ek_model.py:298, 311, 203-209)."""
-    torch.matmul(x, w.t(), out=out)
+    torch.mm(x, w.t(), out=out)
     if lib.recording():
         m, k = x.shape
         n = w.shape[0]
-        lib.record_library_call(f"library_matmul[{n}x{k}]", lambda: torch.matmul(x, w.t(), out=out),
+        lib.record_library_call(f"library_matmul[{n}x{k}]", lambda: torch.mm(x, w.t(), out=out),
                                 bytes=x.element_size() * (m * k + n * k) + out.element_size() * m * n,
                                 flops=2 * m * n * k)
