@@ -1168,6 +1168,17 @@ def swap_k_split(n_out, k, epilogue):
     return 1 << (split.bit_length() - 1)
 
 
+def narrow_k_split(n_out, k, epilogue):
+    """:func:`swap_k_split`, or more where that leaves SMs without a block: a block takes its K blocks one after the other,
+    0.16 us each, so products whose blocks have an SM each (or up to a tenth more than there are) go down to 4 K blocks a
+    block.  Decoding, us a layer with at least 8 and by this rule: attention of width 1,024 at 1 and 40 tokens 18.7 / 17.5 and
+    31.3 / 27.0, latents at 8 tokens 43.8 / 40.4, a window over 20 heads at 20 tokens 35.8 / 34.1.  (4 blocks in all 296
+    places: one token through 33 tiles of 32 K blocks 27.5, so 26.7.)"""
+    tiles = -(-n_out // (64 if epilogue in (EPI_SWIGLU, EPI_GEGLU) else 128))
+    split = max(1, min(sm_count() * 11 // 10 // tiles, -(-k // 64) // 4, TC_MAX_CLUSTER))
+    return max(swap_k_split(n_out, k, epilogue), 1 << (split.bit_length() - 1))
+
+
 def gemm_tc_bf16(out, x, w, epilogue=EPI_BF16, n_rows=None, swap=None, k_split=None, cluster=True,
                  row_scale=None, residual=None, gate_limit=0.0):
     """out = x . w^T (or the SwiGLU of it) on tcgen05 tensor cores with TMA-staged operands.
@@ -1203,7 +1214,7 @@ def gemm_tc_bf16(out, x, w, epilogue=EPI_BF16, n_rows=None, swap=None, k_split=N
     _need(not swap or m <= TC_SWAP_MAX_ROWS, "gemm_tc_bf16: the swapped form takes at most 64 rows")
     partials, tickets = split_scratch(x.device)
     if k_split is None:
-        k_split = swap_k_split(n_out, k, epilogue) if swap else 1
+        k_split = narrow_k_split(n_out, k, epilogue) if swap else 1
     if row_scale is not None or residual is not None:
         cluster, k_split = True, min(k_split, TC_MAX_CLUSTER)     # these forms have no scratch path
     ss_in, ss_tiles, size, eps = None, 0, 0, 0.0
@@ -1316,7 +1327,7 @@ def gemm_tc_qkv_rope(qkv, x, w, n_rows, q_gain, k_gain, qk_eps, cos, sin, positi
               and ss_in.shape[0] >= m, "gemm_tc_qkv_rope: row_scale needs 32-bit sums [rows, tiles]")
         ss_tiles = ss_in.shape[1]
     if k_split is None:
-        k_split = swap_k_split(n, k, EPI_BF16)
+        k_split = narrow_k_split(n, k, EPI_BF16)
     if lib.recording():
         lib.annotate(bytes=2 * (n * k + m * k + m * n), flops=2 * m * n * k)
     _gemm_tc_qkv(qkv, x, w, m, k, x.stride(0), w.stride(0), qkv.stride(0), k_split,
@@ -1376,7 +1387,7 @@ def gemm_tc_qkv_prepare(qkv, x, w, n_rows, q_gain, k_gain, qk_eps, cos, sin, pos
               and ss_in.shape[0] >= m, "gemm_tc_qkv_prepare: row_scale needs 32-bit sums [rows, tiles]")
         ss_tiles = ss_in.shape[1]
     if k_split is None:
-        k_split = swap_k_split(n, k, EPI_BF16)
+        k_split = narrow_k_split(n, k, EPI_BF16)
     if lib.recording():
         lib.annotate(bytes=2 * (n * k + m * k + m * n), flops=2 * m * n * k)
     _gemm_tc_qkv_prepare(qkv, x, w, m, k, x.stride(0), w.stride(0), qkv.stride(0), k_split,

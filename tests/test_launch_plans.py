@@ -25,6 +25,14 @@ def test_k_split_of_the_swapped_form(n_out, k, epi):
     assert split == 1 or k_blocks // split >= 8            # a block keeps a ring's worth of K
 
 
+@pytest.mark.parametrize("n_out,k,split", [(4096, 1024, 4), (1024, 2048, 8), (2560, 4096, 8), (6144, 2560, 4), (4160, 2048, 4),
+                                           (3072, 768, 2), (128, 64, 1), (151936, 2560, 1)])
+def test_k_split_of_narrow_products(n_out, k, split):
+    assert kernels.narrow_k_split(n_out, k, kernels.EPI_BF16) == split
+    tiles, most = -(-n_out // 128), kernels.swap_k_split(n_out, k, kernels.EPI_BF16)
+    assert split == most or (tiles * split <= 1.1 * kernels.sm_count() and -(-k // 64) // split >= 4)
+
+
 def test_the_benchmark_shape_gets_the_splits_the_profiles_name():
     assert kernels.swap_k_split(6144, 2560, kernels.EPI_BF16) == 4      # q/k/v
     assert kernels.swap_k_split(2560, 4096, kernels.EPI_BF16) == 8      # attention output
