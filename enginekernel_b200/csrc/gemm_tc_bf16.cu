@@ -18,8 +18,12 @@
 //     a thread-block cluster: each leaves its partial tile in its own shared memory and sums
 //     its share of the tile's columns over all of them, in split order, through distributed
 //     shared memory (with at most 8 sequences each block sends its partial sums to the
-//     owning block instead, by stores that count their bytes on a barrier of the owner, and
-//     only the owner waits - for those bytes, not for the cluster).  More splits than that go through scratch in global memory, and
+//     owning block instead, from the registers they are in, by stores that count their bytes on a
+//     barrier of the owner, and only the owner waits - for those bytes, not for the cluster).
+//     What counts here is the chain, not the bytes: weights are asked for before the block is set
+//     up (0.3 us after its start instead of 1.1), and sums that pass through no staging and no
+//     block barrier on either side took the rest - one token's layer of width 1,024 17.5 -> 16.4
+//     us, 4 tokens at 4,096 32.0 -> 28.5.  More splits than that go through scratch in global memory, and
 //     the block that delivers the last partial of a tile adds them in split order.
 //   * direct (prompts): P = activations, Q = weights, 128 x 256 tiles.
 // Epilogues: bfloat16, 32-bit, or SwiGLU (the tile holds gate rows/columns in its first
@@ -152,6 +156,41 @@ gemm_tc_bf16_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
   constexpr bool kCanPush = CL && BN == 16;
   const int push_slots = (prm.rows_q + n_split - 1) / n_split;     // sequences a block owns at most
   const bool push = kCanPush && n_split * push_slots <= kTcPushRows;
+  bool ok = (smem_u32(smem) & 1023u) == 0;       // never seen otherwise; the swizzled tiles would be wrong
+  // The rows that the operands' tiles begin with.
+  int p_row0, p_row1 = 0, q_row0, q_row1 = 0;
+  if (EPI == TC_EPI_SWIGLU && SWAP) {            // weights on the P side: 64 gate rows + 64 up rows
+    p_row0 = tile_p * 64;
+    p_row1 = prm.swiglu_half + tile_p * 64;
+  } else {
+    p_row0 = tile_p * kTcBM;
+  }
+  if (EPI == TC_EPI_SWIGLU && !SWAP) {           // weights on the Q side: BN/2 gate + BN/2 up rows
+    q_row0 = tile_q * (BN / 2);
+    q_row1 = prm.swiglu_half + tile_q * (BN / 2);
+  } else {
+    q_row0 = tile_q * BN;
+  }
+  const uint64_t stream_policy = l2_policy_evict_first();
+  auto load_p = [&](int it) {
+    const int s = it % STAGES;
+    const uint32_t full = full0 + 8 * s, pd = smem_u32(p_tiles + s * kBytesP);
+    const int k0 = (kb_begin + it) * kTcBK;
+    if (SWAP) {                                  // the weights are read once: first out of L2
+      tma_load_2d_hint(pd, &map_p, k0, p_row0, full, stream_policy);
+      if (EPI == TC_EPI_SWIGLU) tma_load_2d_hint(pd + kBytesP / 2, &map_p, k0, p_row1, full, stream_policy);
+    } else {
+      tma_load_2d(pd, &map_p, k0, p_row0, full);
+    }
+  };
+  auto load_q = [&](int it) {
+    const int s = it % STAGES;
+    const uint32_t full = full0 + 8 * s, qd = smem_u32(q_tiles + s * kBytesQ);
+    const int k0 = (kb_begin + it) * kTcBK;
+    tma_load_2d(qd, &map_q, k0, q_row0, full);
+    if (EPI == TC_EPI_SWIGLU && !SWAP) tma_load_2d(qd + kBytesQ / 2, &map_q, k0, q_row1, full);
+  };
+  const int first_loads = ok ? min(n_iter, STAGES) : 0;
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full0 + 8 * s, 1);
@@ -160,6 +199,12 @@ gemm_tc_bf16_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
     mbar_init(accum_bar, TWO ? 2 : 1);
     mbar_init(recv_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    // The weight operand does not depend on the kernel before this one: the first ring of weight tiles is requested
+    // before anything else is set up, the activations after the wait for that kernel.
+    for (int it = 0; it < first_loads; ++it) {
+      mbar_expect_tx(full0 + 8 * (it % STAGES), kBytesP + kBytesQ);
+      if (SWAP) load_p(it); else load_q(it);
+    }
     if (push) {                                  // the sequences split, split + n_split, ...: 512 bytes from every block each
       const int mine = prm.rows_q > split ? (prm.rows_q - split + n_split - 1) / n_split : 0;
       mbar_expect_tx(recv_bar, (uint32_t)(n_split * mine * kTcBM * 4));
@@ -167,64 +212,25 @@ gemm_tc_bf16_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
   }
   // (the barrier exists in every block of the cluster before a store from another block reaches it:
   // arrive here, wait just before the first such store)
-  if (kCanPush) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  // (.relaxed: a releasing arrive waits for the copies asked for above)
+  __syncwarp();
+  if (kCanPush) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   if (warp == 0) tmem_alloc(smem_u32(tmem_slot), kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  bool ok = (smem_u32(smem) & 1023u) == 0;       // never seen otherwise; the swizzled tiles would be wrong
   if (!ok && tid == 0) atomicCAS(prm.status, 0, 9);
   int fillings = 0;                              // stage fillings this thread has asked TMA for
   if (tid == 0) {
     // ---------------------------------------------------------------- TMA producer
-    int p_row0, p_row1 = 0;
-    if (EPI == TC_EPI_SWIGLU && SWAP) {        // weights on the P side: 64 gate rows + 64 up rows
-      p_row0 = tile_p * 64;
-      p_row1 = prm.swiglu_half + tile_p * 64;
-    } else {
-      p_row0 = tile_p * kTcBM;
-    }
-    int q_row0, q_row1 = 0;
-    if (EPI == TC_EPI_SWIGLU && !SWAP) {       // weights on the Q side: BN/2 gate + BN/2 up rows
-      q_row0 = tile_q * (BN / 2);
-      q_row1 = prm.swiglu_half + tile_q * (BN / 2);
-    } else {
-      q_row0 = tile_q * BN;
-    }
-    const uint64_t stream_policy = l2_policy_evict_first();
-    auto load_p = [&](int it) {
-      const int s = it % STAGES;
-      const uint32_t full = full0 + 8 * s, pd = smem_u32(p_tiles + s * kBytesP);
-      const int k0 = (kb_begin + it) * kTcBK;
-      if (SWAP) {                              // the weights are read once: first out of L2
-        tma_load_2d_hint(pd, &map_p, k0, p_row0, full, stream_policy);
-        if (EPI == TC_EPI_SWIGLU) tma_load_2d_hint(pd + kBytesP / 2, &map_p, k0, p_row1, full, stream_policy);
-      } else {
-        tma_load_2d(pd, &map_p, k0, p_row0, full);
-      }
-    };
-    auto load_q = [&](int it) {
-      const int s = it % STAGES;
-      const uint32_t full = full0 + 8 * s, qd = smem_u32(q_tiles + s * kBytesQ);
-      const int k0 = (kb_begin + it) * kTcBK;
-      tma_load_2d(qd, &map_q, k0, q_row0, full);
-      if (EPI == TC_EPI_SWIGLU && !SWAP) tma_load_2d(qd + kBytesQ / 2, &map_q, k0, q_row1, full);
-    };
-    // The weight operand does not depend on the kernel before this one: the first ring of
-    // weight tiles is requested before waiting for that kernel, the activations after.
-    const int first = ok ? min(n_iter, STAGES) : 0;
-    for (int it = 0; it < first; ++it) {
-      mbar_expect_tx(full0 + 8 * (it % STAGES), kBytesP + kBytesQ);
-      if (SWAP) load_p(it); else load_q(it);
-    }
     pdl_wait();
-    for (int it = 0; it < first; ++it) {
+    for (int it = 0; it < first_loads; ++it) {
       if (SWAP) load_q(it); else load_p(it);
     }
-    fillings = first;
-    for (int it = first; it < n_iter && ok; ++it) {
+    fillings = first_loads;
+    for (int it = first_loads; it < n_iter && ok; ++it) {
       const int s = it % STAGES;
       const uint32_t phase = (it / STAGES) & 1;
       ok = mbar_wait(empty0 + 8 * s, phase ^ 1, prm.status, 1);
@@ -360,14 +366,14 @@ gemm_tc_bf16_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
     // block takes the sequences split, split + n_split, ...  Every block of a cluster passes
     // the barriers whatever happened to it, so that none waits for one that gave up.
     // With at most kTcPushRows sequences (narrowest clustered form) a block does not wait to be
-    // read: it sends each sequence's partial sums (16 bytes a store) into the shared memory of the
+    // read: it sends each sequence's partial sums (a thread its row's) into the shared memory of the
     // block that owns the sequence (a buffer beside the ring - the owner may still be
-    // multiplying), and after ONE cluster barrier every block has all it needs at home.
+    // multiplying), which adds them up when its barrier has counted their bytes.
     float* red = (float*)smem;
     constexpr int NS = CL ? kTcMaxCluster : 1;
     const int slots = push_slots;
     if (kCanPush) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (!failed) {
+    if (!failed && !push) {
 #pragma unroll 1
       for (int c0 = 0; c0 < BN && c0 < prm.rows_q; c0 += 16) {
         float v[16];
@@ -382,13 +388,24 @@ gemm_tc_bf16_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
       }
     }
     if (push) {
-      __syncthreads();
-      if (!failed) {
-        for (int f = tid; f < prm.rows_q * (kTcBM / 4); f += 128) {
-          const int m = f / (kTcBM / 4), c = 4 * (f % (kTcBM / 4));
-          st_async_f32x4(&recv[(split * slots + m / n_split) * kTcBM + c], (unsigned)(m % n_split),
-                         *reinterpret_cast<const float4*>(&red[m * kTcBM + c]), recv_bar);
+      if (!failed) {                             // from the registers it is in: a warp's 32 rows of a sequence side by side
+        float v[16];
+        if (n_iter > 0) {
+          acc_ld16(0, v);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = 0.f;
         }
+        int to = 0, slot = 0;
+#pragma unroll
+        for (int m = 0; m < kTcPushRows; ++m)
+          if (m < prm.rows_q) {
+            st_async_f32(&recv[(split * slots + slot) * kTcBM + row], (unsigned)to, v[m], recv_bar);
+            if (++to == n_split) {
+              to = 0;
+              ++slot;
+            }
+          }
       }
       // what this block owns has arrived when its barrier has counted the bytes (a block that gave
       // up sends nothing: the others' waits run out and say so)
@@ -402,44 +419,61 @@ gemm_tc_bf16_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
       // One 16-byte load a block of the cluster and thread; all loads of a batch are issued before
       // the first sum.
       const bool wide_ok = (prm.ldo & 3) == 0 && ((uintptr_t)prm.out & 15) == 0;
-      auto fetch4 = [&](int m, int idx, int col, int sp) {   // 4 weight rows from `col` of split sp's tile
-        if (push) return *reinterpret_cast<const float4*>(&recv[(sp * slots + idx) * kTcBM + col]);
+      auto fetch4 = [&](int m, int col, int sp) {           // 4 weight rows from `col` of split sp's tile
         const float* p = &red[m * kTcBM + col];
         return CL ? ld_cluster_f32x4(p, (unsigned)sp) : *reinterpret_cast<const float4*>(p);
       };
+      auto add4 = [](float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
 #pragma unroll 1
       for (int base = 0; base < owned; base += P * 4 * MPW) {
-        float4 part[P][NS], part_up[P][NS];
+        float4 sum[P], sum_up[P];
         if (base > 0) ask(base);                 // (the first batch was asked for before the barrier)
+        if (kCanPush && push) {                  // (at most four sequences, a warp each: one pass)
+          const int idx = warp * MPW + sub;
+          auto total = [&](int col) {
+            float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (idx < owned) {
+              const float4* p = reinterpret_cast<const float4*>(&recv[idx * kTcBM + col]);
+              t = *p;
+              for (int sp = 1; sp < n_split; ++sp) add4(t, p[sp * slots * (kTcBM / 4)]);
+            }
+            return t;
+          };
+          sum[0] = total(r0);
+          if (EPI == TC_EPI_SWIGLU) sum_up[0] = total(r0 + 64);
+        } else {
+          float4 part[P][NS], part_up[P][NS];
 #pragma unroll
-        for (int ps = 0; ps < P; ++ps) {
-          const int idx = base + (ps * 4 + warp) * MPW + sub;
-          const int m = first + idx * step;
+          for (int ps = 0; ps < P; ++ps) {
+            const int idx = base + (ps * 4 + warp) * MPW + sub;
+            const int m = first + idx * step;
 #pragma unroll
-          for (int sp = 0; sp < NS; ++sp) {
-            const bool live = idx < owned && sp < n_split;
-            part[ps][sp] = live ? fetch4(m, idx, r0, sp) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (EPI == TC_EPI_SWIGLU)
-              part_up[ps][sp] = live ? fetch4(m, idx, r0 + 64, sp) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int sp = 0; sp < NS; ++sp) {
+              const bool live = idx < owned && sp < n_split;
+              part[ps][sp] = live ? fetch4(m, r0, sp) : make_float4(0.f, 0.f, 0.f, 0.f);
+              if (EPI == TC_EPI_SWIGLU)
+                part_up[ps][sp] = live ? fetch4(m, r0 + 64, sp) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+          }
+#pragma unroll
+          for (int ps = 0; ps < P; ++ps) {
+            sum[ps] = part[ps][0];
+            if (EPI == TC_EPI_SWIGLU) sum_up[ps] = part_up[ps][0];
+#pragma unroll
+            for (int sp = 1; sp < NS; ++sp)
+              if (sp < n_split) {
+                add4(sum[ps], part[ps][sp]);
+                if (EPI == TC_EPI_SWIGLU) add4(sum_up[ps], part_up[ps][sp]);
+              }
           }
         }
 #pragma unroll
         for (int ps = 0; ps < P; ++ps) {
           const int idx = base + (ps * 4 + warp) * MPW + sub;
           const int m = first + idx * step;
-          float4 acc = part[ps][0];
-          float4 up = EPI == TC_EPI_SWIGLU ? part_up[ps][0] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-          for (int sp = 1; sp < NS; ++sp) {
-            if (sp < n_split) {
-              acc.x += part[ps][sp].x; acc.y += part[ps][sp].y;
-              acc.z += part[ps][sp].z; acc.w += part[ps][sp].w;
-              if (EPI == TC_EPI_SWIGLU) {
-                up.x += part_up[ps][sp].x; up.y += part_up[ps][sp].y;
-                up.z += part_up[ps][sp].z; up.w += part_up[ps][sp].w;
-              }
-            }
-          }
+          if (kCanPush && push && ps > 0) break;
+          float4 acc = sum[ps];
+          float4 up = EPI == TC_EPI_SWIGLU ? sum_up[ps] : make_float4(0.f, 0.f, 0.f, 0.f);
           if (prm.ss_in != nullptr && idx < owned) {
             const float rs = rstd_s[m];
             acc.x *= rs; acc.y *= rs; acc.z *= rs; acc.w *= rs;
