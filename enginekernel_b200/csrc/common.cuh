@@ -279,6 +279,14 @@ __device__ __forceinline__ void st_async_f32x4(float* own, unsigned rank, float4
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
                ::"r"(r), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(b) : "memory");
 }
+// Two floats (8-byte aligned), in the same way.
+__device__ __forceinline__ void st_async_f32x2(float* own, unsigned rank, float2 v, unsigned own_bar) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(own), r, b;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(own_bar), "r"(rank));
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
+               ::"r"(r), "f"(v.x), "f"(v.y), "r"(b) : "memory");
+}
 // One float, in the same way.
 __device__ __forceinline__ void st_async_f32(float* own, unsigned rank, float v, unsigned own_bar) {
   unsigned a = (unsigned)__cvta_generic_to_shared(own), r, b;

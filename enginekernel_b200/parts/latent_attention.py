@@ -207,9 +207,11 @@ class LatentAttention(Mixer):
             blocks = t * -(-nh // 16)
             pages = -(-visible // kernels.PAGE)
             # One block an SM, and a cluster's blocks within one group of SMs: 8 blocks a token up to 96 in all, 16 up to
-            # 64, 2 or 4 up to the number of SMs.  Us behind 2,048 rows by blocks a token: 8 tokens 4: 12.4, 8: 10.0, 16 (a
-            # second wave): 17.1 (register-streaming kernel 26.3); 16 tokens 4: 13.0, 8: 19.8; 4 tokens 8: 9.2, 16: 8.3; 64
-            # behind 1,000 1: 16.4, 2: 13.7, 4: 19.8 (44.6); 256 1: 36.1, 2: 52.0 (54.3).  Behind 20 rows 6.2 (12.0).
+            # 64, 2 or 4 up to the number of SMs.  Us behind 2,048 rows by blocks a token: 8 tokens 4: 10.3, 8: 8.2, 16 (a
+            # second wave): 14.0; 16 tokens 4: 10.5, 8: 15.9; 4 tokens 8: 7.8, 16: 7.3; 64 behind 1,000 1: 14.6, 2: 12.1, 4:
+            # 17.9; 256 1: 30.8, 2: 46.7.  A cluster takes a microsecond more to start and to merge than a block, a page
+            # 0.65: four pages and fewer go to one block (behind 100 rows 1: 4.2, 2: 5.7; 20 tokens behind 190 1: 5.6, 2: 6.4,
+            # 4: 6.4), and so do fewer than eight where there would be two (64 behind 300 1: 7.1, 2: 7.9; behind 640 10.2, 9.8).
             most = max(1, kernels.sm_count(self.device) // blocks)
             if most > 4 and 8 * blocks > 96:
                 most = 4
@@ -217,6 +219,8 @@ class LatentAttention(Mixer):
                 most = 8
             splits = min(most, pages, kernels.decode_tma_max_splits(row, self.device))
             splits = 1 << (splits.bit_length() - 1)
+            if pages <= 4 or (splits == 2 and pages < 8):
+                splits = 1
             kernels.attention_decode_tma(out, q, t, ctx.positions, ctx.token_slot, entry.k_pages, entry.k_pages, table, nh, 1, row,
                                          self.scale, self.window, splits, **common)
             return

@@ -358,6 +358,37 @@ def test_attention_decode_tma_rows_that_are_keys_and_values(nq, window, softcap)
     k.check_tc_status(q.device)
 
 
+@pytest.mark.parametrize("splits", [1, 2, 3])
+def test_attention_decode_tma_turns_of_rows_that_are_keys_and_values(splits):
+    """One to fourteen pages a block, so odd and even numbers of them and both ways round the ring of six; NaN behind the
+    last sixteen rows with a visible one stays out, a NaN in a query comes out in its own head alone."""
+    k, d, nq = K(), 256, 5
+    lens = [64 * n - cut for n in (1, 2, 3, 5, 6, 7, 8, 12, 13, 14) for cut in (0, 17)]
+    pages = Pages(len(lens), max(lens), 1, d, torch.bfloat16, seed=6)
+    rows = [rnd(n, 1, d, dtype=torch.bfloat16, seed=40 + s) for s, n in enumerate(lens)]
+    for s, n in enumerate(lens):
+        beyond = torch.full((-n % 16, 1, d), 3.0, dtype=torch.bfloat16, device=DEV)
+        never = torch.full((-(n + -n % 16) % 64, 1, d), float("nan"), dtype=torch.bfloat16, device=DEV)
+        full = torch.cat([rows[s], beyond, never])
+        pages.fill(s, full, full)
+    t = len(lens)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    q = rnd(t, nq * d, dtype=torch.bfloat16, seed=60)
+    q[4, 2 * d + 9] = float("nan")
+    out = torch.zeros((t, nq * d), dtype=torch.bfloat16, device=DEV)
+    k.attention_decode_tma(out, q, t, i32([n - 1 for n in lens]), i32(list(range(t))), pages.k, pages.k, pages.table, nq, 1,
+                           d, d ** -0.5, None, splits)
+    got = out.view(t, nq, d)
+    assert got[4, 2].isnan().all()
+    got[4, 2], q[4, 2 * d:3 * d] = 0.0, 0.0
+    for i, n in enumerate(lens):
+        want = ref_attention(q[i].view(nq, d).cpu(), rows[i].cpu(), rows[i].cpu(), n - 1, d ** -0.5, None)
+        if i == 4:
+            want.view(nq, d)[2] = 0.0
+        assert rel(got[i].reshape(-1), want.reshape(-1)) <= TOL[torch.bfloat16], (i, n)
+    k.check_tc_status(q.device)
+
+
 @pytest.mark.parametrize("nq,nkv,d", [(6, 3, 64), (32, 8, 128), (5, 5, 64), (16, 1, 128), (40, 4, 128),
                                       (3, 1, 64)])
 def test_attention_decode_tma(nq, nkv, d):
