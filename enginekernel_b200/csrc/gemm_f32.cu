@@ -750,7 +750,7 @@ sgemm_terms_kernel(uint4* __restrict__ images, uint32_t* __restrict__ flags, con
   for (int p = 0; p < 4; ++p) {
     const uint4 hi = first_terms(v[p], largest);
     to[p * 256] = hi;
-    if (more) {
+    if (more || !is_w) {                         // (the terms of x are always multiplied, also where they are zero)
       uint4 mid, lo;
       other_terms(v[p], hi, mid, lo);
       to[p * 256 + kTermTile / 16] = mid;

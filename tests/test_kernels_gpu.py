@@ -327,6 +327,31 @@ def test_attention_decode_bf16(nq, nkv, d):
             assert rel(out[i], want) <= TOL[dtype], (window, splits, i)
 
 
+@pytest.mark.parametrize("m,exact_x,exact_w", [(3, True, False), (64, True, True), (65, True, False), (130, True, True), (130, False, True)])
+def test_gemm_f32_of_values_of_one_term(m, exact_x, exact_w):
+    """Stretches of x or of the weights that 16 bits hold exactly, zeros among them, have no second and third terms: what
+    free memory held before (NaN here) must not take their place.  Every product is then exact, and so is every 32-bit sum
+    of these few small whole numbers."""
+    k = K()
+    n, kk = 256, 1024
+    g = torch.Generator().manual_seed(m)
+    whole = lambda *s: torch.randint(-3, 4, s, generator=g).float().to(DEV)
+    x, w = whole(m, kk), whole(n, kk)
+    x[:, 128:320] = 0
+    if not exact_x:
+        x[:, 64:128] += 2.0 ** -12
+    if not exact_w:
+        w[:, 64:128] += 2.0 ** -12
+    poison = [torch.full((1 << 20,), float("nan"), device=DEV) for _ in range(24)]
+    out = torch.empty(m, n, device=DEV)
+    torch.cuda.synchronize()
+    del poison
+    k.gemm_f32(out, x, w)
+    # below 1024 x 9 in steps of 2^-12: 26 bits, so the last two may be rounded off, once for each of the 16 stretches
+    assert (out.double() - x.double() @ w.double().T).abs().max() <= 16 * 2.0 ** -11
+    k.check_tc_status(x.device)
+
+
 @pytest.mark.parametrize("nq,window,softcap", [(1, None, None), (16, None, None), (17, 100, None), (20, None, 30.0), (40, 1, None)])
 def test_attention_decode_tma_rows_that_are_keys_and_values(nq, window, softcap):
     """Rows of 256 read once for both uses by the TMA-fed kernel: blocks of 16 heads, 1 to 16 splits (more than a short
