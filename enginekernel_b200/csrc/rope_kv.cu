@@ -8,6 +8,7 @@
 // Differences: positions and slots come per token (no padded rectangle), the cache is
 // paged, and all arithmetic is 32-bit with one rounding at the end.
 #include "common.cuh"
+#include <type_traits>
 
 namespace ek {
 
@@ -73,8 +74,9 @@ __global__ void qk_norm_rope_kv_kernel(T* qkv, int row_stride,
   }
 
   // Four neighbouring dimensions a lane when the sizes allow (head size a multiple of 4 and
-  // the rotated half a multiple of 4), else one.
-  const bool vec = (d % 4 == 0) && (rot_dim % 8 == 0) && (row_stride % 4 == 0);
+  // the rotated half a multiple of 4) and rows and pages lie on such boundaries, else one.
+  const bool vec = (d % 4 == 0) && (rot_dim % 8 == 0) && (row_stride % 4 == 0) &&
+                   (((uintptr_t)qkv | (uintptr_t)cache.k | (uintptr_t)cache.v) & (4 * sizeof(T) - 1)) == 0;
   if (!is_q && !is_k && ex.v_unit) {          // values over their root mean square
     float y[EK_MAX_HEAD_DIM / 32];
     float ssv = 0.f;
@@ -527,6 +529,140 @@ bool wide_takes<bf16>(const void* qkv, int row_stride, const float* q_gain, cons
          aligned(cos_tab) && aligned(sin_tab) && aligned(k_pages) && aligned(v_pages);
 }
 
+// Norm and rotation for rows of 16 or 32 bits, any part of a head rotated, in either order: the gained norm first, or
+// (UNIT) the rotation and then the head over its root mean square.  LPH lanes a head (those past the head's size idle); a
+// lane holds 4 neighbouring dimensions and the 4 that they turn with, or 8 neighbouring ones that are not rotated.
+// All loads are issued before the position is known.  The kernels of a warp a head move 2 or 4 bytes a lane, one behind the
+// other through shared memory, and look position, page and angle up ahead of them.
+// Us a call, that form / this: 5,137 rows of 16 + 2 x 8 heads of 128, 64 rotated, 16 bits (84 MB, 12.9 us at the copy
+// rate) 77.5 / 24.8; 1,129 of 16 + 2 x 8 of 128, gained, 32 bits (37 MB, 5.7 us) 18.7 / 9.1; one of 32 + 2 x 8 2.9 / 1.9.
+// What is left is a block's chain of three lookups (position, slot, page) and the stores behind them.
+template <typename T, int LPH, int PASSES, bool UNIT>      // PASSES: heads a thread
+__global__ void __launch_bounds__(kWideThreads, 4)
+qk_rows_kernel(T* rows, int row_stride, int k_col, int v_col, const float* __restrict__ q_gain,
+               const float* __restrict__ k_gain, const float* __restrict__ cos_tab, const float* __restrict__ sin_tab,
+               int rot_dim, const int* positions, const int* token_slot, PagedKV cache, int n_q_heads, int norm_dim,
+               float eps, int unit, int write_kv) {
+  using Raw = typename std::conditional<sizeof(T) == 2, uint2, uint4>::type;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int HPP = blockDim.x / LPH;                // heads a pass
+  const int t = blockIdx.x, n_kv = cache.heads, d = cache.head_dim, half = rot_dim >> 1;
+  const int n_heads = n_q_heads + (write_kv ? 2 * n_kv : 0);
+  const int lih = threadIdx.x % LPH, head0 = blockIdx.y * HPP * PASSES + threadIdx.x / LPH;
+  const bool turned = 8 * lih < rot_dim;
+  const int a0 = turned ? 4 * lih : 8 * lih, b0 = turned ? half + 4 * lih : 8 * lih + 4;     // this lane's dimensions
+  T* row = rows + (size_t)t * row_stride;
+  Raw raw_a[PASSES], raw_b[PASSES];
+#pragma unroll
+  for (int p = 0; p < PASSES; ++p) {
+    const int head = head0 + p * HPP;
+    if (head < n_heads && 8 * lih < d) {
+      const T* src = row + (head < n_q_heads ? head * d : head < n_q_heads + n_kv ? k_col + (head - n_q_heads) * d
+                                                                                  : v_col + (head - n_q_heads - n_kv) * d);
+      raw_a[p] = *reinterpret_cast<const Raw*>(src + a0);
+      raw_b[p] = *reinterpret_cast<const Raw*>(src + b0);
+    } else {
+      raw_a[p] = raw_b[p] = Raw{};
+    }
+  }
+  const int pos = positions[t];
+  if (pos < 0) return;                             // a row of a finished sequence
+  size_t page_base = 0;
+  if (write_kv) {
+    const int page = cache.block_table[(size_t)token_slot[t] * cache.table_stride + pos / EK_PAGE];
+    page_base = page_offset(cache, page, 0, pos);
+  }
+  float4 c = make_float4(1.f, 1.f, 1.f, 1.f), s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (turned) {
+    c = *reinterpret_cast<const float4*>(cos_tab + (size_t)pos * half + a0);
+    s = *reinterpret_cast<const float4*>(sin_tab + (size_t)pos * half + a0);
+  }
+#pragma unroll
+  for (int p = 0; p < PASSES; ++p) {
+    const int head = head0 + p * HPP;
+    const bool is_q = head < n_q_heads, is_k = !is_q && head < n_q_heads + n_kv, live = head < n_heads && 8 * lih < d;
+    float4 a = Vec4<T>::load(reinterpret_cast<const T*>(&raw_a[p])), b = Vec4<T>::load(reinterpret_cast<const T*>(&raw_b[p]));
+    float ss = 0.f;
+    auto squares = [&] {
+      ss = a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w + b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
+    };
+    const float* gain = is_q ? q_gain : k_gain;
+    const bool gained = !UNIT && gain != nullptr;
+    if (gained) {
+      squares();
+      if ((is_q || is_k) && 8 * lih < d) {
+        const float4 ga = *reinterpret_cast<const float4*>(gain + a0), gb = *reinterpret_cast<const float4*>(gain + b0);
+        a.x *= ga.x; a.y *= ga.y; a.z *= ga.z; a.w *= ga.w;
+        b.x *= gb.x; b.y *= gb.y; b.z *= gb.z; b.w *= gb.w;
+      }
+    }
+    if (turned) {
+      const float4 x = a;
+      a = make_float4(x.x * c.x - b.x * s.x, x.y * c.y - b.y * s.y, x.z * c.z - b.z * s.z, x.w * c.w - b.w * s.w);
+      b = make_float4(b.x * c.x + x.x * s.x, b.y * c.y + x.y * s.y, b.z * c.z + x.z * s.z, b.w * c.w + x.w * s.w);
+    }
+    if (UNIT) squares();
+    // (whole warps: the heads of one may be of all kinds, and past the last)
+#pragma unroll
+    for (int o = LPH / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o, LPH);
+    if (!live) continue;
+    T* dst = is_q ? row + (size_t)head * d
+                  : (T*)(is_k ? cache.k : cache.v) + page_base + (size_t)(head - n_q_heads - (is_k ? 0 : n_kv)) * EK_PAGE * d;
+    if (!is_q && !is_k) {                          // a value head is copied
+      *reinterpret_cast<Raw*>(dst + a0) = raw_a[p];
+      *reinterpret_cast<Raw*>(dst + b0) = raw_b[p];
+      continue;
+    }
+    if (UNIT ? unit : gained) {
+      const float r = rsqrtf(ss / (float)norm_dim + eps);
+      a.x *= r; a.y *= r; a.z *= r; a.w *= r;
+      b.x *= r; b.y *= r; b.z *= r; b.w *= r;
+    }
+    Vec4<T>::store(dst + a0, a);
+    Vec4<T>::store(dst + b0, b);
+  }
+}
+
+// What it takes: head sizes up to 256 in whole pieces of 8 values, rotated parts too, every access aligned.
+template <typename T>
+static bool rows_take(const void* rows, int row_stride, int k_col, int v_col, const float* q_gain, const float* k_gain,
+                      const float* cos_tab, const float* sin_tab, int rot_dim, const void* k_pages, const void* v_pages,
+                      int head_dim) {
+  const uintptr_t wide = (uintptr_t)q_gain | (uintptr_t)k_gain | (rot_dim ? (uintptr_t)cos_tab | (uintptr_t)sin_tab : 0);
+  const uintptr_t narrow = (uintptr_t)rows | (uintptr_t)k_pages | (uintptr_t)v_pages;
+  return head_dim % 8 == 0 && head_dim <= 256 && rot_dim % 8 == 0 && (wide & 15) == 0 && (narrow & (4 * sizeof(T) - 1)) == 0 &&
+         row_stride % 4 == 0 && k_col % 4 == 0 && v_col % 4 == 0;
+}
+template <typename T, bool UNIT>
+static int launch_rows(T* rows, int row_stride, int k_col, int v_col, const float* q_gain, const float* k_gain,
+                       const float* cos_tab, const float* sin_tab, int rot_dim, const int* positions, const int* token_slot,
+                       const PagedKV& cache, int n_tokens, int n_q_heads, int norm_dim, float eps, int unit, int write_kv,
+                       cudaStream_t stream) {
+  const int heads = n_q_heads + (write_kv ? 2 * cache.heads : 0);
+  auto run = [&](auto kernel, int lanes, int passes) {
+    // the heads in equal shares to the blocks of a token, and as many threads as a share fills
+    const int blocks = (heads * lanes + passes * kWideThreads - 1) / (passes * kWideThreads);
+    const int threads = ((heads + blocks * passes - 1) / (blocks * passes) * lanes + 31) / 32 * 32;
+    const int a_block = threads / lanes * passes;
+    return (int)launch_pdl(kernel, dim3(n_tokens, (heads + a_block - 1) / a_block), dim3(threads), 0, stream, rows, row_stride, k_col, v_col, q_gain,
+                           k_gain, cos_tab, sin_tab, rot_dim, positions, token_slot, cache, n_q_heads, norm_dim, eps, unit,
+                           write_kv);
+  };
+  // 16-bit rows: two heads a thread once the tokens fill the machine several times (one head / two, as an
+  // earlier form of the kernel had it, us by rows of 16 + 2 x 8 heads of 64: 1 2.1 / 2.7, 127 2.6 / 3.2; of 128: 100 2.5 / 2.8,
+  // 2,000 15.7 / 14.3, 5,137 30.3 / 28.1; four 2,048 of 32 + 2 x 8 18.3, two 17.2)
+  if constexpr (sizeof(T) == 2)
+    if (n_tokens >= 1024) {
+      if (cache.head_dim <= 64) return run(qk_rows_kernel<T, 8, 2, UNIT>, 8, 2);
+      if (cache.head_dim <= 128) return run(qk_rows_kernel<T, 16, 2, UNIT>, 16, 2);
+      return run(qk_rows_kernel<T, 32, 2, UNIT>, 32, 2);
+    }
+  if (cache.head_dim <= 64) return run(qk_rows_kernel<T, 8, 1, UNIT>, 8, 1);
+  if (cache.head_dim <= 128) return run(qk_rows_kernel<T, 16, 1, UNIT>, 16, 1);
+  return run(qk_rows_kernel<T, 32, 1, UNIT>, 32, 1);
+}
+
 template <typename T>
 static int launch(void* qkv, int row_stride, const float* q_gain, const float* k_gain,
                   const float* cos_tab, const float* sin_tab, int rot_dim, const int* positions,
@@ -556,12 +692,12 @@ static int launch(void* qkv, int row_stride, const float* q_gain, const float* k
                                       n_tokens, n_q_heads, eps, write_kv, ex, stream);
     }
   }
-  if (plain && wide_takes<T>(qkv, row_stride, q_gain, k_gain, cos_tab, sin_tab, rot_dim, k_pages, v_pages,
-                    n_tokens, head_dim)) {
+  // Many tokens of larger heads: gain x angle multiplied once a token and lane for all its heads (us by rows of heads of
+  // 128, this form / qk_rows_kernel: 600 of 32 + 2 x 8 5.9 / 5.7, 1,000 of 16 + 2 x 8 6.8 / 6.8, 2,048 of 32 14.6 / 17.2,
+  // 9,000 61 / 70; of 64, 128 of 16 + 2 x 8 2.7 / 2.2, 2,048 9.5 / 7.1)
+  if (plain && head_dim > 64 && n_tokens >= 1024 &&
+      wide_takes<T>(qkv, row_stride, q_gain, k_gain, cos_tab, sin_tab, rot_dim, k_pages, v_pages, n_tokens, head_dim)) {
     bf16* rows = (bf16*)qkv;
-    if (head_dim == 64)
-      return launch_wide<64>(rows, row_stride, q_gain, k_gain, cos_tab, sin_tab, positions, token_slot,
-                             cache, n_tokens, n_q_heads, eps, write_kv, stream);
     if (head_dim == 128)
       return launch_wide<128>(rows, row_stride, q_gain, k_gain, cos_tab, sin_tab, positions, token_slot,
                               cache, n_tokens, n_q_heads, eps, write_kv, stream);
@@ -582,6 +718,13 @@ static int launch(void* qkv, int row_stride, const float* q_gain, const float* k
     return launch_wide<256, true>(rows, row_stride, q_gain, k_gain, cos_tab, sin_tab, positions, token_slot,
                                   cache, n_tokens, n_q_heads, eps, write_kv, stream, ex);
   }
+  const int k_col = n_q_heads * head_dim, v_col = k_col + n_kv_heads * head_dim;
+  const bool options = ex.q_bias || ex.k_bias || ex.v_bias || ex.q_temp_coef != 0.f || ex.v_from_k || ex.v_unit;
+  if (!options && rows_take<T>(qkv, row_stride, k_col, v_col, q_gain, k_gain, cos_tab, sin_tab, rot_dim, k_pages, v_pages,
+                               head_dim))
+    return launch_rows<T, false>((T*)qkv, row_stride, k_col, v_col, q_gain, k_gain, cos_tab, sin_tab, rot_dim, positions,
+                                 token_slot, cache, n_tokens, n_q_heads, ex.norm_dim > 0 ? ex.norm_dim : head_dim, eps, 0,
+                                 write_kv, stream);
   const int heads = n_q_heads + (ex.v_from_k ? 1 : 2) * n_kv_heads;
   dim3 grid(n_tokens, (heads + kRopeWarps - 1) / kRopeWarps);
   return (int)launch_pdl(qk_norm_rope_kv_kernel<T>, grid, dim3(kRopeWarps * 32), 0, stream, (T*)qkv,
@@ -794,6 +937,12 @@ static int launch_whole(void* rows, int row_stride, const float* q_gain, const f
         n_kv_heads <= 0)                                                                       \
       return EK_ERR_ARG;                                                                       \
     PagedKV cache{k_pages, v_pages, block_table, table_stride, n_kv_heads, head_dim};          \
+    if (ek::rows_take<T>(rows, row_stride, k_col, v_col, nullptr, nullptr, cos_tab, sin_tab,   \
+                         rot_dim, k_pages, v_pages, head_dim))                                 \
+      return ek::launch_rows<T, true>((T*)rows, row_stride, k_col, v_col, nullptr, nullptr,    \
+                                      cos_tab, sin_tab, rot_dim, positions, token_slot, cache, \
+                                      n_tokens, n_q_heads, norm_dim, eps, unit, write_kv,      \
+                                      stream);                                                 \
     const int heads = n_q_heads + (write_kv ? 2 * n_kv_heads : 0);                             \
     dim3 grid(n_tokens, (heads + kRopeWarps - 1) / kRopeWarps);                                \
     return (int)launch_pdl(qk_rope_unit_kv_kernel<T>, grid, dim3(kRopeWarps * 32), 0, stream,  \

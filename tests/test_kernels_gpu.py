@@ -414,6 +414,50 @@ def test_attention_decode_tma_turns_of_rows_that_are_keys_and_values(splits):
     k.check_tc_status(q.device)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("t,nq,nkv,d,rot", [(1, 1, 1, 8, 0), (3, 5, 1, 24, 8), (2, 33, 3, 64, 64), (40, 20, 10, 128, 64),
+                                            (17, 3, 1, 136, 128), (5, 9, 2, 256, 40), (1023, 2, 1, 64, 16),
+                                            (1024, 3, 2, 72, 64), (1030, 20, 4, 128, 128)])
+@pytest.mark.parametrize("unit", [False, True])
+def test_norm_and_rotation_by_pairs_of_pieces(dtype, t, nq, nkv, d, rot, unit):
+    """The form by lanes of 4 + 4 values against the one of a warp a head, which rows of an odd stride take: heads that
+    leave lanes idle, parts rotated, one and two heads a thread, a finished row, an infinite value, without cache too."""
+    k = K()
+    width = (nq + 2 * nkv) * d
+    g = torch.Generator().manual_seed(t + d)
+    base = torch.randn(t, width, generator=g).to(dtype).to(DEV)
+    base[0, d - 1] = float("inf")
+    angle = torch.rand(t + 3, rot // 2, generator=g).to(DEV) * 6
+    cos, sin = angle.cos().contiguous(), angle.sin().contiguous()
+    gains = [(torch.rand(d, generator=g) + 0.5).to(DEV) for _ in range(2)]
+    positions = torch.arange(t, dtype=torch.int32, device=DEV)
+    if t > 2:
+        positions[2] = -1
+    slots = torch.zeros(t, dtype=torch.int32, device=DEV)
+    table = torch.arange(-(-t // 64), dtype=torch.int32, device=DEV).view(1, -1)
+    for write in (True, False):
+        got = []
+        for odd in (0, 1):
+            rows = torch.zeros(t, width + 8 + odd, dtype=dtype, device=DEV)[:, :width]
+            rows.copy_(base)
+            kp, vp = (torch.zeros(table.numel(), nkv, 64, d, dtype=dtype, device=DEV) for _ in range(2))
+            if unit:
+                k.qk_rope_unit_kv(rows, t, nq * d, (nq + nkv) * d, cos, sin, rot, positions, slots, kp, vp, table, nq, nkv,
+                                  d, max(1, d - 3), 1e-5, write_kv=write)
+            else:
+                k.qk_norm_rope_kv(rows, t, *gains, cos, sin, rot, positions, slots, kp, vp, table, nq, nkv, d, 1e-5,
+                                  write_kv=write)
+            got.append((rows.float(), kp.float(), vp.float()))
+        # a result is a sum of two products below 14 together (normed values below 4.5, gains below 1.5) after four or five
+        # 32-bit roundings (14 x 5 x 2^-24 = 4.2e-6), the mean of squares summed in another order moves it by less than
+        # 2^-22 of itself; in 16 bits the two may then round to neighbours
+        tol = 2 ** -7 if dtype == torch.bfloat16 else 2 ** -22
+        for a, b in zip(*got):
+            assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+            a, b = (x.nan_to_num(0, 0, 0) for x in (a, b))
+            assert ((a - b).abs() <= tol * b.abs() + 4.2e-6).all(), (write, (a - b).abs().max())
+
+
 @pytest.mark.parametrize("nq,nkv,d", [(6, 3, 64), (32, 8, 128), (5, 5, 64), (16, 1, 128), (40, 4, 128),
                                       (3, 1, 64)])
 def test_attention_decode_tma(nq, nkv, d):
