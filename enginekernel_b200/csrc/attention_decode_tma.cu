@@ -376,8 +376,12 @@ attention_decode_tma_kernel(bf16* __restrict__ out, const bf16* q, int q_row_str
 // of the eight warps kept 16 keys and a whole O of its own, fetched the queries for every page, and the merge of eight
 // took 4 us of a block's 14.  All eight warps on one page, two pages a turn, did as well up to four pages a block
 // and worse behind them: they meet, fetch and multiply at the same time.
-// Us by rows behind a token of 16 heads, blocks a token; before, eight warps a page, now: 200, 1: 8.7, 6.1, 5.6; 2,048, 8:
-// 9.5, 8.0, 7.5; 2,048, 1: 29.1, 31.0, 25.3; 8,000, 1: 97.7, 114, 90.6 (0.70 a page); 256 tokens behind 1,000, 1: 38.3, 36.7, 30.8.
+// P is two bfloat16 terms.  One, taken against the set's maximum, is further from 64 bits than one against the maximum of a
+// warp's 16 keys was, where a row's largest weights stay whole: errors of one token behind 300 rows .00197 against
+// .00186, 64 behind 640 .00194 against .00187; with two .00165 and .00166 (a layer 0.4 us more, 2,048 rows in one block
+// 25.3 -> 26.8).  Weights by ex2.approx.ftz: exp2f but for results below 2^-126, which beside the largest, 1, are nothing.
+// Us by rows behind a token of 16 heads, blocks a token; before / now: 190, 1: 8.8, 5.8; 2,048, 8: 9.5, 7.7; 2,048, 1: 29.1,
+// 26.8; 8,000, 1: 97.7, 95.8 (0.75 a page); 256 tokens behind 1,000, 1: 38.3, 32.5.
 template <int D, int STAGES>
 __global__ void __launch_bounds__(kDtThreads<D>)
 attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_row_stride,
@@ -398,8 +402,8 @@ attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_
   float* recv_ml = recv_o + kDtRecvO<D>;
   float* max_s = recv_ml + kDtRecvMl;              // [set][16 heads][warp of the set] maxima of a page, at the end the sums
   float* row_s = max_s + W * 16;                   // [set][16 heads] the set's maximum, at the end
-  unsigned char* p_s = (unsigned char*)(row_s + 2 * 16);       // [set][16 heads][64 keys] P, 16-byte pieces swizzled
-  unsigned char* q_s = p_s + 2 * 16 * 128;             // [16 heads][D], 16-byte pieces swizzled
+  unsigned char* p_s = (unsigned char*)(row_s + 2 * 16);       // [set][16 heads][64 keys] P's first terms, 16-byte pieces swizzled
+  unsigned char* q_s = p_s + 2 * 16 * 128;             // [16 heads][D], 16-byte pieces swizzled; then P's second terms
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
   const int split = blockIdx.x, n_splits = gridDim.x;
@@ -513,12 +517,13 @@ attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks)
         ldsm_x4(smem_u32(q_s) + a_row * (2 * D) + (((2 * ks + (lane >> 4)) ^ (a_row & 7)) << 4), qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3]);
+      together();                                  // (all have read the queries)
       // addresses are a lane's offset and a constant: 16-byte piece p of row r lies at (p ^ r) & 7
       const uint32_t ring = smem_u32(smem);
       const int k_row = 16 * part + (lane & 7) + 8 * (lane >> 4);
       const uint32_t key_at = k_row * 128 + ((((lane >> 3) & 1) ^ (k_row & 7)) << 4);
       const uint32_t value_at = part * kSub + a_row * 128 + (((lane >> 4) ^ (a_row & 7)) << 4);
-      const uint32_t p_from = smem_u32(p_s) + set * 16 * 128, p_at = a_row * 128 + (((lane >> 4) ^ (a_row & 7)) << 4);
+      const uint32_t p_from = smem_u32(p_s) + set * 16 * 128, p_lower = smem_u32(q_s) - smem_u32(p_s), p_at = a_row * 128 + (((lane >> 4) ^ (a_row & 7)) << 4);
       unsigned char* const p_to = p_s + (16 * set + g) * 128 + 4 * tq;
       float* const max_to = max_s + set * 16 * SET + g * SET + part;
       const float4* const max_of = reinterpret_cast<const float4*>(max_s + set * 16 * SET + g * SET);
@@ -554,14 +559,19 @@ attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_
           for (int u = 0; u < 2; ++u)
 #pragma unroll
             for (int e = 0; e < 4; ++e) sc[u][e] = capped_log2(sc[u][e], cap);
+        const bool inside = page0 >= lo && page0 + EK_PAGE - 1 <= hi;
+        if (!inside)
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int key = page0 + 16 * part + 8 * u + 2 * tq + (e & 1);
+              if (key < lo || key > hi) sc[u][e] = -INFINITY;
+            }
 #pragma unroll
         for (int u = 0; u < 2; ++u)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const unsigned from_lo = (unsigned)(page0 + 16 * part + 8 * u + 2 * tq + (e & 1) - lo);
-            sc[u][e] = from_lo <= (unsigned)(hi - lo) ? sc[u][e] : -INFINITY;
-            mx[e >> 1] = fmaxf(mx[e >> 1], sc[u][e]);
-          }
+          for (int e = 0; e < 4; ++e) mx[e >> 1] = fmaxf(mx[e >> 1], sc[u][e]);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
@@ -577,13 +587,15 @@ attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_
         for (int r = 0; r < 2; ++r) {            // (the maximum is finite from the first page on: it has a visible key)
           const float4 a = max_of[8 * r];
           const float m_new = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), m_run[r]);
-          alpha[r] = exp2f(m_run[r] - m_new);
+          alpha[r] = ex2_approx(m_run[r] - m_new);
           m_run[r] = m_new;
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
-            sc[u][2 * r] = exp2f(sc[u][2 * r] - m_new);
-            sc[u][2 * r + 1] = exp2f(sc[u][2 * r + 1] - m_new);
-            *reinterpret_cast<uint32_t*>(p_to + 8 * r * 128 + (((2 * part + u) ^ (g & 7)) << 4)) = pack2_bf16(sc[u][2 * r], sc[u][2 * r + 1]);
+            const float p0 = sc[u][2 * r] = ex2_approx(sc[u][2 * r] - m_new), p1 = sc[u][2 * r + 1] = ex2_approx(sc[u][2 * r + 1] - m_new);
+            unsigned char* const to = p_to + 8 * r * 128 + (((2 * part + u) ^ (g & 7)) << 4);
+            const uint32_t p = pack2_bf16(p0, p1);
+            *reinterpret_cast<uint32_t*>(to) = p;
+            *reinterpret_cast<uint32_t*>(to + (q_s - p_s)) = pack2_bf16(p0 - __uint_as_float(p << 16), p1 - __uint_as_float(p & 0xffff0000u));
           }
           l_run[r] = l_run[r] * alpha[r] + ((sc[0][2 * r] + sc[0][2 * r + 1]) + (sc[1][2 * r] + sc[1][2 * r + 1]));
         }
@@ -593,19 +605,28 @@ attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_
           acc[n][2] *= alpha[1]; acc[n][3] *= alpha[1];
         }
         set_together();
-        // P of 16 keys and their rows (which are keys and values alike), fetched a step ahead of their MMAs
-        uint32_t pa[2][4], vb[4][4];
+        // both terms of P of 16 keys and their rows (which are keys and values alike), fetched a step ahead of their MMAs
+        uint32_t pa[2][4], pb[2][4], vb[4][4];
         auto fetch_p = [&](int k) {
-          ldsm_x4(p_from + (p_at ^ (32 * k)), pa[k & 1][0], pa[k & 1][1], pa[k & 1][2], pa[k & 1][3]);
+          const uint32_t from = p_from + (p_at ^ (32 * k));
+          ldsm_x4(from, pa[k & 1][0], pa[k & 1][1], pa[k & 1][2], pa[k & 1][3]);
+          ldsm_x4(from + p_lower, pb[k & 1][0], pb[k & 1][1], pb[k & 1][2], pb[k & 1][3]);
         };
         auto fetch_v = [&](int k, int x) {
           ldsm_x4_trans(stage + 16 * k * 128 + (value_at ^ (32 * x)), vb[x][0], vb[x][1], vb[x][2], vb[x][3]);
         };
-        auto add = [&](int k, int x) {
-          mma_bf16_16816(acc[2 * x], pa[k & 1][0], pa[k & 1][1], pa[k & 1][2], pa[k & 1][3], vb[x][0], vb[x][1]);
-          mma_bf16_16816(acc[2 * x + 1], pa[k & 1][0], pa[k & 1][1], pa[k & 1][2], pa[k & 1][3], vb[x][2], vb[x][3]);
+        auto add = [&](int k, int x0) {          // to 32 dimensions: four sums in turn
+#pragma unroll
+          for (int term = 0; term < 2; ++term) {
+            const uint32_t (&p)[4] = term == 0 ? pa[k & 1] : pb[k & 1];
+#pragma unroll
+            for (int x = x0; x < x0 + 2; ++x) {
+              mma_bf16_16816(acc[2 * x], p[0], p[1], p[2], p[3], vb[x][0], vb[x][1]);
+              mma_bf16_16816(acc[2 * x + 1], p[0], p[1], p[2], p[3], vb[x][2], vb[x][3]);
+            }
+          }
         };
-        if (page0 >= lo && page0 + EK_PAGE - 1 <= hi) {
+        if (inside) {
           fetch_p(0);
 #pragma unroll
           for (int x = 0; x < 4; ++x) fetch_v(0, x);
@@ -613,9 +634,10 @@ attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_
           for (int k = 0; k < 4; ++k) {
             if (k < 3) fetch_p(k + 1);
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
+            for (int x = 0; x < 4; x += 2) {
               add(k, x);
               if (k < 3) fetch_v(k + 1, x);
+              if (k < 3) fetch_v(k + 1, x + 1);
             }
           }
         } else {
@@ -627,7 +649,7 @@ attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_
 #pragma unroll
               for (int x = 0; x < 4; ++x) fetch_v(k, x);
 #pragma unroll
-              for (int x = 0; x < 4; ++x) add(k, x);
+              for (int x = 0; x < 4; x += 2) add(k, x);
             }
         }
         __syncwarp();
