@@ -230,21 +230,15 @@ constexpr int kStepSpan = kSpan / 64;
 constexpr int kTermTile = 128 * 128;  // bytes of one term of 128 rows, 64 of K
 
 // 8 values as sums of three bfloat16 terms each, exactly: x = hi + mid + lo, every term the nearest to what the ones
-// before it leave.  `largest` gathers the largest magnitude of either half: where it is an infinity or a NaN the terms
-// say nothing.
+// before it leave.  (Of an infinity, a NaN, or a value that rounds to an infinity in 16 bits the third is a NaN, see
+// plain_sum.)
 __device__ __forceinline__ uint32_t two_bf16(float a, float b) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
   return r;
 }
-__device__ __forceinline__ uint4 first_terms(const float (&v)[8], uint32_t& largest) {
-  uint32_t h[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    h[i] = two_bf16(v[2 * i], v[2 * i + 1]);
-    asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(largest) : "r"(largest), "r"(h[i]));
-  }
-  return make_uint4(h[0], h[1], h[2], h[3]);
+__device__ __forceinline__ uint4 first_terms(const float (&v)[8]) {
+  return make_uint4(two_bf16(v[0], v[1]), two_bf16(v[2], v[3]), two_bf16(v[4], v[5]), two_bf16(v[6], v[7]));
 }
 __device__ __forceinline__ void other_terms(const float (&v)[8], const uint4& hi, uint4& mid, uint4& lo) {
   const uint32_t h[4] = {hi.x, hi.y, hi.z, hi.w};
@@ -257,9 +251,6 @@ __device__ __forceinline__ void other_terms(const float (&v)[8], const uint4& hi
   }
   mid = make_uint4(m[0], m[1], m[2], m[3]);
   lo = make_uint4(l[0], l[1], l[2], l[3]);
-}
-__device__ __forceinline__ bool is_odd(uint32_t largest) {
-  return (largest & 0x7f80u) == 0x7f80u || (largest & 0x7f800000u) == 0x7f800000u;
 }
 __device__ __forceinline__ void load_row8(float (&v)[8], const float* from, bool there) {
   if (there) {
@@ -275,25 +266,43 @@ __device__ __forceinline__ void st_shared_16(uint32_t at, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-// The value of one output over columns [k0, k1) of K by FFMA, in the order of chunks and spans, where its rows hold an
-// infinity or a NaN (a term of theirs times a zero would make a NaN of an infinity) or a value that rounds to an
-// infinity in 16 bits.
-__device__ __noinline__ void plain_if_odd(float* out, const float* a, const float* w, int k0, int k1) {
-  bool odd = false;
-  float total = 0.f;
-  for (int s = k0; s < k1; s += kSpan) {
-    float span = 0.f;
-    for (int c = s; c < min(k1, s + kSpan); c += 32) {
-      float chunk = 0.f;
-      for (int k = c; k < min(k1, c + 32); ++k) {
-        odd |= !(fabsf(a[k]) < 0x1.ffp127f) || !(fabsf(w[k]) < 0x1.ffp127f);
-        chunk = fmaf(a[k], w[k], chunk);
-      }
-      span += chunk;
+// One output by FFMA, in the order of chunks and spans.  It takes the place of a result of the terms that is not finite,
+// which tells two kinds of outputs: those that an infinity or a NaN belongs to, and those of a row with a value that
+// rounds to an infinity in 16 bits.  The terms of all these give a NaN or an infinity, here in the wrong place or not: the
+// third term of x is a NaN then, and is multiplied with every row of the weights; weights of one term only are an infinity
+// or a NaN themselves, times three terms of x of which one is zero or all are not.  So nothing has to be looked for while
+// terms are written, and only such rows' (and columns') outputs cost more.  (A flag for the block, and every output of its
+// tiles worked out again to see whether its rows were the ones, took 1,100 x 4096 x 2048 with one infinity from 0.14 to
+// 36 ms.)  A sum that is a NaN stays one.  (Inlined: as a function of its own it costs the kernels registers.)
+__device__ __forceinline__ float plain_sum(const float* a, const float* w, int K) {
+  float total = 0.f, span = 0.f;
+#pragma unroll 1
+  for (int c = 0; c < K; c += 32) {
+    float x[4][8], y[4][8], chunk = 0.f;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      load_row8(x[p], a + c + 8 * p, c + 8 * p < K);
+      load_row8(y[p], w + c + 8 * p, c + 8 * p < K);
     }
-    total += span;
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) chunk = fmaf(x[p][j], y[p][j], chunk);
+    span += chunk;
+    if (span != span) return span;
+    if ((c + 32) % kSpan == 0 || c + 32 >= K) {
+      total += span;
+      span = 0.f;
+    }
   }
-  if (odd) *out = total;
+  return total;
+}
+__device__ __forceinline__ bool is_finite(float v) { return fabsf(v) < INFINITY; }
+// The outputs from `c` on, `count` rows of one column, that are not finite.
+__device__ __forceinline__ void plain_where_not_finite(float* c, const float* a, const float* w, int count, int K, int lda, int ldc) {
+#pragma unroll 1
+  for (int m = 0; m < count; ++m, a += lda, c += ldc)
+    if (!is_finite(*c)) *c = plain_sum(a, w, K);
 }
 
 // The MMAs of one chunk of 32 (c: the stage's first or second) into the NT columns from `acc` on; tile(i) is where
@@ -355,7 +364,6 @@ sgemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   unsigned char* tail = ring + kTermStages * kStage + few_low(SPLIT) + depth * kRaw;
   uint64_t* bars = (uint64_t*)tail;                     // full[2], summed[2], taken[2], done, received, here[4], read[4]
   uint32_t* tmem_slot = (uint32_t*)(bars + 16);
-  volatile int* any_odd = (int*)(tmem_slot + 1);
   unsigned char* more_terms = (unsigned char*)(tmem_slot + 4);     // [stage][CW]: the weights have second or third terms
   float* received = (float*)(tail + 512);               // [span][token of this block][128]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -406,7 +414,6 @@ sgemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     }
     mbar_init(done, 2);
     mbar_init(received0, 1);
-    *any_odd = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     if (SPLIT && mine > 0) mbar_expect_tx(received0, (uint32_t)(all_spans * mine * 512));
   }
@@ -450,15 +457,12 @@ sgemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       const int span_of = (s - 1) / kStepSpan;
       if constexpr (SPLIT) {
         // every token's sum to the block that adds it up
-        const int n = tile * 128 + tid, k0 = k_begin + span_of * kSpan;
-        const bool odd = *any_odd != 0;
+        const int at = k_begin / kSpan + span_of;
         int to = 0, slot = 0;
 #pragma unroll
         for (int t = 0; t < NT; ++t)
           if (t < rows) {
-            float v = span[t];
-            if (odd && n < N) plain_if_odd(&v, A + (size_t)(m0 + t) * lda, W + (size_t)n * ldw, k0, min(k_end, k0 + kSpan));
-            st_async_f32(&received[((size_t)(k0 / kSpan) * slots + slot) * 128 + tid], (unsigned)to, v, received0);
+            st_async_f32(&received[((size_t)at * slots + slot) * 128 + tid], (unsigned)to, span[t], received0);
             if (++to == ranks) {
               to = 0;
               ++slot;
@@ -485,12 +489,14 @@ sgemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         if (last) {
           s = 0;
           const int n = tile * 128 + tid;
+          bool finite = true;
 #pragma unroll
           for (int t = 0; t < NT; ++t)
-            if (n < N && t < rows) C[(size_t)(m0 + t) * ldc + n] = span[t];
-          if (*any_odd && n < N)
-            for (int m = m0; m < m0 + rows; ++m)
-              plain_if_odd(C + (size_t)m * ldc + n, A + (size_t)m * lda, W + (size_t)n * ldw, 0, K);
+            if (n < N && t < rows) {
+              C[(size_t)(m0 + t) * ldc + n] = span[t];
+              finite = finite && is_finite(span[t]);
+            }
+          if (!finite) plain_where_not_finite(C + (size_t)m0 * ldc + n, A + (size_t)m0 * lda, W + (size_t)n * ldw, rows, K, lda, ldc);
           tile += gridDim.x;
         }
       }
@@ -506,7 +512,8 @@ sgemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             const float v = received[((size_t)j * slots + i) * 128 + tid];
             sum = j > 0 ? sum + v : v;
           }
-          C[(size_t)(m0 + rank + i * ranks) * ldc + n] = sum;
+          const size_t m = m0 + rank + i * ranks;
+          C[m * ldc + n] = is_finite(sum) ? sum : plain_sum(A + m * lda, W + (size_t)n * ldw, K);
         }
     }
   } else if (warp < AW + CW) {
@@ -534,7 +541,7 @@ sgemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       if (!(ok = mbar_wait(here0 + 8 * slot, phase, status, 37))) break;
       const uint32_t from = raw0 + (uint32_t)slot * kRaw, at = terms0 + (q & 1) * kStage;
       float w[2][8], x[8];
-      uint32_t low = 0, largest = 0;
+      uint32_t low = 0, low_x = 0;
       // pass n: half n & 1 of the stage's K, rows 8 (n >> 1) ..
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
@@ -549,15 +556,20 @@ sgemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         const uint32_t in = from + 128 * 256 + (cw & 1) * (NT * 128) + (8 * (cw >> 1) + r8) * 128;
         read_16(x, in + even);
         read_16(x + 4, in + odd);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) low_x |= __float_as_uint(x[j]);
       }
       uint4 hi[2], x_hi;
 #pragma unroll
-      for (int p = 0; p < 2; ++p) hi[p] = first_terms(w[p], largest);
-      if (has_x) x_hi = first_terms(x, largest);
-      if (is_odd(largest)) *any_odd = 1;
-      // (every lane has used what it read when the vote is over: the place may be filled again)
-      const bool more = __any_sync(0xffffffffu, (low & 0xffffu) != 0);
-      if (lane == 0) mbar_arrive(read0 + 8 * slot);
+      for (int p = 0; p < 2; ++p) hi[p] = first_terms(w[p]);
+      if (has_x) x_hi = first_terms(x);
+      const uint32_t with_more = __ballot_sync(0xffffffffu, (low & 0xffffu) != 0);
+      const bool more = with_more != 0;
+      // The place may be filled again once every lane has what it asked for.  Nothing but the need for the values keeps an
+      // arrival behind reads that are on their way (neither a fence nor a barrier of the warp does: a form whose arrival had no use
+      // for them found the values of the next filling in half of its rows), so which lane arrives is read from all of them.
+      const uint32_t seen = with_more | (has_x ? __ballot_sync(0xffffffffu, (low_x & 0xffffu) != 0) : 0u);
+      if (lane == 31 - __clz(seen | 1u)) mbar_arrive(read0 + 8 * slot);
       if (q >= kTermStages && !(ok = mbar_wait(summed0 + 8 * (q & 1), ((q >> 1) & 1) ^ 1, status, 31))) break;
 #pragma unroll
       for (int p = 0; p < 2; ++p) st_shared_16(at + to_w[p], hi[p]);
@@ -725,7 +737,7 @@ static int launch_few(float* C, const float* A, const float* W, int M, int N, in
 
 // ------------------------------------------------------------------ many rows: operands converted ahead
 // Images: [row block of 128][64 of K][term] tiles of 16 KB as the MMA reads them (K-major, 128-byte swizzle), and
-// one word a (row block, 64 of K): bit 0 - there are second or third terms, bit 1 - a value is infinite or NaN.
+// one word a (row block of the weights, 64 of K): whether there are second or third terms.
 
 __global__ void __launch_bounds__(256)
 sgemm_terms_kernel(uint4* __restrict__ images, uint32_t* __restrict__ flags, const float* __restrict__ A, const float* __restrict__ W,
@@ -737,7 +749,7 @@ sgemm_terms_kernel(uint4* __restrict__ images, uint32_t* __restrict__ flags, con
   const float* from = is_w ? W : A;
   const size_t ld = is_w ? ldw : lda;
   float v[4][8];
-  uint32_t low = 0, largest = 0;
+  uint32_t low = 0;
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
     load_row8(v[p], from + (size_t)(r0 + row + 32 * p) * ld + k, r0 + row + 32 * p < limit && k < K);
@@ -748,7 +760,7 @@ sgemm_terms_kernel(uint4* __restrict__ images, uint32_t* __restrict__ flags, con
   uint4* to = images + ((size_t)rb * gridDim.x + kb) * (3 * kTermTile / 16) + row * 8 + (piece ^ (row & 7));
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
-    const uint4 hi = first_terms(v[p], largest);
+    const uint4 hi = first_terms(v[p]);
     to[p * 256] = hi;
     if (more || !is_w) {                         // (the terms of x are always multiplied, also where they are zero)
       uint4 mid, lo;
@@ -757,8 +769,7 @@ sgemm_terms_kernel(uint4* __restrict__ images, uint32_t* __restrict__ flags, con
       to[p * 256 + 2 * kTermTile / 16] = lo;
     }
   }
-  const int odd = __syncthreads_or(is_odd(largest));
-  if (tid == 0) flags[(size_t)rb * gridDim.x + kb] = (more ? 1u : 0u) | (odd ? 2u : 0u);
+  if (is_w && tid == 0) flags[(size_t)rb * gridDim.x + kb] = more ? 1u : 0u;
 }
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -783,7 +794,6 @@ sgemm_tc_many_kernel(float* __restrict__ C, const unsigned char* __restrict__ im
   unsigned char* ring = raw + ((1024 - (smem_u32(raw) & 1023)) & 1023);
   uint64_t* bars = (uint64_t*)(ring + kManyRing * kTermTile);   // full[4], freed[4], summed[2], taken[2], done
   uint32_t* tmem_slot = (uint32_t*)(bars + 14);
-  volatile int* any_odd = (int*)(tmem_slot + 1);
   volatile int* more_terms = (int*)(tmem_slot + 2);     // of the stage behind each barrier
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int stages = (K + 63) / 64, all_tiles = w_blocks * ((M + NT - 1) / NT);
@@ -799,7 +809,6 @@ sgemm_tc_many_kernel(float* __restrict__ C, const unsigned char* __restrict__ im
       mbar_init(taken0 + 8 * i, 8);
     }
     mbar_init(done, 2);
-    *any_odd = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 9) tmem_alloc(smem_u32(tmem_slot), 4 * NT);
@@ -839,12 +848,15 @@ sgemm_tc_many_kernel(float* __restrict__ C, const unsigned char* __restrict__ im
       if (!last) { ++s; continue; }
       s = 0;
       const int n = tile % w_blocks * 128 + (warp & 3) * 32 + lane, m0 = tile / w_blocks * NT + (warp >> 2) * COLS;
+      bool finite = true;
 #pragma unroll
       for (int t = 0; t < COLS; ++t)
-        if (n < N && m0 + t < M) C[(size_t)(m0 + t) * ldc + n] = sum[t];
-      if (*any_odd && n < N)
-        for (int m = m0; m < min(M, m0 + COLS); ++m)
-          plain_if_odd(C + (size_t)m * ldc + n, A + (size_t)m * lda, W + (size_t)n * ldw, 0, K);
+        if (n < N && m0 + t < M) {
+          C[(size_t)(m0 + t) * ldc + n] = sum[t];
+          finite = finite && is_finite(sum[t]);
+        }
+      if (!finite)
+        plain_where_not_finite(C + (size_t)m0 * ldc + n, A + (size_t)m0 * lda, W + (size_t)n * ldw, min(COLS, M - m0), K, lda, ldc);
       tile += gridDim.x;
     }
   } else if (warp == 8) {
@@ -852,11 +864,10 @@ sgemm_tc_many_kernel(float* __restrict__ C, const unsigned char* __restrict__ im
       int s = 0, tile = blockIdx.x, at = 0, room = kManyRing, oldest = 0, asked = 0;
       uint32_t sizes = 0;                               // tiles of the stages in flight, 8 bits each, the oldest lowest
       size_t wi = (size_t)(tile % w_blocks) * stages, xi = (size_t)(w_blocks + tile / w_blocks * NT / 128) * stages;
-      uint32_t w_flag = total > 0 ? flags[wi] : 0, x_flag = total > 0 ? flags[xi] : 0;
+      uint32_t w_flag = total > 0 ? flags[wi] : 0;
 #pragma unroll 1
       for (int q = 0; q < total; ++q) {
-        const bool more = w_flag & 1u;
-        if ((w_flag | x_flag) & 2u) *any_odd = 1;
+        const bool more = w_flag != 0;
         const int need = more ? 6 : 4, slot = q % kManySlots;
         while (ok && (room < need || q - oldest >= kManySlots)) {
           ok = mbar_wait(freed0 + 8 * (oldest % kManySlots), (oldest / kManySlots) & 1, status, 31);
@@ -890,10 +901,7 @@ sgemm_tc_many_kernel(float* __restrict__ C, const unsigned char* __restrict__ im
           wi = (size_t)(tile % w_blocks) * stages;
           xi = (size_t)(w_blocks + tile / w_blocks * NT / 128) * stages;
         }
-        if (q + 1 < total) {                            // (their latency passes behind the next wait)
-          w_flag = flags[wi];
-          x_flag = flags[xi];
-        }
+        if (q + 1 < total) w_flag = flags[wi];          // (its latency passes behind the next wait)
       }
       if (!ok)                                          // copies in flight land before the block leaves
         for (int q = oldest; q < asked; ++q) mbar_wait(full0 + 8 * (q % kManySlots), (q / kManySlots) & 1, status, 36);

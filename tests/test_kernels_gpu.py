@@ -643,6 +643,50 @@ def test_gemm_f32_on_tensor_cores_with_infinities(m, n, k_):
     k.check_tc_status(DEV)
 
 
+@pytest.mark.parametrize("m,n,k_", [(5, 140, 1024), (40, 700, 1320), (150, 140, 1024)])
+def test_gemm_f32_of_the_largest_values_does_not_depend_on_the_rows_beside_them(m, n, k_):
+    """Finite values that 16 bits round to an infinity, in one stretch of K: every form gives their row what the one-row
+    product gives, bit for bit, and 64 bits to the bound of chains of 32 products in spans of 256 (as the other forms)."""
+    k = K()
+    x, w = rnd(m, k_, seed=1).to(DEV), rnd(n, k_, seed=2).to(DEV)
+    w[:, 300] *= 2.0 ** -126
+    x[m - 1, 300], x[0, 301] = 3.4e38, -3.4e38
+    w[:, 301] *= 2.0 ** -126
+    out = torch.empty(m, n, device=DEV)
+    k.gemm_f32(out, x, w)
+    want = x.double() @ w.double().t()
+    for r in (0, m // 2, m - 1):
+        one = torch.empty(1, n, device=DEV)
+        k.gemm_f32(one, x[r:r + 1], w)
+        assert torch.equal(one[0], out[r]), r
+        assert (out[r].double() - want[r]).norm() <= 4e-7 * want[r].norm(), r
+    k.check_tc_status(DEV)
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
+def test_gemm_f32_takes_as_long_beside_a_value_that_is_not_finite(value):
+    """Only the outputs of such a value's row are worked out again: one row among 1,100 may add a fraction to the
+    product (all outputs of its block, and of every later tile of the block, made it 260 times as long: 36 ms)."""
+    k = K()
+    x, w = rnd(1100, 2048, seed=1).to(DEV), rnd(4096, 2048, seed=2).to(DEV)
+    out = torch.empty(1100, 4096, device=DEV)
+
+    def took():
+        times = []
+        for _ in range(5):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            k.gemm_f32(out, x, w)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+    plain = took()
+    x[3, 700] = value
+    assert took() <= 4 * plain
+    k.check_tc_status(DEV)
+
+
 @pytest.mark.parametrize("m,n,k_", [(17, 256, 128), (64, 2560, 4096), (33, 1000, 1000), (1, 128, 64),
                                     (48, 331 * 2, 80), (64, 6144, 2560), (24, 1280, 2560),
                                     (24, 20012, 2560)])
