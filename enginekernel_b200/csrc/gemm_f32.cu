@@ -4,8 +4,10 @@
 // A row's result does not depend, bit for bit, on which other rows share the launch: every form that a layout and K
 // can take sums in one order, whatever M is.
 //
-// Rows of whole 32-byte pieces (K and both strides multiples of 8): tcgen05.  A 32-bit value is the sum of three
-// bfloat16 terms exactly, and the products of two terms are exact in 32 bits.  Of the nine products of two values'
+// Rows of whole 32-byte pieces (K and both strides multiples of 8): tcgen05.  2^24 times a 32-bit value is the sum of three
+// bfloat16 terms exactly (unscaled, the last terms of values below 2^-110 would lie below what bfloat16 holds), and the
+// products of two terms are exact in 32 bits; the sums are scaled back at the end.  Values from 2^104 on and sums from 2^80 on
+// go beyond 32 bits that way, see plain_sum.  Of the nine products of two values'
 // terms the three smallest (2^-24 of the value and less) are left out; weights that came from 16 bits have one term,
 // and then nothing is.  The tensor cores cut a sum at its last place instead of rounding it, so no more than 32 of K go
 // into one accumulator: chunks of 32 are added in 32-bit registers, rounded, to spans of 256, and the spans to the result.
@@ -229,9 +231,16 @@ constexpr int kSpan = 256;            // of K: a span's sum is that of its chunk
 constexpr int kStepSpan = kSpan / 64;
 constexpr int kTermTile = 128 * 128;  // bytes of one term of 128 rows, 64 of K
 
-// 8 values as sums of three bfloat16 terms each, exactly: x = hi + mid + lo, every term the nearest to what the ones
-// before it leave.  (Of an infinity, a NaN, or a value that rounds to an infinity in 16 bits the third is a NaN, see
-// plain_sum.)
+// 8 values, 2^24 times as large, as sums of three bfloat16 terms each, exactly: x = hi + mid + lo, every term the nearest to
+// what the ones before it leave; the last bit of the smallest 32-bit number is 2^-125 then, a normal one.  (Of an infinity, a
+// NaN, or a value that rounds to an infinity in 16 bits the third is a NaN, see plain_sum.)
+constexpr float kScaleBack = 0x1p-48f;
+__device__ __forceinline__ void scale_up(float (&v)[8]) {
+  const uint64_t by = 0x4b8000004b800000ull;                     // 2^24, twice
+#pragma unroll
+  for (int i = 0; i < 8; i += 2)
+    asm("{.reg .b64 p; mov.b64 p, {%0, %1}; mul.rn.f32x2 p, p, %2; mov.b64 {%0, %1}, p;}" : "+f"(v[i]), "+f"(v[i + 1]) : "l"(by));
+}
 __device__ __forceinline__ uint32_t two_bf16(float a, float b) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
@@ -267,8 +276,8 @@ __device__ __forceinline__ void st_shared_16(uint32_t at, uint4 v) {
 }
 
 // One output by FFMA, in the order of chunks and spans.  It takes the place of a result of the terms that is not finite,
-// which tells two kinds of outputs: those that an infinity or a NaN belongs to, and those of a row with a value that
-// rounds to an infinity in 16 bits.  The terms of all these give a NaN or an infinity, here in the wrong place or not: the
+// which tells two kinds of outputs: those that an infinity or a NaN belongs to, and those of a row with a value, or of
+// sums, that scaled up are one (2^104 and 2^80).  The terms of all these values give a NaN or an infinity, here in the wrong place or not: the
 // third term of x is a NaN then, and is multiplied with every row of the weights; weights of one term only are an infinity
 // or a NaN themselves, times three terms of x of which one is zero or all are not.  So nothing has to be looked for while
 // terms are written, and only such rows' (and columns') outputs cost more.  (A flag for the block, and every output of its
@@ -493,7 +502,7 @@ sgemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
           for (int t = 0; t < NT; ++t)
             if (n < N && t < rows) {
-              C[(size_t)(m0 + t) * ldc + n] = span[t];
+              C[(size_t)(m0 + t) * ldc + n] = span[t] * kScaleBack;
               finite = finite && is_finite(span[t]);
             }
           if (!finite) plain_where_not_finite(C + (size_t)m0 * ldc + n, A + (size_t)m0 * lda, W + (size_t)n * ldw, rows, K, lda, ldc);
@@ -513,7 +522,7 @@ sgemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             sum = j > 0 ? sum + v : v;
           }
           const size_t m = m0 + rank + i * ranks;
-          C[m * ldc + n] = is_finite(sum) ? sum : plain_sum(A + m * lda, W + (size_t)n * ldw, K);
+          C[m * ldc + n] = is_finite(sum) ? sum * kScaleBack : plain_sum(A + m * lda, W + (size_t)n * ldw, K);
         }
     }
   } else if (warp < AW + CW) {
@@ -561,8 +570,14 @@ sgemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       }
       uint4 hi[2], x_hi;
 #pragma unroll
-      for (int p = 0; p < 2; ++p) hi[p] = first_terms(w[p]);
-      if (has_x) x_hi = first_terms(x);
+      for (int p = 0; p < 2; ++p) {
+        scale_up(w[p]);
+        hi[p] = first_terms(w[p]);
+      }
+      if (has_x) {
+        scale_up(x);
+        x_hi = first_terms(x);
+      }
       const uint32_t with_more = __ballot_sync(0xffffffffu, (low & 0xffffu) != 0);
       const bool more = with_more != 0;
       // The place may be filled again once every lane has what it asked for.  Nothing but the need for the values keeps an
@@ -760,6 +775,7 @@ sgemm_terms_kernel(uint4* __restrict__ images, uint32_t* __restrict__ flags, con
   uint4* to = images + ((size_t)rb * gridDim.x + kb) * (3 * kTermTile / 16) + row * 8 + (piece ^ (row & 7));
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
+    scale_up(v[p]);
     const uint4 hi = first_terms(v[p]);
     to[p * 256] = hi;
     if (more || !is_w) {                         // (the terms of x are always multiplied, also where they are zero)
@@ -852,7 +868,7 @@ sgemm_tc_many_kernel(float* __restrict__ C, const unsigned char* __restrict__ im
 #pragma unroll
       for (int t = 0; t < COLS; ++t)
         if (n < N && m0 + t < M) {
-          C[(size_t)(m0 + t) * ldc + n] = sum[t];
+          C[(size_t)(m0 + t) * ldc + n] = sum[t] * kScaleBack;
           finite = finite && is_finite(sum[t]);
         }
       if (!finite)

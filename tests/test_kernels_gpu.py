@@ -663,6 +663,28 @@ def test_gemm_f32_of_the_largest_values_does_not_depend_on_the_rows_beside_them(
     k.check_tc_status(DEV)
 
 
+@pytest.mark.parametrize("m,n,k_", [(1, 300, 2048), (40, 700, 1320), (150, 140, 1024)])
+@pytest.mark.parametrize("ex,ew", [(-112, 0), (-120, 90), (-126, 100), (0, -120), (90, -124), (-140, 100), (-60, -60)])
+def test_gemm_f32_of_small_values(m, n, k_, ex, ew):
+    """Values near and below the smallest normal number are whole in 32 bits too: against 64 bits as good as any others,
+    and where the results lie below it themselves, to half their last place (2^-150) more; rows of usual size beside them
+    keep their bits."""
+    k = K()
+    x, w = rnd(m, k_, seed=1).to(DEV), rnd(n, k_, seed=2).to(DEV)
+    x, w = x * 2.0 ** ex, w * 2.0 ** ew
+    if m > 1:
+        x[m // 2] = rnd(1, k_, seed=3).to(DEV)[0] * 2.0 ** max(-ew, -60)
+    out = torch.empty(m, n, device=DEV)
+    k.gemm_f32(out, x, w)
+    want = x.double() @ w.double().t()
+    for r in {0, m // 2, m - 1}:
+        one = torch.empty(1, n, device=DEV)
+        k.gemm_f32(one, x[r:r + 1], w)
+        assert torch.equal(one[0], out[r]), r
+        assert (out[r].double() - want[r]).norm() <= 4e-7 * want[r].norm() + n ** 0.5 * 2.0 ** -150, r
+    k.check_tc_status(DEV)
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
 def test_gemm_f32_takes_as_long_beside_a_value_that_is_not_finite(value):
     """Only the outputs of such a value's row are worked out again: one row among 1,100 may add a fraction to the
