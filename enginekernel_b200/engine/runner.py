@@ -101,16 +101,17 @@ class ModelRunner:
         self.workspace = Workspace(self.device)
         self.plan: Optional[PlanBuffers] = None
         self._uploaded = None          # event: the last step's host->device copies are done
-        if model.dtype == torch.bfloat16:
+        if self.device.type == "cuda":              # (these exist before any graph capture)
             from ..ops import kernels
-            kernels.split_scratch(self.device)      # exist before any graph capture
-            kernels.tc_status(self.device)
+            kernels.tc_status(self.device)          # the products of both data types report there
+            if model.dtype == torch.bfloat16:
+                kernels.split_scratch(self.device)
         model.prepare(min(cache.max_len, model.spec.max_positions))
 
     def check_kernels(self) -> None:
-        """Raise if a kernel reported a failure (a tensor-core GEMM whose bounded barrier wait
-        ran out).  Synchronises the device; called where the host waits anyway."""
-        if self.model.dtype == torch.bfloat16 and self.device.type == "cuda":
+        """Raise if a kernel reported a failure (a tensor-core product of either data type, or an attention
+        kernel, whose bounded barrier wait ran out).  Synchronises the device; called where the host waits anyway."""
+        if self.device.type == "cuda":
             from ..ops import kernels
             kernels.check_tc_status(self.device)
 

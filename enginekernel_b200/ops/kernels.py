@@ -1101,13 +1101,19 @@ _SPLIT_TICKETS = 16384
 _split_scratch = {}
 
 
+def _with_index(device):
+    """The device as its tensors name it: "cuda" is the current one."""
+    device = torch.device(device)
+    return device if device.index is not None else torch.device(device.type, torch.cuda.current_device())
+
+
 def split_scratch(device):
     """Per-device scratch of products whose K is split over more blocks than a cluster holds:
     partial tiles and zeroed tickets.  Created on first use; create it before capturing a graph
     (``ModelRunner`` does)."""
     made = _split_scratch.get(device)            # (by the torch.device that launches hand over)
     if made is None:
-        key = torch.device(device)
+        key = _with_index(device)
         if key not in _split_scratch:
             _split_scratch[key] = (torch.empty(_SPLIT_PARTIAL_FLOATS, dtype=torch.float32, device=device),
                                    torch.zeros(_SPLIT_TICKETS, dtype=torch.int32, device=device))
@@ -1123,10 +1129,10 @@ TC_SWAP_MAX_ROWS = 64
 
 
 def tc_status(device):
-    """One int per device that the tensor-core GEMM sets when a barrier wait times out."""
+    """One int per device that the tensor-core kernels set when a barrier wait times out."""
     status = _tc_status.get(device)              # (by the torch.device that launches hand over)
     if status is None:
-        key = torch.device(device)
+        key = _with_index(device)
         if key not in _tc_status:
             _tc_status[key] = torch.zeros(1, dtype=torch.int32, device=device)
         status = _tc_status[key]
@@ -1134,9 +1140,10 @@ def tc_status(device):
 
 
 def check_tc_status(device):
-    """Synchronises; raises if a kernel gave up a bounded barrier wait since the last check (products:
-    1 producer, 2 MMA, 3 epilogue, 4 copies before exit; decode attention 41, 42; others by their
-    kernel) and clears the word, so that the next check speaks of later launches only."""
+    """Synchronises; raises if a kernel gave up a bounded barrier wait since the last check (products in 16 bits:
+    1 producer, 2 MMA, 3 epilogue, 4 copies before exit, 5 sums from the cluster, 41 to 46 on pairs of SMs, experts 51 to 54;
+    products in 32 bits: 31 to 39; prompt attention 11 to 36; decode attention 41 producer, 42 pages, 43 sums from the
+    cluster) and clears the word, so that the next check speaks of later launches only."""
     code = int(tc_status(device).item())
     if code:
         tc_status(device).zero_()

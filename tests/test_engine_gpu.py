@@ -394,3 +394,21 @@ def test_stale_pages_change_nothing(folders, plains, tag, dtype):
     for p, toks in zip(prompts, eng.generate_all(prompts, 20)):
         check_tokens_against_plain(plains[tag], p, toks, dtype)
     assert eng.cache.free_tokens() == eng.cache.num_pages * 64
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_a_wait_that_ran_out_ends_a_call_with_an_error(folders, dtype, monkeypatch):
+    """The products of both data types report a wait that ran out in the device's status word: it exists from an engine's
+    start (ahead of any graph capture), and the call during which it was set raises instead of returning tokens."""
+    from enginekernel_b200 import Engine
+    from enginekernel_b200.ops import kernels
+    from enginekernel_b200.ops.lib import KernelError
+    monkeypatch.setattr(kernels, "_tc_status", {})
+    eng = Engine(folders["E"], dtype, max_tokens=256, max_batch=2)
+    assert list(kernels._tc_status) == [torch.device("cuda", 0)]
+    want = eng.generate_all([[5, 9, 2]], 4)
+    assert kernels.tc_status("cuda") is kernels.tc_status(torch.zeros(1, device="cuda").device)
+    kernels.wait_that_runs_out("cuda", code=77, limit=256)
+    with pytest.raises(KernelError, match="code 77"):
+        eng.generate_all([[5, 9, 2]], 4)
+    assert eng.generate_all([[5, 9, 2]], 4) == want            # the word was cleared, the engine goes on
