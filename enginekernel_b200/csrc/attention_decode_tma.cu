@@ -10,6 +10,7 @@
 //     signalled by an mbarrier.  Old pages do not depend on the kernel before this one (only
 //     the newest key and value do), so their copies are issued BEFORE the programmatic-launch
 //     wait: the cache stream runs while the q/k/v product and the position encoding finish.
+//     (Heads of 64 and 128, whose steps open with a plain launch.)
 //   * warps 0-3: each takes 16 keys of a page.  The G query heads of the group are the 16 rows
 //     of mma.sync.m16n8k16 (padded), K fragments come by ldmatrix, V fragments by
 //     ldmatrix.trans, softmax is online in 32-bit in units of log2, P is rounded to bfloat16
@@ -380,8 +381,8 @@ attention_decode_tma_kernel(bf16* __restrict__ out, const bf16* q, int q_row_str
 // warp's 16 keys was, where a row's largest weights stay whole: errors of one token behind 300 rows .00197 against
 // .00186, 64 behind 640 .00194 against .00187; with two .00165 and .00166 (a layer 0.4 us more, 2,048 rows in one block
 // 25.3 -> 26.8).  Weights by ex2.approx.ftz: exp2f but for results below 2^-126, which beside the largest, 1, are nothing.
-// Us by rows behind a token of 16 heads, blocks a token; before / now: 190, 1: 8.8, 5.8; 2,048, 8: 9.5, 7.7; 2,048, 1: 29.1,
-// 26.8; 8,000, 1: 97.7, 95.8 (0.75 a page); 256 tokens behind 1,000, 1: 38.3, 32.5.
+// Us by rows behind a token of 16 heads, blocks a token; before / now: 190, 1: 8.8, 6.1; 2,048, 8: 9.5, 8.0; 2,048, 1: 29.1,
+// 27.2; 8,000, 1: 97.7, 95.9 (0.75 a page); 256 tokens behind 1,000, 1: 38.3, 33.0.
 template <int D, int STAGES>
 __global__ void __launch_bounds__(kDtThreads<D>)
 attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_row_stride,
@@ -434,12 +435,12 @@ attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_
   // before the first such store)
   __syncwarp();
   if (n_splits > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-  // Read before the wait: positions, slots and block tables must have been written by work that
-  // a plain (not programmatic) launch separates from this kernel.  A step's first kernel, the
-  // embedding lookup, is such a launch, so the state advance of the step before is complete here, in a
-  // captured graph and in eager decoding alike.  Past L1, which may hold the step before's (common.cuh).
-  const int pos = load_past_l1(positions + t);
-  const int slot_t = load_past_l1(token_slot + t);
+  // Nothing is read ahead of the wait.  A latent layer that a program drives by itself has no plain launch between two steps,
+  // and every kernel of its few-row step lets the next one start at its own top: a chain of them may reach this point while
+  // the step before still writes its row to an older page.
+  pdl_wait();
+  const int pos = positions[t];
+  const int slot_t = token_slot[t];
   int lo = 0, hi = -1, pg_first = 0, pg_last = -1;
   if (pos >= 0) {
     lo = first_key(pos, window, chunk);
@@ -451,7 +452,6 @@ attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_
     hi = min(hi, pg_last * EK_PAGE + EK_PAGE - 1);             // (the last of this split)
   }
   const int n_pages = pg_last - pg_first + 1;                  // <= 0: nothing for this split
-  const int new_page = pos >= 0 ? pos / EK_PAGE : -1;          // holds the key written just now
   __syncthreads();
 
   bool ok = true;
@@ -459,19 +459,14 @@ attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_
     // ------------------------------------------------------------------- TMA producer: one thread, for which the
     // warp's lanes fetch 32 entries of the block table at a time
     const int* table = block_table + (size_t)(pos >= 0 ? slot_t : 0) * table_stride + pg_first;
-    bool waited = false;
     const uint64_t stream_policy = l2_policy_evict_first();   // a page is read once a step
     int entry = 0;
     for (int i = 0; i < n_pages; ++i) {
-      if (i % 32 == 0 && i + lane < n_pages) entry = load_past_l1(table + i + lane);
+      if (i % 32 == 0 && i + lane < n_pages) entry = table[i + lane];
       const int page = __shfl_sync(0xffffffffu, entry, i % 32);
       if (lane == 0) {
         const int s = i % STAGES;
         if (i >= STAGES) ok = mbar_wait(empty(s), ((i / STAGES) & 1) ^ 1, status, 41);
-        if (pg_first + i == new_page && !waited) {   // this page was written to by the kernel before
-          pdl_wait();
-          waited = true;
-        }
         if (ok) {
           const int row = (page * n_kv_heads + kv_head) * EK_PAGE;
           const uint32_t dst = smem_u32(smem + s * kStage);
@@ -493,7 +488,6 @@ attention_decode_tma_shared_kernel(bf16* __restrict__ out, const bf16* q, int q_
     // splits are few), asked for here: behind everything else they took a round trip to memory of their own
     const int my_row = n_splits > 1 ? min((split * run + 4 * tid) / D, group - 1) : 0;
     float my_sink = n_splits > 1 && sinks ? sinks[head0 + my_row] * 1.4426950408889634f : sink_log2, my_gate = 1.f;
-    pdl_wait();                                  // the queries come from the kernel before
     if (n_splits > 1 && gate != nullptr) my_gate = __bfloat162float(gate[(size_t)t * gate_stride + head0 + my_row]);
     const int set = warp / SET, part = warp % SET;
     auto together = [] { asm volatile("bar.sync 1, %0;" ::"n"(W * 32) : "memory"); };

@@ -811,10 +811,11 @@ def attention_decode_tma(out, q, n_tokens, positions, token_slot, k_pages, v_pag
     blocks (16 where :func:`decode_tma_max_splits` says so) share a token's pages and merge inside
     a thread-block cluster.
 
-    Precondition: ``positions``, ``token_slot`` and ``block_table`` are read before the kernel
-    waits for the one ahead of it, so whatever wrote them (an upload, the state advance of the
-    step before) must be separated from this launch by a launch that is not programmatic:
-    :func:`embed`, the first kernel of every step, is one."""
+    Precondition for heads of 64 and 128: ``positions``, ``token_slot``, ``block_table`` and every page but the
+    one of the token's own position are read before the kernel waits for the one ahead of it, so
+    whatever wrote them (an upload, the state advance of the step before, the steps before
+    themselves) must be separated from this launch by a launch that is not programmatic:
+    :func:`embed`, the first kernel of every step, is one.  Rows of 256 are read behind the wait."""
     _need_cuda(out, q, positions, token_slot, k_pages, v_pages, block_table)
     shared = k_pages.data_ptr() == v_pages.data_ptr() and attention_decode_tma_shared_supported(q.dtype, head_dim)
     _need(shared or attention_decode_tma_supported(q.dtype, head_dim, n_q_heads, n_kv_heads),

@@ -207,11 +207,12 @@ class LatentAttention(Mixer):
             blocks = t * -(-nh // 16)
             pages = -(-visible // kernels.PAGE)
             # One block an SM, and a cluster's blocks within one group of SMs: 8 blocks a token up to 96 in all, 16 up to
-            # 64, 2 or 4 up to the number of SMs.  Us behind 2,048 rows by blocks a token: 8 tokens 4: 10.9, 8: 8.5, 16 (a
-            # second wave): 14.4; 16 tokens 4: 11.1, 8: 16.5; 4 tokens 8: 7.9, 16: 7.5; 64 behind 1,000 1: 15.7, 2: 12.8, 4:
-            # 18.4; 256 1: 32.5, 2: 48.8.  A cluster takes a microsecond more to start and to merge than a block, a page
-            # 0.75: three pages and fewer go to one block (behind 100 rows 1: 4.5, 2: 5.8; 20 tokens behind 190 1: 6.0, 2: 6.6),
-            # four for more than 16 blocks (a layer of 20 tokens behind 10 to 200 1: 38.3, 4: 39.8; of one behind 200 31.3, 31.1), and so do fewer than eight where there would be two (64 behind 300 1: 7.6, 2: 8.2; behind 640 10.9, 10.2).
+            # 64, 2 or 4 up to the number of SMs.  Us behind 2,048 rows by blocks a token: 8 tokens 4: 11.1, 8: 8.6, 16 (a
+            # second wave): 14.9; 16 tokens 4: 11.4, 8: 17.1; 4 tokens 8: 8.2, 16: 7.4; 64 behind 1,000 1: 16.1, 2: 12.8, 4:
+            # 18.5; 256 1: 33.0, 2: 48.8.  A cluster takes a microsecond more to start and to merge than a block, a page
+            # 0.75: three pages and fewer go to one block (behind 100 rows 1: 4.9, 2: 6.3; 20 tokens behind 190 1: 6.3, 2: 6.9),
+            # four for more than 16 blocks (a layer of 20 tokens behind 10 to 200 1: 38.3, 4: 39.8; of one behind 200 31.3,
+            # 31.1), and so do fewer than eight where there would be two (64 behind 300 1: 8.2, 2: 8.8; behind 640 11.6, 10.7).
             most = max(1, kernels.sm_count(self.device) // blocks)
             if most > 4 and 8 * blocks > 96:
                 most = 4

@@ -86,6 +86,45 @@ def test_a_layer_driven_alone_reads_its_own_steps_table(kind):
         assert torch.equal(y, wants[i % len(steps)]), (i // len(steps), i % len(steps))
 
 
+@pytest.mark.parametrize("seqs", [1, 3])
+def test_a_latent_layer_driven_alone_decodes_over_rows_that_earlier_steps_wrote(seqs):
+    """Decode steps over a page's border (62 to 67 rows, and 126 to 131) with contexts made ahead, nothing between the steps
+    and none waited for: rows that a step wrote to a page are there in the next steps, which read it as an older one."""
+    from enginekernel_b200.cache import SequenceCache
+    from enginekernel_b200.parts.base import Workspace
+    part = layer("latent", heads=20)
+    for past in (62, 126):
+        def decode(waited):
+            cache = SequenceCache([part.cache_spec()], torch.bfloat16, DEV, max_tokens=192 * seqs, max_slots=seqs)
+            slots = [cache.open() for _ in range(seqs)]
+            for s in slots:
+                cache.reserve(s, past + 6)
+            cache.upload_tables()
+            entry, shared = cache.entry(0), Workspace(torch.device(DEV))
+            g = torch.Generator().manual_seed(past)
+            rows = lambda n: torch.randn(n, H, generator=g).to(torch.bfloat16).to(DEV)
+            prompt = helpers.make_context(torch.bfloat16, DEV, [i for _ in slots for i in range(past)],
+                                          [s for s in slots for _ in range(past)], [past * i for i in range(seqs + 1)])
+            steps = [(rows(past * seqs), prompt)]
+            for i in range(6):
+                steps.append((rows(seqs), helpers.make_context(torch.bfloat16, DEV, [past + i] * seqs, slots, list(range(seqs + 1)))))
+            torch.cuda.synchronize()
+            got = []
+            for x, ctx in steps:
+                ctx.workspace = Workspace(torch.device(DEV)) if waited else shared
+                ctx.shared = {}
+                part.begin_step(ctx)
+                got.append(part.forward(x, ctx, entry, True).clone())
+                if waited:
+                    torch.cuda.synchronize()
+            torch.cuda.synchronize()
+            return got[1:]
+        want = decode(True)
+        for _ in range(4):
+            for i, (a, b) in enumerate(zip(decode(False), want)):
+                assert torch.equal(a, b), (past, i)
+
+
 @pytest.mark.parametrize("kind", ["attention", "window"])
 def test_tiles_found_by_the_blocks_are_those_of_the_table(kind):
     """A step with a table of tiles and without one: the same results, for sequences of one token to several tiles."""
