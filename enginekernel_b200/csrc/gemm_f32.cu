@@ -25,7 +25,7 @@
 //                   at about the rate of the MMAs.  1129 x 6144 x 1024 360 -> 87 us, 1129 x 1024 x 3072 219 -> 56,
 //                   4096^3 3,165 -> 515 (267 TFLOP/s).  The three terms of x side by side in one MMA of 192 columns
 //                   read less shared memory but more L2 (128 x 64 tiles): 820 us.
-// Other rows: FFMA, chains of 64 (kRun) whose sums are added in ascending order.
+// Other rows, and K above 131,072: FFMA, chains of 64 (kRun) whose sums are added in ascending order.
 //   few rows (M <= 16)  a lane takes a few columns and one run of K; one thread an output adds the runs' sums in order.
 //   more rows           8 x 8 outputs a thread from tiles in shared memory.
 #include "tc_common.cuh"
@@ -980,6 +980,8 @@ static int launch_many(float* C, const float* A, const float* W, int M, int N, i
 
 constexpr int kFewRows = 64;          // up to here operands are converted on their way in
 constexpr long long kImageBytes = 128ll << 20;    // of weights, and of rows of x, that are converted at a time
+constexpr int kMostK = 1 << 17;       // of K: one block of 128 rows stays below that (longer rows: FFMA)
+static_assert((kMostK / 64) * (3ll * kTermTile + 4) <= kImageBytes, "a block's images");
 
 // Rows whose images are made at a time: equal parts, whole blocks.
 static int image_rows(int rows, int K) {
@@ -1013,9 +1015,9 @@ static int launch_tc(float* C, const float* A, const float* W, int M, int N, int
 
 }  // namespace ek
 
-// Bytes that a product of these sizes wants for its operands' terms (0: none).
+// Bytes that a product of these sizes wants for its operands' terms (0: none), 256 MB at most.
 EK_EXPORT int ek_gemm_f32_scratch(int M, int N, int K) {
-  if (M <= ek::kFewRows || N <= 0 || K <= 0 || K % 8 != 0) return 0;
+  if (M <= ek::kFewRows || N <= 0 || K <= 0 || K % 8 != 0 || K > ek::kMostK) return 0;
   return (int)(ek::terms_bytes(ek::image_rows(M, K), K) + ek::terms_bytes(ek::image_rows(N, K), K));
 }
 
@@ -1024,7 +1026,7 @@ EK_EXPORT int ek_gemm_nt_f32(float* C, const float* A, const float* W, int M, in
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || lda < K || ldw < K || ldc < N) return EK_ERR_ARG;
   // (a rule on the layout and K, not on M: a row's result does not depend on the rows beside it)
-  const bool vec = K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && ((uintptr_t)A & 31) == 0 && ((uintptr_t)W & 31) == 0;
+  const bool vec = K % 8 == 0 && K <= ek::kMostK && lda % 8 == 0 && ldw % 8 == 0 && ((uintptr_t)A & 31) == 0 && ((uintptr_t)W & 31) == 0;
   return vec ? ek::launch_tc(C, A, W, M, N, K, lda, ldw, ldc, (unsigned char*)scratch, status, stream)
              : ek::launch_ffma(C, A, W, M, N, K, lda, ldw, ldc, stream);
 }

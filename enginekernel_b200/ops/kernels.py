@@ -1076,7 +1076,10 @@ def gemm_f32(out, x, w, n_rows=None):
         lib.annotate(bytes=4 * (n * k + m * k + m * n), flops=2 * m * n * k)
     # many rows: the operands' bfloat16 terms, in memory of the current stream
     room = _gemm_f32_scratch(m, n, k)
-    scratch = torch.empty(room, dtype=torch.uint8, device=x.device) if room else None
+    scratch = None
+    if room:
+        scratch = lib.record_scratch(room, x.device) if lib.recording() else torch.empty(room, dtype=torch.uint8, device=x.device)
+        count_extra_launches()               # the kernel that writes the terms
     _gemm_f32(out, x, w, m, n, k, x.stride(0), w.stride(0), out.stride(0),
               scratch, tc_status(x.device).data_ptr(), _stream())
 

@@ -8,6 +8,8 @@ import importlib.util
 import threading
 from typing import Dict
 
+import torch
+
 from . import build
 
 _libs: Dict[str, ctypes.CDLL] = {}
@@ -15,6 +17,7 @@ _lock = threading.Lock()
 _launch_calls = 0          # kernels launched from Python (a captured graph replays them)
 _recorder = None           # the list of the active LaunchRecord
 _pending_cost = None       # what the launcher said about the launch that comes next
+_record_scratch = {}       # device -> scratch that the launches of the active record share
 
 
 def launch_calls() -> int:
@@ -34,7 +37,8 @@ class LaunchRecord:
     An entry is ``(name, issue, cost)``: ``issue(stream)`` launches it again on the raw stream
     handle ``stream`` and ``cost`` is what the launcher said the launch has to move and compute,
     ``{"bytes": ..., "flops": ...}`` (see :func:`annotate`; empty if it said nothing).  The
-    tensors behind the recorded pointers must outlive the record."""
+    record keeps the tensors that the launches were given; what they take by raw pointer must
+    outlive it."""
 
     def __init__(self):
         self.launches = []
@@ -44,12 +48,14 @@ class LaunchRecord:
         if _recorder is not None:
             raise RuntimeError("a launch record is already active")
         _recorder = self.launches
+        _record_scratch.clear()
         return self
 
     def __exit__(self, *exc):
         global _recorder, _pending_cost
         _recorder = None
         _pending_cost = None
+        _record_scratch.clear()
         return False
 
     def names(self):
@@ -83,6 +89,15 @@ class LaunchRecord:
 
 def recording() -> bool:
     return _recorder is not None
+
+
+def record_scratch(room: int, device):
+    """Scratch of ``room`` bytes for a launch of the active record: its launches, issued one after the other, share it
+    (the record keeps what they were given, and each one's own would add up)."""
+    t = _record_scratch.get(device)
+    if t is None or t.numel() < room:
+        t = _record_scratch[device] = torch.empty(room, dtype=torch.uint8, device=device)
+    return t
 
 
 def annotate(bytes: int = 0, flops: int = 0, label: str = "") -> None:

@@ -685,6 +685,45 @@ def test_gemm_f32_of_small_values(m, n, k_, ex, ew):
     k.check_tc_status(DEV)
 
 
+@pytest.mark.parametrize("m,n,k_", [(65, 70, 131072), (65, 70, 131080), (3, 70, 131080)])
+def test_gemm_f32_of_very_long_rows(m, n, k_):
+    """The longest rows whose terms are made ahead and the shortest longer ones: every row equals the one-row product, and
+    scratch stays within 256 MB whatever K is.  (Chains of 64 and a sum of K / 64 of them, each rounded: 2e-6 as above.)"""
+    k = K()
+    x, w = rnd(m, k_, seed=1).to(DEV), rnd(n, k_, seed=2).to(DEV)
+    out = torch.empty(m, n, device=DEV)
+    k.gemm_f32(out, x, w)
+    assert rel(out, x.double() @ w.double().t()) <= 2e-6
+    one = torch.empty(1, n, device=DEV)
+    k.gemm_f32(one, x[m - 1:], w)
+    assert torch.equal(one[0], out[m - 1])
+    k.check_tc_status(DEV)
+    for kk in (8, 4096, 131072, 131080, 1 << 21, (1 << 31) - 8):
+        for rows in (65, 128, 129, 100000, 1 << 30):
+            assert 0 <= k._gemm_f32_scratch(rows, 1 << 20, kk) <= 1 << 28
+
+
+def test_recorded_products_share_their_scratch():
+    """A record of 32-bit products of many rows keeps one scratch for all of them, and issues them again to the same results."""
+    from enginekernel_b200.ops import lib
+    k = K()
+    x, w = rnd(200, 1024, seed=1).to(DEV), [rnd(2048, 1024, seed=2 + i).to(DEV) for i in range(6)]
+    outs = [torch.empty(200, 2048, device=DEV) for _ in w]
+    room = k._gemm_f32_scratch(200, 2048, 1024)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    with lib.LaunchRecord() as record:
+        for o, m in zip(outs, w):
+            k.gemm_f32(o, x, m)
+    assert torch.cuda.memory_allocated() - before <= 2 * room
+    want = [o.clone() for o in outs]
+    for o in outs:
+        o.zero_()
+    assert record.issue(torch.cuda.current_stream().cuda_stream, "ek_gemm_nt_f32") == len(outs)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(outs, want))
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
 def test_gemm_f32_takes_as_long_beside_a_value_that_is_not_finite(value):
     """Only the outputs of such a value's row are worked out again: one row among 1,100 may add a fraction to the
