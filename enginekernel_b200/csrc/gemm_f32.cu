@@ -32,7 +32,6 @@
 
 namespace ek {
 
-constexpr int kSms = 148;              // of a B200: how many blocks a launch should at least have
 constexpr int kRun = 64;              // products summed in one chain
 
 // 8 values of a row from column k on (zeros from K on).
@@ -686,43 +685,47 @@ static bool tensor_map_f32(const float* rows, int n, int k, int ld, int box_rows
                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// How many clusters of b blocks run at a time (a GPU part's SMs are no multiple of b): asked once.
+// How many clusters of b blocks run at a time (a GPU part's SMs are no multiple of b), asked once a device; 0 where it cannot
+// be asked, this time.
 template <int NT>
 static int clusters_at_once(int b) {
-  static int counts[9];
-  static std::once_flag once;
-  std::call_once(once, [] {
-    auto kernel = sgemm_tc_few_kernel<NT, true>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess) return;
-    for (int n = 2; n <= 8; ++n) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(1, n, 1);
-      cfg.blockDim = dim3(kFewThreads);
-      cfg.dynamicSmemBytes = kMaxSmem;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 1;
-      attr[0].val.clusterDim.y = n;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&counts[n], kernel, &cfg) != cudaSuccess) counts[n] = 0;
-    }
+  static std::mutex mu;
+  static int counts[kMaxDevices][9] = {};
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  int& count = counts[device][b];
+  if (count > 0) return count;
+  auto kernel = sgemm_tc_few_kernel<NT, true>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, b, 1);
+  cfg.blockDim = dim3(kFewThreads);
+  cfg.dynamicSmemBytes = kMaxSmem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = b;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) != cudaSuccess) {
+    count = 0;
     cudaGetLastError();
-  });
-  return counts[b];
+  }
+  return count;
 }
 
 template <int NT>
 static int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int* status,
                       cudaStream_t stream) {
-  const int tiles_n = (N + 127) / 128, tiles_m = (M + NT - 1) / NT, spans = (K + kSpan - 1) / kSpan;
+  const int tiles_n = (N + 127) / 128, tiles_m = (M + NT - 1) / NT, spans = (K + kSpan - 1) / kSpan, sms = max(1, sm_count());
   if (tiles_m > 65535) return EK_ERR_ARG;
   // K over the blocks of a cluster where the tiles alone leave SMs idle: the fewest rounds of blocks, a block's cost
   // taken as its spans and one and a half for its start and end
   int blocks = 1, each = spans, kept = 0;
   const long long tiles = (long long)tiles_n * tiles_m;
-  long long best = (tiles + kSms - 1) / kSms * (2 * spans) + 3;
+  long long best = (tiles + sms - 1) / sms * (2 * spans) + 3;
   for (int b = 2; b <= 8 && b <= spans; ++b) {
     const int e = (spans + b - 1) / b, at_once = clusters_at_once<NT>(b);
     const long long sums = (long long)spans * ((min(NT, M) + b - 1) / b) * 512;
@@ -743,7 +746,7 @@ static int launch_few(float* C, const float* A, const float* W, int M, int N, in
   if (!tensor_map_f32(W, N, K, ldw, 128, &map_w) || !tensor_map_f32(A, M, K, lda, NT, &map_x)) return EK_ERR_ARG;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   if (e != cudaSuccess) return (int)e;
-  const dim3 grid(split ? tiles_n : min(tiles_n, max(1, kSms / tiles_m)), blocks, tiles_m);
+  const dim3 grid(split ? tiles_n : min(tiles_n, max(1, sms / tiles_m)), blocks, tiles_m);
   e = split ? launch_pdl_cluster(kernel, grid, dim3(kFewThreads), smem, stream, blocks, map_w, map_x, C, A, W, M, N, K, lda, ldw, ldc,
                                  each, depth, status)
             : launch_pdl(kernel, grid, dim3(kFewThreads), smem, stream, map_w, map_x, C, A, W, M, N, K, lda, ldw, ldc, each, depth, status);
@@ -974,7 +977,7 @@ static int launch_many(float* C, const float* A, const float* W, int M, int N, i
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kManySmem);
   if (e != cudaSuccess) return (int)e;
   const int tiles = w_blocks * ((M + NT - 1) / NT);
-  return (int)launch_pdl(kernel, dim3(min(tiles, kSms)), dim3(kManyThreads), kManySmem, stream, C, (const unsigned char*)scratch,
+  return (int)launch_pdl(kernel, dim3(min(tiles, max(1, sm_count()))), dim3(kManyThreads), kManySmem, stream, C, (const unsigned char*)scratch,
                          (const uint32_t*)flags, A, W, M, N, K, lda, ldw, ldc, w_blocks, status);
 }
 
@@ -996,7 +999,8 @@ static int launch_tc(float* C, const float* A, const float* W, int M, int N, int
     if (scratch == nullptr) return EK_ERR_ARG;
     const int rows_m = min(M, image_rows(M, K)), rows_n = min(N, image_rows(N, K));
     // 64 rows a tile cost three quarters of what 128 do
-    auto rounds = [&](int nt) { return ((long long)((rows_n + 127) / 128) * ((rows_m + nt - 1) / nt) + kSms - 1) / kSms; };
+    const int sms = max(1, sm_count());
+    auto rounds = [&](int nt) { return ((long long)((rows_n + 127) / 128) * ((rows_m + nt - 1) / nt) + sms - 1) / sms; };
     const bool wide = 4 * rounds(128) <= 3 * rounds(64);
     for (int n = 0; n < N; n += rows_n)
       for (int m = 0; m < M; m += rows_m) {
