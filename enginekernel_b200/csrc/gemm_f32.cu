@@ -14,11 +14,14 @@
 // Relative error against 64 bits (normal values, K = 1,024; this and FFMA in chains of 64): 0.9e-7 and 1.6e-7.
 //   up to 64 rows   bound by the weight stream.  TMA brings 32-bit values, 16 warps write their terms for the MMA,
 //                   the weights on its 128-row side; blocks take tile after tile, or a cluster shares K of one and
-//                   every block sends its spans' sums to the one that adds them up.  us, FFMA before: 4 x 1024 x 3072
-//                   (M x N x K) 22.6 -> 17.4, 16 x 151936 x 1024 248 -> 118 (5.3 TB/s), 13 x 6144 x 2560 78 -> 30,
-//                   64 x 6144 x 2560 163 -> 42.  One row of a narrow product is the exception: 1 x 4096 x 1024 11.3 ->
-//                   15.4, the chain from copy to conversion, MMA and sum being longer than FFMA's.  Loads into registers or
-//                   cp.async instead of TMA ran at half this rate (long chains in every converting warp).
+//                   every block sends its spans' sums to the one that adds them up.  us one behind the other in a graph, FFMA
+//                   before, weights of one term (of three): 4 x 1024 x 3072 (M x N x K) 17.5 -> 11.3 (16.1), 16 x
+//                   151936 x 1024 248 -> 112 (163; 5.6 TB/s), 13 x 6144 x 2560 78 -> 23 (36), 64 x 6144 x 2560 163 -> 37 (53).
+//                   One row of a narrow product is the exception: 1 x 4096 x 1024 6.1 -> 9.7, the chain from copy to
+//                   conversion, MMA and sum being longer than FFMA's.  Loads into registers or
+//                   cp.async instead of TMA ran at half this rate (long chains in every converting warp).  Up to 8 rows by
+//                   mma.sync from registers, whose results were the same bits, took 6.5 us there, but in a step, where small
+//                   kernels stand between the products, 1.8 us more a product than this form.
 //   more rows       a kernel of its own writes both operands' terms as the tiles that the MMA reads, so that a value is
 //                   converted once and not by every block that needs it (which took half as long again); the product
 //                   streams these tiles.  128 x 128 outputs a tile read 64 KB of operands for 64 of K, which L2 supplies
@@ -108,6 +111,8 @@ sgemm_few_rows_kernel(float* __restrict__ C, const float* __restrict__ A, const 
 }
 
 // ------------------------------------------------------------------------------ more rows
+// (A stage is written by plain stores three steps ahead of its use: rows here start anywhere, so there is nothing to copy
+// 16 bytes at a time, and one barrier a step serves both the stage that is read and the one that is written.)
 constexpr int kStepK = 16, kStepLd = kStepK + 4, kStages = 4;
 __host__ __device__ constexpr int tile_smem(int bm, int bn) { return kStages * (bm + bn) * kStepLd * 4; }
 
@@ -208,10 +213,10 @@ static int launch_tile(float* C, const float* A, const float* W, int M, int N, i
 }
 
 static int launch_ffma(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
-  // 5 to 16 rows of many columns: x is read often enough for the few-row form to be bound by L1, and there
-  // are columns enough for tiles (16 x 151936 x 1024: 425 us against 248; 12 x 40000 x 1024: 114 against 87;
-  // but 16 x 6144 x 1024: 30 against 74)
-  if (M <= 16 && !(M > 4 && N > 24576)) {
+  // 9 to 16 rows of many columns: x is read often enough for the few-row form to be bound by L1, and there are columns
+  // enough for tiles of 16 x 128 (us, few-row form / tiles: 16 x 40000 x 1025 224 / 165, 12 x 151936 x 1025 713 / 490; but
+  // 16 x 24576 x 1025 137 / 160, 16 x 6144 x 1025 47 / 106, 8 x 151936 x 1025 366 / 489)
+  if (M <= 16 && !(M > 8 && N > 28672)) {
     const int mr = M == 1 ? 1 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
     const int threads = 32 * min(few_warps(mr), (K + 4 * kRun - 1) / (4 * kRun));
     const dim3 grid((N + 8 * few_cols(mr) - 1) / (8 * few_cols(mr)));
@@ -802,7 +807,9 @@ constexpr int kManySlots = 4;         // stages that barriers are kept for
 constexpr int kManySmem = kManyRing * kTermTile + 512 + 1024;
 
 // C tiles of 128 columns x NT rows; a block takes tile after tile.  A stage takes the tiles of the ring that it needs:
-// the weights' first term or all three, then the three terms of x.
+// the weights' first term or all three, then the three terms of x.  (128 rows a tile: an adding thread keeps 128 sums, and of
+// the 168 registers that 11 warps leave it spills 160 bytes, 232 read back a tile's end and span; 64 rows spill nothing but
+// stream half as much again for an output.)
 template <int NT>
 __global__ void __launch_bounds__(kManyThreads, 1)
 sgemm_tc_many_kernel(float* __restrict__ C, const unsigned char* __restrict__ images, const uint32_t* __restrict__ flags,

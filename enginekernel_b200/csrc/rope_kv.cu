@@ -649,9 +649,9 @@ static int launch_rows(T* rows, int row_stride, int k_col, int v_col, const floa
                            k_gain, cos_tab, sin_tab, rot_dim, positions, token_slot, cache, n_q_heads, norm_dim, eps, unit,
                            write_kv);
   };
-  // 16-bit rows: two heads a thread once the tokens fill the machine several times (one head / two, as an
-  // earlier form of the kernel had it, us by rows of 16 + 2 x 8 heads of 64: 1 2.1 / 2.7, 127 2.6 / 3.2; of 128: 100 2.5 / 2.8,
-  // 2,000 15.7 / 14.3, 5,137 30.3 / 28.1; four 2,048 of 32 + 2 x 8 18.3, two 17.2)
+  // 16-bit rows: two heads a thread once the tokens fill the machine several times (one head / two, us by rows of 16 + 2 x 8
+  // heads of 64: 1 2.0 / 2.6, 127 2.1 / 3.0, 512 2.9 / 3.8, 2,048 6.0 / 5.9; of 128, 64 of them rotated: 100 2.7 / 3.2, 600 4.4 /
+  // 3.9, 1,000 6.2 / 6.1, 2,000 11.9 / 11.3, 5,137 27.4 / 25.9; 2,048 of 32 + 2 x 8 16.8 / 17.0)
   if constexpr (sizeof(T) == 2)
     if (n_tokens >= 1024) {
       if (cache.head_dim <= 64) return run(qk_rows_kernel<T, 8, 2, UNIT>, 8, 2);

@@ -1065,7 +1065,10 @@ EPI_BF16_EXTENDED = 4
 
 
 def gemm_f32(out, x, w, n_rows=None):
-    """out[M, N] = x[M, K] . w[N, K]^T in true 32-bit."""
+    """out[M, N] = x[M, K] . w[N, K]^T in true 32-bit.
+
+    ``w`` holds weights: up to 64 rows of ``x``, it is read before the kernel ahead has ended, so it must not be
+    what one of this package's own launches wrote just before."""
     _need_cuda(out, x, w)
     _need(out.dtype == x.dtype == w.dtype == torch.float32, "gemm_f32: float32 tensors")
     _need(x.stride(-1) == 1 and w.stride(-1) == 1 and out.stride(-1) == 1, "gemm_f32: dense rows")

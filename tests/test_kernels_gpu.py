@@ -576,8 +576,8 @@ def test_gemm_f32_is_true_32_bit(m, n, k_):
                                         (8, 33, 4160, 0), (9, 70, 1032, 3), (16, 24577, 72, 8), (17, 63, 200, 0),
                                         (65, 130, 61, 0), (129, 65, 128, 5)])
 def test_gemm_f32_forms_sum_in_one_order(m, n, k_, pad):
-    """Few rows, few rows of many columns and tiles, with rows that are and are not whole 32-byte pieces: every row
-    equals the one-row product bit for bit, and 64 bits to the bound of a chain of 64 products and K / 64 sums (each
+    """Few rows and tiles on FFMA, where rows are not whole 32-byte pieces, and sizes near them on the tensor cores, where they
+    are: every row equals the one-row product bit for bit, and 64 bits to the bound of a chain of 64 products and K / 64 sums (each
     rounding 2^-24 of a partial sum, which random terms keep within a few standard deviations of the result)."""
     k = K()
     xs, ws = rnd(m, k_ + pad, seed=1).to(DEV), rnd(n, k_ + pad, seed=2).to(DEV)
@@ -589,6 +589,13 @@ def test_gemm_f32_forms_sum_in_one_order(m, n, k_, pad):
         one = torch.empty(1, n, device=DEV)
         k.gemm_f32(one, x[r:r + 1], w)
         assert torch.equal(one[0], out[r])
+
+
+@pytest.mark.parametrize("m,n,k_,pad", [(3, 50, 137, 0), (5, 24584, 137, 0), (6, 70, 1032, 3), (8, 33, 4161, 0), (8, 28673, 72, 3),
+                                        (9, 28672, 72, 3), (9, 28673, 137, 0), (16, 28800, 72, 3), (16, 100, 515, 0)])
+def test_gemm_f32_of_rows_that_are_not_whole_pieces(m, n, k_, pad):
+    """The forms on FFMA, each with few rows of few columns and (9 to 16 rows) of many: as above."""
+    test_gemm_f32_forms_sum_in_one_order(m, n, k_, pad)
 
 
 @pytest.mark.parametrize("m,n,k_,pad", [(1, 130, 8, 0), (16, 128, 264, 8), (4, 1000, 2560, 0), (9, 24584, 72, 0), (17, 257, 1032, 0),
