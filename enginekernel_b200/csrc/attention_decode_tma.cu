@@ -369,8 +369,8 @@ attention_decode_tma_kernel(bf16* __restrict__ out, const bf16* q, int q_row_str
 // counts blocks of 16 query heads of a KV head.  grid (splits, blocks of heads, tokens); cluster (splits, 1, 1) when
 // splits > 1.
 // What bounds it is the latency of one block's pages and of what follows them, not the bytes (8 tokens behind 2,048 rows
-// read 8 MB, 1.3 us); of a page's time, most is shared memory: 32 KB come in and are read twice, for the scores and for
-// P.V, 0.4 us at 128 bytes a clock.  So two sets of four warps take the pages in turn, one set's MMAs under the other's
+// read 8 MB, 1.3 us); of a page's 0.75 us, 0.42 are shared memory's (32 KB come in and are read twice, for the scores and for
+// P.V: 811 wavefronts a page by ncu, tensor pipes 40 % active).  So two sets of four warps take the pages in turn, one set's MMAs under the other's
 // fetches, and inside a set a page is spread without reading anything twice: 16 keys of the scores a warp, then 64
 // dimensions of P.V of all keys, the page's maximum and P passing through shared memory.  O lies in the set's registers
 // in parts, and the queries' fragments stay in registers too; only the two sets' results are merged.  Before, each

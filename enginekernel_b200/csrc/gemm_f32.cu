@@ -24,8 +24,9 @@
 //                   kernels stand between the products, 1.8 us more a product than this form.
 //   more rows       a kernel of its own writes both operands' terms as the tiles that the MMA reads, so that a value is
 //                   converted once and not by every block that needs it (which took half as long again); the product
-//                   streams these tiles.  128 x 128 outputs a tile read 64 KB of operands for 64 of K, which L2 supplies
-//                   at about the rate of the MMAs.  1129 x 6144 x 1024 360 -> 87 us, 1129 x 1024 x 3072 219 -> 56,
+//                   streams these tiles.  128 x 128 outputs a tile read 64 KB of operands for 64 of K (96 KB with three
+//                   terms of the weights), two or three such stages in flight: ncu shows tensor pipes 34 % active and L2 at
+//                   10.7 TB/s, 31 % of its sectors' peak, so neither is full.  1129 x 6144 x 1024 360 -> 87 us, 1129 x 1024 x 3072 219 -> 56,
 //                   4096^3 3,165 -> 515 (267 TFLOP/s).  The three terms of x side by side in one MMA of 192 columns
 //                   read less shared memory but more L2 (128 x 64 tiles): 820 us.
 // Other rows, and K above 131,072: FFMA, chains of 64 (kRun) whose sums are added in ascending order.

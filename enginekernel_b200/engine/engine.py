@@ -100,7 +100,7 @@ class Engine:
     def close_sequence(self, slot: int) -> None:
         torch.cuda.current_stream().synchronize()
         self.cache.close(slot)
-        self.runner.check_kernels()
+        self.runner.check_kernels(waited=True)
 
     def step(self, entries: Sequence) -> torch.Tensor:
         """``entries``: (slot, tokens, want) triples or :class:`StepEntry`.  Returns 32-bit

@@ -108,12 +108,13 @@ class ModelRunner:
                 kernels.split_scratch(self.device)
         model.prepare(min(cache.max_len, model.spec.max_positions))
 
-    def check_kernels(self) -> None:
+    def check_kernels(self, waited: bool = False) -> None:
         """Raise if a kernel reported a failure (a tensor-core product of either data type, or an attention
-        kernel, whose bounded barrier wait ran out).  Synchronises the device; called where the host waits anyway."""
+        kernel, whose bounded barrier wait ran out).  Waits for the current stream unless the caller has just done so
+        (``waited``); called where the host waits anyway."""
         if self.device.type == "cuda":
             from ..ops import kernels
-            kernels.check_tc_status(self.device)
+            kernels.check_tc_status(self.device, waited)
 
     def _plan_for(self, n_tokens: int, n_seqs: int) -> PlanBuffers:
         p = self.plan
