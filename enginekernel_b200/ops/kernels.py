@@ -1137,21 +1137,24 @@ TC_SWAP_MAX_ROWS = 64
 
 def tc_status(device):
     """One int per device that the tensor-core kernels set when a barrier wait times out: in pinned host memory, which
-    they write across the bus in that case only, so that looking at it costs the host no copy."""
+    they write across the bus in that case only, so that looking at it costs the host no copy (made while a graph is
+    captured, which pinned memory cannot be: on the device)."""
     status = _tc_status.get(device)              # (by the torch.device that launches hand over)
     if status is None:
         key = _with_index(device)
         if key not in _tc_status:
-            _tc_status[key] = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+            where = dict(device=key) if torch.cuda.is_current_stream_capturing() else dict(pin_memory=True)
+            _tc_status[key] = torch.zeros(1, dtype=torch.int32, **where)
         status = _tc_status[key]
     return status
 
 
 def check_tc_status(device, waited=False):
-    """Waits for the current stream (``waited``: the caller has); raises if a kernel gave up a bounded barrier wait since the last check (products in 16 bits:
-    1 producer, 2 MMA, 3 epilogue, 4 copies before exit, 5 sums from the cluster, 41 to 46 on pairs of SMs, experts 51 to 54;
-    products in 32 bits: 31 to 39; prompt attention 11 to 36; decode attention 41 producer, 42 pages, 43 sums from the
-    cluster) and clears the word, so that the next check speaks of later launches only."""
+    """Waits for the current stream (``waited``: the caller has); raises if a kernel gave up a bounded barrier wait
+    since the last check (products in 16 bits: 1 producer, 2 MMA, 3 epilogue, 4 copies before exit, 5 sums from the
+    cluster, 41 to 46 on pairs of SMs, experts 51 to 54; products in 32 bits: 31 to 39; prompt attention 11 to 36; decode
+    attention 41 producer, 42 pages, 43 sums from the cluster) and clears the word, so that the next check speaks of
+    later launches only."""
     status = tc_status(device)
     if not waited:
         torch.cuda.current_stream(_with_index(device)).synchronize()

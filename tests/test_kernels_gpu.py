@@ -710,6 +710,23 @@ def test_gemm_f32_of_very_long_rows(m, n, k_):
             assert 0 <= k._gemm_f32_scratch(rows, 1 << 20, kk) <= 1 << 28
 
 
+@pytest.mark.parametrize("m", [4, 100])
+def test_a_first_product_may_be_captured(m, monkeypatch):
+    """Where no launch made the status word before a capture, the capture makes it, and checks find it."""
+    k = K()
+    x, w = rnd(m, 512, seed=1).to(DEV), rnd(300, 512, seed=2).to(DEV)
+    want, out = torch.empty(m, 300, device=DEV), torch.empty(m, 300, device=DEV)
+    k.gemm_f32(want, x, w)
+    torch.cuda.synchronize()
+    monkeypatch.setattr(k, "_tc_status", {})
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        k.gemm_f32(out, x, w)
+    graph.replay()
+    k.check_tc_status(x.device)
+    assert len(k._tc_status) == 1 and torch.equal(out, want)
+
+
 def test_recorded_products_share_their_scratch():
     """A record of 32-bit products of many rows keeps one scratch for all of them, and issues them again to the same results."""
     from enginekernel_b200.ops import lib
